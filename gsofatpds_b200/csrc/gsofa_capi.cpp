@@ -321,88 +321,332 @@ MatDesc make_desc(const gsofa_matrix* m, const gsofa_result* r, long long base) 
     return d;
 }
 
+// Whether the counting traversal (gsofa_chain.cu) runs these options: it
+// always reuses closures and searches top-down, and does not scatter per-row L
+// statistics; the diagnostic switches and that option take traverse_kernel.
+bool chain_runs(const gsofa_opts& o) {
+    return !(o.flags & (GSOFA_NO_MERGE | GSOFA_NO_CHAIN | GSOFA_L_ROW_STATS)) && o.bu_alpha <= 0;
+}
+
+int plan_chain(gsofa_ctx* ctx, int32_t nmax, bool all_sym, const gsofa_opts* o, bool serve,
+               ChainCfg* c) {
+    c->words = bitmap_words(nmax);
+    const long long need = (all_sym ? 1 : 2) * c->words;  // X of each direction
+    const size_t fixed = (chain_sparse_bytes() + 15) & ~(size_t)15;
+    size_t bytes = ((size_t)need * 4 + 15) & ~(size_t)15;
+    if (fixed + bytes + 4096 > (size_t)ctx->smem_optin || (o->flags & GSOFA_FORCE_GLOBAL_BITMAP))
+        bytes = 0;
+    c->smem_words = bytes ? need : 0;
+    c->gbm_count = bytes ? 2 : 4;
+    c->smem = fixed + bytes;
+    c->block = o->threads_per_source;
+    if (c->block <= 0) {
+        const long long fit = ctx->smem_per_sm / (long long)(c->smem + 2048);
+        c->block = fit >= 8 ? 128 : fit >= 4 ? 256 : fit >= 2 ? 512 : 1024;
+    }
+    if (c->block != 128 && c->block != 256 && c->block != 512 && c->block != 1024)
+        return set_err(ctx, GSOFA_ERR_ARG, "threads_per_source must be 128, 256, 512 or 1024");
+    const int occ = chain_occupancy(c->block, serve, c->smem);
+    if (occ <= 0)
+        return set_err(ctx, GSOFA_ERR_UNSUPPORTED,
+                       "traversal kernel cannot be resident (block %d, %zu B shared)", c->block,
+                       c->smem);
+    c->grid = occ * ctx->sm_count;
+    if (o->sources_in_flight > 0) c->grid = std::min(c->grid, o->sources_in_flight);
+    return GSOFA_OK;
+}
+
+void fill_chain_launch(ChainLaunch* L, const ChainCfg& c, const gsofa_opts& o, int32_t nmax) {
+    L->queue_stride = std::max(nmax, 1);
+    if (o.flags & GSOFA_DEBUG_QUEUE_CAP) L->queue_stride = std::min<long long>(L->queue_stride, 64);
+    L->list_cap = (int)std::min<long long>(chain_list_cap(), L->queue_stride);
+    L->gbm_count = c.gbm_count;
+    L->bitmap_words = c.words;
+    L->smem_words = c.smem_words;
+}
+
+int32_t method_of(const gsofa_matrix* m) {
+    if (m->n <= kDirectMax) return METHOD_DIRECT;
+    return m->host_sym > 0 ? METHOD_CHAIN : METHOD_HUB;
+}
+
+bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, void* ws,
+              size_t* bytes, HubLaunch* L, HubCfg* c) {
+    *L = HubLaunch{};
+    *c = HubCfg{};
+    long long sources = 0, off = 0, items = 0;
+    int32_t n_max = 0;
+    int hubs = 0;
+    for (MatDesc& d : *descs) {
+        if (d.method == METHOD_CHAIN) continue;
+        sources += 2ll * d.n;
+        n_max = std::max(n_max, d.n);
+        if (d.method != METHOD_HUB) continue;
+        hubs++;
+        d.hub_off = off;
+        d.hub_len = ((long long)d.n + 1 + 31) & ~31ll;
+        off += d.hub_len;
+    }
+    *bytes = 0;
+    if (n_max == 0) return false;
+    const int nm = (int)descs->size(), W = hub_count();
+    c->any_hub = hubs > 0;
+    c->n_max = n_max;
+    c->sm_count = ctx->sm_count;
+    // labels in the shared memory of a cluster: of as many CTAs as leave every
+    // job's cluster room on the GPU at once, and hold the largest matrix's labels
+    c->cluster = 1;
+    while (c->cluster < 16 && 2 * W * hubs * 2 * c->cluster <= ctx->sm_count) c->cluster *= 2;
+    while (c->cluster < 16 && label_smem_bytes(n_max, c->cluster) + 2048 > (size_t)ctx->smem_optin)
+        c->cluster *= 2;
+    if (label_smem_bytes(n_max, c->cluster) + 2048 > (size_t)ctx->smem_optin) c->cluster = 0;
+    L->nmats = nm;
+    L->total = off;
+    // sources per warp and turn: few enough that the GPU's warps all have some
+    long long g = 1;
+    while (g < 16 && sources / (2 * g) >= 2ll * 32 * ctx->sm_count) g *= 2;
+    L->group = (int)g;
+    for (MatDesc& d : *descs) {
+        d.hub_item = items;
+        d.hub_slots = 0;
+        if (d.method == METHOD_CHAIN || d.n == 0) continue;
+        d.hub_slots = 1;
+        while (d.hub_slots < 2 * ((d.n + g - 1) / g)) d.hub_slots *= 2;
+        items += d.hub_slots;
+    }
+    L->total_items = items;
+    // large_kernel: small CTAs for small matrices, whole SMs for large ones
+    L->bitmap_words = bitmap_words(n_max);
+    const size_t bm = ((size_t)L->bitmap_words * 4 + 15) & ~(size_t)15;
+    c->large_block = 256;
+    L->large_smem = 4 * (bm + 2048) <= (size_t)ctx->smem_per_sm && !(o.flags & GSOFA_FORCE_GLOBAL_BITMAP);
+    c->large_smem = L->large_smem ? bm : 0;
+    int occ = large_occupancy(c->large_block, c->large_smem);
+    if (occ <= 0) occ = 1;
+    c->large_grid = occ * ctx->sm_count;
+    L->queue_stride = n_max;
+    if (o.flags & GSOFA_DEBUG_QUEUE_CAP) L->queue_stride = std::min<long long>(L->queue_stride, 64);
+    c->scan_bytes = c->any_hub ? hub_scan_bytes(2 * hub_bases() * off) : 0;
+    // workspace: the zeroed block first
+    size_t at = 0;
+    char* const w = static_cast<char*>(ws);
+    auto place = [&](size_t b) {
+        char* p = w ? w + at : nullptr;
+        at += align256(b);
+        return static_cast<void*>(p);
+    };
+    const size_t T = (size_t)off;
+    L->zeroed = w;
+    L->base = static_cast<Tot*>(place(sizeof(Tot) * 2 * (size_t)hub_bases() * T));
+    L->stamp = static_cast<int32_t*>(place(4 * 2 * (size_t)W * T));
+    L->lcnt = static_cast<int32_t*>(place(16 * 2 * (size_t)W * (size_t)nm));
+    L->fallback = static_cast<int32_t*>(place(4 * (size_t)nm));
+    L->judged = static_cast<int32_t*>(place(8 * (size_t)nm));
+    L->counters = static_cast<unsigned long long*>(place(8 * CNT_SLOTS * (size_t)nm));
+    L->hubs = static_cast<unsigned long long*>(place(8 * (size_t)W * (size_t)nm));
+    L->large_count = static_cast<int*>(place(4));
+    L->work_counter = static_cast<unsigned long long*>(place(16));
+    c->zeroed_bytes = at;
+    L->lam = static_cast<int32_t*>(place(4 * 2 * (size_t)W * T));
+    L->lq = static_cast<int32_t*>(place(8 * 2 * (size_t)W * T));
+    L->large = static_cast<unsigned long long*>(place(8 * (size_t)sources));
+    c->scan_tmp = place(c->scan_bytes);
+    L->queue = static_cast<int32_t*>(place((size_t)c->large_grid * (size_t)L->queue_stride * 4));
+    L->gbm = static_cast<uint32_t*>(
+        place(L->large_smem ? 0 : (size_t)c->large_grid * (size_t)L->bitmap_words * 4));
+    *bytes = at;
+    return true;
+}
+
+long long chain_chunk(const gsofa_opts& o, long long total_sources, int grid) {
+    if (o.chunk_sources > 0) return o.chunk_sources;
+    return std::max(1ll, (total_sources + grid - 1) / grid);
+}
+
 // Runs the traversal (and optionally supernodes / pattern) for `count`
 // matrices in one persistent launch.  results[i] must be freshly allocated.
 int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
                const gsofa_opts* o, gsofa_result** res, long long sample_stride = 1) {
     int32_t nmax = 0;
-    long long items = 0;
-    long long total_sources = 0;
+    long long total_sources = 0, weight = 0;
+    bool all_sym = true;
     for (int32_t i = 0; i < count; i++) {
         nmax = std::max(nmax, mats[i]->n);
-        total_sources += chunk_weight(ctx, mats[i]);
+        weight += chunk_weight(ctx, mats[i]);
+        total_sources += mats[i]->n;
+        all_sym = all_sym && mats[i]->host_sym > 0;
     }
-    LaunchCfg cfg;
-    int rc = plan_launch(ctx, std::max(nmax, 1), o, &cfg);
-    if (rc) return rc;
-    // So few sources that each can have a CTA of its own: chunks of one source
-    // run them all at once (a 115-row matrix: 0.06 instead of 0.23 ms); with
-    // more, chunks share closures between consecutive sources.
-    long long one_each = 0;
-    for (int32_t i = 0; i < count; i++) one_each += 2ll * mats[i]->n;
-    const long long chunk = o->chunk_sources > 0 ? o->chunk_sources
-                            : one_each <= cfg.grid ? 1
-                                                   : default_chunk(total_sources, cfg.grid);
-    for (int32_t i = 0; i < count; i++) items += 2ll * ((mats[i]->n + chunk - 1) / chunk);
-    rc = ensure(ctx, &ctx->queue, &ctx->queue_bytes, (size_t)cfg.grid * (size_t)std::max(nmax, 1) * 4);
-    if (rc) return rc;
-    if (!cfg.smem_bitmap) {
-        rc = ensure(ctx, &ctx->gbitmap, &ctx->gbitmap_bytes, (size_t)cfg.grid * (size_t)cfg.words * 4);
-        if (rc) return rc;
-    }
-    const bool merge = !(o->flags & GSOFA_NO_MERGE);
-    int ring = o->cached_closures > 0 ? o->cached_closures : kDefaultRing;
-    if (ring > kMaxRing) ring = kMaxRing;
-    while (ring & (ring - 1)) ring &= ring - 1;  // power of 2
-    if (merge) {
-        rc = ensure(ctx, &ctx->gprev, &ctx->gprev_bytes,
-                    (size_t)cfg.grid * (size_t)ring * (size_t)cfg.words * 4);
-        if (rc) return rc;
-    }
+    const bool chain = chain_runs(*o);
+    const bool pattern = (o->flags & GSOFA_PATTERN) != 0;
+    const bool traverse = !chain || pattern;
+    int rc = GSOFA_OK;
     // matrix descriptors, largest matrices first
     const std::vector<int32_t> order = batch_order(mats, count);
     std::vector<MatDesc> descs((size_t)count);
-    long long base = 0;
-    for (int32_t k = 0; k < count; k++) {
-        const int32_t i = order[(size_t)k];
-        descs[(size_t)k] = make_desc(mats[i], res[i], base);
-        base += 2ll * ((mats[i]->n + chunk - 1) / chunk);
+    auto place = [&](long long chunk, int per_chunk) {
+        long long base = 0;
+        for (int32_t k = 0; k < count; k++) {
+            const int32_t i = order[(size_t)k];
+            descs[(size_t)k] = make_desc(mats[i], res[i], base);
+            base += per_chunk * ((mats[i]->n + chunk - 1) / chunk);
+        }
+        return base;
+    };
+    unsigned long long* wc = nullptr;
+    int32_t* dstatus = work_counter_status(ctx, &wc);
+    const long long stride = sample_stride > 1 ? sample_stride : 1;
+
+    ChainCfg ccfg;
+    ChainLaunch CL{};
+    HubLaunch HL{};
+    HubCfg hcfg;
+    bool hub = false;
+    if (chain) {
+        long long chain_sources = 0;
+        bool chain_sym = true;
+        for (int32_t i = 0; i < count; i++) {
+            if (method_of(mats[i]) != METHOD_CHAIN) continue;
+            chain_sources += mats[i]->n;
+            chain_sym = chain_sym && mats[i]->host_sym > 0;
+        }
+        // with none of its own, the chain's shape is that of what it may be left
+        if (chain_sources == 0) {
+            chain_sources = total_sources;
+            chain_sym = all_sym;
+        }
+        rc = plan_chain(ctx, std::max(nmax, 1), chain_sym, o, false, &ccfg);
+        if (rc) return rc;
+        CL.chunk = (int)chain_chunk(*o, chain_sources, ccfg.grid);
+        long long items = 0;
+        place(CL.chunk, 1);
+        for (int32_t k = 0; k < count; k++) {
+            const gsofa_matrix* m = mats[order[(size_t)k]];
+            MatDesc& d = descs[(size_t)k];
+            d.method = method_of(m);
+            d.item_base = items;
+            if (d.method == METHOD_CHAIN) items += (m->n + CL.chunk - 1) / CL.chunk;
+        }
+        size_t hub_bytes = 0;
+        if (plan_hub(ctx, &descs, *o, nullptr, &hub_bytes, &HL, &hcfg)) {
+            rc = ensure(ctx, &ctx->hub_ws, &ctx->hub_ws_bytes, hub_bytes);
+            if (rc) return rc;
+            hub = plan_hub(ctx, &descs, *o, ctx->hub_ws, &hub_bytes, &HL, &hcfg);
+            HL.status = dstatus;
+        }
+        ccfg.grid = (int)std::max(1ll, std::min<long long>(ccfg.grid, items));
+        rc = ensure(ctx, &ctx->queue, &ctx->queue_bytes, (size_t)ccfg.grid * (size_t)std::max(nmax, 1) * 4);
+        if (!rc)
+            rc = ensure(ctx, &ctx->gbitmap, &ctx->gbitmap_bytes,
+                        (size_t)ccfg.grid * (size_t)ccfg.gbm_count * (size_t)ccfg.words * 4);
+        if (rc) return rc;
+        fill_chain_launch(&CL, ccfg, *o, nmax);
+        CL.nmats = count;
+        CL.total_items = (items + stride - 1) / stride;
+        CL.sample_stride = stride;
+        CL.work_counter = wc;
+        CL.queue = reinterpret_cast<int32_t*>(ctx->queue);
+        CL.gbm = reinterpret_cast<uint32_t*>(ctx->gbitmap);
+        CL.status = dstatus;
+    }
+    LaunchCfg cfg;
+    TraverseLaunch L{};
+    if (traverse) {
+        rc = plan_launch(ctx, std::max(nmax, 1), o, &cfg);
+        if (rc) return rc;
+        // So few sources that each can have a CTA of its own: chunks of one source
+        // run them all at once; with more, chunks share closures between
+        // consecutive sources.
+        const long long chunk = o->chunk_sources > 0 ? o->chunk_sources
+                                : 2 * total_sources <= cfg.grid ? 1
+                                                                : default_chunk(weight, cfg.grid);
+        const long long items = chain ? 0 : place(chunk, 2);
+        rc = ensure(ctx, &ctx->queue, &ctx->queue_bytes, (size_t)cfg.grid * (size_t)std::max(nmax, 1) * 4);
+        if (!rc && !cfg.smem_bitmap)
+            rc = ensure(ctx, &ctx->gbitmap, &ctx->gbitmap_bytes, (size_t)cfg.grid * (size_t)cfg.words * 4);
+        const bool merge = !(o->flags & GSOFA_NO_MERGE);
+        int ring = o->cached_closures > 0 ? o->cached_closures : kDefaultRing;
+        if (ring > kMaxRing) ring = kMaxRing;
+        while (ring & (ring - 1)) ring &= ring - 1;  // power of 2
+        if (!rc && merge)
+            rc = ensure(ctx, &ctx->gprev, &ctx->gprev_bytes,
+                        (size_t)cfg.grid * (size_t)ring * (size_t)cfg.words * 4);
+        if (rc) return rc;
+        L.nmats = count;
+        L.total_items = (items + stride - 1) / stride;
+        L.sample_stride = stride;
+        L.work_counter = wc;
+        L.queue = reinterpret_cast<int32_t*>(ctx->queue);
+        L.queue_stride = std::max(nmax, 1);
+        if (o->flags & GSOFA_DEBUG_QUEUE_CAP) L.queue_stride = std::min<long long>(L.queue_stride, 64);
+        L.gbitmap = reinterpret_cast<uint32_t*>(ctx->gbitmap);
+        L.bitmap_words = cfg.words;
+        L.status = dstatus;
+        L.pattern_pass = 0;
+        L.bu_alpha = o->bu_alpha > 0 ? o->bu_alpha : (o->bu_alpha < 0 ? 0 : kDefaultBuAlpha);
+        L.bu_beta = o->bu_beta > 0 ? o->bu_beta : kDefaultBuBeta;
+        L.bu_min_src = o->bu_min_source > 0 ? o->bu_min_source : kBuMinSource;
+        L.gprev = reinterpret_cast<uint32_t*>(ctx->gprev);
+        L.merge = merge ? 1 : 0;
+        L.chain = merge && !(o->flags & GSOFA_NO_CHAIN) ? 1 : 0;
+        L.chain_wait_ns = chain_wait_ns(*o);
+        L.ring = ring;
+        L.chunk = (int)chunk;
+        L.heavy_len = o->heavy_row > 0 ? ((o->heavy_row + 3) & ~3) : kDefaultHeavyRow;
+        // both traversals share the queue and bitmap buffers, which may have grown
+        CL.queue = L.queue;
+        CL.gbm = L.gbitmap;
     }
     void* ddesc = nullptr;
     rc = dev_alloc(ctx, sizeof(MatDesc) * (size_t)count, &ddesc);
     if (rc) return rc;
     CK(cudaMemcpyAsync(ddesc, descs.data(), sizeof(MatDesc) * (size_t)count, cudaMemcpyHostToDevice,
                        ctx->stream));
-    unsigned long long* wc = nullptr;
-    int32_t* dstatus = work_counter_status(ctx, &wc);
     CK(cudaMemsetAsync(ctx->small, 0, 128, ctx->stream));
-
-    TraverseLaunch L{};
-    L.mats = reinterpret_cast<const MatDesc*>(ddesc);
-    L.nmats = count;
-    L.total_items = sample_stride > 1 ? (items + sample_stride - 1) / sample_stride : items;
-    L.sample_stride = sample_stride > 1 ? sample_stride : 1;
-    L.work_counter = wc;
-    L.queue = reinterpret_cast<int32_t*>(ctx->queue);
-    L.queue_stride = std::max(nmax, 1);
-    if (o->flags & GSOFA_DEBUG_QUEUE_CAP) L.queue_stride = std::min<long long>(L.queue_stride, 64);
-    L.gbitmap = reinterpret_cast<uint32_t*>(ctx->gbitmap);
-    L.bitmap_words = cfg.words;
-    L.status = dstatus;
-    L.pattern_pass = 0;
-    L.bu_alpha = o->bu_alpha > 0 ? o->bu_alpha : (o->bu_alpha < 0 ? 0 : kDefaultBuAlpha);
-    L.bu_beta = o->bu_beta > 0 ? o->bu_beta : kDefaultBuBeta;
-    L.bu_min_src = o->bu_min_source > 0 ? o->bu_min_source : kBuMinSource;
-    L.gprev = reinterpret_cast<uint32_t*>(ctx->gprev);
-    L.merge = merge ? 1 : 0;
-    L.chain = merge && !(o->flags & GSOFA_NO_CHAIN) ? 1 : 0;
-    L.chain_wait_ns = chain_wait_ns(*o);
-    L.ring = ring;
-    L.chunk = (int)chunk;
-    L.heavy_len = o->heavy_row > 0 ? ((o->heavy_row + 3) & ~3) : kDefaultHeavyRow;
+    L.mats = CL.mats = HL.mats = reinterpret_cast<const MatDesc*>(ddesc);
 
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    if (items > 0) CK(launch_traverse(L, cfg.block, cfg.grid, cfg.smem_bitmap, cfg.smem, ctx->stream));
+    if (chain) {
+        if (hub) {
+            CK(launch_hub(HL, hcfg, (o->flags & GSOFA_DIGESTS) != 0, ctx->stream));
+            // left to the chain: known before the supernodes are looked for
+            ctx->h_fallback.assign((size_t)count, 0);
+            CK(cudaMemcpyAsync(ctx->h_fallback.data(), HL.fallback, 4 * (size_t)count,
+                               cudaMemcpyDeviceToHost, ctx->stream));
+            CK(cudaStreamSynchronize(ctx->stream));
+            bool any = false;
+            for (int32_t k = 0; k < count; k++) any = any || ctx->h_fallback[(size_t)k];
+            if (any) {
+                long long items = 0;
+                bool sym = true;
+                for (int32_t k = 0; k < count; k++) {
+                    MatDesc& d = descs[(size_t)k];
+                    if (ctx->h_fallback[(size_t)k]) d.method = METHOD_CHAIN;
+                    d.item_base = items;
+                    if (d.method != METHOD_CHAIN) continue;
+                    items += (d.n + CL.chunk - 1) / CL.chunk;
+                    sym = sym && mats[order[(size_t)k]]->host_sym > 0;
+                }
+                rc = plan_chain(ctx, std::max(nmax, 1), sym, o, false, &ccfg);
+                if (rc) return rc;
+                ccfg.grid = (int)std::max(1ll, std::min<long long>(ccfg.grid, items));
+                rc = ensure(ctx, &ctx->queue, &ctx->queue_bytes,
+                            (size_t)ccfg.grid * (size_t)std::max(nmax, 1) * 4);
+                if (!rc)
+                    rc = ensure(ctx, &ctx->gbitmap, &ctx->gbitmap_bytes,
+                                (size_t)ccfg.grid * (size_t)ccfg.gbm_count * (size_t)ccfg.words * 4);
+                if (rc) return rc;
+                fill_chain_launch(&CL, ccfg, *o, nmax);
+                CL.queue = L.queue = reinterpret_cast<int32_t*>(ctx->queue);
+                CL.gbm = L.gbitmap = reinterpret_cast<uint32_t*>(ctx->gbitmap);
+                CL.total_items = (items + stride - 1) / stride;
+                CK(cudaMemcpyAsync(ddesc, descs.data(), sizeof(MatDesc) * (size_t)count,
+                                   cudaMemcpyHostToDevice, ctx->stream));
+            }
+        }
+        if (CL.total_items > 0) CK(launch_chain(CL, ccfg.block, false, ccfg.grid, ccfg.smem, ctx->stream));
+    } else if (L.total_items > 0) {
+        CK(launch_traverse(L, cfg.block, cfg.grid, cfg.smem_bitmap, cfg.smem, ctx->stream));
+    }
     CK(cudaEventRecord(ctx->evt, ctx->stream));
     for (int32_t i = 0; i < count; i++) {
         if ((o->flags & GSOFA_SUPERNODES) && mats[i]->n > 0)
@@ -422,7 +666,7 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
     CK(cudaEventElapsedTime(&ms_trav, ctx->ev0, ctx->evt));
 
     // pattern pass (second traversal writing sorted ids)
-    if (o->flags & GSOFA_PATTERN) {
+    if (pattern) {
         for (int32_t k = 0; k < count; k++) {
             const int32_t i = order[(size_t)k];
             gsofa_result* r = res[i];
@@ -446,13 +690,14 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
             if (rc) return rc;
             CK(launch_pattern_ptrs(r->n, r->nnz_u, r->nnz_lc, r->uptr, r->lptr, ctx->scan_tmp,
                                    ctx->scan_tmp_bytes, ctx->stream));
-            descs[(size_t)k] = make_desc(mats[i], r, descs[(size_t)k].item_base);
         }
+        L.total_items = place(L.chunk, 2);
         CK(cudaMemcpyAsync(ddesc, descs.data(), sizeof(MatDesc) * (size_t)count,
                            cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaMemsetAsync(ctx->small, 0, 128, ctx->stream));
         L.pattern_pass = 1;
-        if (items > 0)
+        L.sample_stride = 1;
+        if (L.total_items > 0)
             CK(launch_traverse(L, cfg.block, cfg.grid, cfg.smem_bitmap, cfg.smem, ctx->stream));
         CK(cudaMemcpyAsync(ctx->h_status, dstatus, 4, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
@@ -686,7 +931,7 @@ int gsofa::host::ingest_csr(gsofa_ctx* ctx, cudaStream_t stream, int32_t* dstatu
         return cuda_fail(ctx, e, "ingest upload");
     }
     rc = matrix_build(ctx, stream, dstatus, m, nnz, dbeg, dcol_in,
-                      maxd <= kSymmetryCheckMaxRow ? 1 : 0);
+                      maxd <= kSymmetryCheckMaxRow ? 1 : 0, 1);
     dev_free_on(ctx, sblk, stage, stream);  // stream-ordered: after the build
     if (rc) { matrix_free_on(m, stream); return rc; }
     *out = m;
@@ -734,7 +979,8 @@ void gsofa::host::matrix_free_on(gsofa_matrix* m, cudaStream_t stream) {
 
 int gsofa::host::matrix_build(gsofa_ctx* ctx, cudaStream_t stream, int32_t* dstatus,
                               gsofa_matrix* m, int64_t nnz_in, const int32_t* dbeg,
-                              const int32_t* dcol_in, int check_symmetry) {
+                              const int32_t* dcol_in, int check_symmetry,
+                              int check_dup) {
     const int32_t n = m->n;
     const size_t N1 = (size_t)n + 1;
     size_t scan_bytes = canonicalize_scan_bytes(n);
@@ -757,7 +1003,7 @@ int gsofa::host::matrix_build(gsofa_ctx* ctx, cudaStream_t stream, int32_t* dsta
     if (e == cudaSuccess)
         e = launch_canonicalize(n, nnz_in, dbeg, dcol_in, m->rowptr, m->col, tcount, tpad,
                                 m->trowptr, m->tcol, tfill, m->wdeg, m->dplanes, m->nplanes,
-                                m->asym, check_symmetry, scan_tmp, scan_bytes, dstatus, stream);
+                                m->asym, check_symmetry, check_dup, scan_tmp, scan_bytes, dstatus, stream);
     dev_free_on(ctx, sblk, stage, stream);  // stream-ordered: after the build
     return e == cudaSuccess ? GSOFA_OK : cuda_fail(ctx, e, "matrix build");
 }
@@ -858,6 +1104,7 @@ int gsofa_destroy(gsofa_ctx* ctx) {
         dev_free(ctx, ctx->gbitmap, ctx->gbitmap_bytes);
         dev_free(ctx, ctx->gprev, ctx->gprev_bytes);
         dev_free(ctx, ctx->scan_tmp, ctx->scan_tmp_bytes);
+        dev_free(ctx, ctx->hub_ws, ctx->hub_ws_bytes);
         dev_free(ctx, ctx->small, 256);
         cudaStreamSynchronize(ctx->stream);
         cudaStreamSynchronize(ctx->own_stream);
@@ -906,7 +1153,10 @@ int gsofa_load_csr(gsofa_ctx* ctx, int32_t n, int64_t nnz, const int32_t* row_be
     int rc = ingest_csr(ctx, ctx->stream, dstatus, n, nnz, row_begin, row_end, col, &m);
     if (rc) return rc;
     cudaError_t e = cudaMemcpyAsync(ctx->h_status, dstatus, 4, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(ctx->h_status + 1, m->asym, 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) m->host_sym = n > 0 && ctx->h_status[1] == 0;
     rc = e != cudaSuccess ? cuda_fail(ctx, e, "load") : check_status(ctx);
     if (rc) {
         dev_free(ctx, m->rowptr, m->bytes);
@@ -1200,7 +1450,13 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
         nmax = std::max(nmax, mats[i]->n);
     }
     if (cudaSetDevice(ctx->device) != cudaSuccess) return set_err(ctx, GSOFA_ERR_CUDA, "cudaSetDevice");
-    for (int32_t i = 0; i < count; i++) total_sources += chunk_weight(ctx, mats[i]);
+    long long weight = 0;
+    bool all_sym = true;
+    for (int32_t i = 0; i < count; i++) {
+        weight += chunk_weight(ctx, mats[i]);
+        total_sources += mats[i]->n;
+        all_sym = all_sym && mats[i]->host_sym > 0;
+    }
     gsofa_batch* b = new (std::nothrow) gsofa_batch();
     if (!b) return set_err(ctx, GSOFA_ERR_OOM_BUDGET, "host allocation failed");
     b->ctx = ctx;
@@ -1216,11 +1472,20 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
         if (rc) return fail(rc);
         b->res[(size_t)i]->batch_owned = true;
     }
+    const bool chain = chain_runs(o);
+    ChainCfg ccfg;
     LaunchCfg cfg;
-    rc = plan_launch(ctx, nmax, &o, &cfg);
+    // the chain's shape: that of the matrices it takes, or of all if it takes none
+    long long chain_sources = 0;
+    for (int32_t i = 0; i < count; i++)
+        if (method_of(mats[i]) == METHOD_CHAIN) chain_sources += mats[i]->n;
+    if (chain_sources == 0) chain_sources = total_sources;
+    rc = chain ? plan_chain(ctx, nmax, all_sym, &o, false, &ccfg) : plan_launch(ctx, nmax, &o, &cfg);
     if (rc) return fail(rc);
-    const long long chunk =
-        o.chunk_sources > 0 ? o.chunk_sources : default_chunk(total_sources, cfg.grid);
+    const long long chunk = chain ? chain_chunk(o, chain_sources, ccfg.grid)
+                            : o.chunk_sources > 0 ? o.chunk_sources
+                                                  : default_chunk(weight, cfg.grid);
+    const long long per_chunk = chain ? 1 : 2;  // work items
     const bool merge = !(o.flags & GSOFA_NO_MERGE);
     int ring = o.cached_closures > 0 ? o.cached_closures : kDefaultRing;
     if (ring > kMaxRing) ring = kMaxRing;
@@ -1233,18 +1498,28 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     for (int32_t k = 0; k < count; k++) {
         const int32_t i = order[(size_t)k];
         descs[(size_t)k] = make_desc(mats[i], b->res[(size_t)i], base);
-        base += 2ll * ((mats[i]->n + chunk - 1) / chunk);
+        base += per_chunk * ((mats[i]->n + chunk - 1) / chunk);
         seg[(size_t)k + 1] = seg[(size_t)k] + supernode_segment_count(mats[i]->n, o.max_supernode_size);
     }
     b->items = base;
+    HubLaunch HL{};
+    HubCfg hcfg;
+    size_t sz_hub = 0;
+    bool hub = false;
+    for (int32_t k = 0; k < count && chain; k++)
+        descs[(size_t)k].method = method_of(mats[order[(size_t)k]]);
+    if (chain) hub = plan_hub(ctx, &descs, o, nullptr, &sz_hub, &HL, &hcfg);
     const size_t sz_small = 256;
     const size_t sz_desc = align256(sizeof(MatDesc) * (size_t)count);
     const size_t sz_seg = align256(sizeof(long long) * ((size_t)count + 1));
     const size_t sz_cnt = align256(8ull * CNT_SLOTS * (size_t)count);
-    const size_t sz_q = align256((size_t)cfg.grid * (size_t)nmax * 4);
-    const size_t sz_ring = merge ? align256((size_t)cfg.grid * (size_t)ring * (size_t)cfg.words * 4) : 0;
-    const size_t sz_gbm = cfg.smem_bitmap ? 0 : align256((size_t)cfg.grid * (size_t)cfg.words * 4);
-    b->ws_bytes = sz_small + sz_desc + sz_seg + sz_cnt + sz_q + sz_ring + sz_gbm;
+    const size_t sz_q = align256((size_t)(chain ? ccfg.grid : cfg.grid) * (size_t)nmax * 4);
+    const size_t sz_ring =
+        merge && !chain ? align256((size_t)cfg.grid * (size_t)ring * (size_t)cfg.words * 4) : 0;
+    const size_t sz_gbm =
+        chain ? align256((size_t)ccfg.grid * (size_t)ccfg.gbm_count * (size_t)ccfg.words * 4)
+        : cfg.smem_bitmap ? 0 : align256((size_t)cfg.grid * (size_t)cfg.words * 4);
+    b->ws_bytes = sz_small + sz_desc + sz_seg + sz_cnt + sz_q + sz_ring + sz_gbm + sz_hub;
     rc = dev_alloc(ctx, b->ws_bytes, &b->ws);
     if (rc) return fail(rc);
     char* p = reinterpret_cast<char*>(b->ws);
@@ -1259,9 +1534,15 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     p += sz_cnt;
     int32_t* dq = reinterpret_cast<int32_t*>(p);
     p += sz_q;
-    uint32_t* dring = merge ? reinterpret_cast<uint32_t*>(p) : nullptr;
+    uint32_t* dring = sz_ring ? reinterpret_cast<uint32_t*>(p) : nullptr;
     p += sz_ring;
-    uint32_t* dgbm = cfg.smem_bitmap ? nullptr : reinterpret_cast<uint32_t*>(p);
+    uint32_t* dgbm = sz_gbm ? reinterpret_cast<uint32_t*>(p) : nullptr;
+    p += sz_gbm;
+    if (hub) {
+        plan_hub(ctx, &descs, o, p, &sz_hub, &HL, &hcfg);
+        HL.mats = ddesc;
+        HL.status = dstatus;
+    }
     for (int32_t k = 0; k < count; k++)  // matrix i's counters at slot i, whatever its launch order
         descs[(size_t)k].counters = dcnt + (size_t)order[(size_t)k] * CNT_SLOTS;
     cudaError_t e;
@@ -1298,13 +1579,28 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     L.chain_wait_ns = chain_wait_ns(o);
     L.ring = ring;
     L.sample_stride = 1;
+    ChainLaunch CL{};
+    CL.mats = ddesc;
+    CL.nmats = count;
+    CL.total_items = b->items;
+    CL.work_counter = wc;
+    CL.queue = dq;
+    CL.gbm = dgbm;
+    CL.chunk = (int)chunk;
+    CL.sample_stride = 1;
+    CL.status = dstatus;
+    if (chain) fill_chain_launch(&CL, ccfg, o, nmax);
+    CL.fallback = hub ? HL.fallback : nullptr;
 
     // capture: reset -> traversal -> supernodes -> read-back
     if ((e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed)) != cudaSuccess)
         return fail(cuda_fail(ctx, e, "cudaStreamBeginCapture"));
     e = cudaMemsetAsync(b->ws, 0, 128, ctx->stream);
     if (e == cudaSuccess) e = launch_batch_reset(ddesc, count, ctx->stream);
-    if (e == cudaSuccess && b->items > 0)
+    if (e == cudaSuccess && hub) e = launch_hub(HL, hcfg, (o.flags & GSOFA_DIGESTS) != 0, ctx->stream);
+    if (e == cudaSuccess && b->items > 0 && chain)  // with what the hubs' launch leaves it
+        e = launch_chain(CL, ccfg.block, false, ccfg.grid, ccfg.smem, ctx->stream);
+    else if (e == cudaSuccess && b->items > 0)
         e = launch_traverse(L, cfg.block, cfg.grid, cfg.smem_bitmap, cfg.smem, ctx->stream);
     if (e == cudaSuccess && (o.flags & GSOFA_SUPERNODES))
         e = launch_supernodes_batch(ddesc, count, o.max_supernode_size, dseg, seg[(size_t)count],

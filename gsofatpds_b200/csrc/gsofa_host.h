@@ -42,6 +42,9 @@ struct gsofa_ctx {
     void* small = nullptr;  // work counter (8 B) + status (4 B)
     void* scan_tmp = nullptr;
     size_t scan_tmp_bytes = 0;
+    void* hub_ws = nullptr;
+    size_t hub_ws_bytes = 0;
+    std::vector<int32_t> h_fallback;
 };
 
 struct gsofa_matrix {
@@ -55,7 +58,8 @@ struct gsofa_matrix {
     int32_t* wdeg = nullptr;
     uint32_t* dplanes = nullptr;
     int32_t nplanes = 0;
-    int32_t* asym = nullptr;  // device word: 0 iff the pattern is symmetric
+    // device words: [0] 0 iff the pattern is symmetric, [1] non-zero when a row may hold an id twice
+    int32_t* asym = nullptr;
     size_t bytes = 0;
     mutable int host_sym = -1;  // the device word read back once (-1: not yet)
 };
@@ -141,6 +145,29 @@ long long default_chunk(long long total_sources, int grid);
 // ctx->stream) and keeps it with m.
 long long chunk_weight(gsofa_ctx* ctx, const gsofa_matrix* m);
 int default_block(int32_t nmax, int smem_per_sm);
+// The counting traversal's launch shape (gsofa_chain.cu).
+struct ChainCfg {
+    int block = 512;
+    int grid = 0;
+    size_t smem = 0;
+    long long words = 0;       // of the largest matrix's bitmap
+    long long smem_words = 0;  // bitmap words in shared memory (0: bitmaps in global memory)
+    int gbm_count = 2;         // global bitmaps per CTA
+};
+bool chain_runs(const gsofa_opts& o);
+int plan_chain(gsofa_ctx* ctx, int32_t nmax, bool all_sym, const gsofa_opts* o, bool serve,
+               ChainCfg* c);
+// The launch's fields that follow from the shape, the options and the largest order.
+void fill_chain_launch(ChainLaunch* L, const ChainCfg& c, const gsofa_opts& o, int32_t nmax);
+// Which counting traversal a matrix takes (its host_sym must be known).
+int32_t method_of(const gsofa_matrix* m);
+// A launch of gsofa_hub.cu over descriptors whose methods are set: fills their
+// hub_* fields, `L` and `c`, and places the workspace of *bytes in `ws` (null:
+// sizes only).  False: no matrix takes it.
+bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, void* ws,
+              size_t* bytes, HubLaunch* L, HubCfg* c);
+// Consecutive sources per work item.
+long long chain_chunk(const gsofa_opts& o, long long total_sources, int grid);
 // Result arrays of an n-row matrix, zero-initialised on `stream`.
 int result_alloc_on(gsofa_ctx* ctx, int32_t n, uint32_t flags, int32_t mss, cudaStream_t stream,
                     gsofa_result** out);
@@ -179,7 +206,8 @@ void matrix_free_on(gsofa_matrix* m, cudaStream_t stream);
 // must already be on the device (or queued); row v of the input is
 // dcol_in[dbeg[v] ...] with the length m->rowptr gives it.
 int matrix_build(gsofa_ctx* ctx, cudaStream_t stream, int32_t* dstatus, gsofa_matrix* m,
-                 int64_t nnz_in, const int32_t* dbeg, const int32_t* dcol_in, int check_symmetry);
+                 int64_t nnz_in, const int32_t* dbeg, const int32_t* dcol_in, int check_symmetry,
+                 int check_dup);
 // Device bytes ingest_csr holds for a matrix (kept) and while it runs (staging).
 void ingest_bytes(int32_t n, int64_t nnz, size_t* kept, size_t* staging);
 size_t result_bytes(int32_t n, uint32_t flags);

@@ -1,0 +1,925 @@
+// gsofa_hub.cu -- the counting traversal for matrices with a large strongly
+// connected core: every source searched on its own, on top of what a hub
+// reaches.
+//
+// For a vertex b let label(v) be the smallest value, over all paths b -> v, of
+// the path's largest id before v (b included).  Then b reaches v through ids
+// below s exactly when label(v) < s, for every s at once.  With the labels of
+// one well connected b in A and in A^T (`lam` of the two directions), a source
+// s that reaches b through ids below s -- one comparison, label of s in the
+// other direction below s -- has
+//     F(s) = { v : label(v) < s }  u  what s reaches beyond it,
+// and the first set's sizes and digest are known for every s in advance: each v
+// joins it at s = label(v) + 1 and leaves the part above s at s = v, so the
+// totals are prefix sums over s of the changes at these times (its digest too:
+// a 32-id word's term changes only there).  What is left per source is the
+// search beyond the hub's set: on the circuit-like n = 659,033 matrix 21 ids on
+// average, and no source waits for another.  gsofa_chain.cu, where a chunk's
+// sources are a chain, took 450 ms on that matrix.
+//
+// Three hubs serve three windows of s (above n/16, n/16 down to n/256, below),
+// each among the ids below its window's, so that early sources have one too;
+// the smaller windows' labels expand only ids below their end.
+//
+//   hub_kernel     per matrix and window: the vertex of largest in-degree times
+//                  out-degree below the window's start
+//   label_*_kernel label-correcting rounds, by one CTA per (matrix, window,
+//                  direction) in shared memory up to 50,000 rows, else one launch
+//                  of the whole GPU per round (46 and 93 rounds on the
+//                  circuit-like matrix, 3.5 to 5.2 reads per entry)
+//   event_kernel   a warp per word of 32 ids: the changes of the totals
+//   (a scan)       the totals of the hub's set for every s
+//   extra_kernel   a warp per (source, direction): the search beyond, in a
+//                  table in shared memory
+//   large_kernel   the sources whose search outgrew the table: a CTA each, in
+//                  a bitmap
+//
+// A matrix of at most kDirectMax rows has every source searched alone, without
+// a hub.  A matrix in which more than a quarter of the searches outgrow the
+// table (no core that the hub lies in: meshes) is left to gsofa_chain.cu, and
+// so are matrices with repeated entries in a row.
+#include <algorithm>
+#include <climits>
+
+#include <cub/device/device_scan.cuh>
+
+#include "gsofa_device.cuh"
+
+namespace gsofa {
+
+namespace {
+
+constexpr int kWindows = 3;
+constexpr int kHubs = 4;  // two for the first window, one for each other
+constexpr int kBases = 2;  // arrays of totals: a source has at most two hubs to choose from
+constexpr int kMaxRounds = 192;  // label rounds before a matrix is left to the chain
+constexpr int kLabelThreads = 1024;
+constexpr int kNoLabel = 0x7f7f7f7f;
+constexpr int kExtraThreads = 256;
+constexpr int kJudgeAfter = 512;  // searches before a matrix may be left to the chain
+
+struct WarpTable {
+    uint32_t key[kSlots];
+    uint32_t msk[kSlots];
+    int32_t list[kListRoom];
+};
+
+// sources of window l: above window_end(n, l + 1), up to window_end(n, l); its
+// labels expand ids below window_end(n, l); its hub lies below window_end(n, l + 1)
+__host__ __device__ __forceinline__ int window_end(int n, int l) { return n >> (4 * l); }
+
+__device__ __forceinline__ int window_of(int n, int s) {
+    return s > window_end(n, 1) ? 0 : s > window_end(n, 2) ? 1 : 2;
+}
+
+// hubs 0 and 1 serve the first window, 2 and 3 the others
+__host__ __device__ __forceinline__ int window_of_hub(int h) { return h < 2 ? 0 : h - 1; }
+
+__device__ __forceinline__ long long lam_at(const HubLaunch& P, const MatDesc& M, int h, int d) {
+    return (2ll * h + d) * P.total + M.hub_off;
+}
+
+// Per matrix and hub, several CTAs: the largest key (degree product, then
+// smallest id).  The first window's two hubs are the best of the even and of
+// the odd ids.
+__global__ void hub_kernel(HubLaunch P) {
+    const int mi = blockIdx.x / kHubs, h = blockIdx.x % kHubs;
+    const MatDesc& M = P.mats[mi];
+    if (M.method != METHOD_HUB) return;
+    const int lim = max(2, window_end(M.n, window_of_hub(h) + 1));
+    const int step = h < 2 ? 2 : 1;
+    unsigned long long mine = 0;
+    for (int v = (h == 1) + step * (blockIdx.y * blockDim.x + threadIdx.x); v < lim;
+         v += step * gridDim.y * blockDim.x) {
+        const unsigned long long a = (unsigned)row_degree<false>(M.rowptr, v);
+        const unsigned long long b = (unsigned)row_degree<false>(M.trowptr, v);
+        const unsigned long long p = min(a * b, 0xfffffffeull) + 1ull;
+        mine = max(mine, p << 32 | (0xffffffffu - (unsigned)v));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mine = max(mine, __shfl_xor_sync(FULL_MASK, mine, o));
+    if ((threadIdx.x & 31) == 0 && mine) atomicMax(P.hubs + blockIdx.x, mine);
+}
+
+__device__ __forceinline__ int hub_of(const HubLaunch& P, int mi, int h) {
+    return (int)(0xffffffffu - (unsigned)P.hubs[mi * kHubs + h]);
+}
+
+__device__ __forceinline__ unsigned cluster_size() {
+    unsigned x;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(x));
+    return x;
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned x;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(x));
+    return x;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// A shared-memory address of this CTA, as the same place in CTA `rank`.
+__device__ __forceinline__ unsigned at_rank(unsigned addr, unsigned rank) {
+    unsigned x;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(x) : "r"(addr), "r"(rank));
+    return x;
+}
+__device__ __forceinline__ int dsm_ld(unsigned a) {
+    int x;
+    asm volatile("ld.volatile.shared::cluster.s32 %0, [%1];" : "=r"(x) : "r"(a) : "memory");
+    return x;
+}
+__device__ __forceinline__ int dsm_min(unsigned a, int v) {
+    int x;
+    asm volatile("atom.relaxed.cluster.shared::cluster.min.s32 %0, [%1], %2;" : "=r"(x) : "r"(a), "r"(v) : "memory");
+    return x;
+}
+__device__ __forceinline__ unsigned dsm_or(unsigned a, unsigned v) {
+    unsigned x;
+    asm volatile("atom.relaxed.cluster.shared::cluster.or.b32 %0, [%1], %2;" : "=r"(x) : "r"(a), "r"(v) : "memory");
+    return x;
+}
+__device__ __forceinline__ void dsm_and(unsigned a, unsigned v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.and.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ int dsm_add(unsigned a, int v) {
+    int x;
+    asm volatile("atom.relaxed.cluster.shared::cluster.add.s32 %0, [%1], %2;" : "=r"(x) : "r"(a), "r"(v) : "memory");
+    return x;
+}
+
+// Labels of one (matrix, hub, direction) by one thread block cluster, spread
+// over its CTAs' shared memory: the labels and one bit per id that is queued,
+// 32-id words dealt out in turn.  A round expands the ids queued in the one
+// before; an id's bit is cleared before its label is read, so an improvement
+// is either read there or queues the id again.  Queues are in global memory.
+__global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch P) {
+    extern __shared__ uint4 dyn_smem[];
+    __shared__ int cnt[3];  // of rank 0: queued ids per round, in turn
+    const unsigned C = cluster_size(), rank = cluster_rank();
+    const unsigned shift = 31 - __clz(C);
+    const int job = blockIdx.x / C;
+    const int mi = job / (2 * kHubs), h = (job >> 1) % kHubs, d = job & 1;
+    const MatDesc& M = P.mats[mi];
+    if (M.method != METHOD_HUB) return;
+    const int l = window_of_hub(h);
+    const int n = M.n, nw = (n + 31) >> 5;
+    const int bound = l == 0 ? n : window_end(n, l) + 1;  // sources of the window lie below
+    const Graph G = d ? Graph{M.trowptr, M.tcol} : Graph{M.rowptr, M.col};
+    const long long at = lam_at(P, M, h, d);
+    const int mine = (nw + (int)C - 1) >> shift;  // words of this CTA, at most
+    int32_t* const lam = reinterpret_cast<int32_t*>(dyn_smem);
+    uint32_t* const inq = reinterpret_cast<uint32_t*>(lam + 32 * mine);
+    const unsigned lam_a = (unsigned)__cvta_generic_to_shared(lam);
+    const unsigned inq_a = (unsigned)__cvta_generic_to_shared(inq);
+    const unsigned cnt_a = at_rank((unsigned)__cvta_generic_to_shared(cnt), 0);
+    auto group_sync = [&]() {
+        if (C == 1) __syncthreads();
+        else cluster_sync();
+    };
+    auto lam_of = [&](int v) {
+        const unsigned w = (unsigned)v >> 5;
+        return at_rank(lam_a + 4 * (32 * (w >> shift) + ((unsigned)v & 31)), w & (C - 1));
+    };
+    auto inq_of = [&](int v) {
+        const unsigned w = (unsigned)v >> 5;
+        return at_rank(inq_a + 4 * (w >> shift), w & (C - 1));
+    };
+    int32_t* const q[2] = {P.lq + 2 * at, P.lq + 2 * at + M.hub_len};
+    const int lane = threadIdx.x & 31;
+    const int gw = (int)(rank * kLabelThreads + threadIdx.x) >> 5;
+    const int nwarps = (int)C * (kLabelThreads / 32);
+    for (int v = threadIdx.x; v < 32 * mine; v += kLabelThreads) lam[v] = kNoLabel;
+    for (int w = threadIdx.x; w < mine; w += kLabelThreads) inq[w] = 0u;
+    if (threadIdx.x == 0) {
+        cnt[0] = 1;
+        cnt[1] = cnt[2] = 0;
+    }
+    group_sync();
+    if (rank == 0 && threadIdx.x == 0) {
+        const int hub = hub_of(P, mi, h);
+        dsm_min(lam_of(hub), hub);
+        __stcg(q[0], hub);
+    }
+    group_sync();
+    int r = 0, count = 0;
+    for (; r < kMaxRounds; r++) {
+        count = dsm_ld(cnt_a + 4 * (r % 3));
+        if (count == 0) break;
+        const int32_t* cur = q[r & 1];
+        int32_t* const next = q[(r + 1) & 1];
+        const unsigned nc = cnt_a + 4 * ((r + 1) % 3);
+        if (rank == 0 && threadIdx.x == 0) cnt[(r + 2) % 3] = 0;
+        // few ids queued: fewer per warp, so that more warps work
+        const int per = count >= 32 * nwarps ? 32 : (count + nwarps - 1) / nwarps;
+        for (int base = gw * per; base < count; base += nwarps * per) {
+            int s0 = 0, its = 0, nl = 0;
+            if (lane < per && base + lane < count) {
+                const int u = __ldcg(cur + base + lane);
+                const int a0 = __ldg(G.rp + u), a1 = __ldg(G.rp + u + 1);
+                dsm_and(inq_of(u), ~(1u << (u & 31)));
+                nl = max(dsm_ld(lam_of(u)), u);
+                s0 = a0 & ~3;
+                its = ((a1 & ~3) - s0) >> 2;
+            }
+            const int incl = warp_incl_sum(its, lane);
+            const int total = __shfl_sync(FULL_MASK, incl, 31);
+            int o;
+            int p = flat_int4(lane, total, s0, its, incl, &o);
+            int4 e = p >= 0 ? ld_row4<false>(G.cl + p) : make_int4(-1, -1, -1, -1);
+            for (int j0 = 0; j0 < total; j0 += 32) {
+                const int onl = __shfl_sync(FULL_MASK, nl, o);
+                int4 en = make_int4(-1, -1, -1, -1);
+                if (j0 + 32 < total) {
+                    p = flat_int4(j0 + 32 + lane, total, s0, its, incl, &o);
+                    if (p >= 0) en = ld_row4<false>(G.cl + p);
+                }
+                const int ws[4] = {e.x, e.y, e.z, e.w};
+                int lw[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) lw[c] = ws[c] >= 0 ? dsm_ld(lam_of(ws[c])) : -1;
+#pragma unroll
+                for (int c = 0; c < 4; c++) lw[c] = onl < lw[c] ? dsm_min(lam_of(ws[c]), onl) : -1;
+                unsigned was[4], bal[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    was[c] = lw[c] > onl && ws[c] < bound ? dsm_or(inq_of(ws[c]), 1u << (ws[c] & 31)) : ~0u;
+                int k = 0;
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    bal[c] = __ballot_sync(FULL_MASK, !((was[c] >> (ws[c] & 31)) & 1u));
+                    k += __popc(bal[c]);
+                }
+                if (k) {
+                    int to = 0;
+                    if (lane == 0) to = dsm_add(nc, k);
+                    to = __shfl_sync(FULL_MASK, to, 0);
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        // a round lists an id once, so at most n
+                        const int x = to + __popc(bal[c] & ((1u << lane) - 1u));
+                        if (((bal[c] >> lane) & 1u) && x < M.hub_len) __stcg(next + x, ws[c]);
+                        to += __popc(bal[c]);
+                    }
+                }
+                e = en;
+            }
+        }
+        group_sync();
+    }
+    if (r == kMaxRounds && dsm_ld(cnt_a + 4 * (r % 3)) != 0 && rank == 0 && threadIdx.x == 0)
+        atomicExch(P.fallback + mi, 1);  // unfinished labels are too large
+    for (int w = (int)rank + (int)C * (threadIdx.x >> 5); w < nw; w += (int)C * (kLabelThreads / 32)) {
+        // whole words: the ids from n on keep kNoLabel
+        P.lam[at + 32ll * w + lane] = lam[32 * (w >> shift) + lane];
+    }
+    group_sync();  // no CTA leaves while another may still read its counts
+}
+
+// The same by the whole GPU, one launch per round (labels, queues, counts in
+// global memory): blockIdx.y is the job, a launch that finds nothing queued
+// ends at once.  `last`: the matrix goes to the chain if this round leaves ids
+// queued.
+__global__ void label_start_kernel(HubLaunch P) {
+    const int job = blockIdx.x;
+    const int mi = job / (2 * kHubs), h = (job >> 1) % kHubs, d = job & 1;
+    const MatDesc& M = P.mats[mi];
+    if (M.method != METHOD_HUB || threadIdx.x) return;
+    const long long at = lam_at(P, M, h, d);
+    const int hub = hub_of(P, mi, h);
+    P.lam[at + hub] = hub;
+    P.lq[2 * at] = hub;
+    P.lcnt[4ll * job] = 1;
+}
+
+__global__ void __launch_bounds__(kLabelThreads) label_round_kernel(HubLaunch P, int r, int last) {
+    const int job = blockIdx.y;
+    int32_t* const cnt = P.lcnt + 4ll * job;
+    const int count = cnt[r % 3];
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt[(r + 2) % 3] = 0;
+    if (count == 0) return;
+    const int mi = job / (2 * kHubs), h = (job >> 1) % kHubs, d = job & 1;
+    if (last && blockIdx.x == 0 && threadIdx.x == 0) atomicExch(P.fallback + mi, 1);
+    const int lane = threadIdx.x & 31;
+    const int gw = (blockIdx.x * kLabelThreads + threadIdx.x) >> 5;
+    const int nwarps = (int)gridDim.x * (kLabelThreads / 32);
+    // few ids queued: fewer per warp, so that more warps work
+    const int per = count >= 32 * nwarps ? 32 : (count + nwarps - 1) / nwarps;
+    if (gw * per >= count) return;
+    const MatDesc& M = P.mats[mi];
+    const int n = M.n;
+    const int l = window_of_hub(h);
+    const int bound = l == 0 ? n : window_end(n, l) + 1;
+    const Graph G = d ? Graph{M.trowptr, M.tcol} : Graph{M.rowptr, M.col};
+    const long long at = lam_at(P, M, h, d);
+    int32_t* const lam = P.lam + at;
+    int32_t* const stamp = P.stamp + at;
+    const int32_t* cur = P.lq + 2 * at + (r & 1) * M.hub_len;
+    int32_t* const next = P.lq + 2 * at + ((r + 1) & 1) * M.hub_len;
+    for (int base = gw * per; base < count; base += nwarps * per) {
+        int s0 = 0, its = 0, nl = 0;
+        if (lane < per && base + lane < count) {
+            const int u = cur[base + lane];
+            const int a0 = __ldg(G.rp + u), a1 = __ldg(G.rp + u + 1);
+            nl = max(__ldcg(lam + u), u);
+            s0 = a0 & ~3;
+            its = ((a1 & ~3) - s0) >> 2;
+        }
+        const int incl = warp_incl_sum(its, lane);
+        const int total = __shfl_sync(FULL_MASK, incl, 31);
+        int o;
+        int p = flat_int4(lane, total, s0, its, incl, &o);
+        int4 e = p >= 0 ? ld_row4<false>(G.cl + p) : make_int4(-1, -1, -1, -1);
+        for (int j0 = 0; j0 < total; j0 += 32) {
+            const int onl = __shfl_sync(FULL_MASK, nl, o);
+            int4 en = make_int4(-1, -1, -1, -1);
+            if (j0 + 32 < total) {
+                p = flat_int4(j0 + 32 + lane, total, s0, its, incl, &o);
+                if (p >= 0) en = ld_row4<false>(G.cl + p);
+            }
+            const int ws[4] = {e.x, e.y, e.z, e.w};
+            int lw[4], old[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) lw[c] = ws[c] >= 0 ? __ldcg(lam + ws[c]) : -1;
+#pragma unroll
+            for (int c = 0; c < 4; c++) old[c] = onl < lw[c] ? atomicMin(lam + ws[c], onl) : -1;
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                old[c] = old[c] > onl && ws[c] < bound ? atomicExch(stamp + ws[c], r + 1) : r + 1;
+            unsigned bal[4];
+            int k = 0;
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                bal[c] = __ballot_sync(FULL_MASK, old[c] != r + 1);
+                k += __popc(bal[c]);
+            }
+            if (k) {
+                int to = 0;
+                if (lane == 0) to = atomicAdd(cnt + (r + 1) % 3, k);
+                to = __shfl_sync(FULL_MASK, to, 0);
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    // a round lists an id once, so at most n
+                    const int x = to + __popc(bal[c] & ((1u << lane) - 1u));
+                    if (((bal[c] >> lane) & 1u) && x < M.hub_len) next[x] = ws[c];
+                    to += __popc(bal[c]);
+                }
+            }
+            e = en;
+        }
+    }
+}
+
+// The changes over s of the hub set's totals.  A warp per word: lane j is id
+// v = 32 w + j, in the set from s = label + 1 on, above s until s = v.
+__global__ void event_kernel(HubLaunch P, int digests) {
+    const int mi = blockIdx.y / (2 * kHubs), h = (blockIdx.y >> 1) % kHubs, d = blockIdx.y & 1;
+    const MatDesc& M = P.mats[mi];
+    if (M.method != METHOD_HUB) return;
+    const int n = M.n;
+    const int l = window_of_hub(h);
+    const int lo = l == kWindows - 1 ? 0 : window_end(n, l + 1) + 1;  // the window's sources
+    const int hi = l == 0 ? n - 1 : window_end(n, l);
+    if (lo > hi) return;
+    const int32_t* lam = P.lam + lam_at(P, M, h, d);
+    Tot* const D = P.base + (2ll * (h == 1) + d) * P.total + M.hub_off;
+    const int lane = threadIdx.x & 31;
+    const int nw = (n + 31) >> 5;
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nw;
+         w += (gridDim.x * blockDim.x) >> 5) {
+        const int v = 32 * w + lane;
+        const int lv = v < n ? __ldg(lam + v) : INT_MAX;
+        int in = -1, out = -1, ve = -1, deg = 0;
+        if (lv < hi) {
+            in = max(lv + 1, lo);
+            out = min(v, hi + 1);
+            if (in >= out) in = out = -1;
+            ve = max(max(lv, v) + 1, lo);
+            if (ve > hi) ve = -1;
+            else if (d == 0) deg = row_degree<false>(M.rowptr, v);
+        }
+        if (!__any_sync(FULL_MASK, in >= 0 || ve >= 0)) continue;
+        uint32_t m_in = 0, m_in1 = 0, m_out = 0, m_out1 = 0;  // the word at and before the lane's times
+        int c_in = 0, c_out = 0, c_ve = 0;
+        unsigned long long s_ve = 0;
+        bool lead_in = in >= 0, lead_out = out >= 0, lead_ve = ve >= 0, in_at_out = false;
+        for (int i = 0; i < 32; i++) {
+            const int ti = __shfl_sync(FULL_MASK, in, i), to = __shfl_sync(FULL_MASK, out, i);
+            const int te = __shfl_sync(FULL_MASK, ve, i), dg = __shfl_sync(FULL_MASK, deg, i);
+            const uint32_t bit = 1u << i;
+            if (ti >= 0) {
+                if (ti <= in && in < to) m_in |= bit;
+                if (ti <= in - 1 && in - 1 < to) m_in1 |= bit;
+                if (ti <= out && out < to) m_out |= bit;
+                if (ti <= out - 1 && out - 1 < to) m_out1 |= bit;
+                if (ti == in) {
+                    c_in++;
+                    if (i < lane) lead_in = false;
+                }
+                if (to == out) {
+                    c_out++;
+                    if (i < lane) lead_out = false;
+                }
+                if (ti == out) in_at_out = true;
+            }
+            if (te >= 0 && te == ve) {
+                c_ve++;
+                s_ve += (unsigned)dg;
+                if (i < lane) lead_ve = false;
+            }
+        }
+        if (lead_in) {
+            atomicAdd(&D[in].gt, c_in);
+            if (digests) atomicAdd(&D[in].dig, word_digest(w, m_in) - word_digest(w, m_in1));
+        }
+        if (lead_out) {
+            atomicAdd(&D[out].gt, -c_out);
+            if (digests && !in_at_out)
+                atomicAdd(&D[out].dig, word_digest(w, m_out) - word_digest(w, m_out1));
+        }
+        if (lead_ve) {
+            atomicAdd(&D[ve].v, c_ve);
+            if (d == 0) atomicAdd(&D[ve].e, s_ve);
+        }
+        // the ids below s leave with the window
+        const int all = __reduce_add_sync(FULL_MASK, ve >= 0 ? 1 : 0);
+        const unsigned long long sum = warp_sum64((unsigned long long)(unsigned)deg);
+        if (lane == 0 && all) {
+            atomicAdd(&D[hi + 1].v, -all);
+            if (d == 0) atomicAdd(&D[hi + 1].e, 0ull - sum);
+        }
+    }
+}
+
+struct TotSum {
+    __host__ __device__ Tot operator()(const Tot& a, const Tot& b) const {
+        return Tot{a.gt + b.gt, a.v + b.v, a.e + b.e, a.dig + b.dig};
+    }
+};
+
+// A search's base: the hub's labels in its direction (null: none), and the
+// totals of the hub's set.
+struct Base {
+    const int32_t* lam;
+    Tot t;
+};
+
+__device__ __forceinline__ Base base_of(const HubLaunch& P, const MatDesc& M, int s, int d, bool sym) {
+    Base b{nullptr, {0, 0, 0ull, 0ull}};
+    if (M.method != METHOD_HUB) return b;
+    const int l = window_of(M.n, s);
+    // the hubs s reaches; of two the one that reaches more
+    for (int h = l == 0 ? 0 : l + 1; h <= (l == 0 ? 1 : l + 1); h++) {
+        if (__ldg(P.lam + lam_at(P, M, h, sym ? d : 1 - d) + s) >= s) continue;
+        const Tot t = P.base[(2ll * (h == 1) + d) * P.total + M.hub_off + s];
+        if (b.lam && t.gt + t.v <= b.t.gt + b.t.v) continue;
+        b.lam = P.lam + lam_at(P, M, h, d);
+        b.t = t;
+    }
+    return b;
+}
+
+// the hub set's ids above s in word w
+__device__ __forceinline__ uint32_t base_word(const Base& b, int w, int s, int n) {
+    if (!b.lam) return 0u;
+    uint32_t m = 0;
+    const int4* p = reinterpret_cast<const int4*>(b.lam + 32 * w);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int4 x = __ldg(p + k);  // the array is padded to whole words
+        m |= (x.x < s ? 1u : 0u) << (4 * k) | (x.y < s ? 2u : 0u) << (4 * k) |
+             (x.z < s ? 4u : 0u) << (4 * k) | (x.w < s ? 8u : 0u) << (4 * k);
+    }
+    return m & above(w, s);
+}
+
+// Bits of the hub's set among the 128 ids after s: word `lane` for lanes 0..3.
+__device__ __forceinline__ uint32_t base_next128(const Base& b, int s, int n) {
+    const int lane = threadIdx.x & 31;
+    uint32_t mine = 0;
+    if (!b.lam) return 0u;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int v = s + 1 + 32 * j + lane;
+        const uint32_t x = __ballot_sync(FULL_MASK, v < n && __ldg(b.lam + v) < s);
+        if (lane == j) mine = x;
+    }
+    return mine;
+}
+
+__global__ void __launch_bounds__(kExtraThreads, 1024 / kExtraThreads) extra_kernel(HubLaunch P) {
+    extern __shared__ uint4 dyn_smem[];
+    const int lane = threadIdx.x & 31;
+    WarpTable& T = reinterpret_cast<WarpTable*>(dyn_smem)[threadIdx.x >> 5];
+    bool dirty = true;
+    for (;;) {
+        unsigned long long item = 0;
+        if (lane == 0) item = atomicAdd(P.work_counter, 1ull);
+        item = __shfl_sync(FULL_MASK, item, 0);
+        if ((long long)item >= P.total_items) return;
+        int mi = 0;
+        {
+            int lo = 0, hi = P.nmats - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (P.mats[mid].hub_item <= (long long)item) lo = mid;
+                else hi = mid - 1;
+            }
+            mi = lo;
+        }
+        const MatDesc& M = P.mats[mi];
+        if (ld_vol_i32(P.fallback + mi)) continue;
+        if (M.asym[1] != 0) {  // repeated entries: the chain counts a row's distinct ids
+            if (lane == 0) atomicExch(P.fallback + mi, 1);
+            continue;
+        }
+        const int n = M.n;
+        const bool sym = M.asym[0] == 0;
+        const bool digests = M.dig_u != nullptr;
+        const int dirs = sym ? 1 : 2;
+        const int groups = (n + P.group - 1) / P.group;
+        // the matrix's items in an order that spreads the first ones over all
+        // of it (an odd multiplier permutes a power of two)
+        const unsigned slots = (unsigned)M.hub_slots;
+        const unsigned x = ((unsigned)((long long)item - M.hub_item) * 0x9E3779B1u) & (slots - 1);
+        if (x >= (unsigned)(groups * dirs)) continue;
+        const int d = sym ? 0 : (int)(x & 1u);
+        const int g = sym ? (int)x : (int)(x >> 1);
+        const Graph G = d ? Graph{M.trowptr, M.tcol} : Graph{M.rowptr, M.col};
+        const int s_first = g * P.group, s_end = min(n, s_first + P.group);
+        unsigned long long a_fill = 0, a_e = 0, a_v = 0, a_nnz = 0, a_trav = 0;
+        int a_hub = 0, a_large = 0;
+        int r0 = __ldg(G.rp + s_first), r1 = __ldg(G.rp + s_first + 1);
+        int4 pre = make_int4(-1, -1, -1, -1);
+        if (4 * lane < (r1 & ~3) - (r0 & ~3)) pre = ld_row4<false>(G.cl + (r0 & ~3) + 4 * lane);
+        for (int s = s_first; s < s_end; s++) {
+            const int r2 = s + 2 <= n ? __ldg(G.rp + s + 2) : r1;
+            const Base B = base_of(P, M, s, d, sym);
+            if (dirty) {
+                for (int i = lane; i < kSlots; i += 32) {
+                    T.key[i] = kFree;
+                    T.msk[i] = 0u;
+                }
+                dirty = false;
+                __syncwarp();
+            }
+            int found = 0, words = 0, raw = 0, v = 0, trav = 0;
+            unsigned e = 0;
+            bool large = false;
+            auto visit = [&](const int4& q4, bool own_row) -> bool {
+                const int ws[4] = {q4.x, q4.y, q4.z, q4.w};
+                bool todo[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    todo[c] = ws[c] >= 0 && ws[c] != s;
+                    if (own_row) raw += ws[c] > s;
+                }
+                if (B.lam) {
+                    int lw[4];
+#pragma unroll
+                    for (int c = 0; c < 4; c++) lw[c] = todo[c] ? __ldg(B.lam + ws[c]) : -1;
+#pragma unroll
+                    for (int c = 0; c < 4; c++) todo[c] = todo[c] && lw[c] >= s;
+                }
+                if (!__any_sync(FULL_MASK, todo[0] || todo[1] || todo[2] || todo[3])) return true;
+                dirty = true;
+                int nslots = 0, k = 0;
+                bool full = false;
+                unsigned bal[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    bool fresh = false;
+                    if (todo[c]) {
+                        const int i = sparse_slot(T.key, ws[c] >> 5, &nslots);
+                        const uint32_t bit = 1u << (ws[c] & 31);
+                        if (i < 0) full = true;
+                        else fresh = !(atomicOr(T.msk + i, bit) & bit);
+                    }
+                    bal[c] = __ballot_sync(FULL_MASK, fresh);
+                    k += __popc(bal[c]);
+                }
+                words += __reduce_add_sync(FULL_MASK, nslots);
+                int to = found;
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    if ((bal[c] >> lane) & 1u) T.list[to + __popc(bal[c] & ((1u << lane) - 1u))] = ws[c];
+                    to += __popc(bal[c]);
+                }
+                found = to;
+                __syncwarp();
+                return found <= kListCap && words <= kSlotsMax && !__any_sync(FULL_MASK, full);
+            };
+            {
+                const int b = r0 & ~3, plen = (r1 & ~3) - b;
+                int4 q4 = pre;
+                for (int k0 = 0; k0 < plen && !large; k0 += 128) {
+                    int4 qn = make_int4(-1, -1, -1, -1);
+                    if (k0 + 128 + 4 * lane < plen) qn = ld_row4<false>(G.cl + b + k0 + 128 + 4 * lane);
+                    large = !visit(q4, true);
+                    q4 = qn;
+                }
+                trav += plen;
+            }
+            pre = make_int4(-1, -1, -1, -1);
+            if (4 * lane < (r2 & ~3) - (r1 & ~3)) pre = ld_row4<false>(G.cl + (r1 & ~3) + 4 * lane);
+            for (int h = 0; h < found && !large;) {
+                const int end = found;
+                const int u = h + lane < end ? T.list[h + lane] : INT_MAX;
+                int s0 = 0, its = 0;
+                if (u < s) {
+                    const int a0 = __ldg(G.rp + u), a1 = __ldg(G.rp + u + 1);
+                    s0 = a0 & ~3;
+                    its = ((a1 & ~3) - s0) >> 2;
+                    v++;
+                    e += (unsigned)(4 * its - (a1 & 3));
+                }
+                const int incl = warp_incl_sum(its, lane);
+                const int total = __shfl_sync(FULL_MASK, incl, 31);
+                trav += 4 * total;
+                int o;
+                int at = flat_int4(lane, total, s0, its, incl, &o);
+                int4 q4 = at >= 0 ? ld_row4<false>(G.cl + at) : make_int4(-1, -1, -1, -1);
+                for (int j0 = 0; j0 < total && !large; j0 += 32) {
+                    int4 qn = make_int4(-1, -1, -1, -1);
+                    if (j0 + 32 < total) {
+                        at = flat_int4(j0 + 32 + lane, total, s0, its, incl, &o);
+                        if (at >= 0) qn = ld_row4<false>(G.cl + at);
+                    }
+                    large = !visit(q4, false);
+                    q4 = qn;
+                }
+                h = min(h + 32, end);
+            }
+            if (large) {
+                a_large++;
+                if (lane == 0) {
+                    // room for every (source, direction) of the launch
+                    const int p = atomicAdd(P.large_count, 1);
+                    P.large[p] = (unsigned long long)mi << 33 | (unsigned long long)d << 32 | (unsigned)s;
+                }
+            } else {
+                Tot t = B.t;
+                raw = __reduce_add_sync(FULL_MASK, raw);
+                if (found) {
+                    // the found ids word by word: occupied slots listed first
+                    int k = 0;
+                    __syncwarp();
+                    for (int i = lane; i < kSlots; i += 32) {
+                        const bool has = T.key[i] != kFree && (T.msk[i] & above((int)T.key[i], s));
+                        const unsigned b = __ballot_sync(FULL_MASK, has);
+                        if (has) T.list[k + __popc(b & ((1u << lane) - 1u))] = i;
+                        k += __popc(b);
+                    }
+                    __syncwarp();
+                    int gt = 0;
+                    unsigned long long dig = 0;
+                    for (int i = lane; i < k; i += 32) {
+                        const int slot = T.list[i];
+                        const int w = (int)T.key[slot];
+                        const uint32_t hi = T.msk[slot] & above(w, s);
+                        gt += __popc(hi);
+                        if (digests) {
+                            const uint32_t bw = base_word(B, w, s, n);
+                            dig += word_digest(w, bw | hi) - word_digest(w, bw);
+                        }
+                    }
+                    t.gt += __reduce_add_sync(FULL_MASK, gt);
+                    t.v += __reduce_add_sync(FULL_MASK, v);
+                    t.e += (unsigned)__reduce_add_sync(FULL_MASK, e);
+                    if (digests && k) t.dig += warp_sum64(dig);
+                }
+                if (lane == 0) write_row(M, s, d, sym, t, raw, raw);
+                if (d == 1 || sym) {
+                    uint32_t word = base_next128(B, s, n);
+                    if (found) {
+                        const uint32_t x5 = lane < 5 ? sparse_word(T.key, T.msk, ((s + 1) >> 5) + lane) : 0u;
+                        word |= next128(x5, s);
+                    }
+                    if (lane < 4) M.lmask[4ll * s + lane] = word;
+                }
+                a_fill += (unsigned long long)(t.gt - raw) * (sym ? 2 : 1);
+                a_nnz += (unsigned)t.gt;
+                a_trav += (unsigned)trav;
+                a_hub += B.lam != nullptr;
+                if (d == 0) {
+                    a_e += t.e;
+                    a_v += (unsigned)t.v;
+                }
+            }
+            r0 = r1;
+            r1 = r2;
+        }
+        if (lane == 0) {
+            unsigned long long* c = P.counters + (long long)mi * CNT_SLOTS;
+            atomicAdd(c + CNT_FILLS, a_fill);
+            atomicAdd(c + CNT_EDGES_TRAV, a_trav);
+            if (d == 0) {
+                atomicAdd(c + CNT_EDGES_ALG, a_e);
+                atomicAdd(c + CNT_VERTS_ALG, a_v);
+                atomicAdd(c + CNT_NNZ_U, a_nnz);
+            }
+            if (d == 1 || sym) atomicAdd(c + CNT_NNZ_L, a_nnz);
+            if (a_hub) atomicAdd(c + CNT_CHAINED, (unsigned long long)a_hub);
+            const int done = atomicAdd(P.judged + 2 * mi, s_end - s_first) + s_end - s_first;
+            if (a_large) {
+                const int big = atomicAdd(P.judged + 2 * mi + 1, a_large) + a_large;
+                if (M.n > kDirectMax && done >= kJudgeAfter && 4ll * big > done) atomicExch(P.fallback + mi, 1);
+            }
+        }
+    }
+}
+
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) large_kernel(HubLaunch P) {
+    extern __shared__ uint4 dyn_smem[];
+    __shared__ BfsSmem bfs;
+    __shared__ long long item;
+    __shared__ unsigned long long red[BLOCK / 32][4];
+    __shared__ int row[2];
+    const int lane = threadIdx.x & 31;
+    uint32_t* const bm = P.large_smem ? reinterpret_cast<uint32_t*>(dyn_smem)
+                                      : P.gbm + (long long)blockIdx.x * P.bitmap_words;
+    int32_t* const q = P.queue + (long long)blockIdx.x * P.queue_stride;
+    const int count = *P.large_count;
+    if (count == 0) return;
+    for (long long i = threadIdx.x; i < P.bitmap_words; i += BLOCK) bm[i] = 0u;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const unsigned long long k = atomicAdd(P.work_counter + 1, 1ull);
+            item = k < (unsigned long long)count ? (long long)P.large[k] : -1;
+        }
+        __syncthreads();
+        if (item < 0) return;
+        const int mi = (int)(item >> 33), d = (int)(item >> 32) & 1, s = (int)(item & 0xffffffff);
+        const MatDesc& M = P.mats[mi];
+        if (P.fallback[mi]) continue;
+        const int n = M.n, nw = (n + 31) >> 5;
+        const bool sym = M.asym[0] == 0;
+        const bool digests = M.dig_u != nullptr;
+        const Graph G = d ? Graph{M.trowptr, M.tcol} : Graph{M.rowptr, M.col};
+        const Base B = base_of(P, M, s, d, sym);
+        if (threadIdx.x < 32) {
+            const int b = __ldg(G.rp + s) & ~3, e = __ldg(G.rp + s + 1) & ~3;
+            int raw = 0;
+            for (int j = b + lane; j < e; j += 32) raw += __ldg(G.cl + j) > s;
+            raw = __reduce_add_sync(FULL_MASK, raw);
+            if (lane == 0) {
+                row[0] = raw;
+                bfs.rtrav = 0;
+                q[0] = s;
+            }
+        }
+        __syncthreads();
+        if (B.lam)
+            block_bfs<BLOCK, false, true>(bfs, G, bm, q, P.queue_stride, 1, s, s, false, P.status, B.lam);
+        else
+            block_bfs<BLOCK, false, false>(bfs, G, bm, q, P.queue_stride, 1, s, s, false, P.status);
+        unsigned long long vals[4] = {0, 0, 0, 0};  // found above, below, degrees below, digest change
+        for (int w = threadIdx.x; w < nw; w += BLOCK) {
+            const uint32_t x = bm[w];
+            if (!x) continue;
+            const uint32_t hi = x & above(w, s), low = x & below(w, s);
+            vals[0] += __popc(hi);
+            vals[1] += __popc(low);
+            if (digests && hi) {
+                const uint32_t bw = base_word(B, w, s, n);
+                vals[3] += word_digest(w, bw | hi) - word_digest(w, bw);
+            }
+            if (d != 0 || !low) continue;
+            if (__popc(low) <= 2) {
+                for (uint32_t t = low; t; t &= t - 1)
+                    vals[2] += (unsigned)row_degree<false>(M.rowptr, 32 * w + __ffs(t) - 1);
+            } else {
+                for (int k = 0; k < M.nplanes; k++)
+                    vals[2] += (unsigned long long)__popc(low & __ldg(M.dplanes + (long long)k * nw + w)) << k;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            vals[j] = warp_sum64(vals[j]);
+            if (lane == 0) red[threadIdx.x >> 5][j] = vals[j];
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            if (d == 1 || sym) {
+                uint32_t word = base_next128(B, s, n);
+                word |= next128(lane < 5 ? bm[((s + 1) >> 5) + lane] : 0u, s);
+                if (lane < 4) M.lmask[4ll * s + lane] = word;
+            }
+            if (lane == 0) {
+                Tot t = B.t;
+                for (int i = 0; i < BLOCK / 32; i++) {
+                    t.gt += (int)red[i][0];
+                    t.v += (int)red[i][1];
+                    t.e += red[i][2];
+                    t.dig += red[i][3];
+                }
+                write_row(M, s, d, sym, t, row[0], row[0]);
+                unsigned long long* c = P.counters + (long long)mi * CNT_SLOTS;
+                atomicAdd(c + CNT_FILLS, (unsigned long long)(t.gt - row[0]) * (sym ? 2 : 1));
+                atomicAdd(c + CNT_EDGES_TRAV, bfs.rtrav);
+                if (d == 0) {
+                    atomicAdd(c + CNT_EDGES_ALG, t.e);
+                    atomicAdd(c + CNT_VERTS_ALG, (unsigned long long)(unsigned)t.v);
+                    atomicAdd(c + CNT_NNZ_U, (unsigned long long)(unsigned)t.gt);
+                }
+                if (d == 1 || sym) atomicAdd(c + CNT_NNZ_L, (unsigned long long)(unsigned)t.gt);
+                if (B.lam) atomicAdd(c + CNT_CHAINED, 1ull);
+            }
+        }
+        __syncthreads();
+        block_clear<BLOCK>(bm, nw);
+    }
+}
+
+// The counters of every matrix that was not left to the chain.
+__global__ void commit_kernel(HubLaunch P) {
+    const int mi = blockIdx.x;
+    const MatDesc& M = P.mats[mi];
+    if (M.method != METHOD_CHAIN && !P.fallback[mi] && threadIdx.x < CNT_SLOTS)
+        M.counters[threadIdx.x] += P.counters[(long long)mi * CNT_SLOTS + threadIdx.x];
+}
+
+}  // namespace
+
+
+int hub_count() { return kHubs; }
+int hub_bases() { return kBases; }
+
+// The largest cluster's shared memory per CTA for a matrix of order n.
+size_t label_smem_bytes(int32_t n, int cluster) {
+    const size_t words = (((size_t)n + 31) / 32 + (size_t)cluster - 1) / (size_t)cluster;
+    return 33 * 4 * words + 16;
+}
+
+size_t hub_scan_bytes(long long count) {
+    size_t b = 0;
+    cub::DeviceScan::InclusiveScan(nullptr, b, (const Tot*)nullptr, (Tot*)nullptr, TotSum(), (int)count);
+    return b;
+}
+
+int large_occupancy(int block, size_t smem) {
+    int occ = 0;
+    cudaError_t e;
+    if (block == 256) {
+        e = cudaFuncSetAttribute(large_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, large_kernel<256>, 256, smem);
+    } else {
+        e = cudaFuncSetAttribute(large_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, large_kernel<1024>, 1024, smem);
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess ? occ : 0;
+}
+
+cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(L.zeroed, 0, c.zeroed_bytes, st);
+    if (e != cudaSuccess) return e;
+    if (c.any_hub) {
+        const int jobs = L.nmats * 2 * kHubs;
+        hub_kernel<<<dim3((unsigned)(L.nmats * kHubs), 16), 256, 0, st>>>(L);
+        if (c.cluster > 0) {
+            const size_t smem = label_smem_bytes(c.n_max, c.cluster);
+            e = cudaFuncSetAttribute(label_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e == cudaSuccess && c.cluster > 8)
+                e = cudaFuncSetAttribute(label_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (e != cudaSuccess) return e;
+            cudaLaunchConfig_t cfg{};
+            cudaLaunchAttribute attr{};
+            cfg.gridDim = dim3((unsigned)(jobs * c.cluster));
+            cfg.blockDim = dim3(kLabelThreads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = (unsigned)c.cluster;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            if ((e = cudaLaunchKernelEx(&cfg, label_cluster_kernel, L)) != cudaSuccess) return e;
+        } else {
+            e = cudaMemsetAsync(L.lam, 0x7f, 4ull * 2 * kHubs * (size_t)L.total, st);
+            if (e != cudaSuccess) return e;
+            label_start_kernel<<<jobs, 32, 0, st>>>(L);
+            const dim3 grid((unsigned)std::max(8, 2 * c.sm_count / std::min(L.nmats, 8)), (unsigned)jobs);
+            for (int r = 0; r < kMaxRounds; r++)
+                label_round_kernel<<<grid, kLabelThreads, 0, st>>>(L, r, r == kMaxRounds - 1);
+        }
+        const int words = (int)((c.n_max + 31) / 32);
+        event_kernel<<<dim3((unsigned)std::min((words + 7) / 8, 1024), (unsigned)jobs), 256, 0, st>>>(L, digests);
+        size_t sb = c.scan_bytes;
+        e = cub::DeviceScan::InclusiveScan(c.scan_tmp, sb, L.base, L.base, TotSum(), (int)(2 * kBases * L.total), st);
+        if (e != cudaSuccess) return e;
+    }
+    const size_t smem = sizeof(WarpTable) * (kExtraThreads / 32);
+    if ((e = cudaFuncSetAttribute(extra_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+        return e;
+    const long long want = (L.total_items + kExtraThreads / 32 - 1) / (kExtraThreads / 32);
+    extra_kernel<<<(int)std::min<long long>(want, (long long)c.sm_count * (1024 / kExtraThreads)), kExtraThreads, smem, st>>>(L);
+    if (c.large_block == 256) large_kernel<256><<<c.large_grid, 256, c.large_smem, st>>>(L);
+    else large_kernel<1024><<<c.large_grid, 1024, c.large_smem, st>>>(L);
+    commit_kernel<<<L.nmats, 32, 0, st>>>(L);
+    return cudaGetLastError();
+}
+
+}  // namespace gsofa

@@ -48,10 +48,11 @@ struct MatDesc {
     const int32_t* wdeg;        // ceil(n/32): sum of A's row lengths per 32-vertex word
     const uint32_t* dplanes;    // nplanes * ceil(n/32): degree bit-planes of A's rows
     int32_t nplanes;            // bits of A's largest row length
-    int32_t pad0;
+    int32_t method;             // METHOD_*: which counting traversal takes it
     // 0 when A's pattern equals A^T's (set by the ingest's check): the L
     // column searches in A^T then repeat the U row searches in A, and the
-    // direction-0 census writes both halves
+    // direction-0 census writes both halves.  asym[1]: non-zero when a row
+    // may hold an id twice
     const int32_t* asym;
     int32_t* nnz_u;             // n: |U row|
     int32_t* nz_row_u;          // n: reference nz_row_U counter
@@ -74,6 +75,12 @@ struct MatDesc {
     // in the other direction reads it (see traverse_kernel: chained starts)
     uint8_t* link;
     long long item_base;        // first work item of this matrix
+    // gsofa_hub.cu: place of the matrix in its arrays (a multiple of 32), the
+    // room there (n + 1 rounded up), first work item and items (a power of two)
+    long long hub_off;
+    long long hub_len;
+    long long hub_item;
+    long long hub_slots;
     // serving only (zero elsewhere)
     long long n_items;          // work items of this request
     unsigned long long seq;     // request number (claim word tag, done flag value)
@@ -141,6 +148,100 @@ struct TraverseLaunch {
     ServeLaunch serve;          // serving kernel only
 };
 
+// The counting traversal (gsofa_chain.cu).  Per CTA: a queue of queue_stride
+// ints and gbm_count bitmaps of bitmap_words words in global memory (two that
+// are zero between uses; two more for the dense base when it does not fit in
+// shared memory).
+struct ChainLaunch {
+    const MatDesc* mats;               // device array
+    int32_t nmats;
+    long long total_items;             // chunks of all matrices
+    unsigned long long* work_counter;  // device, zeroed before launch
+    int32_t* queue;
+    long long queue_stride;
+    uint32_t* gbm;
+    int gbm_count;
+    long long bitmap_words;            // covers the largest n + padding
+    long long smem_words;              // bitmap words that fit in shared memory
+    int chunk;                         // consecutive sources per work item
+    int list_cap;                      // new ids of a search before the whole CTA takes it
+    long long sample_stride;           // > 1: only every stride-th item (autotuner timing)
+    int32_t* status;                   // device error word
+    const int32_t* fallback;           // or null: per matrix, gsofa_hub.cu left it to the chain
+    ServeLaunch serve;                 // serving kernel only
+};
+// sizes of a set relative to the current source: ids above it, ids below it,
+// the degree sum of those below, the digest of those above
+struct Tot {
+    int gt, v;
+    unsigned long long e, dig;
+};
+
+// How a matrix's counting traversal runs.
+enum : int32_t {
+    METHOD_CHAIN = 0,   // gsofa_chain.cu
+    METHOD_HUB = 1,     // gsofa_hub.cu
+    METHOD_DIRECT = 2,  // gsofa_hub.cu without a hub: every source searched alone
+};
+// A matrix of at most this many rows is METHOD_DIRECT.
+constexpr int kDirectMax = 1024;
+
+// The traversal of gsofa_hub.cu over the launch's matrices of the methods hub
+// and direct.  `total` is the sum of their hub_len.
+struct HubLaunch {
+    const MatDesc* mats;
+    int32_t nmats;
+    int group;                         // consecutive sources per work item
+    long long total;
+    long long total_items;
+    unsigned long long* work_counter;  // [0] extra_kernel, [1] large_kernel
+    // zeroed before every launch, in one block: Tot base[2 * hub_bases() * total], stamp,
+    // label counts, fallback, judged, counters, large_count
+    void* zeroed;
+    Tot* base;                         // per base, direction and source: the hub set's totals
+    int32_t* stamp;                    // as lam
+    int32_t* lcnt;                     // 4 per label job
+    int32_t* fallback;                 // per matrix: left to the chain
+    int32_t* judged;                   // per matrix: searches done, searches too large
+    unsigned long long* counters;      // per matrix, CNT_SLOTS
+    int* large_count;
+    int32_t* lam;                      // labels: hubs x 2 directions x total
+    int32_t* lq;                       // label queues: twice lam
+    unsigned long long* hubs;          // per matrix and hub (zeroed too)
+    unsigned long long* large;         // (matrix, direction, source) of large searches
+    int32_t* queue;                    // large_kernel: per CTA queue_stride ints
+    long long queue_stride;
+    uint32_t* gbm;                     // large_kernel: per CTA bitmap_words (not with large_smem)
+    long long bitmap_words;
+    int large_smem;                    // its bitmaps are in shared memory
+    int32_t* status;
+};
+struct HubCfg {
+    bool any_hub = false;
+    int cluster = 0;          // CTAs per label job, labels in shared memory (0: in global memory)
+    int32_t n_max = 0;
+    int sm_count = 0;
+    size_t zeroed_bytes = 0;
+    void* scan_tmp = nullptr;
+    size_t scan_bytes = 0;
+    int large_block = 256, large_grid = 0;
+    size_t large_smem = 0;
+};
+int hub_count();  // hubs per matrix
+int hub_bases();  // arrays of totals per direction
+size_t label_smem_bytes(int32_t n, int cluster);
+size_t hub_scan_bytes(long long count);
+int large_occupancy(int block, size_t smem);
+cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStream_t stream);
+
+// Shared memory of a CTA besides its bitmaps; the largest list_cap.
+size_t chain_sparse_bytes();
+int chain_list_cap();
+// Resident CTAs per SM with `smem` dynamic bytes (0 = cannot run).
+int chain_occupancy(int block, bool serve, size_t smem);
+cudaError_t launch_chain(const ChainLaunch& L, int block, bool serve, int grid, size_t smem,
+                         cudaStream_t stream);
+
 // Launch helpers (gsofa_kernels.cu).  All asynchronous on `stream`.
 int traverse_block_sizes(int* sizes, int max_sizes);
 // Returns the resident CTAs per SM for the given configuration (0 = cannot run).
@@ -159,7 +260,7 @@ cudaError_t launch_canonicalize(int32_t n, long long nnz_in, const int32_t* beg,
                                 const int32_t* col_in, const int32_t* rp, int32_t* col_out,
                                 int32_t* tcount, int32_t* tpad, int32_t* trp, int32_t* tcol,
                                 int32_t* tfill, int32_t* wdeg, uint32_t* dplanes, int nplanes,
-                                int32_t* asym, int check_symmetry, void* scan_tmp,
+                                int32_t* asym, int check_symmetry, int check_dup, void* scan_tmp,
                                 size_t scan_tmp_bytes, int32_t* status, cudaStream_t stream);
 size_t canonicalize_scan_bytes(int32_t n);
 // *sum (zeroed by the caller) += sum over A's entries (v, c) of |v - c|.

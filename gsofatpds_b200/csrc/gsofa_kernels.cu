@@ -36,58 +36,10 @@
 #include <cub/block/block_scan.cuh>
 #include <cub/device/device_scan.cuh>
 
-#include "gsofa_internal.h"
+#include "gsofa_device.cuh"
 #include "../../include/gsofa.h"
 
 namespace gsofa {
-
-#define FULL_MASK 0xffffffffu
-
-// Digest mixing: splitmix64 finaliser (Steele, Lea, Flood 2014).  A U-row
-// or L-column digest sums mix64((w << 32) | mask) over the set's non-zero
-// 32-id words w; an L-row digest (scattered) sums mix64(id) over its ids.
-__host__ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
-    x += 0x9E3779B97F4A7C15ull;
-    x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
-    x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
-    return x ^ (x >> 31);
-}
-
-__device__ __forceinline__ int find_matrix(const MatDesc* mats, int nmats, long long item) {
-    int lo = 0, hi = nmats - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (mats[mid].item_base <= item) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-
-__device__ __forceinline__ uint32_t ld_vol(const uint32_t* p) {
-    return *reinterpret_cast<const volatile uint32_t*>(p);
-}
-
-// Loads of matrix data.  CG = false: the read-only path (L1-cached), valid
-// because nothing writes a matrix while a launch reads it.  CG = true (the
-// serving kernel): L2 only.  A serving launch outlives the matrices it reads;
-// their memory is freed and reused for later requests while it runs, so a
-// line it once cached in L1 could be stale.
-template <bool CG>
-__device__ __forceinline__ int ld_i32(const int32_t* p) {
-    return CG ? __ldcg(p) : __ldg(p);
-}
-
-template <bool CG>
-__device__ __forceinline__ int4 ld_row4(const int32_t* p) {
-    const int4* q = reinterpret_cast<const int4*>(p);
-    return CG ? __ldcg(q) : __ldg(q);
-}
-
-// Original (unpadded) length of row v of a padded graph.
-template <bool CG>
-__device__ __forceinline__ int row_degree(const int32_t* rp, int v) {
-    const int a = ld_i32<CG>(rp + v), b = ld_i32<CG>(rp + v + 1);
-    return (b & ~3) - (a & ~3) - (b & 3);
-}
 
 // Ring slot masks: one bit per closure-ring slot (up to 64 slots).
 typedef unsigned long long rmask_t;
@@ -132,12 +84,6 @@ struct TraverseSmem {
     int chain;            // the next source starts from this source's bitmap
     int premerge;         // else: ring slot of a cached source the next one is known to reach
 };
-
-// Bitmap words of a matrix of order n: n bits plus zero padding read by the
-// 128-bit L-mask extraction past the last vertex.
-__host__ __device__ __forceinline__ long long bitmap_words_for(int32_t n) {
-    return (((long long)n + 31) >> 5) + 6;
-}
 
 struct Src {
     int32_t src, n;
@@ -614,20 +560,6 @@ __device__ __forceinline__ rmask_t merge_reached(const Src& S, rmask_t reached, 
     return mm;
 }
 
-__device__ __forceinline__ unsigned long long ld_vol64(const unsigned long long* p) {
-    return *reinterpret_cast<const volatile unsigned long long*>(p);
-}
-
-__device__ __forceinline__ int ld_vol_i32(const int32_t* p) {
-    return *reinterpret_cast<const volatile int32_t*>(p);
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 // Called by the 32 lanes of warp 0 when source nx = src + 1 cannot start
 // from src's closure: the ring slot of the largest cached source t < src that
 // nx is known to reach, or -1.  nx reaches t when the other direction's
@@ -663,121 +595,6 @@ __device__ int premerge_candidate(const Src& S, const MatDesc& M, int32_t src, i
         if (b) return (src - 1 - k0 - (__ffs(b) - 1)) & (S.ring - 1);
     }
     return -1;
-}
-
-// Serving, called by all 32 lanes of warp 0: claims a work item of any
-// published request.  Each lane checks one list entry (rotating start); the
-// claimable entry with the fewest unclaimed items is taken with
-// compare-and-swap on its claim word.  Returns false (in every
-// lane) when the host says to take no more items (ctrl[1]), when nothing is
-// claimable and the host asks idle CTAs to exit (ctrl[0]), after idle_ns of
-// finding nothing, or after max_idle_polls polls.
-__device__ bool serve_claim(const TraverseLaunch& P, int* slot_out, long long* item_out) {
-    const ServeLaunch& V = P.serve;
-    const int lane = threadIdx.x & 31;
-    unsigned ns = 32;
-    const unsigned long long t0 = global_ns();
-    for (long long polls = 0; polls < V.max_idle_polls; polls++) {
-        int c0 = 0, c1 = 0, n = 0;
-        unsigned r = 0;
-        if (lane == 0) {
-            c1 = ld_vol_i32(V.ctrl + 1);
-            c0 = ld_vol_i32(V.ctrl);
-            n = min(ld_vol_i32(V.ctrl + 2), V.nslots);
-            if (!c1 && n > 0) r = atomicAdd(V.rr, 1u);
-        }
-        c0 = __shfl_sync(FULL_MASK, c0, 0);
-        c1 = __shfl_sync(FULL_MASK, c1, 0);
-        n = __shfl_sync(FULL_MASK, n, 0);
-        r = __shfl_sync(FULL_MASK, r, 0);
-        if (c1) return false;
-        for (int base = 0; base < n; base += 32) {
-            const int k = base + lane;
-            bool ok = false;
-            int slot = -1;
-            unsigned seq = 0;
-            unsigned long long v = 0;
-            long long nit = 0;
-            if (k < n) {
-                const unsigned long long e = ld_vol64(V.list + (r + (unsigned)k) % (unsigned)n);
-                slot = (int)(e >> 32);
-                seq = (unsigned)e;
-                if (slot >= 0 && slot < V.nslots) {
-                    v = ld_vol64(V.claim + slot);
-                    if ((unsigned)(v >> 32) == seq) {
-                        __threadfence();  // the descriptor was written before the claim word
-                        nit = __ldcg(&V.slots[slot].n_items);
-                        ok = (long long)(v & 0xffffffffull) < nit;
-                    }
-                }
-            }
-            // shortest remaining work first (fewest unclaimed items), ties in
-            // rotation order: small requests overtake large ones item by item
-            unsigned rem = 0xffffffffu;
-            if (ok) rem = (unsigned)min(nit - (long long)(v & 0xffffffffull), 0xfffffffell);
-            for (int round = 0; round < 32; round++) {
-                const unsigned best = __reduce_min_sync(FULL_MASK, rem);
-                if (best == 0xffffffffu) break;
-                const int l = __ffs(__ballot_sync(FULL_MASK, rem == best)) - 1;
-                int got = 0;
-                long long it = 0;
-                if (lane == l) {
-                    for (int tries = 0; tries < 256; tries++) {
-                        if ((unsigned)(v >> 32) != seq || (long long)(v & 0xffffffffull) >= nit) break;
-                        const unsigned long long old = atomicCAS(V.claim + slot, v, v + 1ull);
-                        if (old == v) {
-                            got = 1;
-                            it = (long long)(v & 0xffffffffull);
-                            break;
-                        }
-                        v = old;
-                    }
-                    rem = 0xffffffffu;  // taken or gone: this entry is done
-                }
-                if (__shfl_sync(FULL_MASK, got, l)) {
-                    *slot_out = __shfl_sync(FULL_MASK, slot, l);
-                    *item_out = __shfl_sync(FULL_MASK, it, l);
-                    return true;
-                }
-            }
-        }
-        if (c0) return false;
-        if (global_ns() - t0 > (unsigned long long)V.idle_ns) return false;
-        __nanosleep(ns);
-        if (ns < 2048) ns <<= 1;
-    }
-    return false;
-}
-
-// Serving: takes a free per-CTA workspace slot, or returns -1.
-__device__ int take_cta_slot(const ServeLaunch& V) {
-    const int nw = (V.n_cta_slots + 31) >> 5;
-    for (int w = 0; w < nw; w++) {
-        unsigned v = ld_vol_i32(reinterpret_cast<const int32_t*>(V.cta_slots + w));
-        for (int tries = 0; tries < 64 && ~v; tries++) {
-            const int b = __ffs(~v) - 1;
-            if (w * 32 + b >= V.n_cta_slots) break;
-            const unsigned old = atomicOr(V.cta_slots + w, 1u << b);
-            if (!(old & (1u << b))) {
-                atomicAdd(V.alive, 1);
-                __threadfence();
-                return w * 32 + b;
-            }
-            v = old | (1u << b);
-        }
-    }
-    return -1;
-}
-
-// Thread 0 copies a matrix descriptor to shared memory (through L2 when it
-// may have been rewritten since the launch began).
-template <bool CG>
-__device__ __forceinline__ void copy_desc(MatDesc* dst, const MatDesc* src) {
-    static_assert(sizeof(MatDesc) % 8 == 0, "descriptor copied in 8-byte words");
-    const unsigned long long* a = reinterpret_cast<const unsigned long long*>(src);
-    unsigned long long* b = reinterpret_cast<unsigned long long*>(dst);
-#pragma unroll
-    for (int k = 0; k < (int)(sizeof(MatDesc) / 8); k++) b[k] = CG ? __ldcg(a + k) : a[k];
 }
 
 __device__ __forceinline__ void flush_counters(unsigned long long* c, unsigned long long* acc) {
@@ -840,7 +657,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) traverse_kernel(TraverseL
             if (warp == 0) {
                 int slot = 0;
                 long long it = -1;
-                const bool got = serve_claim(P, &slot, &it);
+                const bool got = serve_claim(P.serve, &slot, &it);
                 if (lane == 0) {
                     if (got) {
                         copy_desc<true>(&SD, P.serve.slots + slot);
@@ -1375,12 +1192,17 @@ cudaError_t launch_serve(const TraverseLaunch& L, int block, int grid, size_t sm
 //
 // The host computes A's padded row pointers (pad counts in the low 2 bits).
 // One warp per row copies the row into its padded slot, writes the padding
-// (the row's own id) and counts the entries per column for A^T.
+// (the row's own id) and counts the entries per column for A^T.  *dup becomes
+// non-zero when a row holds an id twice: a strictly increasing row cannot;
+// the others are compared pairwise up to kDupCheckMaxRow entries, and longer
+// unsorted rows count as holding one (a matrix so marked has its rows'
+// distinct ids counted in every search: slower, the same results).
+constexpr int kDupCheckMaxRow = 1024;
 
 __global__ void gather_rows_kernel(int32_t n, long long nnz_in, const int32_t* __restrict__ beg,
                                    const int32_t* __restrict__ rp,
                                    const int32_t* __restrict__ col_in, int32_t* __restrict__ col_out,
-                                   int32_t* __restrict__ tcount, int32_t* status) {
+                                   int32_t* __restrict__ tcount, int32_t* dup, int32_t* status) {
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -1390,6 +1212,7 @@ __global__ void gather_rows_kernel(int32_t n, long long nnz_in, const int32_t* _
         const long long o = r0 & ~3;
         const long long plen = (long long)(r1 & ~3) - o;
         const long long d = plen - (r1 & 3);
+        bool unsorted = false;
         for (long long j = lane; j < plen; j += 32) {
             if (j >= d) {
                 col_out[o + j] = (int32_t)v;
@@ -1413,7 +1236,16 @@ __global__ void gather_rows_kernel(int32_t n, long long nnz_in, const int32_t* _
             }
             col_out[o + j] = c;
             atomicAdd(&tcount[c], 1);
+            unsorted |= j > 0 && src > 0 && col_in[src - 1] >= c;
         }
+        if (!dup || !__any_sync(FULL_MASK, unsorted)) continue;
+        bool twice = d > kDupCheckMaxRow;
+        for (long long j = lane; j < d && !twice; j += 32) {
+            if (b + j < 0 || b + j >= nnz_in) break;  // reported above
+            const int32_t c = col_in[b + j];
+            for (long long i = 0; i < j && !twice; i++) twice = b + i >= 0 && col_in[b + i] == c;
+        }
+        if (twice) atomicOr(dup, 1);
     }
 }
 
@@ -1553,9 +1385,10 @@ cudaError_t launch_canonicalize(int32_t n, long long nnz_in, const int32_t* beg,
                                 const int32_t* col_in, const int32_t* rp, int32_t* col_out,
                                 int32_t* tcount, int32_t* tpad, int32_t* trp, int32_t* tcol,
                                 int32_t* tfill, int32_t* wdeg, uint32_t* dplanes, int nplanes,
-                                int32_t* asym, int check_symmetry, void* scan_tmp,
+                                int32_t* asym, int check_symmetry, int check_dup, void* scan_tmp,
                                 size_t scan_tmp_bytes, int32_t* status, cudaStream_t st) {
     cudaError_t e0 = cudaMemsetAsync(asym, check_symmetry ? 0 : 1, 4, st);
+    if (e0 == cudaSuccess) e0 = cudaMemsetAsync(asym + 1, check_dup ? 0 : 1, 4, st);
     if (e0 != cudaSuccess) return e0;
     if (n <= 0) return cudaSuccess;
     const int threads = 256;
@@ -1563,7 +1396,8 @@ cudaError_t launch_canonicalize(int32_t n, long long nnz_in, const int32_t* beg,
     int grid = (int)(grid_w > 148 * 64 ? 148 * 64 : grid_w);
     long long grid_t = ((long long)n + threads) / threads;
     int gridt = (int)(grid_t > 148 * 16 ? 148 * 16 : grid_t);
-    gather_rows_kernel<<<grid, threads, 0, st>>>(n, nnz_in, beg, rp, col_in, col_out, tcount, status);
+    gather_rows_kernel<<<grid, threads, 0, st>>>(n, nnz_in, beg, rp, col_in, col_out, tcount,
+                                                 check_dup ? asym + 1 : nullptr, status);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     pad_counts_kernel<<<gridt, threads, 0, st>>>(n, tcount, tpad);

@@ -929,13 +929,13 @@ extern "C" int gsofa_matrix_permute(gsofa_ctx* ctx, const gsofa_matrix* mat, con
         }
         encode_rows_kernel<<<grid_for((long long)n + 1, kThreads), kThreads, 0, st>>>(n, incl, pads,
                                                                                       m->rowptr);
-        rc = matrix_build(ctx, st, dstatus, m, padded, dbeg, cols, 0);
+        rc = matrix_build(ctx, st, dstatus, m, padded, dbeg, cols, 0, 0);
         if (rc) {
             matrix_free_on(m, st);
             return rc;
         }
-        // P A P^T is symmetric exactly when A is
-        e = cudaMemcpyAsync(m->asym, mat->asym, 4, cudaMemcpyDeviceToDevice, st);
+        // P A P^T is symmetric, and its rows hold ids twice, exactly when A's do
+        e = cudaMemcpyAsync(m->asym, mat->asym, 8, cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_status, dstatus, 4, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e == cudaSuccess) e = cudaGetLastError();
