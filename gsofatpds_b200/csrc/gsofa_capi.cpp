@@ -92,6 +92,21 @@ int ensure(gsofa_ctx* ctx, void** p, size_t* have, size_t need) {
     return GSOFA_OK;
 }
 
+// Pinned words for the totals and flags of `count` matrices.
+int ensure_pinned(gsofa_ctx* ctx, size_t count) {
+    if (ctx->h_counters_cap >= count) return GSOFA_OK;
+    if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
+    if (ctx->h_fallback) cudaFreeHost(ctx->h_fallback);
+    ctx->h_counters = nullptr;
+    ctx->h_fallback = nullptr;
+    ctx->h_counters_cap = 0;
+    cudaError_t e = cudaMallocHost((void**)&ctx->h_counters, 8 * CNT_SLOTS * count);
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&ctx->h_fallback, 4 * count);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "pinned totals");
+    ctx->h_counters_cap = count;
+    return GSOFA_OK;
+}
+
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 long long bitmap_words(int32_t n) { return (((long long)n + 31) >> 5) + 6; }
@@ -211,16 +226,17 @@ static size_t result_layout(int32_t n, uint32_t flags, size_t off[12]) {
     size_t sz[12];
     sz[0] = 4 * N;                       // nnz_u
     sz[1] = 4 * N;                       // nz_row_u
-    sz[2] = dig ? 8 * N : 0;             // dig_u
-    sz[3] = 4 * N;                       // nnz_lc
+    sz[2] = 4 * N;                       // nnz_lc
+    sz[3] = dig ? 8 * N : 0;             // dig_u
     sz[4] = dig ? 8 * N : 0;             // dig_lc
     sz[5] = 16 * N;                      // lmask
-    sz[6] = lrow ? 4 * N : 0;            // nnz_lr
-    sz[7] = lrow ? 8 * N : 0;            // dig_lr
-    sz[8] = N;                           // supernode flags
-    sz[9] = 8 * CNT_SLOTS;               // counters
-    sz[10] = 2 * N;                      // link (chained starts)
-    sz[11] = 16 * N;                     // umask (chained starts)
+    sz[6] = 16 * N;                      // umask (chained starts)
+    // zeroed from here on
+    sz[7] = lrow ? 4 * N : 0;            // nnz_lr
+    sz[8] = lrow ? 8 * N : 0;            // dig_lr
+    sz[9] = N;                           // supernode flags
+    sz[10] = 8 * CNT_SLOTS;              // counters
+    sz[11] = 2 * N;                      // link (chained starts)
     size_t total = 0;
     for (int i = 0; i < 12; i++) {
         off[i] = total;
@@ -243,7 +259,6 @@ int result_alloc_on(gsofa_ctx* ctx, int32_t n, uint32_t flags, int32_t mss, cuda
     r->n = n;
     r->flags = flags;
     r->mss = mss;
-    const size_t N = (size_t)std::max(n, 1);
     const bool dig = flags & GSOFA_DIGESTS;
     const bool lrow = flags & GSOFA_L_ROW_STATS;
     size_t off[12];
@@ -257,25 +272,18 @@ int result_alloc_on(gsofa_ctx* ctx, int32_t n, uint32_t flags, int32_t mss, cuda
     char* b = reinterpret_cast<char*>(r->arena);
     r->nnz_u = reinterpret_cast<int32_t*>(b + off[0]);
     r->nz_row_u = reinterpret_cast<int32_t*>(b + off[1]);
-    r->dig_u = dig ? reinterpret_cast<uint64_t*>(b + off[2]) : nullptr;
-    r->nnz_lc = reinterpret_cast<int32_t*>(b + off[3]);
+    r->nnz_lc = reinterpret_cast<int32_t*>(b + off[2]);
+    r->dig_u = dig ? reinterpret_cast<uint64_t*>(b + off[3]) : nullptr;
     r->dig_lc = dig ? reinterpret_cast<uint64_t*>(b + off[4]) : nullptr;
     r->lmask = reinterpret_cast<uint32_t*>(b + off[5]);
-    r->nnz_lr = lrow ? reinterpret_cast<int32_t*>(b + off[6]) : nullptr;
-    r->dig_lr = lrow ? reinterpret_cast<uint64_t*>(b + off[7]) : nullptr;
-    r->sflags = reinterpret_cast<int8_t*>(b + off[8]);
-    r->counters = reinterpret_cast<unsigned long long*>(b + off[9]);
-    r->link = reinterpret_cast<uint8_t*>(b + off[10]);
-    r->umask = reinterpret_cast<uint32_t*>(b + off[11]);
-    // zero the scatter targets, the counters and the flags
-    cudaError_t e = cudaSuccess;
-    if (lrow) {
-        e = cudaMemsetAsync(r->nnz_lr, 0, 4 * N, stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(r->dig_lr, 0, 8 * N, stream);
-    }
-    if (e == cudaSuccess) e = cudaMemsetAsync(r->counters, 0, 8 * CNT_SLOTS, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(r->sflags, 0, N, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(r->link, 0, 2 * N, stream);
+    r->umask = reinterpret_cast<uint32_t*>(b + off[6]);
+    r->nnz_lr = lrow ? reinterpret_cast<int32_t*>(b + off[7]) : nullptr;
+    r->dig_lr = lrow ? reinterpret_cast<uint64_t*>(b + off[8]) : nullptr;
+    r->sflags = reinterpret_cast<int8_t*>(b + off[9]);
+    r->counters = reinterpret_cast<unsigned long long*>(b + off[10]);
+    r->link = reinterpret_cast<uint8_t*>(b + off[11]);
+    // zero the scatter targets, the flags, the counters and the links
+    cudaError_t e = cudaMemsetAsync(b + off[7], 0, total - off[7], stream);
     if (e != cudaSuccess) {
         dev_free_on(ctx, r->arena, r->bytes, stream);
         delete r;
@@ -332,7 +340,8 @@ int plan_chain(gsofa_ctx* ctx, int32_t nmax, bool all_sym, const gsofa_opts* o, 
                ChainCfg* c) {
     c->words = bitmap_words(nmax);
     const long long need = (all_sym ? 1 : 2) * c->words;  // X of each direction
-    const size_t fixed = (chain_sparse_bytes() + 15) & ~(size_t)15;
+    c->sides = all_sym ? 1 : 2;
+    const size_t fixed = (chain_sparse_bytes(c->sides) + 15) & ~(size_t)15;
     size_t bytes = ((size_t)need * 4 + 15) & ~(size_t)15;
     if (fixed + bytes + 4096 > (size_t)ctx->smem_optin || (o->flags & GSOFA_FORCE_GLOBAL_BITMAP))
         bytes = 0;
@@ -342,7 +351,7 @@ int plan_chain(gsofa_ctx* ctx, int32_t nmax, bool all_sym, const gsofa_opts* o, 
     c->block = o->threads_per_source;
     if (c->block <= 0) {
         const long long fit = ctx->smem_per_sm / (long long)(c->smem + 2048);
-        c->block = fit >= 8 ? 128 : fit >= 4 ? 256 : fit >= 2 ? 512 : 1024;
+        c->block = fit >= 4 ? 256 : fit >= 2 ? 512 : 1024;
     }
     if (c->block != 128 && c->block != 256 && c->block != 512 && c->block != 1024)
         return set_err(ctx, GSOFA_ERR_ARG, "threads_per_source must be 128, 256, 512 or 1024");
@@ -363,6 +372,7 @@ void fill_chain_launch(ChainLaunch* L, const ChainCfg& c, const gsofa_opts& o, i
     L->gbm_count = c.gbm_count;
     L->bitmap_words = c.words;
     L->smem_words = c.smem_words;
+    L->sides = c.sides;
 }
 
 int32_t method_of(const gsofa_matrix* m) {
@@ -458,9 +468,16 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     return true;
 }
 
-long long chain_chunk(const gsofa_opts& o, long long total_sources, int grid) {
+long long chain_chunk(const gsofa_opts& o, long long total_sources, int grid, bool sym) {
     if (o.chunk_sources > 0) return o.chunk_sources;
-    return std::max(1ll, (total_sources + grid - 1) / grid);
+    // A chunk's first source is searched from nothing.  Symmetric patterns:
+    // about two items per CTA, at most 128 sources each, since their items
+    // differ in cost (64^3 mesh: 3.3 ms with 128 sources, 4.0 with 443; 40^3:
+    // 0.92 with 54, 1.09 with 108).  The others come here without a core that a
+    // hub lies in, and such first searches may read most of the matrix: one
+    // item per CTA.
+    if (!sym) return std::max(1ll, (total_sources + grid - 1) / grid);
+    return std::max(1ll, std::min(128ll, (total_sources + 2ll * grid - 1) / (2ll * grid)));
 }
 
 // Runs the traversal (and optionally supernodes / pattern) for `count`
@@ -516,7 +533,7 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
         }
         rc = plan_chain(ctx, std::max(nmax, 1), chain_sym, o, false, &ccfg);
         if (rc) return rc;
-        CL.chunk = (int)chain_chunk(*o, chain_sources, ccfg.grid);
+        CL.chunk = (int)chain_chunk(*o, chain_sources, ccfg.grid, chain_sym);
         long long items = 0;
         place(CL.chunk, 1);
         for (int32_t k = 0; k < count; k++) {
@@ -596,70 +613,89 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
         CL.queue = L.queue;
         CL.gbm = L.gbitmap;
     }
-    void* ddesc = nullptr;
-    rc = dev_alloc(ctx, sizeof(MatDesc) * (size_t)count, &ddesc);
+    rc = ensure(ctx, &ctx->desc, &ctx->desc_bytes, sizeof(MatDesc) * (size_t)count);
+    if (!rc) rc = ensure_pinned(ctx, (size_t)count);
     if (rc) return rc;
+    void* const ddesc = ctx->desc;
     CK(cudaMemcpyAsync(ddesc, descs.data(), sizeof(MatDesc) * (size_t)count, cudaMemcpyHostToDevice,
                        ctx->stream));
     CK(cudaMemsetAsync(ctx->small, 0, 128, ctx->stream));
     L.mats = CL.mats = HL.mats = reinterpret_cast<const MatDesc*>(ddesc);
 
-    CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    if (chain) {
-        if (hub) {
-            CK(launch_hub(HL, hcfg, (o->flags & GSOFA_DIGESTS) != 0, ctx->stream));
-            // left to the chain: known before the supernodes are looked for
-            ctx->h_fallback.assign((size_t)count, 0);
-            CK(cudaMemcpyAsync(ctx->h_fallback.data(), HL.fallback, 4 * (size_t)count,
-                               cudaMemcpyDeviceToHost, ctx->stream));
-            CK(cudaStreamSynchronize(ctx->stream));
-            bool any = false;
-            for (int32_t k = 0; k < count; k++) any = any || ctx->h_fallback[(size_t)k];
-            if (any) {
-                long long items = 0;
-                bool sym = true;
-                for (int32_t k = 0; k < count; k++) {
-                    MatDesc& d = descs[(size_t)k];
-                    if (ctx->h_fallback[(size_t)k]) d.method = METHOD_CHAIN;
-                    d.item_base = items;
-                    if (d.method != METHOD_CHAIN) continue;
-                    items += (d.n + CL.chunk - 1) / CL.chunk;
-                    sym = sym && mats[order[(size_t)k]]->host_sym > 0;
-                }
-                rc = plan_chain(ctx, std::max(nmax, 1), sym, o, false, &ccfg);
-                if (rc) return rc;
-                ccfg.grid = (int)std::max(1ll, std::min<long long>(ccfg.grid, items));
-                rc = ensure(ctx, &ctx->queue, &ctx->queue_bytes,
-                            (size_t)ccfg.grid * (size_t)std::max(nmax, 1) * 4);
-                if (!rc)
-                    rc = ensure(ctx, &ctx->gbitmap, &ctx->gbitmap_bytes,
-                                (size_t)ccfg.grid * (size_t)ccfg.gbm_count * (size_t)ccfg.words * 4);
-                if (rc) return rc;
-                fill_chain_launch(&CL, ccfg, *o, nmax);
-                CL.queue = L.queue = reinterpret_cast<int32_t*>(ctx->queue);
-                CL.gbm = L.gbitmap = reinterpret_cast<uint32_t*>(ctx->gbitmap);
-                CL.total_items = (items + stride - 1) / stride;
-                CK(cudaMemcpyAsync(ddesc, descs.data(), sizeof(MatDesc) * (size_t)count,
-                                   cudaMemcpyHostToDevice, ctx->stream));
-            }
+    // the supernodes and the read-back of the matrices of `mine` (all: null)
+    auto finish = [&](const std::vector<char>* mine) -> int {
+        for (int32_t k = 0; k < count; k++) {
+            const int32_t i = order[(size_t)k];
+            if (mine && !(*mine)[(size_t)k]) continue;
+            if ((o->flags & GSOFA_SUPERNODES) && mats[i]->n > 0)
+                CK(launch_supernodes(mats[i]->n, o->max_supernode_size, res[i]->nz_row_u, res[i]->lmask,
+                                     res[i]->sflags, res[i]->counters, ctx->stream));
         }
-        if (CL.total_items > 0) CK(launch_chain(CL, ccfg.block, false, ccfg.grid, ccfg.smem, ctx->stream));
-    } else if (L.total_items > 0) {
+        CK(cudaEventRecord(ctx->ev1, ctx->stream));
+        for (int32_t k = 0; k < count; k++) {
+            const int32_t i = order[(size_t)k];
+            if (mine && !(*mine)[(size_t)k]) continue;
+            CK(cudaMemcpyAsync(ctx->h_counters + (size_t)i * CNT_SLOTS, res[i]->counters, 8 * CNT_SLOTS,
+                               cudaMemcpyDeviceToHost, ctx->stream));
+        }
+        CK(cudaMemcpyAsync(ctx->h_status, dstatus, 4, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        return check_status(ctx);
+    };
+    CK(cudaEventRecord(ctx->ev0, ctx->stream));
+    if (hub) {
+        CK(launch_hub(HL, hcfg, (o->flags & GSOFA_DIGESTS) != 0, ctx->stream));
+        CK(cudaMemcpyAsync(ctx->h_fallback, HL.fallback, 4 * (size_t)count, cudaMemcpyDeviceToHost,
+                           ctx->stream));
+    }
+    if (chain && CL.total_items > 0)
+        CK(launch_chain(CL, ccfg.block, false, ccfg.grid, ccfg.smem, ctx->stream));
+    if (!chain && L.total_items > 0)
         CK(launch_traverse(L, cfg.block, cfg.grid, cfg.smem_bitmap, cfg.smem, ctx->stream));
-    }
     CK(cudaEventRecord(ctx->evt, ctx->stream));
-    for (int32_t i = 0; i < count; i++) {
-        if ((o->flags & GSOFA_SUPERNODES) && mats[i]->n > 0)
-            CK(launch_supernodes(mats[i]->n, o->max_supernode_size, res[i]->nz_row_u, res[i]->lmask,
-                                 res[i]->sflags, res[i]->counters, ctx->stream));
-    }
-    CK(cudaEventRecord(ctx->ev1, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->h_status, dstatus, 4, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    rc = check_status(ctx);
-    if (rc) {
-        dev_free(ctx, ddesc, sizeof(MatDesc) * (size_t)count);
-        return rc;
+    rc = finish(nullptr);
+    if (rc) return rc;
+    // matrices the hubs' launch left to the chain (few: no core, repeated entries)
+    std::vector<char> left((size_t)count, 0);
+    bool any = false;
+    for (int32_t k = 0; k < count && hub; k++) any |= (left[(size_t)k] = ctx->h_fallback[k] != 0);
+    if (any) {
+        long long items = 0, sources = 0;
+        bool sym = true;
+        for (int32_t k = 0; k < count; k++) {
+            if (!left[(size_t)k]) continue;
+            sources += descs[(size_t)k].n;
+            sym = sym && mats[order[(size_t)k]]->host_sym > 0;
+        }
+        rc = plan_chain(ctx, std::max(nmax, 1), sym, o, false, &ccfg);
+        if (rc) return rc;
+        CL.chunk = (int)chain_chunk(*o, sources, ccfg.grid, sym);
+        for (int32_t k = 0; k < count; k++) {
+            MatDesc& d = descs[(size_t)k];
+            // the others have no items now
+            d.method = left[(size_t)k] ? METHOD_CHAIN : d.method;
+            d.item_base = items;
+            if (!left[(size_t)k]) continue;
+            items += (d.n + CL.chunk - 1) / CL.chunk;
+            CK(cudaMemsetAsync(res[order[(size_t)k]]->counters, 0, 8 * CNT_SLOTS, ctx->stream));
+        }
+        ccfg.grid = (int)std::max(1ll, std::min<long long>(ccfg.grid, items));
+        rc = ensure(ctx, &ctx->queue, &ctx->queue_bytes, (size_t)ccfg.grid * (size_t)std::max(nmax, 1) * 4);
+        if (!rc)
+            rc = ensure(ctx, &ctx->gbitmap, &ctx->gbitmap_bytes,
+                        (size_t)ccfg.grid * (size_t)ccfg.gbm_count * (size_t)ccfg.words * 4);
+        if (rc) return rc;
+        fill_chain_launch(&CL, ccfg, *o, nmax);
+        CL.queue = L.queue = reinterpret_cast<int32_t*>(ctx->queue);
+        CL.gbm = L.gbitmap = reinterpret_cast<uint32_t*>(ctx->gbitmap);
+        CL.total_items = (items + stride - 1) / stride;
+        CK(cudaMemsetAsync(ctx->small, 0, 128, ctx->stream));
+        CK(cudaMemcpyAsync(ddesc, descs.data(), sizeof(MatDesc) * (size_t)count, cudaMemcpyHostToDevice,
+                           ctx->stream));
+        CK(launch_chain(CL, ccfg.block, false, ccfg.grid, ccfg.smem, ctx->stream));
+        CK(cudaEventRecord(ctx->evt, ctx->stream));
+        rc = finish(&left);
+        if (rc) return rc;
     }
     float ms = 0.f, ms_trav = 0.f;
     CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
@@ -670,11 +706,9 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
         for (int32_t k = 0; k < count; k++) {
             const int32_t i = order[(size_t)k];
             gsofa_result* r = res[i];
-            CK(cudaMemcpyAsync(ctx->h_counters, r->counters, 8 * CNT_SLOTS, cudaMemcpyDeviceToHost,
-                               ctx->stream));
-            CK(cudaStreamSynchronize(ctx->stream));
+            const unsigned long long* c = ctx->h_counters + (size_t)i * CNT_SLOTS;
             const size_t N = (size_t)r->n + 1;
-            const size_t nu = ctx->h_counters[CNT_NNZ_U], nl = ctx->h_counters[CNT_NNZ_L];
+            const size_t nu = c[CNT_NNZ_U], nl = c[CNT_NNZ_L];
             size_t total = align256(8 * N) * 2 + align256(4 * std::max<size_t>(nu, 1)) +
                            align256(4 * std::max<size_t>(nl, 1));
             rc = dev_alloc(ctx, total, &r->parena);
@@ -702,19 +736,12 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
         CK(cudaMemcpyAsync(ctx->h_status, dstatus, 4, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         rc = check_status(ctx);
-        if (rc) {
-            dev_free(ctx, ddesc, sizeof(MatDesc) * (size_t)count);
-            return rc;
-        }
+        if (rc) return rc;
     }
-    dev_free(ctx, ddesc, sizeof(MatDesc) * (size_t)count);
 
     for (int32_t i = 0; i < count; i++) {
         gsofa_result* r = res[i];
-        CK(cudaMemcpyAsync(ctx->h_counters, r->counters, 8 * CNT_SLOTS, cudaMemcpyDeviceToHost,
-                           ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        const unsigned long long* c = ctx->h_counters;
+        const unsigned long long* c = ctx->h_counters + (size_t)i * CNT_SLOTS;
         gsofa_counts& k = r->counts;
         k.n = r->n;
         k.fill_count = c[CNT_FILLS];
@@ -1062,6 +1089,10 @@ int gsofa_create(int device, size_t budget_bytes, gsofa_ctx** out) {
         if (ctx->ev1) cudaEventDestroy(ctx->ev1);
         if (ctx->evt) cudaEventDestroy(ctx->evt);
         if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
+        if (ctx->h_fallback) cudaFreeHost(ctx->h_fallback);
+        if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+        for (cudaEvent_t ev : ctx->stage_ev)
+            if (ev) cudaEventDestroy(ev);
         if (ctx->h_status) cudaFreeHost(ctx->h_status);
         if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
         delete ctx;
@@ -1081,7 +1112,10 @@ int gsofa_create(int device, size_t budget_bytes, gsofa_ctx** out) {
     if ((e = cudaEventCreate(&ctx->ev0)) != cudaSuccess) return fail(e);
     if ((e = cudaEventCreate(&ctx->ev1)) != cudaSuccess) return fail(e);
     if ((e = cudaEventCreate(&ctx->evt)) != cudaSuccess) return fail(e);
-    if ((e = cudaMallocHost((void**)&ctx->h_counters, 8 * CNT_SLOTS)) != cudaSuccess) return fail(e);
+    if (ensure_pinned(ctx, 1) != GSOFA_OK) return fail(cudaErrorMemoryAllocation);
+    if ((e = cudaMallocHost((void**)&ctx->h_stage, kStageBytes)) != cudaSuccess) return fail(e);
+    for (cudaEvent_t& ev : ctx->stage_ev)
+        if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return fail(e);
     if ((e = cudaMallocHost((void**)&ctx->h_status, 64)) != cudaSuccess) return fail(e);
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
@@ -1105,6 +1139,7 @@ int gsofa_destroy(gsofa_ctx* ctx) {
         dev_free(ctx, ctx->gprev, ctx->gprev_bytes);
         dev_free(ctx, ctx->scan_tmp, ctx->scan_tmp_bytes);
         dev_free(ctx, ctx->hub_ws, ctx->hub_ws_bytes);
+        dev_free(ctx, ctx->desc, ctx->desc_bytes);
         dev_free(ctx, ctx->small, 256);
         cudaStreamSynchronize(ctx->stream);
         cudaStreamSynchronize(ctx->own_stream);
@@ -1113,6 +1148,9 @@ int gsofa_destroy(gsofa_ctx* ctx) {
         cudaEventDestroy(ctx->ev1);
         cudaEventDestroy(ctx->evt);
         cudaFreeHost(ctx->h_counters);
+        cudaFreeHost(ctx->h_fallback);
+        cudaFreeHost(ctx->h_stage);
+        for (cudaEvent_t ev : ctx->stage_ev) cudaEventDestroy(ev);
         cudaFreeHost(ctx->h_status);
         cudaMemPoolDestroy(ctx->pool);
     }
@@ -1482,7 +1520,7 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     if (chain_sources == 0) chain_sources = total_sources;
     rc = chain ? plan_chain(ctx, nmax, all_sym, &o, false, &ccfg) : plan_launch(ctx, nmax, &o, &cfg);
     if (rc) return fail(rc);
-    const long long chunk = chain ? chain_chunk(o, chain_sources, ccfg.grid)
+    const long long chunk = chain ? chain_chunk(o, chain_sources, ccfg.grid, all_sym)
                             : o.chunk_sources > 0 ? o.chunk_sources
                                                   : default_chunk(weight, cfg.grid);
     const long long per_chunk = chain ? 1 : 2;  // work items
@@ -1676,34 +1714,86 @@ int gsofa_result_counts(const gsofa_result* r, gsofa_counts* out) {
     return GSOFA_OK;
 }
 
+// Arrays from the device to the caller's memory, through pinned staging: the
+// copies of small ones share one wait (of three 80 KB arrays: 36 -> 16 us), and
+// a large one's piece is moved on while the next arrives.
+struct Fetch {
+    void* dst;
+    const void* src;
+    size_t bytes;
+};
+
+static int fetch_all(const gsofa_result* r, const Fetch* f, int count) {
+    gsofa_ctx* ctx = r->ctx;
+    size_t total = 0;
+    for (int k = 0; k < count; k++) {
+        if (!f[k].dst) continue;
+        if (!f[k].src) return set_err(ctx, GSOFA_ERR_ARG, "requested array was not computed (option off)");
+        total += f[k].bytes;
+    }
+    std::lock_guard<std::recursive_mutex> g(ctx->mu);
+    cudaError_t e = cudaSuccess;
+    if (total <= kStageBytes) {
+        size_t at = 0;
+        for (int k = 0; k < count && e == cudaSuccess; k++) {
+            if (!f[k].dst || !f[k].bytes) continue;
+            e = cudaMemcpyAsync(ctx->h_stage + at, f[k].src, f[k].bytes, cudaMemcpyDeviceToHost, ctx->stream);
+            at += f[k].bytes;
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        at = 0;
+        for (int k = 0; k < count && e == cudaSuccess; k++) {
+            if (!f[k].dst || !f[k].bytes) continue;
+            memcpy(f[k].dst, ctx->h_stage + at, f[k].bytes);
+            at += f[k].bytes;
+        }
+    } else {
+        constexpr size_t kHalf = kStageBytes / 2;
+        struct { void* dst; size_t bytes; } held[2] = {{nullptr, 0}, {nullptr, 0}};
+        int h = 0;
+        auto deliver = [&](int x) {
+            if (!held[x].bytes) return;
+            e = cudaEventSynchronize(ctx->stage_ev[x]);
+            if (e == cudaSuccess) memcpy(held[x].dst, ctx->h_stage + x * kHalf, held[x].bytes);
+            held[x].bytes = 0;
+        };
+        for (int k = 0; k < count; k++) {
+            if (!f[k].dst) continue;
+            for (size_t at = 0; at < f[k].bytes && e == cudaSuccess; at += kHalf, h ^= 1) {
+                deliver(h);
+                if (e != cudaSuccess) break;
+                const size_t b = std::min(kHalf, f[k].bytes - at);
+                e = cudaMemcpyAsync(ctx->h_stage + h * kHalf, static_cast<const char*>(f[k].src) + at, b,
+                                    cudaMemcpyDeviceToHost, ctx->stream);
+                if (e == cudaSuccess) e = cudaEventRecord(ctx->stage_ev[h], ctx->stream);
+                held[h].dst = static_cast<char*>(f[k].dst) + at;
+                held[h].bytes = b;
+            }
+        }
+        for (int x = 0; x < 2 && e == cudaSuccess; x++, h ^= 1) deliver(h);
+    }
+    return e == cudaSuccess ? GSOFA_OK : cuda_fail(ctx, e, "result fetch");
+}
+
 static int fetch(const gsofa_result* r, void* dst, const void* src, size_t bytes) {
-    if (!dst) return GSOFA_OK;
-    if (!src) return set_err(r->ctx, GSOFA_ERR_ARG, "requested array was not computed (option off)");
-    std::lock_guard<std::recursive_mutex> g(r->ctx->mu);
-    cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, r->ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(r->ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(r->ctx, e, "result fetch");
-    return GSOFA_OK;
+    const Fetch f{dst, src, bytes};
+    return fetch_all(r, &f, 1);
 }
 
 int gsofa_result_row_counts(const gsofa_result* r, int32_t* nnz_u_row, int32_t* nz_row_u,
                             int32_t* nnz_l_col, int32_t* nnz_l_row) {
     if (!r) return GSOFA_ERR_ARG;
     const size_t b = 4 * (size_t)r->n;
-    int rc;
-    if ((rc = fetch(r, nnz_u_row, r->nnz_u, b))) return rc;
-    if ((rc = fetch(r, nz_row_u, r->nz_row_u, b))) return rc;
-    if ((rc = fetch(r, nnz_l_col, r->nnz_lc, b))) return rc;
-    return fetch(r, nnz_l_row, r->nnz_lr, b);
+    const Fetch f[4] = {{nnz_u_row, r->nnz_u, b}, {nz_row_u, r->nz_row_u, b},
+                        {nnz_l_col, r->nnz_lc, b}, {nnz_l_row, r->nnz_lr, b}};
+    return fetch_all(r, f, 4);
 }
 
 int gsofa_result_digests(const gsofa_result* r, uint64_t* du, uint64_t* dlc, uint64_t* dlr) {
     if (!r) return GSOFA_ERR_ARG;
     const size_t b = 8 * (size_t)r->n;
-    int rc;
-    if ((rc = fetch(r, du, r->dig_u, b))) return rc;
-    if ((rc = fetch(r, dlc, r->dig_lc, b))) return rc;
-    return fetch(r, dlr, r->dig_lr, b);
+    const Fetch f[3] = {{du, r->dig_u, b}, {dlc, r->dig_lc, b}, {dlr, r->dig_lr, b}};
+    return fetch_all(r, f, 3);
 }
 
 int gsofa_result_lmask(const gsofa_result* r, uint32_t* mask4n) {
@@ -1716,10 +1806,10 @@ int gsofa_result_supernodes(const gsofa_result* r, int8_t* flags, int32_t* bound
     if (!r) return GSOFA_ERR_ARG;
     if (!(r->flags & GSOFA_SUPERNODES))
         return set_err(r->ctx, GSOFA_ERR_ARG, "supernode detection was not requested");
-    std::vector<int8_t> f((size_t)r->n);
-    int rc = fetch(r, f.data(), r->sflags, (size_t)r->n);
+    std::vector<int8_t> own(flags ? 0 : (size_t)r->n);
+    int8_t* const f = flags ? flags : own.data();
+    int rc = fetch(r, f, r->sflags, (size_t)r->n);
     if (rc) return rc;
-    if (flags) memcpy(flags, f.data(), (size_t)r->n);
     int64_t k = 0;
     for (int32_t v = 0; v < r->n; v++) {
         if (f[v]) {

@@ -57,12 +57,15 @@ struct Sparse {
     uint32_t key[2][kSlots];
     uint32_t msk[2][kSlots];
     int32_t list[kListRoom];
+    uint32_t was[kListRoom];  // the id's word before it joined
 };
 
 // per-direction counters of an item
 struct Acc {
     unsigned long long fills, e, v, trav, nnz, chained;
 };
+
+constexpr int kIdleT = 16;  // sources that do not meet T before it is dropped
 
 enum : int { PUB_X = 1, PUB_T = 2, PUB_LARGE = 4, PUB_DROP = 8 };
 
@@ -141,6 +144,14 @@ __device__ void block_census(ChainSmem<BLOCK>& SM, const MatDesc& M, const uint3
     __syncthreads();
 }
 
+// The change of word w's digest when its bit s stops being above the source:
+// lane 1 digests the word with the bit, the others without.
+__device__ __forceinline__ unsigned long long pass_digest(int w, uint32_t x, int s) {
+    const bool with = (threadIdx.x & 31) == 1;
+    const unsigned long long h = word_digest(w, x & (with ? ~0u << (s & 31) : above(w, s)));
+    return __shfl_sync(FULL_MASK, h, 0) - __shfl_sync(FULL_MASK, h, 1);
+}
+
 // ---- one warp's walk through a chunk ----------------------------------------------------
 
 // What a warp needs of its direction.
@@ -186,6 +197,7 @@ __device__ void warp_walk(ChainSmem<BLOCK>& SM, const MatDesc& M, const Side& D,
     int pend_fill = 0, pend_trav = 0, pend_chained = 0;
     bool large = false;
     int mode = 0, found = 0, hits = 0;
+    int idle = 0;  // sources since one met T
     for (;; s++) {
         pair_sync();
         const int f0 = SM.pub[s & 1][0], f1 = sym ? f0 : SM.pub[s & 1][1];
@@ -204,9 +216,11 @@ __device__ void warp_walk(ChainSmem<BLOCK>& SM, const MatDesc& M, const Side& D,
         pend.gt = pend.v = 0;
         pend.e = 0ull;
         if (s >= s_end) break;
+        if (idle >= kIdleT) have_t = false;
         // xs: the base reaches s (direction 0) / s reaches the base (1); ts: the same for T
         const bool xs0 = have && (f0 & PUB_X), xs1 = have && (f1 & PUB_X);
         const bool ts0 = have_t && (f0 & PUB_T), ts1 = have_t && (f1 & PUB_T);
+        idle = ts0 || ts1 ? 0 : idle + 1;
         const bool on_x = d ? xs0 : xs1, keep_x = d ? xs1 : xs0;
         const bool on_t = d ? ts0 : ts1, keep_t = d ? ts1 : ts0;
         hits = (xs0 ? 1 : 0) | (xs1 ? 2 : 0);
@@ -219,9 +233,8 @@ __device__ void warp_walk(ChainSmem<BLOCK>& SM, const MatDesc& M, const Side& D,
             const int w = s >> 5, wp = (s - 1) >> 5;
             if (have) {
                 if (keep_x) {
-                    const uint32_t x = ld_vol(D.X + w);
                     bx.gt--;
-                    if (digests) bx.dig += word_digest(w, x & above(w, s)) - word_digest(w, x & (~0u << (s & 31)));
+                    if (digests) bx.dig += pass_digest(w, ld_vol(D.X + w), s);
                 }
                 if (s > 0 && in_x(s - 1)) {
                     bx.v++;
@@ -230,9 +243,8 @@ __device__ void warp_walk(ChainSmem<BLOCK>& SM, const MatDesc& M, const Side& D,
             }
             if (have_t) {
                 if (keep_t) {
-                    const uint32_t x = sparse_word(P.key[tsel], P.msk[tsel], w);
                     bt.gt--;
-                    if (digests) bt.dig += word_digest(w, x & above(w, s)) - word_digest(w, x & (~0u << (s & 31)));
+                    if (digests) bt.dig += pass_digest(w, sparse_word(P.key[tsel], P.msk[tsel], w), s);
                 }
                 if (s > 0 && (sparse_word(P.key[tsel], P.msk[tsel], wp) >> ((s - 1) & 31)) & 1u) {
                     bt.v++;
@@ -254,23 +266,26 @@ __device__ void warp_walk(ChainSmem<BLOCK>& SM, const MatDesc& M, const Side& D,
         }
         large = false;
         found = 0;
-        int gt = 0, v = 0, raw = 0, trav = 0;  // this lane's
+        int v = 0, raw = 0, trav = 0;  // this lane's
         unsigned e = 0;
-        unsigned long long dig = 0;
         // marks the four entries and lists the new ids; false: too many for a warp
-        auto visit = [&](const int4& q4, bool own_row) -> bool {
+        auto visit = [&](const int4& q4) -> bool {
             const int ws[4] = {q4.x, q4.y, q4.z, q4.w};
-            uint32_t cur[4], old[4];
+            uint32_t old[4];
             int nslots = 0;
             bool full = false;
             if (mode == 0) {
+                bool any = false;
 #pragma unroll
-                for (int c = 0; c < 4; c++)
-                    cur[c] = ws[c] >= 0 && ws[c] != s ? ld_vol(D.X + (ws[c] >> 5)) : ~0u;
+                for (int c = 0; c < 4; c++) {
+                    old[c] = ws[c] >= 0 && ws[c] != s ? ld_vol(D.X + (ws[c] >> 5)) : ~0u;
+                    any |= !((old[c] >> (ws[c] & 31)) & 1u);
+                }
+                if (!__any_sync(FULL_MASK, any)) return true;  // all of them known
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     const uint32_t bit = 1u << (ws[c] & 31);
-                    old[c] = cur[c] & bit ? ~0u : atomicOr(D.X + (ws[c] >> 5), bit);
+                    old[c] = old[c] & bit ? ~0u : atomicOr(D.X + (ws[c] >> 5), bit);
                 }
             } else {
 #pragma unroll
@@ -284,24 +299,18 @@ __device__ void warp_walk(ChainSmem<BLOCK>& SM, const MatDesc& M, const Side& D,
                 words += __reduce_add_sync(FULL_MASK, nslots);
             }
             unsigned bal[4];
-            int n = 0;
+            int to = found;
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const uint32_t bit = 1u << (ws[c] & 31);
-                const bool fresh = !(old[c] & bit);
-                if (own_row) raw += ws[c] > s;
-                if (fresh && ws[c] > s) {
-                    gt++;
-                    if (digests) dig += digest_step(ws[c] >> 5, old[c], old[c] | bit, s);
-                }
-                bal[c] = __ballot_sync(FULL_MASK, fresh);
-                n += __popc(bal[c]);
-            }
-            if (n) {
-                int to = found;
+            for (int c = 0; c < 4; c++)
+                bal[c] = __ballot_sync(FULL_MASK, !((old[c] >> (ws[c] & 31)) & 1u));
+            if (bal[0] | bal[1] | bal[2] | bal[3]) {
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                    if ((bal[c] >> lane) & 1u) P.list[to + __popc(bal[c] & ((1u << lane) - 1u))] = ws[c];
+                    if ((bal[c] >> lane) & 1u) {
+                        const int k = to + __popc(bal[c] & ((1u << lane) - 1u));
+                        P.list[k] = ws[c];
+                        P.was[k] = old[c];
+                    }
                     to += __popc(bal[c]);
                 }
                 found = to;
@@ -316,7 +325,8 @@ __device__ void warp_walk(ChainSmem<BLOCK>& SM, const MatDesc& M, const Side& D,
             for (int k0 = 0; k0 < plen && !large; k0 += 128) {
                 int4 qn = make_int4(-1, -1, -1, -1);
                 if (k0 + 128 + 4 * lane < plen) qn = ld_row4<CG>(D.G.cl + b + k0 + 128 + 4 * lane);
-                large = !visit(q4, true);
+                raw += (q4.x > s) + (q4.y > s) + (q4.z > s) + (q4.w > s);
+                large = !visit(q4);
                 q4 = qn;
             }
             if (lane == 0) trav += plen;
@@ -347,7 +357,7 @@ __device__ void warp_walk(ChainSmem<BLOCK>& SM, const MatDesc& M, const Side& D,
                     at = flat_int4(j0 + 32 + lane, total, s0, its, incl, &o);
                     if (at >= 0) qn = ld_row4<CG>(D.G.cl + at);
                 }
-                large = !visit(q4, false);
+                large = !visit(q4);
                 q4 = qn;
             }
             // a partial group of 32: the ids found meanwhile start the next one
@@ -358,10 +368,19 @@ __device__ void warp_walk(ChainSmem<BLOCK>& SM, const MatDesc& M, const Side& D,
         if (!large) {
             Tot t = mode == 0 ? bx : mode == 1 ? bt : Tot{0, 0, 0ull, 0ull};
             if (found) {
-                t.gt += __reduce_add_sync(FULL_MASK, gt);
+                int gt = 0;
+                unsigned long long dig = 0;
+                for (int i = lane; i < found; i += 32) {
+                    const int w = P.list[i];
+                    if (w < s) continue;
+                    gt++;
+                    if (digests) dig += digest_step(w >> 5, P.was[i], P.was[i] | (1u << (w & 31)), s);
+                }
+                gt = __reduce_add_sync(FULL_MASK, gt);
+                t.gt += gt;
                 t.v += __reduce_add_sync(FULL_MASK, v);
                 t.e += (unsigned)__reduce_add_sync(FULL_MASK, e);  // distinct rows: below 2^31
-                if (digests && __any_sync(FULL_MASK, gt != 0)) t.dig += warp_sum64(dig);
+                if (digests && gt) t.dig += warp_sum64(dig);
             }
             raw = __reduce_add_sync(FULL_MASK, raw);
             const int orig = dup ? row_distinct<CG>(D.G, s, D.g) : raw;
@@ -478,6 +497,7 @@ __device__ void warp_walk(ChainSmem<BLOCK>& SM, const MatDesc& M, const Side& D,
                 used = words;
                 bt = t;
                 have_t = true;
+                idle = 0;
             }
             __syncwarp();
             if (lane == 0 && s + 1 < M.n)
@@ -511,6 +531,7 @@ __device__ void warp_walk(ChainSmem<BLOCK>& SM, const MatDesc& M, const Side& D,
         if (d == 0) {
             SM.s = s;
             SM.hits = hits;
+            SM.tsel = tsel;
         }
     }
 }
@@ -595,6 +616,32 @@ struct Large {
         block_census<BLOCK, CG>(SM, M, D[d].X, s, d, digests);
         emit(d, s, D[d].X, false);
         if (threadIdx.x == 0) SM.base[d] = SM.tot;
+        __syncthreads();
+    }
+
+    // Symmetric patterns: s's search has outgrown its table.  Every id in the
+    // table is reached by s (with T's base, which s reaches), and all but those
+    // of the list are expanded: the table becomes X, and the search goes on there.
+    __device__ void promote(int s, bool digests) {
+        const Sparse& P = *D[0].P;
+        const int found = SM.found[0];
+        const int which = SM.mode[0] == 1 ? SM.tsel : 1 - SM.tsel;
+        row_stats(0, s);
+        block_clear<BLOCK>(D[0].X, words);
+        __syncthreads();
+        for (int i = threadIdx.x; i < kSlots; i += BLOCK)
+            if (P.key[which][i] != kFree) D[0].X[P.key[which][i]] = P.msk[which][i];
+        for (int i = threadIdx.x; i <= found; i += BLOCK) {
+            if (i < qcap) q[i] = i ? P.list[i - 1] : s;
+            else atomicOr(status, DEV_ERR_QUEUE);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) D[0].X[s >> 5] |= 1u << (s & 31);
+        __syncthreads();
+        block_bfs<BLOCK, CG>(SM.bfs, D[0].G, D[0].X, q, qcap, found + 1, s, s, false, status);
+        block_census<BLOCK, CG>(SM, M, D[0].X, s, 0, digests);
+        emit(0, s, D[0].X, SM.mode[0] == 1);
+        if (threadIdx.x == 0) SM.base[0] = SM.tot;
         __syncthreads();
     }
 
@@ -728,10 +775,13 @@ struct Large {
                     rebuilt = true;
                 }
             }
-            if (rebuild) {
-                for (int k = 0; k < (sym ? 1 : 2); k++) block_clear<BLOCK>(D[k].X, words);
+            if (rebuild && sym) {
+                promote(s, digests);
+                rebuilt = true;
+            } else if (rebuild) {
+                for (int k = 0; k < 2; k++) block_clear<BLOCK>(D[k].X, words);
                 __syncthreads();
-                for (int k = 0; k < (sym ? 1 : 2); k++) rebuild_from(k, s, digests);
+                for (int k = 0; k < 2; k++) rebuild_from(k, s, digests);
                 rebuilt = true;
             }
         }
@@ -775,7 +825,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) chain_kernel(ChainLaunch 
     }
     const long long cta = SERVE ? SM.cta : blockIdx.x;
     Sparse* const sparse = reinterpret_cast<Sparse*>(dyn_smem);
-    uint32_t* const sbm = reinterpret_cast<uint32_t*>(sparse + 2);
+    uint32_t* const sbm = reinterpret_cast<uint32_t*>(sparse + P.sides);
     uint32_t* const gb = P.gbm + cta * P.gbm_count * P.bitmap_words;
     int32_t* const q = P.queue + cta * P.queue_stride;
     for (long long i = threadIdx.x; i < 2 * P.bitmap_words; i += BLOCK) gb[i] = 0u;
@@ -821,6 +871,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) chain_kernel(ChainLaunch 
         const int s_first = (int)(chunk * clen);
         const int s_end = SM.skip ? s_first : (int)min((long long)n, (chunk + 1) * clen);
         const long long words = bitmap_words_for(n);
+        // (a launch planned for symmetric patterns alone has tables for one direction)
         const bool in_smem = (sym ? 1 : 2) * words <= P.smem_words;
         uint32_t* const x0 = in_smem ? sbm : gb + 2 * P.bitmap_words;
         uint32_t* const x1 = in_smem ? sbm + words : gb + 3 * P.bitmap_words;
@@ -907,7 +958,7 @@ cudaError_t launch_one(const ChainLaunch& L, int grid, size_t smem, cudaStream_t
 
 }  // namespace
 
-size_t chain_sparse_bytes() { return 2 * sizeof(Sparse); }
+size_t chain_sparse_bytes(int sides) { return (size_t)sides * sizeof(Sparse); }
 int chain_list_cap() { return kListCap; }
 
 int chain_occupancy(int block, bool serve, size_t smem) {

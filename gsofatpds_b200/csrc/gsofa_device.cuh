@@ -336,9 +336,13 @@ __device__ __forceinline__ void write_row(const MatDesc& M, int s, int dir, bool
     }
 }
 
+constexpr int kBfsCap = 512;
+
 struct BfsSmem {
-    int cnt[3], grab[3];       // per level, in turn
+    int cnt[3];                // ids queued per level, in turn
     unsigned long long rtrav;  // entries read
+    // the rows of a level's first kBfsCap ids: first entry, int4s
+    int2 row[2][kBfsCap];
 };
 
 // Breadth-first search in the bitmap bm from the frontier q[0, tail), whose
@@ -346,41 +350,32 @@ struct BfsSmem {
 // `bound`, and s, is expanded; ids found are marked and queued (ids from
 // `bound` on only when `all`).  Returns the queue's length.  With LAM, ids
 // whose label is below s count as marked.  Block-wide.
+//
+// What bounds it is the chain of dependent accesses per level (a mesh has
+// hundreds of narrow levels): in narrow levels an id's row pointers are loaded
+// when it is found and its row is kept in shared memory, so that a level is row
+// entries -> bitmap -> row pointers -> barrier; wide ones read the queue two
+// groups ahead.
 template <int BLOCK, bool CG, bool LAM = false>
 __device__ long long block_bfs(BfsSmem& SM, const Graph& G, uint32_t* bm, int32_t* q,
                                long long qcap, long long tail, int s, int bound, bool all,
                                int32_t* status, const int32_t* lam = nullptr) {
-    const int lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) {
-        SM.cnt[0] = 0;
-        SM.grab[0] = 0;
-    }
+    constexpr int NW = BLOCK / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) SM.cnt[0] = 0;
     __syncthreads();
     long long lb = 0, le = min(tail, qcap);
     unsigned long long trav = 0;
+    bool kept = false;
     for (int level = 0; lb < le; level++) {
-        int* cnt = &SM.cnt[level % 3];
-        int* grab = &SM.grab[level % 3];
-        if (threadIdx.x == 0) {
-            SM.cnt[(level + 1) % 3] = 0;
-            SM.grab[(level + 1) % 3] = 0;
-        }
-        int c0 = 0;
-        if (lane == 0) c0 = atomicAdd(grab, 1);
-        long long base = lb + 32ll * __shfl_sync(FULL_MASK, c0, 0);
-        int u = base + lane < le ? q[base + lane] : -1;
-        while (base < le) {
-            // the next chunk's entries load while this one is expanded
-            int cn = 0;
-            if (lane == 0) cn = atomicAdd(grab, 1);
-            const long long nbase = lb + 32ll * __shfl_sync(FULL_MASK, cn, 0);
-            const int nu = nbase + lane < le ? q[nbase + lane] : -1;
-            int s0 = 0, its = 0;
-            if (u >= 0 && (u < bound || u == s)) {
-                const int a0 = ld_i32<CG>(G.rp + u), a1 = ld_i32<CG>(G.rp + u + 1);
-                s0 = a0 & ~3;
-                its = ((a1 & ~3) - s0) >> 2;
-            }
+        int* const cnt = &SM.cnt[level % 3];
+        int2* const next = SM.row[(level + 1) & 1];
+        const int2* const cur = SM.row[level & 1];
+        if (threadIdx.x == 0) SM.cnt[(level + 1) % 3] = 0;
+        const long long n = le - lb;
+        const bool keep = n <= BLOCK;  // this level is narrow: the next one's rows are kept
+        // the entries of up to 32 rows, 128 at a time: marks them, queues the new ids
+        auto expand = [&](int s0, int its) {
             const int incl = warp_incl_sum(its, lane);
             const int total = __shfl_sync(FULL_MASK, incl, 31);
             if (lane == 0) trav += 4ull * total;
@@ -394,49 +389,97 @@ __device__ long long block_bfs(BfsSmem& SM, const Graph& G, uint32_t* bm, int32_
                     if (at >= 0) en = ld_row4<CG>(G.cl + at);
                 }
                 const int ws[4] = {e.x, e.y, e.z, e.w};
-                uint32_t cur[4], old[4];
+                e = en;
+                uint32_t old[4];
 #pragma unroll
                 for (int c = 0; c < 4; c++)
-                    cur[c] = ws[c] >= 0 && ws[c] != s ? ld_vol(bm + (ws[c] >> 5)) : ~0u;
+                    old[c] = ws[c] >= 0 && ws[c] != s ? ld_vol(bm + (ws[c] >> 5)) : ~0u;
                 if constexpr (LAM) {
                     // what the hub reaches through ids below s is not looked at
 #pragma unroll
                     for (int c = 0; c < 4; c++)
-                        if (ws[c] >= 0 && __ldg(lam + ws[c]) < s) cur[c] = ~0u;
+                        if (ws[c] >= 0 && __ldg(lam + ws[c]) < s) old[c] = ~0u;
                 }
+                bool any = false;
+#pragma unroll
+                for (int c = 0; c < 4; c++) any |= !((old[c] >> (ws[c] & 31)) & 1u);
+                if (!__any_sync(FULL_MASK, any)) continue;
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     const uint32_t bit = 1u << (ws[c] & 31);
-                    old[c] = cur[c] & bit ? ~0u : atomicOr(bm + (ws[c] >> 5), bit);
+                    old[c] = old[c] & bit ? ~0u : atomicOr(bm + (ws[c] >> 5), bit);
                 }
                 unsigned bal[4];
-                int n = 0;
+                int k = 0;
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                    const bool fresh = !(old[c] & (1u << (ws[c] & 31)));
-                    bal[c] = __ballot_sync(FULL_MASK, fresh && (all || ws[c] < bound));
-                    n += __popc(bal[c]);
+                    bal[c] = __ballot_sync(FULL_MASK, !((old[c] >> (ws[c] & 31)) & 1u) &&
+                                                          (all || ws[c] < bound));
+                    k += __popc(bal[c]);
                 }
-                if (n) {
-                    int p = 0;
-                    if (lane == 0) p = atomicAdd(cnt, n);
-                    long long to = le + __shfl_sync(FULL_MASK, p, 0);
+                if (!k) continue;
+                int to = 0;
+                if (lane == 0) to = atomicAdd(cnt, k);
+                to = __shfl_sync(FULL_MASK, to, 0);
+                int x[4];
 #pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        if ((bal[c] >> lane) & 1u) {
-                            const long long k = to + __popc(bal[c] & ((1u << lane) - 1u));
-                            if (k < qcap) q[k] = ws[c];
-                            else atomicOr(status, DEV_ERR_QUEUE);
-                        }
-                        to += __popc(bal[c]);
+                for (int c = 0; c < 4; c++) {
+                    x[c] = ((bal[c] >> lane) & 1u) ? to + __popc(bal[c] & ((1u << lane) - 1u)) : -1;
+                    to += __popc(bal[c]);
+                    if (x[c] < 0) continue;
+                    if (le + x[c] < qcap) q[le + x[c]] = ws[c];
+                    else atomicOr(status, DEV_ERR_QUEUE);
+                }
+                if (!keep) continue;
+                int a0[4], a1[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    a0[c] = a1[c] = 0;
+                    if (x[c] >= 0 && ws[c] < bound) {
+                        a0[c] = ld_i32<CG>(G.rp + ws[c]);
+                        a1[c] = ld_i32<CG>(G.rp + ws[c] + 1);
                     }
                 }
-                e = en;
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (x[c] >= 0 && x[c] < kBfsCap)
+                        next[x[c]] = make_int2(a0[c] & ~3, ((a1[c] & ~3) - (a0[c] & ~3)) >> 2);
             }
-            base = nbase;
-            u = nu;
+        };
+        if (kept && n <= kBfsCap) {
+            const int per = n >= 32 * NW ? 32 : (int)((n + NW - 1) / NW);
+            for (long long base = (long long)warp * per; base < n; base += NW * per) {
+                int2 r = make_int2(0, 0);
+                if (lane < per && base + lane < n) r = cur[base + lane];
+                expand(r.x, r.y);
+            }
+        } else {
+            // two groups of 32 ahead: the queue entries load while the group
+            // before is expanded, the row pointers while the one before that is
+            auto id_of = [&](long long k) { return k < le ? q[k] : -1; };
+            auto row_of = [&](int u, int& a0, int& a1) {
+                a0 = a1 = 0;
+                if (u >= 0 && (u < bound || u == s)) {
+                    a0 = ld_i32<CG>(G.rp + u);
+                    a1 = ld_i32<CG>(G.rp + u + 1);
+                }
+            };
+            long long base = lb + 32ll * warp;
+            int nu = id_of(base + lane), a0, a1;
+            row_of(nu, a0, a1);
+            nu = id_of(base + 32 * NW + lane);
+            for (; base < le; base += 32 * NW) {
+                const int nnu = id_of(base + 64 * NW + lane);
+                int na0, na1;
+                row_of(nu, na0, na1);
+                expand(a0 & ~3, ((a1 & ~3) - (a0 & ~3)) >> 2);
+                nu = nnu;
+                a0 = na0;
+                a1 = na1;
+            }
         }
         __syncthreads();
+        kept = keep;
         lb = le;
         le = min(le + *cnt, qcap);
     }

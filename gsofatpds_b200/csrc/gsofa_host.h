@@ -29,9 +29,17 @@ struct gsofa_ctx {
     // autotuner choices per class (log2 n, mean row length, locality: half-
     // octaves of the mean |i - j| of the entries over n)
     std::map<std::tuple<int, int, int>, gsofa_opts> tuned;
-    // pinned staging
-    unsigned long long* h_counters = nullptr;  // CNT_SLOTS
+    // pinned staging: totals of h_counters_cap matrices, the status words and
+    // h_fallback_cap flags, and results on their way to the caller's arrays
+    unsigned long long* h_counters = nullptr;
+    size_t h_counters_cap = 0;
     int32_t* h_status = nullptr;
+    int32_t* h_fallback = nullptr;
+    char* h_stage = nullptr;
+    cudaEvent_t stage_ev[2] = {};
+    // matrix descriptors of the current launch
+    void* desc = nullptr;
+    size_t desc_bytes = 0;
     // grown workspace
     void* queue = nullptr;
     size_t queue_bytes = 0;
@@ -44,7 +52,6 @@ struct gsofa_ctx {
     size_t scan_tmp_bytes = 0;
     void* hub_ws = nullptr;
     size_t hub_ws_bytes = 0;
-    std::vector<int32_t> h_fallback;
 };
 
 struct gsofa_matrix {
@@ -153,6 +160,7 @@ struct ChainCfg {
     long long words = 0;       // of the largest matrix's bitmap
     long long smem_words = 0;  // bitmap words in shared memory (0: bitmaps in global memory)
     int gbm_count = 2;         // global bitmaps per CTA
+    int sides = 2;
 };
 bool chain_runs(const gsofa_opts& o);
 int plan_chain(gsofa_ctx* ctx, int32_t nmax, bool all_sym, const gsofa_opts* o, bool serve,
@@ -167,7 +175,7 @@ int32_t method_of(const gsofa_matrix* m);
 bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, void* ws,
               size_t* bytes, HubLaunch* L, HubCfg* c);
 // Consecutive sources per work item.
-long long chain_chunk(const gsofa_opts& o, long long total_sources, int grid);
+long long chain_chunk(const gsofa_opts& o, long long total_sources, int grid, bool sym);
 // Result arrays of an n-row matrix, zero-initialised on `stream`.
 int result_alloc_on(gsofa_ctx* ctx, int32_t n, uint32_t flags, int32_t mss, cudaStream_t stream,
                     gsofa_result** out);
@@ -232,6 +240,8 @@ struct DeviceScratch {
         for (auto& b : blocks) dev_free_on(ctx, b.first, b.second, ctx->stream);
     }
 };
+
+constexpr size_t kStageBytes = 8u << 20;  // ctx->h_stage
 
 constexpr int kDefaultBuAlpha = 0;  // top-down only unless a caller asks
 constexpr int kDefaultBuBeta = 24;

@@ -163,6 +163,7 @@ struct ChainLaunch {
     int gbm_count;
     long long bitmap_words;            // covers the largest n + padding
     long long smem_words;              // bitmap words that fit in shared memory
+    int sides;                         // directions with tables: 1 when every pattern is symmetric
     int chunk;                         // consecutive sources per work item
     int list_cap;                      // new ids of a search before the whole CTA takes it
     long long sample_stride;           // > 1: only every stride-th item (autotuner timing)
@@ -235,7 +236,7 @@ int large_occupancy(int block, size_t smem);
 cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStream_t stream);
 
 // Shared memory of a CTA besides its bitmaps; the largest list_cap.
-size_t chain_sparse_bytes();
+size_t chain_sparse_bytes(int sides);
 int chain_list_cap();
 // Resident CTAs per SM with `smem` dynamic bytes (0 = cannot run).
 int chain_occupancy(int block, bool serve, size_t smem);
