@@ -293,6 +293,13 @@ int result_alloc_on(gsofa_ctx* ctx, int32_t n, uint32_t flags, int32_t mss, cuda
     return GSOFA_OK;
 }
 
+// The arrays a factorization finds zeroed.
+cudaError_t result_clear(gsofa_result* r, cudaStream_t stream) {
+    size_t off[12];
+    const size_t total = result_layout(r->n, r->flags, off);
+    return cudaMemsetAsync(static_cast<char*>(r->arena) + off[7], 0, total - off[7], stream);
+}
+
 int result_alloc(gsofa_ctx* ctx, int32_t n, uint32_t flags, int32_t mss, gsofa_result** out) {
     return result_alloc_on(ctx, n, flags, mss, ctx->stream, out);
 }
@@ -329,11 +336,16 @@ MatDesc make_desc(const gsofa_matrix* m, const gsofa_result* r, long long base) 
     return d;
 }
 
-// Whether the counting traversal (gsofa_chain.cu) runs these options: it
-// always reuses closures and searches top-down, and does not scatter per-row L
-// statistics; the diagnostic switches and that option take traverse_kernel.
-bool chain_runs(const gsofa_opts& o) {
-    return !(o.flags & (GSOFA_NO_MERGE | GSOFA_NO_CHAIN | GSOFA_L_ROW_STATS)) && o.bu_alpha <= 0;
+// Whether the counting traversals (gsofa_chain.cu, gsofa_hub.cu) run these
+// options: they always reuse closures and search top-down, so the diagnostic
+// switches take traverse_kernel.  Per-row L statistics come from gsofa_hub.cu
+// alone: with them, only matrices that all go there.
+bool chain_runs(const gsofa_opts& o, const gsofa_matrix* const* mats, int32_t count) {
+    if ((o.flags & (GSOFA_NO_MERGE | GSOFA_NO_CHAIN)) || o.bu_alpha > 0) return false;
+    if (o.flags & GSOFA_L_ROW_STATS)
+        for (int32_t i = 0; i < count; i++)
+            if (method_of(mats[i]) == METHOD_CHAIN) return false;
+    return true;
 }
 
 int plan_chain(gsofa_ctx* ctx, int32_t nmax, bool all_sym, const gsofa_opts* o, bool serve,
@@ -436,7 +448,9 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     c->large_grid = occ * ctx->sm_count;
     L->queue_stride = n_max;
     if (o.flags & GSOFA_DEBUG_QUEUE_CAP) L->queue_stride = std::min<long long>(L->queue_stride, 64);
-    c->scan_bytes = c->any_hub ? hub_scan_bytes(2 * hub_bases() * off) : 0;
+    c->l_rows = (o.flags & GSOFA_L_ROW_STATS) != 0;
+    const long long uses = c->l_rows ? (long long)W * off : 0;
+    c->scan_bytes = c->any_hub ? hub_scan_bytes(2ll * hub_bases() * off, uses) : 0;
     // workspace: the zeroed block first
     size_t at = 0;
     char* const w = static_cast<char*>(ws);
@@ -448,6 +462,7 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     const size_t T = (size_t)off;
     L->zeroed = w;
     L->base = static_cast<Tot*>(place(sizeof(Tot) * 2 * (size_t)hub_bases() * T));
+    L->l_use = static_cast<LRowUse*>(place(sizeof(LRowUse) * (size_t)uses));
     L->stamp = static_cast<int32_t*>(place(4 * 2 * (size_t)W * T));
     L->lcnt = static_cast<int32_t*>(place(16 * 2 * (size_t)W * (size_t)nm));
     L->fallback = static_cast<int32_t*>(place(4 * (size_t)nm));
@@ -483,7 +498,8 @@ long long chain_chunk(const gsofa_opts& o, long long total_sources, int grid, bo
 // Runs the traversal (and optionally supernodes / pattern) for `count`
 // matrices in one persistent launch.  results[i] must be freshly allocated.
 int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
-               const gsofa_opts* o, gsofa_result** res, long long sample_stride = 1) {
+               const gsofa_opts* o, gsofa_result** res, long long sample_stride = 1,
+               bool counting = true) {
     int32_t nmax = 0;
     long long total_sources = 0, weight = 0;
     bool all_sym = true;
@@ -493,7 +509,7 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
         total_sources += mats[i]->n;
         all_sym = all_sym && mats[i]->host_sym > 0;
     }
-    const bool chain = chain_runs(*o);
+    const bool chain = counting && chain_runs(*o, mats, count);
     const bool pattern = (o->flags & GSOFA_PATTERN) != 0;
     const bool traverse = !chain || pattern;
     int rc = GSOFA_OK;
@@ -659,6 +675,11 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
     std::vector<char> left((size_t)count, 0);
     bool any = false;
     for (int32_t k = 0; k < count && hub; k++) any |= (left[(size_t)k] = ctx->h_fallback[k] != 0);
+    if (any && (o->flags & GSOFA_L_ROW_STATS)) {
+        // the chain does not make them: all of it again
+        for (int32_t i = 0; i < count; i++) CK(result_clear(res[i], ctx->stream));
+        return run_factor(ctx, mats, count, o, res, sample_stride, false);
+    }
     if (any) {
         long long items = 0, sources = 0;
         bool sym = true;
@@ -1035,6 +1056,43 @@ int gsofa::host::matrix_build(gsofa_ctx* ctx, cudaStream_t stream, int32_t* dsta
     return e == cudaSuccess ? GSOFA_OK : cuda_fail(ctx, e, "matrix build");
 }
 
+// Small arrays share one wait through pinned staging (three 80 KB arrays: 36 ->
+// 16 us); large ones go straight to the caller's pages, which the driver's own
+// staging fills faster (46 MB: 2.4 ms, against 3.2 through 16 MB pinned pieces and
+// four copying threads).
+int gsofa::host::fetch_all(gsofa_ctx* ctx, const Fetch* f, int count) {
+    size_t total = 0;
+    for (int k = 0; k < count; k++) {
+        if (!f[k].dst) continue;
+        if (!f[k].src)
+            return set_err(ctx, GSOFA_ERR_ARG, "requested array was not computed (option off)");
+        total += f[k].bytes;
+    }
+    std::lock_guard<std::recursive_mutex> g(ctx->mu);
+    cudaError_t e = cudaSuccess;
+    if (total <= kStageBytes) {
+        size_t at = 0;
+        for (int k = 0; k < count && e == cudaSuccess; k++) {
+            if (!f[k].dst || !f[k].bytes) continue;
+            e = cudaMemcpyAsync(ctx->h_stage + at, f[k].src, f[k].bytes, cudaMemcpyDeviceToHost, ctx->stream);
+            at += f[k].bytes;
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        at = 0;
+        for (int k = 0; k < count && e == cudaSuccess; k++) {
+            if (!f[k].dst || !f[k].bytes) continue;
+            memcpy(f[k].dst, ctx->h_stage + at, f[k].bytes);
+            at += f[k].bytes;
+        }
+        return e == cudaSuccess ? GSOFA_OK : cuda_fail(ctx, e, "result fetch");
+    }
+    for (int k = 0; k < count && e == cudaSuccess; k++)
+        if (f[k].dst && f[k].bytes)
+            e = cudaMemcpyAsync(f[k].dst, f[k].src, f[k].bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    return e == cudaSuccess ? GSOFA_OK : cuda_fail(ctx, e, "result fetch");
+}
+
 // ============================================================================
 extern "C" {
 
@@ -1091,8 +1149,6 @@ int gsofa_create(int device, size_t budget_bytes, gsofa_ctx** out) {
         if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
         if (ctx->h_fallback) cudaFreeHost(ctx->h_fallback);
         if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
-        for (cudaEvent_t ev : ctx->stage_ev)
-            if (ev) cudaEventDestroy(ev);
         if (ctx->h_status) cudaFreeHost(ctx->h_status);
         if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
         delete ctx;
@@ -1114,8 +1170,6 @@ int gsofa_create(int device, size_t budget_bytes, gsofa_ctx** out) {
     if ((e = cudaEventCreate(&ctx->evt)) != cudaSuccess) return fail(e);
     if (ensure_pinned(ctx, 1) != GSOFA_OK) return fail(cudaErrorMemoryAllocation);
     if ((e = cudaMallocHost((void**)&ctx->h_stage, kStageBytes)) != cudaSuccess) return fail(e);
-    for (cudaEvent_t& ev : ctx->stage_ev)
-        if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return fail(e);
     if ((e = cudaMallocHost((void**)&ctx->h_status, 64)) != cudaSuccess) return fail(e);
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
@@ -1150,7 +1204,6 @@ int gsofa_destroy(gsofa_ctx* ctx) {
         cudaFreeHost(ctx->h_counters);
         cudaFreeHost(ctx->h_fallback);
         cudaFreeHost(ctx->h_stage);
-        for (cudaEvent_t ev : ctx->stage_ev) cudaEventDestroy(ev);
         cudaFreeHost(ctx->h_status);
         cudaMemPoolDestroy(ctx->pool);
     }
@@ -1510,7 +1563,8 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
         if (rc) return fail(rc);
         b->res[(size_t)i]->batch_owned = true;
     }
-    const bool chain = chain_runs(o);
+    // (per-row L statistics could not be made again inside the captured launch)
+    const bool chain = !(o.flags & GSOFA_L_ROW_STATS) && chain_runs(o, mats, count);
     ChainCfg ccfg;
     LaunchCfg cfg;
     // the chain's shape: that of the matrices it takes, or of all if it takes none
@@ -1714,70 +1768,10 @@ int gsofa_result_counts(const gsofa_result* r, gsofa_counts* out) {
     return GSOFA_OK;
 }
 
-// Arrays from the device to the caller's memory, through pinned staging: the
-// copies of small ones share one wait (of three 80 KB arrays: 36 -> 16 us), and
-// a large one's piece is moved on while the next arrives.
-struct Fetch {
-    void* dst;
-    const void* src;
-    size_t bytes;
-};
-
-static int fetch_all(const gsofa_result* r, const Fetch* f, int count) {
-    gsofa_ctx* ctx = r->ctx;
-    size_t total = 0;
-    for (int k = 0; k < count; k++) {
-        if (!f[k].dst) continue;
-        if (!f[k].src) return set_err(ctx, GSOFA_ERR_ARG, "requested array was not computed (option off)");
-        total += f[k].bytes;
-    }
-    std::lock_guard<std::recursive_mutex> g(ctx->mu);
-    cudaError_t e = cudaSuccess;
-    if (total <= kStageBytes) {
-        size_t at = 0;
-        for (int k = 0; k < count && e == cudaSuccess; k++) {
-            if (!f[k].dst || !f[k].bytes) continue;
-            e = cudaMemcpyAsync(ctx->h_stage + at, f[k].src, f[k].bytes, cudaMemcpyDeviceToHost, ctx->stream);
-            at += f[k].bytes;
-        }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        at = 0;
-        for (int k = 0; k < count && e == cudaSuccess; k++) {
-            if (!f[k].dst || !f[k].bytes) continue;
-            memcpy(f[k].dst, ctx->h_stage + at, f[k].bytes);
-            at += f[k].bytes;
-        }
-    } else {
-        constexpr size_t kHalf = kStageBytes / 2;
-        struct { void* dst; size_t bytes; } held[2] = {{nullptr, 0}, {nullptr, 0}};
-        int h = 0;
-        auto deliver = [&](int x) {
-            if (!held[x].bytes) return;
-            e = cudaEventSynchronize(ctx->stage_ev[x]);
-            if (e == cudaSuccess) memcpy(held[x].dst, ctx->h_stage + x * kHalf, held[x].bytes);
-            held[x].bytes = 0;
-        };
-        for (int k = 0; k < count; k++) {
-            if (!f[k].dst) continue;
-            for (size_t at = 0; at < f[k].bytes && e == cudaSuccess; at += kHalf, h ^= 1) {
-                deliver(h);
-                if (e != cudaSuccess) break;
-                const size_t b = std::min(kHalf, f[k].bytes - at);
-                e = cudaMemcpyAsync(ctx->h_stage + h * kHalf, static_cast<const char*>(f[k].src) + at, b,
-                                    cudaMemcpyDeviceToHost, ctx->stream);
-                if (e == cudaSuccess) e = cudaEventRecord(ctx->stage_ev[h], ctx->stream);
-                held[h].dst = static_cast<char*>(f[k].dst) + at;
-                held[h].bytes = b;
-            }
-        }
-        for (int x = 0; x < 2 && e == cudaSuccess; x++, h ^= 1) deliver(h);
-    }
-    return e == cudaSuccess ? GSOFA_OK : cuda_fail(ctx, e, "result fetch");
-}
-
 static int fetch(const gsofa_result* r, void* dst, const void* src, size_t bytes) {
+    if (dst && !src) return set_err(r->ctx, GSOFA_ERR_ARG, "requested array was not computed (option off)");
     const Fetch f{dst, src, bytes};
-    return fetch_all(r, &f, 1);
+    return fetch_all(r->ctx, &f, 1);
 }
 
 int gsofa_result_row_counts(const gsofa_result* r, int32_t* nnz_u_row, int32_t* nz_row_u,
@@ -1786,14 +1780,14 @@ int gsofa_result_row_counts(const gsofa_result* r, int32_t* nnz_u_row, int32_t* 
     const size_t b = 4 * (size_t)r->n;
     const Fetch f[4] = {{nnz_u_row, r->nnz_u, b}, {nz_row_u, r->nz_row_u, b},
                         {nnz_l_col, r->nnz_lc, b}, {nnz_l_row, r->nnz_lr, b}};
-    return fetch_all(r, f, 4);
+    return fetch_all(r->ctx, f, 4);
 }
 
 int gsofa_result_digests(const gsofa_result* r, uint64_t* du, uint64_t* dlc, uint64_t* dlr) {
     if (!r) return GSOFA_ERR_ARG;
     const size_t b = 8 * (size_t)r->n;
     const Fetch f[3] = {{du, r->dig_u, b}, {dlc, r->dig_lc, b}, {dlr, r->dig_lr, b}};
-    return fetch_all(r, f, 3);
+    return fetch_all(r->ctx, f, 3);
 }
 
 int gsofa_result_lmask(const gsofa_result* r, uint32_t* mask4n) {

@@ -56,15 +56,30 @@ __device__ __forceinline__ long long lower_bound_i32(const int32_t* a, long long
     return lo;
 }
 
-// cnt[c] = entries of list c (sorted) at or beyond the end of c's block
+// Does the next list of c's block hold everything of list c past it?  For L
+// columns it does when U(c, c + 1) != 0: a row r that reaches c reaches c + 1
+// through c.  For U rows, when L(c + 1, c) != 0.  (optr, oidx: the other side's
+// lists; ids above c, ascending.)  Then list c adds nothing to the block's
+// union, so only the last list of each such run is emitted and sorted: of the
+// 40^3 mesh's 21.3M ids a side 5.7M, and most blocks are one sorted list.
+__device__ __forceinline__ bool held_by_next(int32_t c, int32_t l, const int64_t* __restrict__ optr,
+                                             const int32_t* __restrict__ oidx) {
+    if (c + 1 >= l) return false;
+    const long long b = optr[c];
+    return b < optr[c + 1] && oidx[b] == c + 1;
+}
+
+// cnt[c] = entries of list c (sorted) at or beyond the end of c's block, 0 for
+// a list that the next one holds
 __global__ void count_kernel(int32_t n, const int64_t* __restrict__ ptr,
-                             const int32_t* __restrict__ idx, const int32_t* __restrict__ blk,
+                             const int32_t* __restrict__ idx, const int64_t* __restrict__ optr,
+                             const int32_t* __restrict__ oidx, const int32_t* __restrict__ blk,
                              const int32_t* __restrict__ start, long long* __restrict__ cnt) {
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n;
          c += (long long)gridDim.x * blockDim.x) {
         const int32_t l = start[blk[c] + 1];
         const long long b = ptr[c], e = ptr[c + 1];
-        cnt[c] = e - lower_bound_i32(idx, b, e, l);
+        cnt[c] = held_by_next((int32_t)c, l, optr, oidx) ? 0 : e - lower_bound_i32(idx, b, e, l);
     }
 }
 
@@ -78,6 +93,7 @@ __global__ void emit_kernel(int32_t n, const int64_t* __restrict__ ptr,
     for (long long c = gw; c < n; c += nwarps) {  // a warp per list
         const int32_t l = start[blk[c] + 1];
         const long long b = ptr[c], e = ptr[c + 1];
+        if (off[c + 1] == off[c]) continue;  // adds nothing
         const long long first = lower_bound_i32(idx, b, e, l);
         for (long long j = first + lane; j < e; j += 32) ids[off[c] + (j - first)] = idx[j];
     }
@@ -131,14 +147,15 @@ int grid_for(long long items, int threads) {
 // Sorted union per block of one side's lists past the block end: fills
 // out_ptr (nblocks + 1) and allocates *out_idx (*out_count ids).
 int one_side(gsofa_ctx* ctx, DeviceScratch& S, int32_t n, long long nblocks, const int64_t* ptr,
-             const int32_t* idx, const int32_t* blk, const int32_t* start, int64_t* out_ptr,
+             const int32_t* idx, const int64_t* optr, const int32_t* oidx, const int32_t* blk,
+             const int32_t* start, int64_t* out_ptr,
              int32_t** out_idx, long long* out_count) {
     cudaStream_t st = ctx->stream;
     long long* cnt = static_cast<long long*>(S.get(8 * ((size_t)n + 1)));
     long long* off = static_cast<long long*>(S.get(8 * ((size_t)n + 1)));
     if (!cnt || !off) return GSOFA_ERR_OOM_BUDGET;
     cudaMemsetAsync(cnt + n, 0, 8, st);
-    count_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, ptr, idx, blk, start, cnt);
+    count_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, ptr, idx, optr, oidx, blk, start, cnt);
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, off, (int)n + 1, st);
     void* tmp = S.get(tb);
@@ -234,10 +251,10 @@ int build(gsofa_result* r) {
     cudaStreamSynchronize(st);  // the copy's source is on this stack frame
     // L: rows of each column; U: columns of each row
     long long nl = 0, nu = 0;
-    int rc = one_side(ctx, S, n, nb, r->lptr, r->lrows, blk, start, lp, &r->sn_lrows, &nl);
+    int rc = one_side(ctx, S, n, nb, r->lptr, r->lrows, r->uptr, r->ucols, blk, start, lp, &r->sn_lrows, &nl);
     if (rc) return rc;
     r->sn_nl = nl;  // recorded at once: a failure below frees it with its size
-    rc = one_side(ctx, S, n, nb, r->uptr, r->ucols, blk, start, up, &r->sn_ucols, &nu);
+    rc = one_side(ctx, S, n, nb, r->uptr, r->ucols, r->lptr, r->lrows, blk, start, up, &r->sn_ucols, &nu);
     if (rc) return rc;
     r->sn_nu = nu;
     if (cudaStreamSynchronize(st) != cudaSuccess)
@@ -283,16 +300,10 @@ extern "C" int gsofa_result_supernodal(const gsofa_result* res, int64_t* nblocks
     if (nl) *nl = r->sn_nl;
     if (nu) *nu = r->sn_nu;
     const size_t nb = (size_t)r->sn_nblocks + 1;
-    cudaStream_t st = ctx->stream;
-    cudaError_t e = cudaSuccess;
-    if (block_start) e = cudaMemcpyAsync(block_start, r->sn_start, 4 * nb, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && lptr) e = cudaMemcpyAsync(lptr, r->sn_lptr, 8 * nb, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && uptr) e = cudaMemcpyAsync(uptr, r->sn_uptr, 8 * nb, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && lrows && r->sn_nl > 0)
-        e = cudaMemcpyAsync(lrows, r->sn_lrows, 4 * (size_t)r->sn_nl, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && ucols && r->sn_nu > 0)
-        e = cudaMemcpyAsync(ucols, r->sn_ucols, 4 * (size_t)r->sn_nu, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return set_err(ctx, GSOFA_ERR_CUDA, "supernodal form: %s", cudaGetErrorString(e));
-    return GSOFA_OK;
+    const Fetch f[5] = {{block_start, r->sn_start, 4 * nb},
+                        {lptr, r->sn_lptr, 8 * nb},
+                        {lrows, r->sn_lrows, 4 * (size_t)r->sn_nl},
+                        {uptr, r->sn_uptr, 8 * nb},
+                        {ucols, r->sn_ucols, 4 * (size_t)r->sn_nu}};
+    return fetch_all(ctx, f, 5);
 }

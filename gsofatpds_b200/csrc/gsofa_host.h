@@ -36,7 +36,6 @@ struct gsofa_ctx {
     int32_t* h_status = nullptr;
     int32_t* h_fallback = nullptr;
     char* h_stage = nullptr;
-    cudaEvent_t stage_ev[2] = {};
     // matrix descriptors of the current launch
     void* desc = nullptr;
     size_t desc_bytes = 0;
@@ -162,7 +161,7 @@ struct ChainCfg {
     int gbm_count = 2;         // global bitmaps per CTA
     int sides = 2;
 };
-bool chain_runs(const gsofa_opts& o);
+bool chain_runs(const gsofa_opts& o, const gsofa_matrix* const* mats, int32_t count);
 int plan_chain(gsofa_ctx* ctx, int32_t nmax, bool all_sym, const gsofa_opts* o, bool serve,
                ChainCfg* c);
 // The launch's fields that follow from the shape, the options and the largest order.
@@ -241,7 +240,14 @@ struct DeviceScratch {
     }
 };
 
-constexpr size_t kStageBytes = 8u << 20;  // ctx->h_stage
+constexpr size_t kStageBytes = 2u << 20;  // ctx->h_stage
+// Device arrays to the caller's memory, complete on return.
+struct Fetch {
+    void* dst;
+    const void* src;
+    size_t bytes;
+};
+int fetch_all(gsofa_ctx* ctx, const Fetch* f, int count);
 
 constexpr int kDefaultBuAlpha = 0;  // top-down only unless a caller asks
 constexpr int kDefaultBuBeta = 24;

@@ -462,10 +462,11 @@ struct TotSum {
 struct Base {
     const int32_t* lam;
     Tot t;
+    int hub;
 };
 
 __device__ __forceinline__ Base base_of(const HubLaunch& P, const MatDesc& M, int s, int d, bool sym) {
-    Base b{nullptr, {0, 0, 0ull, 0ull}};
+    Base b{nullptr, {0, 0, 0ull, 0ull}, 0};
     if (M.method != METHOD_HUB) return b;
     const int l = window_of(M.n, s);
     // the hubs s reaches; of two the one that reaches more
@@ -475,8 +476,25 @@ __device__ __forceinline__ Base base_of(const HubLaunch& P, const MatDesc& M, in
         if (b.lam && t.gt + t.v <= b.t.gt + b.t.v) continue;
         b.lam = P.lam + lam_at(P, M, h, d);
         b.t = t;
+        b.hub = h;
     }
     return b;
+}
+
+// Per-row L statistics of L column s: the ids `bits` (of word w, above s) that
+// its search found.
+__device__ __forceinline__ void lrow_found(const MatDesc& M, int w, uint32_t bits, int s) {
+    const unsigned long long ds = mix64((uint64_t)(uint32_t)s);
+    for (; bits; bits &= bits - 1) {
+        const int v = 32 * w + __ffs(bits) - 1;
+        atomicAdd(&M.nnz_lr[v], 1);
+        atomicAdd((unsigned long long*)&M.dig_lr[v], ds);
+    }
+}
+
+// That column s also holds its hub's set above s: noted for lrow_kernel.
+__device__ __forceinline__ void lrow_hub(const HubLaunch& P, const MatDesc& M, const Base& b, int s) {
+    if (b.lam) P.l_use[(long long)b.hub * P.total + M.hub_off + s] = LRowUse{1ull, mix64((uint64_t)(uint32_t)s)};
 }
 
 // the hub set's ids above s in word w
@@ -678,6 +696,7 @@ __global__ void __launch_bounds__(kExtraThreads, 1024 / kExtraThreads) extra_ker
                         const int w = (int)T.key[slot];
                         const uint32_t hi = T.msk[slot] & above(w, s);
                         gt += __popc(hi);
+                        if (M.nnz_lr && (d == 1 || sym)) lrow_found(M, w, hi, s);
                         if (digests) {
                             const uint32_t bw = base_word(B, w, s, n);
                             dig += word_digest(w, bw | hi) - word_digest(w, bw);
@@ -688,7 +707,10 @@ __global__ void __launch_bounds__(kExtraThreads, 1024 / kExtraThreads) extra_ker
                     t.e += (unsigned)__reduce_add_sync(FULL_MASK, e);
                     if (digests && k) t.dig += warp_sum64(dig);
                 }
-                if (lane == 0) write_row(M, s, d, sym, t, raw, raw);
+                if (lane == 0) {
+                    write_row(M, s, d, sym, t, raw, raw);
+                    if (M.nnz_lr && (d == 1 || sym)) lrow_hub(P, M, B, s);
+                }
                 if (d == 1 || sym) {
                     uint32_t word = base_next128(B, s, n);
                     if (found) {
@@ -782,6 +804,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) large_kernel(HubLaunch P)
             const uint32_t hi = x & above(w, s), low = x & below(w, s);
             vals[0] += __popc(hi);
             vals[1] += __popc(low);
+            if (M.nnz_lr && (d == 1 || sym)) lrow_found(M, w, hi, s);
             if (digests && hi) {
                 const uint32_t bw = base_word(B, w, s, n);
                 vals[3] += word_digest(w, bw | hi) - word_digest(w, bw);
@@ -816,6 +839,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) large_kernel(HubLaunch P)
                     t.dig += red[i][3];
                 }
                 write_row(M, s, d, sym, t, row[0], row[0]);
+                if (M.nnz_lr && (d == 1 || sym)) lrow_hub(P, M, B, s);
                 unsigned long long* c = P.counters + (long long)mi * CNT_SLOTS;
                 atomicAdd(c + CNT_FILLS, (unsigned long long)(t.gt - row[0]) * (sym ? 2 : 1));
                 atomicAdd(c + CNT_EDGES_TRAV, bfs.rtrav);
@@ -830,6 +854,36 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) large_kernel(HubLaunch P)
         }
         __syncthreads();
         block_clear<BLOCK>(bm, nw);
+    }
+}
+
+struct UseSum {
+    __host__ __device__ LRowUse operator()(const LRowUse& a, const LRowUse& b) const {
+        return LRowUse{a.count + b.count, a.dig + b.dig};
+    }
+};
+
+// Per-row L statistics from the hubs' sets: row v is in the set of column s
+// when label(v) < s < v, so it gains the columns that took hub h's set between
+// those two ids: a difference of prefix sums (l_use, scanned).
+__global__ void lrow_kernel(HubLaunch P) {
+    const int mi = blockIdx.y;
+    const MatDesc& M = P.mats[mi];
+    if (M.method != METHOD_HUB || P.fallback[mi]) return;
+    const int d = M.asym[0] == 0 ? 0 : 1;
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < M.n; v += gridDim.x * blockDim.x) {
+        unsigned long long count = 0, dig = 0;
+        for (int h = 0; h < kHubs; h++) {
+            const int l = __ldg(P.lam + lam_at(P, M, h, d) + v);
+            if (l >= v - 1) continue;
+            const LRowUse* u = P.l_use + (long long)h * P.total + M.hub_off;
+            const LRowUse a = u[l], b = u[v - 1];
+            count += b.count - a.count;
+            dig += b.dig - a.dig;
+        }
+        if (!count) continue;
+        M.nnz_lr[v] += (int)count;
+        M.dig_lr[v] += dig;
     }
 }
 
@@ -853,10 +907,12 @@ size_t label_smem_bytes(int32_t n, int cluster) {
     return 33 * 4 * words + 16;
 }
 
-size_t hub_scan_bytes(long long count) {
-    size_t b = 0;
-    cub::DeviceScan::InclusiveScan(nullptr, b, (const Tot*)nullptr, (Tot*)nullptr, TotSum(), (int)count);
-    return b;
+size_t hub_scan_bytes(long long tots, long long uses) {
+    size_t b = 0, c = 0;
+    cub::DeviceScan::InclusiveScan(nullptr, b, (const Tot*)nullptr, (Tot*)nullptr, TotSum(), (int)tots);
+    if (uses)
+        cub::DeviceScan::InclusiveScan(nullptr, c, (const LRowUse*)nullptr, (LRowUse*)nullptr, UseSum(), (int)uses);
+    return std::max(b, c);
 }
 
 int large_occupancy(int block, size_t smem) {
@@ -918,6 +974,12 @@ cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStr
     extra_kernel<<<(int)std::min<long long>(want, (long long)c.sm_count * (1024 / kExtraThreads)), kExtraThreads, smem, st>>>(L);
     if (c.large_block == 256) large_kernel<256><<<c.large_grid, 256, c.large_smem, st>>>(L);
     else large_kernel<1024><<<c.large_grid, 1024, c.large_smem, st>>>(L);
+    if (c.any_hub && c.l_rows) {
+        size_t sb = c.scan_bytes;
+        e = cub::DeviceScan::InclusiveScan(c.scan_tmp, sb, L.l_use, L.l_use, UseSum(), (int)(kHubs * L.total), st);
+        if (e != cudaSuccess) return e;
+        lrow_kernel<<<dim3((unsigned)std::min((c.n_max + 255) / 256, 1024), (unsigned)L.nmats), 256, 0, st>>>(L);
+    }
     commit_kernel<<<L.nmats, 32, 0, st>>>(L);
     return cudaGetLastError();
 }

@@ -178,6 +178,11 @@ struct Tot {
     unsigned long long e, dig;
 };
 
+// sources counted and the sum of their digests
+struct LRowUse {
+    unsigned long long count, dig;
+};
+
 // How a matrix's counting traversal runs.
 enum : int32_t {
     METHOD_CHAIN = 0,   // gsofa_chain.cu
@@ -199,6 +204,7 @@ struct HubLaunch {
     // zeroed before every launch, in one block: Tot base[2 * hub_bases() * total], stamp,
     // label counts, fallback, judged, counters, large_count
     void* zeroed;
+    LRowUse* l_use;                    // per hub and source (with per-row L statistics): see lrow_kernel
     Tot* base;                         // per base, direction and source: the hub set's totals
     int32_t* stamp;                    // as lam
     int32_t* lcnt;                     // 4 per label job
@@ -227,11 +233,12 @@ struct HubCfg {
     size_t scan_bytes = 0;
     int large_block = 256, large_grid = 0;
     size_t large_smem = 0;
+    bool l_rows = false;      // per-row L statistics are wanted
 };
 int hub_count();  // hubs per matrix
 int hub_bases();  // arrays of totals per direction
 size_t label_smem_bytes(int32_t n, int cluster);
-size_t hub_scan_bytes(long long count);
+size_t hub_scan_bytes(long long tots, long long uses);
 int large_occupancy(int block, size_t smem);
 cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStream_t stream);
 

@@ -75,9 +75,9 @@ def test_counts_against_the_oracle(ctx, name):  # noqa: F811
     r, rt = oracle_full(beg, end, col)
     # the default shape, one chunk per CTA and short ones, bitmaps in global memory
     for kw in (dict(), dict(chunk_sources=1000, threads_per_source=512), dict(chunk_sources=37),
-               dict(global_bitmap=True)):
+               dict(global_bitmap=True), dict(l_row_stats=True)):
         res = ctx.factor(m, **kw)
-        check_full(res, r, rt, l_rows=False)
+        check_full(res, r, rt, l_rows="l_row_stats" in kw)
         res.close()
     m.close()
 
@@ -96,8 +96,8 @@ def test_repeated_entries(ctx, n):  # noqa: F811
     col = np.concatenate(parts).astype(np.int32)
     m = ctx.load_csr(beg, end, col)
     r, rt = oracle_full(beg, end, col)
-    res = ctx.factor(m)
-    check_full(res, r, rt, l_rows=False)
+    res = ctx.factor(m, l_row_stats=True)
+    check_full(res, r, rt)
     res.close()
     m.close()
 
