@@ -65,6 +65,7 @@ struct Acc {
     unsigned long long fills, e, v, trav, nnz, chained;
 };
 
+constexpr int kPoor = 3;  // large searches a base may miss before another is looked for
 constexpr int kIdleT = 16;  // sources that do not meet T before it is dropped
 
 enum : int { PUB_X = 1, PUB_T = 2, PUB_LARGE = 4, PUB_DROP = 8 };
@@ -82,6 +83,7 @@ struct ChainSmem {
     int large[2], mode[2], found[2];
     int hits;              // of the source in hand: 1: in X0, 2: in X1
     int hub, hub_at, hub_fails, hub_wait;
+    int poor;              // large searches since the base was built that it did not keep
     int raw, orig, plen;
     Tot tot;
     Acc acc[2];
@@ -685,8 +687,8 @@ struct Large {
     }
 
     // A hub for the one-sided search of direction d: its reach set in the
-    // other direction first, in the global bitmap; too small: no base.
-    __device__ bool try_hub(int d, int s, bool digests) {
+    // other direction first, in the global bitmap; not above `least`: no base.
+    __device__ bool try_hub(int d, int s, int least, bool digests) {
         if (threadIdx.x < 32) {
             const int lane = threadIdx.x;
             const int32_t* rp = D[1 - d].G.rp;
@@ -718,7 +720,7 @@ struct Large {
             g[hub >> 5] = 1u << (hub & 31);
         }
         long long size = block_bfs<BLOCK, CG>(SM.bfs, D[o].G, g, q, qcap, 1, -1, s, false, status);
-        const bool ok = size > kListCap;
+        const bool ok = size > least;
         if (ok) {
             for (long long i = threadIdx.x; i < words; i += BLOCK) {
                 D[o].X[i] = g[i];
@@ -743,6 +745,17 @@ struct Large {
         return ok;
     }
 
+    // Failed attempts are further and further apart; one a source, so that every
+    // pass through take() makes progress.
+    __device__ void note_hub(bool ok, int s) {
+        if (threadIdx.x == 0) {
+            SM.hub_at = s;
+            SM.hub_fails = ok ? 0 : min(SM.hub_fails + 1, 6);
+            SM.hub_wait = ok ? 0 : (1 << SM.hub_fails) - 1;
+        }
+        __syncthreads();
+    }
+
     // Source SM.s, whose search in at least one direction is large.  Leaves
     // SM.s at the source to go on with.
     __device__ void take() {
@@ -754,18 +767,26 @@ struct Large {
         const bool tried = SM.hub_at == s;  // once a source: every pass through here makes progress
         __syncthreads();
         bool done = true, rebuilt = false;
+        // a base that search after search outgrows lies beside the core: a hub
+        // among what this one found takes its place if its other set is larger
+        // than the base's smaller one
+        const int miss = sym ? -1 : l0 && !(hits & 1) ? 0 : l1 && !(hits & 2) ? 1 : -1;
+        if (hits && miss >= 0 && !tried && hub_wait == 0 && SM.poor >= kPoor) {
+            const bool ok = try_hub(miss, s, max(kListCap, min(SM.base[0].v, SM.base[1].v)), digests);
+            note_hub(ok, s);
+            if (ok) {
+                rebuilt = true;
+                done = false;
+            }
+        }
         if (!hits) {
             // neither direction met the base
             bool rebuild = sym || (l0 && l1) || !have || tried;
             if (!sym && !(l0 && l1) && !tried) {
                 bool ok = false;
                 if (hub_wait == 0) {
-                    if (threadIdx.x == 0) SM.hub_at = s;
-                    ok = try_hub(l0 ? 0 : 1, s, digests);
-                    if (threadIdx.x == 0) {
-                        SM.hub_fails = ok ? 0 : min(SM.hub_fails + 1, 6);
-                        SM.hub_wait = ok ? 0 : (1 << SM.hub_fails) - 1;
-                    }
+                    ok = try_hub(l0 ? 0 : 1, s, kListCap, digests);
+                    note_hub(ok, s);
                 } else if (threadIdx.x == 0) {
                     SM.hub_wait = hub_wait - 1;
                 }
@@ -798,7 +819,13 @@ struct Large {
         }
         __syncthreads();
         if (threadIdx.x == 0) {
-            if (rebuilt) SM.have = 1;
+            if (rebuilt) {
+                SM.have = 1;
+                SM.poor = 0;
+            } else if (miss >= 0) {
+                SM.poor++;
+                if (SM.hub_wait > 0 && hits) SM.hub_wait--;
+            }
             SM.have_t = 0;
             SM.tsel = 0;
             SM.s = done ? s + 1 : s;
@@ -881,6 +908,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) chain_kernel(ChainLaunch 
             SM.have = SM.have_t = SM.tsel = 0;
             SM.hub_fails = SM.hub_wait = 0;
             SM.hub_at = -1;
+            SM.poor = 0;
             for (int d = 0; d < 2; d++) {
                 SM.used[d] = 0;
                 SM.large[d] = 0;

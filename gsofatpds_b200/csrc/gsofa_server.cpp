@@ -1,8 +1,8 @@
 // gsofa_server.cpp -- the serving request loop (continuous batching).
 //
 // One host thread per server drives:
-//   * a persistent traversal kernel (traverse_kernel, serving mode) on the
-//     kernel stream.  Its CTAs claim work items of every published request;
+//   * a persistent traversal kernel (chain_kernel; traverse_kernel for the
+//     diagnostic options and per-row L statistics) on the kernel stream.  Its CTAs claim work items of every published request;
 //     it stays on the device while published work is waiting and ends by
 //     itself when its CTAs have found nothing to claim for a short while;
 //   * a side stream for everything else: the upload and padded-CSR build of
@@ -101,6 +101,7 @@ struct gsofa_server {
     long long smem_words = 0, words = 0;
     int ring = 32;
     bool merge = true;
+    bool chain = true;  // gsofa_chain.cu serves; else traverse_kernel (diagnostics, per-row L statistics)
     cudaStream_t ks[kKernelStreams] = {};  // serving launches (low priority)
     cudaEvent_t kdone[kKernelStreams] = {};
     bool krun[kKernelStreams] = {};
@@ -193,6 +194,10 @@ size_t request_footprint(const gsofa_server* s, int32_t n, int64_t nnz) {
 // cap is no tighter because every item's first source starts cold.
 int request_chunk(const gsofa_server* s, int32_t n) {
     if (s->opts.chunk_sources > 0) return s->opts.chunk_sources;
+    if (s->chain) {
+        // about one item per CTA; an item's first source is searched from nothing
+        return (int)std::max(8ll, std::min(128ll, ((long long)n + s->grid - 1) / s->grid));
+    }
     long long cap = 512;
     while (cap > 16 && cap * (long long)std::max(n, 1) > (1ll << 28)) cap >>= 1;
     return (int)std::min<long long>(default_chunk(2ll * n, 4 * s->grid), cap);
@@ -283,7 +288,7 @@ bool admit_one(gsofa_server* s) {
         r = s->queued.front();
         if (s->in_use + r->footprint > s->budget) return false;
         chunk = request_chunk(s, r->n);
-        items = 2ll * (((long long)r->n + chunk - 1) / chunk);
+        items = (s->chain ? 1ll : 2ll) * (((long long)r->n + chunk - 1) / chunk);
         s->queued.pop_front();
         slot = s->free_slots.back();
         s->free_slots.pop_back();
@@ -394,7 +399,26 @@ bool launch_kernel(gsofa_server* s, int k, int grid) {
     V.cta_slots = s->d_cta_slots;
     V.n_cta_slots = s->grid;
     V.alive = s->d_alive;
-    cudaError_t e = launch_serve(L, s->block, grid, s->smem, s->ks[k]);
+    cudaError_t e;
+    if (s->chain) {
+        ChainLaunch C{};
+        C.work_counter = s->d_work;
+        C.queue = s->queue;
+        C.queue_stride = std::max(s->max_n, 1);
+        C.gbm = s->gbm;
+        C.gbm_count = 4;
+        C.bitmap_words = s->words;
+        C.smem_words = s->smem_words;
+        C.sides = 2;
+        C.chunk = 1;
+        C.list_cap = (int)std::min<long long>(chain_list_cap(), C.queue_stride);
+        C.sample_stride = 1;
+        C.status = s->d_status;
+        C.serve = V;
+        e = launch_chain(C, s->block, true, grid, s->smem, s->ks[k]);
+    } else {
+        e = launch_serve(L, s->block, grid, s->smem, s->ks[k]);
+    }
     if (e == cudaSuccess) e = cudaEventRecord(s->kdone[k], s->ks[k]);
     if (e != cudaSuccess) {
         server_err(s, "serving kernel launch: %s", cudaGetErrorString(e));
@@ -663,10 +687,17 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
         return set_err(ctx, GSOFA_ERR_ARG, "invalid serving options");
     if (o.flags & GSOFA_PATTERN)
         return set_err(ctx, GSOFA_ERR_UNSUPPORTED, "GSOFA_PATTERN is not served");
-    // default CTA size: the plain path's for the largest order served (the
-    // widest bitmap then fits in shared memory up to n of about 1.8M)
+    const bool chain = chain_runs(o, nullptr, 0) && !(o.flags & GSOFA_L_ROW_STATS);
+    // default CTA size of traverse_kernel: the plain path's for the largest
+    // order served (the widest bitmap then fits in shared memory up to n of
+    // about 1.8M).  The chain's throughput is its CTAs' number, whatever max_n:
+    // four of 256 threads per SM, or as many as keep one bitmap of max_n in shared
+    // memory while that takes at most 64 KB (a symmetric pattern's only one: the
+    // 64^3 mesh at max_n = 300,000 took 11.8 ms with it in global memory); wider
+    // ones are in global memory.
     const int block = o.threads_per_source > 0 ? o.threads_per_source
-                                                : std::max(256, default_block(max_n, ctx->smem_per_sm));
+                      : chain ? 256
+                              : std::max(256, default_block(max_n, ctx->smem_per_sm));
     if (block != 256 && block != 512 && block != 1024)
         return set_err(ctx, GSOFA_ERR_ARG, "serving threads_per_source must be 256, 512 or 1024");
     if (cudaSetDevice(ctx->device) != cudaSuccess) return set_err(ctx, GSOFA_ERR_CUDA, "cudaSetDevice");
@@ -678,6 +709,7 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
     s->max_n = max_n;
     s->budget = budget_bytes ? budget_bytes : kDefaultBudget;
     s->block = block;
+    s->chain = chain;
     s->merge = !(o.flags & GSOFA_NO_MERGE);
     s->ring = o.cached_closures > 0 ? std::min(o.cached_closures, kMaxRing) : kDefaultRing;
     while (s->ring & (s->ring - 1)) s->ring &= s->ring - 1;
@@ -692,20 +724,27 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
 
     // shared-memory bitmap: the widest that keeps the block's full residency
     // (none with the diagnostic GSOFA_FORCE_GLOBAL_BITMAP)
+    s->words = (((long long)max_n + 31) >> 5) + 6;
     const int occ_target = 1024 / block;
+    const size_t fixed = chain ? (chain_sparse_bytes(2) + 15) & ~(size_t)15 : 0;
+    auto occupancy = [&](size_t bytes) {
+        return chain ? chain_occupancy(block, true, fixed + bytes) : serve_occupancy(block, bytes);
+    };
     size_t smem = 0;
     if (!(o.flags & GSOFA_FORCE_GLOBAL_BITMAP)) {
         smem = (size_t)std::min(ctx->smem_optin, ctx->smem_per_sm / occ_target - 8 * 1024);
         smem &= ~(size_t)1023;
-        while (smem >= 4096 && serve_occupancy(block, smem) < occ_target) smem -= 1024;
+        while (smem >= 4096 && occupancy(smem) < occ_target) smem -= 1024;
         if (smem < 4096) smem = 0;
+        const size_t one = ((size_t)s->words * 4 + 1023) & ~(size_t)1023;
+        if (chain && one <= 64 * 1024 && smem < one && occupancy(one) > 0) smem = one;
     }
-    if (serve_occupancy(block, smem) <= 0)
+    if (chain) smem = std::min(smem, ((size_t)s->words * 8 + 1023) & ~(size_t)1023);  // both directions
+    s->occ = occupancy(smem);
+    if (s->occ <= 0)
         return fail(GSOFA_ERR_UNSUPPORTED, "serving kernel cannot be resident", cudaSuccess);
-    s->smem = smem;
+    s->smem = fixed + smem;
     s->smem_words = (long long)(smem / 4);
-    s->occ = serve_occupancy(block, smem);
-    s->words = (((long long)max_n + 31) >> 5) + 6;
     s->grid = s->occ * std::max(1, ctx->sm_count - kReserveSms);
     if (o.sources_in_flight > 0) s->grid = std::min(s->grid, o.sources_in_flight);
 
@@ -754,11 +793,11 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
 
     // device workspace: per-CTA queues, closure rings and global bitmaps
     // (only when max_n's bitmap exceeds shared memory), then the tables
-    const bool need_gbm = s->words > s->smem_words;
+    const bool need_gbm = chain || s->words > s->smem_words;
     const size_t G = (size_t)s->grid;
     const size_t qb = align256(G * (size_t)max_n * 4);
-    const size_t rb = s->merge ? align256(G * (size_t)s->ring * (size_t)s->words * 4) : 0;
-    const size_t gb = need_gbm ? align256(G * (size_t)s->words * 4) : 0;
+    const size_t rb = s->merge && !chain ? align256(G * (size_t)s->ring * (size_t)s->words * 4) : 0;
+    const size_t gb = need_gbm ? align256(G * (chain ? 4 : 1) * (size_t)s->words * 4) : 0;
     const size_t tb = align256(sizeof(MatDesc) * kSlots) + align256(8 * kSlots) * 2 +
                       align256(4 * kSlots) + 256 + align256(4 * (size_t)((s->grid + 31) / 32)) +
                       align256(kCtlBytes);
@@ -778,7 +817,7 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
     char* b = static_cast<char*>(s->ws);
     s->queue = reinterpret_cast<int32_t*>(b);
     b += qb;
-    s->rings = s->merge ? reinterpret_cast<uint32_t*>(b) : nullptr;
+    s->rings = rb ? reinterpret_cast<uint32_t*>(b) : nullptr;
     b += rb;
     s->gbm = need_gbm ? reinterpret_cast<uint32_t*>(b) : nullptr;
     b += gb;
