@@ -75,6 +75,7 @@ struct Graph {
     const int32_t* col;
     const int32_t* trp;
     const int32_t* tcol;
+    int sides;  // 1: the pattern is symmetric, A^T's rows repeat A's
 };
 
 int grid_for(long long items, int threads) {
@@ -144,7 +145,7 @@ __global__ void cc_hook_kernel(Graph g, int32_t n, const int32_t* __restrict__ p
         const int v = (int)vv;
         const int p = __ldg(part + v);
         if (p < 0) continue;
-        for (int side = 0; side < 2; side++) {
+        for (int side = 0; side < g.sides; side++) {
             const int32_t* rp = side ? g.trp : g.rp;
             const int32_t* cl = side ? g.tcol : g.col;
             const int b = __ldg(rp + v) & ~3, e = __ldg(rp + v + 1) & ~3;
@@ -321,7 +322,7 @@ __global__ void __launch_bounds__(kBfsThreads) bfs_kernel(BfsArgs a) {
             const int u = __ldcg(qin + i);
             const int p = __ldg(a.part + u);
             int found = 0;
-            for (int side = 0; side < 2; side++) {
+            for (int side = 0; side < a.g.sides; side++) {
                 const int32_t* rp = side ? a.g.trp : a.g.rp;
                 const int32_t* cl = side ? a.g.tcol : a.g.col;
                 const int b = __ldg(rp + u) & ~3, e = __ldg(rp + u + 1) & ~3;
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(kLocalThreads) bfs_local_kernel(
         for (int L = 0; lb < le; L++) {
             for (int i = lb + warp; i < le; i += NW) {
                 const int u = q[base + i];
-                for (int side = 0; side < 2; side++) {
+                for (int side = 0; side < g.sides; side++) {
                     const int32_t* rp = side ? g.trp : g.rp;
                     const int32_t* cl = side ? g.tcol : g.col;
                     const int b = __ldg(rp + u) & ~3, e = __ldg(rp + u + 1) & ~3;
@@ -500,7 +501,7 @@ __global__ void separator_kernel(Graph g, int32_t n, const int32_t* __restrict__
         const int m = pm[k];
         if (dist[v] != m) continue;
         bool any = false;
-        for (int side = 0; side < 2 && !any; side++) {
+        for (int side = 0; side < g.sides && !any; side++) {
             const int32_t* rp = side ? g.trp : g.rp;
             const int32_t* cl = side ? g.tcol : g.col;
             const int b = __ldg(rp + v) & ~3, e = __ldg(rp + v + 1) & ~3;
@@ -705,14 +706,17 @@ int order_impl(gsofa_ctx* ctx, const gsofa_matrix* mat, int32_t leaf, int32_t ma
         pml = i32(N);
         if (!mside || !msep || !pns || !pna || !pnb || !pml)
             return set_err(ctx, GSOFA_ERR_OOM_BUDGET, "ordering workspace exceeds the budget");
-        int rc = sym_graph_build(ctx, S, n, mat->rowptr, mat->col, mat->trowptr, mat->tcol, &Hg);
+        chunk_weight(ctx, mat);
+        int rc = sym_graph_build(ctx, S, n, mat->rowptr, mat->col, mat->trowptr, mat->tcol,
+                                 mat->host_sym > 0, &Hg);
         if (rc) return rc;
     }
     int32_t* nroots = small;
     unsigned* bar = reinterpret_cast<unsigned*>(small + 8);
     int32_t* err = small + 10;
     unsigned long long* tot = reinterpret_cast<unsigned long long*>(small + 16);
-    Graph g{mat->rowptr, mat->col, mat->trowptr, mat->tcol};
+    chunk_weight(ctx, mat);  // reads the symmetry word back, once per matrix
+    Graph g{mat->rowptr, mat->col, mat->trowptr, mat->tcol, mat->host_sym > 0 ? 1 : 2};
 
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bfs_kernel, kBfsThreads, 0) !=
@@ -949,6 +953,7 @@ extern "C" int gsofa_matrix_permute(gsofa_ctx* ctx, const gsofa_matrix* mat, con
         matrix_free_on(m, st);
         return rc;
     }
+    m->host_sym = mat->host_sym;
     *out = m;
     return GSOFA_OK;
 }
@@ -983,7 +988,7 @@ extern "C" int gsofa_order_wait_selftest(gsofa_ctx* ctx, double limit_ms) {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bfs_kernel, kBfsThreads, 0);
     if (e != cudaSuccess || occ <= 0) return set_err(ctx, GSOFA_ERR_CUDA, "self-test setup");
     const int grid = ctx->sm_count * std::min(occ, kBfsBlocksPerSm);
-    Graph g{rp, col, rp, col};
+    Graph g{rp, col, rp, col, 2};
     BfsArgs a{g, part, plo, dist, q0, q1, lcnt, H, bar, err, 3, (unsigned)grid + 1u,
               (unsigned long long)(limit_ms * 1e6)};
     void* args[] = {&a};

@@ -36,19 +36,19 @@
 // level-0 index space (a part's vertices in increasing id); every level keeps
 // that layout for the parts still present, so a part is a contiguous range
 // and per-part work is a segmented scan, sort or reduction:
-//   matching     one thread per vertex per proposal round;
+//   matching     a lane per vertex per proposal round, a warp per long row;
 //   coarse ids   an exclusive scan of the "pair's smaller member" flags;
 //   contraction  64-bit (coarse u, coarse w) keys radix-sorted with their
 //                weights and reduced by key: the coarse CSR, rows sorted;
-//   BFS order    parts of up to 256 vertices: one thread each, a plain
+//   BFS order    parts of up to 256 vertices: one warp each, a plain
 //                sequential BFS; larger parts: one CTA each, level by level
 //                with block barriers, each new vertex appended by its first
 //                parent in queue order (the smallest queue position among its
 //                frontier neighbours) at an offset from a block scan, in
 //                adjacency order: exactly the queue order of a sequential BFS
 //                that visits neighbours in id order;
-//   refinement   gains and candidates one thread per vertex; candidates
-//                compacted in increasing id; then one thread per part
+//   refinement   gains and candidates a lane per vertex, a warp per long row;
+//                candidates compacted in increasing id; then one warp per part
 //                accepts them in order against the balance bounds (the one
 //                sequential step; a pass has few candidates).
 #include <cub/block/block_scan.cuh>
@@ -75,8 +75,8 @@ constexpr int32_t kCoarsenMin = 200;   // graphs of at most this many vertices a
 constexpr int kMatchRounds = 3;
 constexpr int kRefinePasses = 10;
 constexpr unsigned long long kNoKey = ~0ull;
-// parts of at most this many vertices are searched by one thread each (a
-// plain sequential BFS, all such parts at once); larger ones by one CTA each
+// parts of at most this many vertices are searched by one warp each (a plain
+// sequential BFS, all such parts at once); larger ones by one CTA each
 constexpr int32_t kSeqBfsMax = 256;
 constexpr int kCtaBfsThreads = 1024;
 
@@ -89,17 +89,57 @@ int blocks_for(long long items) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (count); \
          i += (long long)gridDim.x * blockDim.x)
 
+// Rows of a graph, 32 vertices per warp: each lane walks its own row when that
+// has at most kLaneRow entries, and the warp walks the longer ones together
+// (a contracted graph's hubs have thousands: with one thread per row the
+// proposals took 30 ms of a 100,000-row circuit-like ordering, now 1.9).
+// take(x): whether row x is walked; entry(x, j, acc) folds entry j of row x;
+// merge(a, b) joins two partial results; done(x, acc) gets the whole row's.
+constexpr int kLaneRow = 24;
+
+template <class T, class Take, class Entry, class Merge, class Done>
+__device__ __forceinline__ void over_rows(long long V, const int32_t* __restrict__ xadj, T zero, Take take,
+                                          Entry entry, Merge merge, Done done) {
+    const int lane = threadIdx.x & 31;
+    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long base = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5 << 5; base < V; base += nw * 32) {
+        const long long x = base + lane;
+        const bool mine = x < V && take(x);
+        int b = 0, e = 0;
+        if (mine) {
+            b = xadj[x];
+            e = xadj[x + 1];
+        }
+        unsigned lng = __ballot_sync(0xffffffffu, e - b > kLaneRow);
+        if (mine && e - b <= kLaneRow) {
+            T acc = zero;
+            for (int j = b; j < e; j++) entry(x, j, acc);
+            done(x, acc);
+        }
+        while (lng) {
+            const int l = __ffs(lng) - 1;
+            lng &= lng - 1;
+            const int rb = __shfl_sync(0xffffffffu, b, l), re = __shfl_sync(0xffffffffu, e, l);
+            T acc = zero;
+            for (int j = rb + lane; j < re; j += 32) entry(base + l, j, acc);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc = merge(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+            if (lane == l) done(base + l, acc);
+        }
+    }
+}
+
 // ---- A + A^T: distinct sorted neighbours, no self loops -------------------------
 
 // keys (v << 32 | w) for the entries of row v of A and of A^T, w != v;
 // padding (which repeats v) and loops become kNoKey
 __global__ void sym_keys_kernel(int32_t n, const int32_t* __restrict__ rp,
                                 const int32_t* __restrict__ col, const int32_t* __restrict__ trp,
-                                const int32_t* __restrict__ tcol, long long tbase,
+                                const int32_t* __restrict__ tcol, int sides, long long tbase,
                                 unsigned long long* __restrict__ keys) {
     GRID_LOOP(vv, n) {
         const int v = (int)vv;
-        for (int side = 0; side < 2; side++) {
+        for (int side = 0; side < sides; side++) {
             const int32_t* r = side ? trp : rp;
             const int32_t* c = side ? tcol : col;
             const long long off = side ? tbase : 0;
@@ -187,21 +227,22 @@ __global__ void propose_kernel(long long V, const int32_t* __restrict__ xadj,
                                const int32_t* __restrict__ adj, const int32_t* __restrict__ ew,
                                const int32_t* __restrict__ vpart, const int32_t* __restrict__ pn,
                                const int32_t* __restrict__ match, int32_t* __restrict__ prop) {
-    GRID_LOOP(x, V) {
-        int best = -1, bw = -1;
-        if (match[x] < 0 && pn[vpart[x]] > kCoarsenMin) {
-            for (int j = xadj[x]; j < xadj[x + 1]; j++) {
-                const int y = adj[j];
-                if (match[y] >= 0) continue;
-                const int w = ew[j];
-                if (w > bw || (w == bw && y > best)) {
-                    bw = w;
-                    best = y;
-                }
-            }
-        }
-        prop[x] = best;
-    }
+    // (edge weight, id) as one key: weights are at least 1, so 0 is none
+    over_rows(
+        V, xadj, 0ull,
+        [&](long long x) {
+            if (match[x] < 0 && pn[vpart[x]] > kCoarsenMin) return true;
+            prop[x] = -1;
+            return false;
+        },
+        [&](long long, int j, unsigned long long& best) {
+            const int y = adj[j];
+            if (match[y] >= 0) return;
+            const unsigned long long key = (unsigned long long)(uint32_t)ew[j] << 32 | (uint32_t)y;
+            if (key > best) best = key;
+        },
+        [](unsigned long long a, unsigned long long c) { return a > c ? a : c; },
+        [&](long long x, unsigned long long best) { prop[x] = best ? (int32_t)(uint32_t)best : -1; });
 }
 
 __global__ void resolve_kernel(long long V, const int32_t* __restrict__ prop, int32_t* match) {
@@ -269,9 +310,10 @@ __global__ void coarse_keys_kernel(long long V, const int32_t* __restrict__ xadj
                                    const int32_t* __restrict__ adj, const int32_t* __restrict__ ew,
                                    const int32_t* __restrict__ cmap,
                                    unsigned long long* __restrict__ keys, int32_t* __restrict__ vals) {
-    GRID_LOOP(x, V) {
-        const int cx = cmap[x];
-        for (int j = xadj[x]; j < xadj[x + 1]; j++) {
+    over_rows(
+        V, xadj, 0, [](long long) { return true; },
+        [&](long long x, int j, int&) {
+            const int cx = cmap[x];
             const int cy = cx >= 0 ? cmap[adj[j]] : cx;
             if (cx < 0 || cy == cx) {
                 keys[j] = kNoKey;
@@ -280,8 +322,8 @@ __global__ void coarse_keys_kernel(long long V, const int32_t* __restrict__ xadj
                 keys[j] = ((unsigned long long)(uint32_t)cx << 32) | (uint32_t)cy;
                 vals[j] = ew[j];
             }
-        }
-    }
+        },
+        [](int a, int) { return a; }, [](long long, int) {});
 }
 
 __global__ void coarse_rows_kernel(long long m, const unsigned long long* __restrict__ ukeys,
@@ -295,31 +337,70 @@ __global__ void coarse_rows_kernel(long long m, const unsigned long long* __rest
 
 // ---- breadth-first search in exact queue order ---------------------------------
 
-// one thread per part: the sequential BFS from start[k], its queue in qord
-__global__ void seq_bfs_kernel(int R, const int32_t* __restrict__ on,
-                               const int32_t* __restrict__ start, const int32_t* __restrict__ pb,
-                               const int32_t* __restrict__ pn, const int32_t* __restrict__ xadj,
-                               const int32_t* __restrict__ adj, int32_t* __restrict__ lev,
-                               int32_t* __restrict__ qord, int32_t* __restrict__ cnt) {
-    GRID_LOOP(k, R) {
+// One warp per part of at most kSeqBfsMax vertices: the sequential BFS from
+// start[k], its queue in qord.  The queue and the marks are in shared memory; a
+// vertex's neighbours are read by the lanes together and appended in adjacency
+// order (a ballot's prefix counts), the next vertex's row a step ahead.  (One
+// thread per part, everything in global memory: 23 ms of a 100,000-row
+// circuit-like ordering.)
+constexpr int kSeqWarps = 8;
+__global__ void __launch_bounds__(32 * kSeqWarps) seq_bfs_kernel(
+    int R, const int32_t* __restrict__ on, const int32_t* __restrict__ start,
+    const int32_t* __restrict__ pb, const int32_t* __restrict__ pn, const int32_t* __restrict__ xadj,
+    const int32_t* __restrict__ adj, int32_t* __restrict__ qord, int32_t* __restrict__ cnt) {
+    __shared__ int16_t queue[kSeqWarps][kSeqBfsMax];
+    __shared__ unsigned seen[kSeqWarps][kSeqBfsMax / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int16_t* const q = queue[warp];
+    unsigned* const mark = seen[warp];
+    for (int k = blockIdx.x * kSeqWarps + warp; k < R; k += gridDim.x * kSeqWarps) {
         if (!on[k]) continue;
         const int base = pb[k], size = pn[k];
-        for (int i = base; i < base + size; i++) lev[i] = -1;
-        const int s = start[k];
-        qord[base] = s;
-        lev[s] = 0;
-        int h = 0, t = 1;
-        while (h < t) {
-            const int u = qord[base + h++];
-            for (int j = xadj[u]; j < xadj[u + 1]; j++) {
-                const int y = adj[j];
-                if (lev[y] == -1 && t < size) {
-                    lev[y] = 0;
-                    qord[base + t++] = y;
-                }
+        for (int i = lane; i < kSeqBfsMax / 32; i += 32) mark[i] = 0u;
+        __syncwarp();
+        const int s = start[k] - base;
+        if (lane == 0) {
+            q[0] = (int16_t)s;
+            mark[s >> 5] = 1u << (s & 31);
+        }
+        __syncwarp();
+        int t = 1, ready = -1;  // ready: the queue position whose row has been requested
+        int nb = 0, ne = 0, ny = -1;
+        for (int h = 0; h < t; h++) {
+            int b, e, y;
+            if (ready == h) {
+                b = nb;
+                e = ne;
+                y = ny;
+            } else {
+                const int u = base + q[h];
+                b = xadj[u];
+                e = xadj[u + 1];
+                y = b + lane < e ? adj[b + lane] - base : -1;
+            }
+            if (h + 1 < t) {
+                const int u = base + q[h + 1];
+                nb = xadj[u];
+                ne = xadj[u + 1];
+                ny = nb + lane < ne ? adj[nb + lane] - base : -1;
+                ready = h + 1;
+            }
+            for (int j = b; j < e; j += 32) {
+                if (j > b) y = j + lane < e ? adj[j + lane] - base : -1;
+                // a row's ids are distinct, so no two lanes mark the same one
+                const bool fresh = y >= 0 && !((mark[y >> 5] >> (y & 31)) & 1u);
+                const unsigned m = __ballot_sync(0xffffffffu, fresh);
+                if (!m) continue;
+                const int at = t + __popc(m & ((1u << lane) - 1u));
+                if (fresh && at < size) q[at] = (int16_t)y;
+                if (fresh) atomicOr(mark + (y >> 5), 1u << (y & 31));
+                t = min(t + __popc(m), size);
+                __syncwarp();
             }
         }
-        cnt[k] = t;
+        for (int i = lane; i < t; i += 32) qord[base + i] = base + q[i];
+        if (lane == 0) cnt[k] = t;
+        __syncwarp();
     }
 }
 
@@ -466,62 +547,76 @@ __global__ void gain_kernel(long long V, const int32_t* __restrict__ xadj,
                             const int32_t* __restrict__ adj, const int32_t* __restrict__ ew,
                             const int32_t* __restrict__ vpart, const int32_t* __restrict__ done,
                             const int32_t* __restrict__ side, int32_t* __restrict__ gain) {
-    GRID_LOOP(x, V) {
-        if (done[vpart[x]]) continue;
-        const int s = side[x];
-        int g = 0;
-        for (int j = xadj[x]; j < xadj[x + 1]; j++) g += side[adj[j]] != s ? ew[j] : -ew[j];
-        gain[x] = g;
-    }
+    over_rows(
+        V, xadj, 0, [&](long long x) { return !done[vpart[x]]; },
+        [&](long long x, int j, int& g) { g += side[adj[j]] != side[x] ? ew[j] : -ew[j]; },
+        [](int a, int c) { return a + c; }, [&](long long x, int g) { gain[x] = g; });
 }
 
 __global__ void cand_kernel(long long V, const int32_t* __restrict__ xadj,
                             const int32_t* __restrict__ adj, const int32_t* __restrict__ vpart,
                             const int32_t* __restrict__ done, const int32_t* __restrict__ gain,
                             int32_t* __restrict__ cand, int32_t* __restrict__ ccount) {
-    GRID_LOOP(x, V) {
-        const int k = vpart[x];
-        int c = 0;
-        if (!done[k]) {
-            const int g = gain[x];
-            if (g > 0) {
-                c = 1;
-                for (int j = xadj[x]; j < xadj[x + 1] && c; j++) {
-                    const int y = adj[j];
-                    const int gy = gain[y];
-                    if (gy > g || (gy == g && y < x)) c = 0;
-                }
-            }
-        }
-        cand[x] = c;
-        if (c) atomicAdd(ccount + k, 1);
-    }
+    over_rows(
+        V, xadj, 0,
+        [&](long long x) {
+            if (!done[vpart[x]] && gain[x] > 0) return true;
+            cand[x] = 0;
+            return false;
+        },
+        [&](long long x, int j, int& beaten) {
+            const int g = gain[x], y = adj[j];
+            const int gy = gain[y];
+            if (gy > g || (gy == g && y < x)) beaten = 1;
+        },
+        [](int a, int c) { return a | c; },
+        [&](long long x, int beaten) {
+            cand[x] = !beaten;
+            if (!beaten) atomicAdd(ccount + vpart[x], 1);
+        });
 }
 
-// one thread per part: its candidates in increasing id, each moved when
-// side 0's weight stays within 40..60 % of the total
+// One warp per part: its candidates in increasing id, each moved when side 0's
+// weight stays within 40..60 % of the total.  The lanes load 32 candidates
+// together; the decisions, a chain through side 0's weight, run on broadcasts.
+// (One thread per part waited for three loads per candidate: 18 ms of a
+// 100,000-row circuit-like ordering.)
 __global__ void accept_kernel(int R, const int32_t* __restrict__ cstart,
                               const int32_t* __restrict__ ccount, const int32_t* __restrict__ clist,
                               const int32_t* __restrict__ vw, const long long* __restrict__ ptotal,
                               long long* __restrict__ pw0, int32_t* __restrict__ side,
                               int32_t* __restrict__ done, int32_t* any_moved) {
-    GRID_LOOP(k, R) {
+    const int lane = threadIdx.x & 31;
+    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long k = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < R; k += nw) {
         if (done[k]) continue;
         const long long total = ptotal[k];
+        const long long low = total * 40, high = total * 60;
         long long w0 = pw0[k];
         int moved = 0;
         const int b = cstart[k], e = b + ccount[k];
-        for (int i = b; i < e; i++) {
-            const int x = clist[i];
-            const long long nw0 = side[x] ? w0 + vw[x] : w0 - vw[x];
-            if (nw0 * 100 < total * 40 || nw0 * 100 > total * 60) continue;
-            side[x] ^= 1;
-            w0 = nw0;
-            moved++;
+        for (int i0 = b; i0 < e; i0 += 32) {
+            const int x = i0 + lane < e ? clist[i0 + lane] : -1;
+            int step = 0, s = 0;
+            if (x >= 0) {
+                s = side[x];
+                step = s ? vw[x] : -vw[x];
+            }
+            bool go = false;
+            for (int i = 0; i < min(32, e - i0); i++) {
+                const long long nw0 = w0 + __shfl_sync(0xffffffffu, step, i);
+                if (nw0 * 100 < low || nw0 * 100 > high) continue;
+                w0 = nw0;
+                moved++;
+                if (lane == i) go = true;
+            }
+            if (go) side[x] = s ^ 1;
         }
-        pw0[k] = w0;
-        if (!moved) done[k] = 1;
-        else *any_moved = 1;
+        if (lane == 0) {
+            pw0[k] = w0;
+            if (!moved) done[k] = 1;
+            else *any_moved = 1;
+        }
     }
 }
 
@@ -539,13 +634,14 @@ __global__ void boundary_kernel(long long V, const int32_t* __restrict__ xadj,
                                 const int32_t* __restrict__ adj, const int32_t* __restrict__ vpart,
                                 const int32_t* __restrict__ side, int32_t* __restrict__ isb,
                                 int32_t* __restrict__ bnd) {
-    GRID_LOOP(x, V) {
-        const int s = side[x];
-        int b = 0;
-        for (int j = xadj[x]; j < xadj[x + 1] && !b; j++) b = side[adj[j]] != s;
-        isb[x] = b;
-        if (b) atomicAdd(bnd + 2 * vpart[x] + s, 1);
-    }
+    over_rows(
+        V, xadj, 0, [](long long) { return true; },
+        [&](long long x, int j, int& other) { other |= side[adj[j]] != side[x]; },
+        [](int a, int c) { return a | c; },
+        [&](long long x, int other) {
+            isb[x] = other;
+            if (other) atomicAdd(bnd + 2 * vpart[x] + side[x], 1);
+        });
 }
 
 __global__ void ml_result_kernel(long long V, const int32_t* __restrict__ xid,
@@ -611,14 +707,16 @@ namespace gsofa {
 namespace host {
 
 int sym_graph_build(gsofa_ctx* ctx, DeviceScratch& S, int32_t n, const int32_t* rp,
-                    const int32_t* col, const int32_t* trp, const int32_t* tcol, SymGraph* out) {
+                    const int32_t* col, const int32_t* trp, const int32_t* tcol, bool symmetric,
+                    SymGraph* out) {
     cudaStream_t st = ctx->stream;
     int32_t h[2] = {0, 0};
     if (cudaMemcpyAsync(&h[0], rp + n, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaMemcpyAsync(&h[1], trp + n, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
         return set_err(ctx, GSOFA_ERR_CUDA, "hybrid ordering: row pointer read-back");
-    const long long pa = h[0] & ~3, pt = h[1] & ~3, m = pa + pt;
+    // a symmetric pattern: A^T adds nothing
+    const long long pa = h[0] & ~3, pt = symmetric ? 0 : h[1] & ~3, m = pa + pt;
     auto* keys = static_cast<unsigned long long*>(S.get(8 * (size_t)std::max(m, 1ll)));
     auto* sorted = static_cast<unsigned long long*>(S.get(8 * (size_t)std::max(m, 1ll)));
     auto* flag = static_cast<int32_t*>(S.get(4 * (size_t)std::max(m, 1ll)));
@@ -631,7 +729,7 @@ int sym_graph_build(gsofa_ctx* ctx, DeviceScratch& S, int32_t n, const int32_t* 
     cub::DeviceRadixSort::SortKeys(nullptr, b1, keys, sorted, (int)m, 0, 64, st);
     cub::DeviceScan::ExclusiveSum(nullptr, b2, flag, fpos, (int)m, st);
     if (!T.need(std::max(b1, b2))) return fail(ctx, "sort storage");
-    sym_keys_kernel<<<blocks_for(n), kT, 0, st>>>(n, rp, col, trp, tcol, pa, keys);
+    sym_keys_kernel<<<blocks_for(n), kT, 0, st>>>(n, rp, col, trp, tcol, symmetric ? 1 : 2, pa, keys);
     size_t tb = T.bytes;
     cub::DeviceRadixSort::SortKeys(T.p, tb, keys, sorted, (int)m, 0, 64, st);
     cudaMemsetAsync(hdeg, 0, 4 * ((size_t)n + 1), st);
@@ -868,11 +966,11 @@ int ml_round(gsofa_ctx* ctx, const SymGraph& H, int32_t n, const int32_t* part, 
     if (int rc = sync("hybrid ordering: coarsest levels")) return rc;
 
     // one exact-order search of the parts flagged in `on` at level c, from
-    // start[]: the small ones (on_small) one thread each, the others (on_big)
+    // start[]: the small ones (on_small) one warp each, the others (on_big)
     // one CTA each
     auto bfs = [&](Level& c, int nbig) -> int {
-        seq_bfs_kernel<<<blocks_for(R), kT, 0, st>>>(R, on_small, start, c.pb, c.pn, c.xadj, c.adj,
-                                                     lev, qord, bcnt);
+        seq_bfs_kernel<<<std::min((R + kSeqWarps - 1) / kSeqWarps, ctx->sm_count * 8), 32 * kSeqWarps, 0, st>>>(
+            R, on_small, start, c.pb, c.pn, c.xadj, c.adj, qord, bcnt);
         if (nbig > 0)
             cta_bfs_kernel<<<std::min(nbig, 2 * ctx->sm_count), kCtaBfsThreads, 0, st>>>(
                 R, on_big, start, c.pb, c.pn, c.xadj, c.adj, lev, par, qord, bcnt);
@@ -944,7 +1042,7 @@ int ml_round(gsofa_ctx* ctx, const SymGraph& H, int32_t n, const int32_t* part, 
             // parts that moved nothing are done and skip later passes; the
             // host looks every other pass whether any part is left
             if (pass % 2 == 0) cudaMemsetAsync(err + 1, 0, 4, st);
-            accept_kernel<<<blocks_for(R), kT, 0, st>>>(R, cstart, ccount, clist, c.vw, ptotal, pw0,
+            accept_kernel<<<blocks_for(32ll * R), kT, 0, st>>>(R, cstart, ccount, clist, c.vw, ptotal, pw0,
                                                         c.side, done, err + 1);
             if (pass % 2 == 1) {
                 int32_t moved = 0;

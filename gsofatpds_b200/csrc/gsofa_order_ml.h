@@ -21,7 +21,8 @@ struct SymGraph {
 // Builds the structure of A + A^T from the padded CSR of A (rp, col) and of
 // A^T (trp, tcol) into memory held by S.  Synchronous on ctx->stream.
 int sym_graph_build(gsofa_ctx* ctx, DeviceScratch& S, int32_t n, const int32_t* rp,
-                    const int32_t* col, const int32_t* trp, const int32_t* tcol, SymGraph* out);
+                    const int32_t* col, const int32_t* trp, const int32_t* tcol, bool symmetric,
+                    SymGraph* out);
 
 // The multilevel bisection of every part of one round: part[v] (device, n
 // entries) is v's part in [0, R) or -1; parts with psize[k] > leaf (device,
