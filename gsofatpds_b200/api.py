@@ -394,7 +394,7 @@ class Result:
         cnt = ctypes.c_int64()
         self.ctx._check(self.ctx._L.gsofa_result_supernodes(self._h, _ptr(flags), None, 0,
                                                             ctypes.byref(cnt)), "supernodes")
-        return flags, np.nonzero(flags)[0].astype(np.int32)
+        return flags, np.flatnonzero(flags != 0).astype(np.int32)
 
     def lmask(self):
         """(n, 4) uint32: bit j of column f's mask is L(f+1+j, f) != 0."""

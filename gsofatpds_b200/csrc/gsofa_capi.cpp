@@ -348,14 +348,14 @@ bool chain_runs(const gsofa_opts& o, const gsofa_matrix* const* mats, int32_t co
     return true;
 }
 
-int plan_chain(gsofa_ctx* ctx, int32_t nmax, bool all_sym, const gsofa_opts* o, bool serve,
-               ChainCfg* c) {
+int plan_chain(gsofa_ctx* ctx, int32_t nmax, long long total_sources, bool all_sym, const gsofa_opts* o,
+               bool serve, ChainCfg* c) {
     c->words = bitmap_words(nmax);
     const long long need = (all_sym ? 1 : 2) * c->words;  // X of each direction
     c->sides = all_sym ? 1 : 2;
     const size_t fixed = (chain_sparse_bytes(c->sides) + 15) & ~(size_t)15;
     size_t bytes = ((size_t)need * 4 + 15) & ~(size_t)15;
-    if (fixed + bytes + 4096 > (size_t)ctx->smem_optin || (o->flags & GSOFA_FORCE_GLOBAL_BITMAP))
+    if (fixed + bytes + 20 * 1024 > (size_t)ctx->smem_optin || (o->flags & GSOFA_FORCE_GLOBAL_BITMAP))
         bytes = 0;
     c->smem_words = bytes ? need : 0;
     c->gbm_count = bytes ? 2 : 4;
@@ -363,7 +363,12 @@ int plan_chain(gsofa_ctx* ctx, int32_t nmax, bool all_sym, const gsofa_opts* o, 
     c->block = o->threads_per_source;
     if (c->block <= 0) {
         const long long fit = ctx->smem_per_sm / (long long)(c->smem + 2048);
-        c->block = fit >= 4 ? 256 : fit >= 2 ? 512 : 1024;
+        // Many small matrices: more chunks at a time (a batch of 64: 5.0 -> 3.9 ms
+        // with 128 threads against 256).  A few: their chunks' first searches
+        // are the longest chain, shorter with more threads (170 x 170 mesh:
+        // 0.97 against 0.82 ms).
+        c->block = fit >= 8 && total_sources >= 8ll * nmax ? 128 : fit >= 4 ? 256 : fit >= 2 ? 512 : 1024;
+
     }
     if (c->block != 128 && c->block != 256 && c->block != 512 && c->block != 1024)
         return set_err(ctx, GSOFA_ERR_ARG, "threads_per_source must be 128, 256, 512 or 1024");
@@ -483,7 +488,52 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     return true;
 }
 
-long long chain_chunk(const gsofa_opts& o, long long total_sources, int grid, bool sym) {
+// The last separators of a mesh in nested-dissection order reach almost
+// everything: their chunks' first searches, from nothing, take as long as all
+// the rest of the launch (500 x 500 mesh: 4.0 of 4.6 ms by 256 threads).  From
+// 131,072 rows on, the chunks of the last 2 % of them go to CTAs of 1,024 threads,
+// at most one per SM, beside the rest (3.55 ms; the 64^3 mesh 3.3 either way).
+// Smaller meshes lose more by the SMs those CTAs take (170 x 170: 0.82 -> 1.0 ms,
+// a batch of 64 matrices 5.9 -> 7.2).
+long long chain_top_items(const gsofa_opts& o, int32_t n, long long chunk, bool sym) {
+    if (!sym || o.threads_per_source > 0 || o.sources_in_flight > 0 || n < 131072) return 0;
+    const long long chunks = (n + chunk - 1) / chunk;
+    return std::min(chunks - 1, (n / 50 + chunk - 1) / chunk);
+}
+
+constexpr int kTopBlock = 1024;
+
+size_t chain_queue_bytes(const gsofa_ctx* ctx, const ChainCfg& c, int32_t nmax, bool top) {
+    return ((size_t)c.grid + (top ? (size_t)ctx->sm_count : 0)) * (size_t)std::max(nmax, 1) * 4;
+}
+
+size_t chain_gbm_bytes(const gsofa_ctx* ctx, const ChainCfg& c, bool top) {
+    return ((size_t)c.grid + (top ? (size_t)ctx->sm_count : 0)) * (size_t)c.gbm_count * (size_t)c.words * 4;
+}
+
+cudaError_t launch_chain_both(gsofa_ctx* ctx, const ChainLaunch& L, const ChainCfg& c, long long top_items) {
+    cudaError_t e = cudaSuccess;
+    if (top_items > 0) {
+        ChainLaunch T = L;
+        T.items = ITEMS_TOP;
+        T.total_items = top_items;
+        T.sample_stride = 1;
+        T.work_counter = L.work_counter + 1;
+        T.queue = L.queue + (size_t)c.grid * (size_t)L.queue_stride;
+        T.gbm = L.gbm + (size_t)c.grid * (size_t)c.gbm_count * (size_t)c.words;
+        e = cudaEventRecord(ctx->fork, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->side_stream, ctx->fork, 0);
+        if (e == cudaSuccess)
+            e = launch_chain(T, kTopBlock, false, (int)std::min<long long>(top_items, ctx->sm_count), c.smem,
+                             ctx->side_stream);
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->join, ctx->side_stream);
+    }
+    if (e == cudaSuccess && L.total_items > 0) e = launch_chain(L, c.block, false, c.grid, c.smem, ctx->stream);
+    if (e == cudaSuccess && top_items > 0) e = cudaStreamWaitEvent(ctx->stream, ctx->join, 0);
+    return e;
+}
+
+long long chain_chunk(const gsofa_opts& o, long long total_sources, int32_t nmax, int grid, bool sym) {
     if (o.chunk_sources > 0) return o.chunk_sources;
     // A chunk's first source is searched from nothing.  Symmetric patterns:
     // about two items per CTA, at most 128 sources each, since their items
@@ -492,7 +542,9 @@ long long chain_chunk(const gsofa_opts& o, long long total_sources, int grid, bo
     // hub lies in, and such first searches may read most of the matrix: one
     // item per CTA.
     if (!sym) return std::max(1ll, (total_sources + grid - 1) / grid);
-    return std::max(1ll, std::min(128ll, (total_sources + 2ll * grid - 1) / (2ll * grid)));
+    // (64 where no matrix has the 1,024-thread launch: a batch's meshes of up to
+    // 30,000 rows 5.9 -> 5.3 ms)
+    return std::max(1ll, std::min(nmax < 131072 ? 64ll : 128ll, (total_sources + 2ll * grid - 1) / (2ll * grid)));
 }
 
 // Runs the traversal (and optionally supernodes / pattern) for `count`
@@ -534,6 +586,7 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
     HubLaunch HL{};
     HubCfg hcfg;
     bool hub = false;
+    long long top_items = 0;
     if (chain) {
         long long chain_sources = 0;
         bool chain_sym = true;
@@ -547,9 +600,9 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
             chain_sources = total_sources;
             chain_sym = all_sym;
         }
-        rc = plan_chain(ctx, std::max(nmax, 1), chain_sym, o, false, &ccfg);
+        rc = plan_chain(ctx, std::max(nmax, 1), chain_sources, chain_sym, o, false, &ccfg);
         if (rc) return rc;
-        CL.chunk = (int)chain_chunk(*o, chain_sources, ccfg.grid, chain_sym);
+        CL.chunk = (int)chain_chunk(*o, chain_sources, nmax, ccfg.grid, chain_sym);
         long long items = 0;
         place(CL.chunk, 1);
         for (int32_t k = 0; k < count; k++) {
@@ -557,7 +610,11 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
             MatDesc& d = descs[(size_t)k];
             d.method = method_of(m);
             d.item_base = items;
-            if (d.method == METHOD_CHAIN) items += (m->n + CL.chunk - 1) / CL.chunk;
+            d.top_base = top_items;
+            if (d.method != METHOD_CHAIN) continue;
+            d.top_items = stride > 1 ? 0 : chain_top_items(*o, m->n, CL.chunk, m->host_sym > 0);
+            top_items += d.top_items;
+            items += (m->n + CL.chunk - 1) / CL.chunk - d.top_items;
         }
         size_t hub_bytes = 0;
         if (plan_hub(ctx, &descs, *o, nullptr, &hub_bytes, &HL, &hcfg)) {
@@ -567,10 +624,9 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
             HL.status = dstatus;
         }
         ccfg.grid = (int)std::max(1ll, std::min<long long>(ccfg.grid, items));
-        rc = ensure(ctx, &ctx->queue, &ctx->queue_bytes, (size_t)ccfg.grid * (size_t)std::max(nmax, 1) * 4);
+        rc = ensure(ctx, &ctx->queue, &ctx->queue_bytes, chain_queue_bytes(ctx, ccfg, nmax, top_items > 0));
         if (!rc)
-            rc = ensure(ctx, &ctx->gbitmap, &ctx->gbitmap_bytes,
-                        (size_t)ccfg.grid * (size_t)ccfg.gbm_count * (size_t)ccfg.words * 4);
+            rc = ensure(ctx, &ctx->gbitmap, &ctx->gbitmap_bytes, chain_gbm_bytes(ctx, ccfg, top_items > 0));
         if (rc) return rc;
         fill_chain_launch(&CL, ccfg, *o, nmax);
         CL.nmats = count;
@@ -664,8 +720,7 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
         CK(cudaMemcpyAsync(ctx->h_fallback, HL.fallback, 4 * (size_t)count, cudaMemcpyDeviceToHost,
                            ctx->stream));
     }
-    if (chain && CL.total_items > 0)
-        CK(launch_chain(CL, ccfg.block, false, ccfg.grid, ccfg.smem, ctx->stream));
+    if (chain) CK(launch_chain_both(ctx, CL, ccfg, top_items));
     if (!chain && L.total_items > 0)
         CK(launch_traverse(L, cfg.block, cfg.grid, cfg.smem_bitmap, cfg.smem, ctx->stream));
     CK(cudaEventRecord(ctx->evt, ctx->stream));
@@ -688,14 +743,15 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
             sources += descs[(size_t)k].n;
             sym = sym && mats[order[(size_t)k]]->host_sym > 0;
         }
-        rc = plan_chain(ctx, std::max(nmax, 1), sym, o, false, &ccfg);
+        rc = plan_chain(ctx, std::max(nmax, 1), sources, sym, o, false, &ccfg);
         if (rc) return rc;
-        CL.chunk = (int)chain_chunk(*o, sources, ccfg.grid, sym);
+        CL.chunk = (int)chain_chunk(*o, sources, nmax, ccfg.grid, sym);
         for (int32_t k = 0; k < count; k++) {
             MatDesc& d = descs[(size_t)k];
             // the others have no items now
             d.method = left[(size_t)k] ? METHOD_CHAIN : d.method;
             d.item_base = items;
+            d.top_items = 0;
             if (!left[(size_t)k]) continue;
             items += (d.n + CL.chunk - 1) / CL.chunk;
             CK(cudaMemsetAsync(res[order[(size_t)k]]->counters, 0, 8 * CNT_SLOTS, ctx->stream));
@@ -1070,20 +1126,31 @@ int gsofa::host::fetch_all(gsofa_ctx* ctx, const Fetch* f, int count) {
     }
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     cudaError_t e = cudaSuccess;
-    if (total <= kStageBytes) {
-        size_t at = 0;
-        for (int k = 0; k < count && e == cudaSuccess; k++) {
-            if (!f[k].dst || !f[k].bytes) continue;
-            e = cudaMemcpyAsync(ctx->h_stage + at, f[k].src, f[k].bytes, cudaMemcpyDeviceToHost, ctx->stream);
-            at += f[k].bytes;
+    if (total + 256 * (size_t)count <= kStageBytes && count <= 8) {
+        // arrays that lie one after another (256-byte steps) share a copy too
+        size_t at[8] = {}, used = 0;
+        for (int k = 0; k < count && e == cudaSuccess;) {
+            if (!f[k].dst || !f[k].bytes) {
+                k++;
+                continue;
+            }
+            const char* first = static_cast<const char*>(f[k].src);
+            at[k] = used;
+            size_t span = f[k].bytes;
+            int next = k + 1;
+            for (; next < count && f[next].dst && f[next].bytes; next++) {
+                const char* s = static_cast<const char*>(f[next].src);
+                if (s < first + span || s - (first + span) >= 256) break;
+                at[next] = used + (size_t)(s - first);
+                span = (size_t)(s - first) + f[next].bytes;
+            }
+            e = cudaMemcpyAsync(ctx->h_stage + used, first, span, cudaMemcpyDeviceToHost, ctx->stream);
+            used += span;
+            k = next;
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        at = 0;
-        for (int k = 0; k < count && e == cudaSuccess; k++) {
-            if (!f[k].dst || !f[k].bytes) continue;
-            memcpy(f[k].dst, ctx->h_stage + at, f[k].bytes);
-            at += f[k].bytes;
-        }
+        for (int k = 0; k < count && e == cudaSuccess; k++)
+            if (f[k].dst && f[k].bytes) memcpy(f[k].dst, ctx->h_stage + at[k], f[k].bytes);
         return e == cudaSuccess ? GSOFA_OK : cuda_fail(ctx, e, "result fetch");
     }
     for (int k = 0; k < count && e == cudaSuccess; k++)
@@ -1146,6 +1213,12 @@ int gsofa_create(int device, size_t budget_bytes, gsofa_ctx** out) {
         if (ctx->ev0) cudaEventDestroy(ctx->ev0);
         if (ctx->ev1) cudaEventDestroy(ctx->ev1);
         if (ctx->evt) cudaEventDestroy(ctx->evt);
+        if (ctx->side_stream) cudaStreamDestroy(ctx->side_stream);
+        if (ctx->fork) cudaEventDestroy(ctx->fork);
+        if (ctx->join) cudaEventDestroy(ctx->join);
+        if (ctx->hub_stream) cudaStreamDestroy(ctx->hub_stream);
+        if (ctx->hub_fork) cudaEventDestroy(ctx->hub_fork);
+        if (ctx->hub_join) cudaEventDestroy(ctx->hub_join);
         if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
         if (ctx->h_fallback) cudaFreeHost(ctx->h_fallback);
         if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
@@ -1168,6 +1241,13 @@ int gsofa_create(int device, size_t budget_bytes, gsofa_ctx** out) {
     if ((e = cudaEventCreate(&ctx->ev0)) != cudaSuccess) return fail(e);
     if ((e = cudaEventCreate(&ctx->ev1)) != cudaSuccess) return fail(e);
     if ((e = cudaEventCreate(&ctx->evt)) != cudaSuccess) return fail(e);
+    if ((e = cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&ctx->join, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaStreamCreateWithFlags(&ctx->hub_stream, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&ctx->hub_fork, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&ctx->hub_join, cudaEventDisableTiming)) != cudaSuccess)
+        return fail(e);
     if (ensure_pinned(ctx, 1) != GSOFA_OK) return fail(cudaErrorMemoryAllocation);
     if ((e = cudaMallocHost((void**)&ctx->h_stage, kStageBytes)) != cudaSuccess) return fail(e);
     if ((e = cudaMallocHost((void**)&ctx->h_status, 64)) != cudaSuccess) return fail(e);
@@ -1201,6 +1281,12 @@ int gsofa_destroy(gsofa_ctx* ctx) {
         cudaEventDestroy(ctx->ev0);
         cudaEventDestroy(ctx->ev1);
         cudaEventDestroy(ctx->evt);
+        cudaStreamDestroy(ctx->side_stream);
+        cudaEventDestroy(ctx->fork);
+        cudaEventDestroy(ctx->join);
+        cudaStreamDestroy(ctx->hub_stream);
+        cudaEventDestroy(ctx->hub_fork);
+        cudaEventDestroy(ctx->hub_join);
         cudaFreeHost(ctx->h_counters);
         cudaFreeHost(ctx->h_fallback);
         cudaFreeHost(ctx->h_stage);
@@ -1534,7 +1620,6 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     if (o.flags & GSOFA_PATTERN)
         return set_err(ctx, GSOFA_ERR_UNSUPPORTED, "a captured batch cannot materialise patterns");
     int32_t nmax = 1;
-    long long total_sources = 0;
     for (int32_t i = 0; i < count; i++) {
         if (!mats[i] || mats[i]->ctx != ctx)
             return set_err(ctx, GSOFA_ERR_ARG, "matrix %d is null or from another context", i);
@@ -1542,12 +1627,7 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     }
     if (cudaSetDevice(ctx->device) != cudaSuccess) return set_err(ctx, GSOFA_ERR_CUDA, "cudaSetDevice");
     long long weight = 0;
-    bool all_sym = true;
-    for (int32_t i = 0; i < count; i++) {
-        weight += chunk_weight(ctx, mats[i]);
-        total_sources += mats[i]->n;
-        all_sym = all_sym && mats[i]->host_sym > 0;
-    }
+    for (int32_t i = 0; i < count; i++) weight += chunk_weight(ctx, mats[i]);
     gsofa_batch* b = new (std::nothrow) gsofa_batch();
     if (!b) return set_err(ctx, GSOFA_ERR_OOM_BUDGET, "host allocation failed");
     b->ctx = ctx;
@@ -1567,16 +1647,27 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     const bool chain = !(o.flags & GSOFA_L_ROW_STATS) && chain_runs(o, mats, count);
     ChainCfg ccfg;
     LaunchCfg cfg;
-    // the chain's shape: that of the matrices it takes, or of all if it takes none
-    long long chain_sources = 0;
-    for (int32_t i = 0; i < count; i++)
-        if (method_of(mats[i]) == METHOD_CHAIN) chain_sources += mats[i]->n;
-    if (chain_sources == 0) chain_sources = total_sources;
-    rc = chain ? plan_chain(ctx, nmax, all_sym, &o, false, &ccfg) : plan_launch(ctx, nmax, &o, &cfg);
+    // the chain's shape for the symmetric matrices it takes, and for those that
+    // the hubs' launch may leave it
+    long long chain_sources = 0, left_sources = 0;
+    int32_t chain_nmax = 1, left_nmax = 1;
+    for (int32_t i = 0; i < count; i++) {
+        const bool mine = method_of(mats[i]) == METHOD_CHAIN;
+        (mine ? chain_sources : left_sources) += mats[i]->n;
+        (mine ? chain_nmax : left_nmax) = std::max(mine ? chain_nmax : left_nmax, mats[i]->n);
+    }
+    ChainCfg lcfg;
+    if (chain) {
+        rc = plan_chain(ctx, chain_nmax, chain_sources, true, &o, false, &ccfg);
+        if (!rc) rc = plan_chain(ctx, left_nmax, left_sources, false, &o, false, &lcfg);
+    } else {
+        rc = plan_launch(ctx, nmax, &o, &cfg);
+    }
     if (rc) return fail(rc);
-    const long long chunk = chain ? chain_chunk(o, chain_sources, ccfg.grid, all_sym)
+    const long long chunk = chain ? chain_chunk(o, chain_sources, chain_nmax, ccfg.grid, true)
                             : o.chunk_sources > 0 ? o.chunk_sources
                                                   : default_chunk(weight, cfg.grid);
+    const long long left_chunk = chain_chunk(o, left_sources, left_nmax, lcfg.grid > 0 ? lcfg.grid : 1, false);
     const long long per_chunk = chain ? 1 : 2;  // work items
     const bool merge = !(o.flags & GSOFA_NO_MERGE);
     int ring = o.cached_closures > 0 ? o.cached_closures : kDefaultRing;
@@ -1598,18 +1689,38 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     HubCfg hcfg;
     size_t sz_hub = 0;
     bool hub = false;
-    for (int32_t k = 0; k < count && chain; k++)
-        descs[(size_t)k].method = method_of(mats[order[(size_t)k]]);
+    long long top_items = 0, left_items = 0;
+    if (chain) {
+        long long items = 0;
+        for (int32_t k = 0; k < count; k++) {
+            MatDesc& d = descs[(size_t)k];
+            const gsofa_matrix* m = mats[order[(size_t)k]];
+            d.method = method_of(m);
+            d.item_base = items;
+            d.top_base = top_items;
+            d.left_base = left_items;
+            if (d.method == METHOD_CHAIN) {
+                d.top_items = chain_top_items(o, m->n, chunk, true);
+                top_items += d.top_items;
+                items += (m->n + chunk - 1) / chunk - d.top_items;
+            } else {
+                left_items += (m->n + left_chunk - 1) / left_chunk;
+            }
+        }
+        b->items = items;
+    }
     if (chain) hub = plan_hub(ctx, &descs, o, nullptr, &sz_hub, &HL, &hcfg);
     const size_t sz_small = 256;
     const size_t sz_desc = align256(sizeof(MatDesc) * (size_t)count);
     const size_t sz_seg = align256(sizeof(long long) * ((size_t)count + 1));
     const size_t sz_cnt = align256(8ull * CNT_SLOTS * (size_t)count);
-    const size_t sz_q = align256((size_t)(chain ? ccfg.grid : cfg.grid) * (size_t)nmax * 4);
+    const size_t sz_q = align256(chain ? std::max(chain_queue_bytes(ctx, ccfg, chain_nmax, top_items > 0),
+                                                  chain_queue_bytes(ctx, lcfg, left_nmax, false))
+                                       : (size_t)cfg.grid * (size_t)nmax * 4);
     const size_t sz_ring =
         merge && !chain ? align256((size_t)cfg.grid * (size_t)ring * (size_t)cfg.words * 4) : 0;
     const size_t sz_gbm =
-        chain ? align256((size_t)ccfg.grid * (size_t)ccfg.gbm_count * (size_t)ccfg.words * 4)
+        chain ? align256(std::max(chain_gbm_bytes(ctx, ccfg, top_items > 0), chain_gbm_bytes(ctx, lcfg, false)))
         : cfg.smem_bitmap ? 0 : align256((size_t)cfg.grid * (size_t)cfg.words * 4);
     b->ws_bytes = sz_small + sz_desc + sz_seg + sz_cnt + sz_q + sz_ring + sz_gbm + sz_hub;
     rc = dev_alloc(ctx, b->ws_bytes, &b->ws);
@@ -1681,18 +1792,37 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     CL.chunk = (int)chunk;
     CL.sample_stride = 1;
     CL.status = dstatus;
-    if (chain) fill_chain_launch(&CL, ccfg, o, nmax);
-    CL.fallback = hub ? HL.fallback : nullptr;
+    ChainLaunch LL = CL;  // what the hubs' launch leaves
+    if (chain) {
+        fill_chain_launch(&CL, ccfg, o, chain_nmax);
+        fill_chain_launch(&LL, lcfg, o, left_nmax);
+        LL.chunk = (int)left_chunk;
+        LL.items = ITEMS_LEFT;
+        LL.total_items = left_items;
+        LL.work_counter = wc + 2;
+        LL.fallback = HL.fallback;
+    }
 
     // capture: reset -> traversal -> supernodes -> read-back
     if ((e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed)) != cudaSuccess)
         return fail(cuda_fail(ctx, e, "cudaStreamBeginCapture"));
     e = cudaMemsetAsync(b->ws, 0, 128, ctx->stream);
     if (e == cudaSuccess) e = launch_batch_reset(ddesc, count, ctx->stream);
-    if (e == cudaSuccess && hub) e = launch_hub(HL, hcfg, (o.flags & GSOFA_DIGESTS) != 0, ctx->stream);
-    if (e == cudaSuccess && b->items > 0 && chain)  // with what the hubs' launch leaves it
-        e = launch_chain(CL, ccfg.block, false, ccfg.grid, ccfg.smem, ctx->stream);
-    else if (e == cudaSuccess && b->items > 0)
+    if (e == cudaSuccess && chain) {
+        // the two traversals side by side, then what the first leaves to the chain
+        if (hub) {
+            e = cudaEventRecord(ctx->hub_fork, ctx->stream);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->hub_stream, ctx->hub_fork, 0);
+            if (e == cudaSuccess) e = launch_hub(HL, hcfg, (o.flags & GSOFA_DIGESTS) != 0, ctx->hub_stream);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->hub_join, ctx->hub_stream);
+        }
+        if (e == cudaSuccess) e = launch_chain_both(ctx, CL, ccfg, top_items);
+        if (e == cudaSuccess && hub) {
+            e = cudaStreamWaitEvent(ctx->stream, ctx->hub_join, 0);
+            if (e == cudaSuccess) e = launch_chain(LL, lcfg.block, false, lcfg.grid, lcfg.smem, ctx->stream);
+        }
+    }
+    if (e == cudaSuccess && b->items > 0 && !chain)
         e = launch_traverse(L, cfg.block, cfg.grid, cfg.smem_bitmap, cfg.smem, ctx->stream);
     if (e == cudaSuccess && (o.flags & GSOFA_SUPERNODES))
         e = launch_supernodes_batch(ddesc, count, o.max_supernode_size, dseg, seg[(size_t)count],
@@ -1805,6 +1935,11 @@ int gsofa_result_supernodes(const gsofa_result* r, int8_t* flags, int32_t* bound
     int rc = fetch(r, f, r->sflags, (size_t)r->n);
     if (rc) return rc;
     int64_t k = 0;
+    if (!boundaries) {
+        for (int32_t v = 0; v < r->n; v++) k += f[v] != 0;
+        if (count) *count = k;
+        return GSOFA_OK;
+    }
     for (int32_t v = 0; v < r->n; v++) {
         if (f[v]) {
             if (boundaries && k < cap) boundaries[k] = v;

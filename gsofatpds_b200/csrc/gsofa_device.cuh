@@ -17,11 +17,12 @@ __host__ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
     return x ^ (x >> 31);
 }
 
+template <long long MatDesc::*BASE = &MatDesc::item_base>
 __device__ __forceinline__ int find_matrix(const MatDesc* mats, int nmats, long long item) {
     int lo = 0, hi = nmats - 1;
     while (lo < hi) {
         int mid = (lo + hi + 1) >> 1;
-        if (mats[mid].item_base <= item) lo = mid; else hi = mid - 1;
+        if (mats[mid].*BASE <= item) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
@@ -336,13 +337,15 @@ __device__ __forceinline__ void write_row(const MatDesc& M, int s, int dir, bool
     }
 }
 
-constexpr int kBfsCap = 512;
+// rows kept of a narrow level by a CTA of BLOCK threads
+__host__ __device__ constexpr int bfs_cap(int block) { return block >= 1024 ? 1024 : 512; }
 
+template <int BLOCK>
 struct BfsSmem {
     int cnt[3];                // ids queued per level, in turn
     unsigned long long rtrav;  // entries read
-    // the rows of a level's first kBfsCap ids: first entry, int4s
-    int2 row[2][kBfsCap];
+    // the rows of a level's first ids: first entry, int4s
+    int2 row[2][bfs_cap(BLOCK)];
 };
 
 // Breadth-first search in the bitmap bm from the frontier q[0, tail), whose
@@ -357,10 +360,10 @@ struct BfsSmem {
 // entries -> bitmap -> row pointers -> barrier; wide ones read the queue two
 // groups ahead.
 template <int BLOCK, bool CG, bool LAM = false>
-__device__ long long block_bfs(BfsSmem& SM, const Graph& G, uint32_t* bm, int32_t* q,
+__device__ long long block_bfs(BfsSmem<BLOCK>& SM, const Graph& G, uint32_t* bm, int32_t* q,
                                long long qcap, long long tail, int s, int bound, bool all,
                                int32_t* status, const int32_t* lam = nullptr) {
-    constexpr int NW = BLOCK / 32;
+    constexpr int NW = BLOCK / 32, kCap = bfs_cap(BLOCK);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) SM.cnt[0] = 0;
     __syncthreads();
@@ -442,11 +445,11 @@ __device__ long long block_bfs(BfsSmem& SM, const Graph& G, uint32_t* bm, int32_
                 }
 #pragma unroll
                 for (int c = 0; c < 4; c++)
-                    if (x[c] >= 0 && x[c] < kBfsCap)
+                    if (x[c] >= 0 && x[c] < kCap)
                         next[x[c]] = make_int2(a0[c] & ~3, ((a1[c] & ~3) - (a0[c] & ~3)) >> 2);
             }
         };
-        if (kept && n <= kBfsCap) {
+        if (kept && n <= kCap) {
             const int per = n >= 32 * NW ? 32 : (int)((n + NW - 1) / NW);
             for (long long base = (long long)warp * per; base < n; base += NW * per) {
                 int2 r = make_int2(0, 0);

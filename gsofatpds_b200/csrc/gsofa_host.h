@@ -24,6 +24,12 @@ struct gsofa_ctx {
     cudaStream_t stream = nullptr;
     cudaMemPool_t pool = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evt = nullptr;
+    // the chain's two launches run side by side
+    cudaStream_t side_stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    // a captured batch runs the hubs' launches beside the chain's
+    cudaStream_t hub_stream = nullptr;
+    cudaEvent_t hub_fork = nullptr, hub_join = nullptr;
     std::recursive_mutex mu;
     std::string err;
     // autotuner choices per class (log2 n, mean row length, locality: half-
@@ -162,8 +168,16 @@ struct ChainCfg {
     int sides = 2;
 };
 bool chain_runs(const gsofa_opts& o, const gsofa_matrix* const* mats, int32_t count);
-int plan_chain(gsofa_ctx* ctx, int32_t nmax, bool all_sym, const gsofa_opts* o, bool serve,
-               ChainCfg* c);
+int plan_chain(gsofa_ctx* ctx, int32_t nmax, long long total_sources, bool all_sym, const gsofa_opts* o,
+               bool serve, ChainCfg* c);
+// The chunks of a matrix of n rows that the launch of larger CTAs takes.
+long long chain_top_items(const gsofa_opts& o, int32_t n, long long chunk, bool sym);
+// Both launches of the chain on ctx->stream and beside it: `top` (`top_items`
+// items, workspace after the first launch's) and the rest.
+cudaError_t launch_chain_both(gsofa_ctx* ctx, const ChainLaunch& L, const ChainCfg& c, long long top_items);
+// Queue and bitmap bytes of both launches.
+size_t chain_queue_bytes(const gsofa_ctx* ctx, const ChainCfg& c, int32_t nmax, bool top);
+size_t chain_gbm_bytes(const gsofa_ctx* ctx, const ChainCfg& c, bool top);
 // The launch's fields that follow from the shape, the options and the largest order.
 void fill_chain_launch(ChainLaunch* L, const ChainCfg& c, const gsofa_opts& o, int32_t nmax);
 // Which counting traversal a matrix takes (its host_sym must be known).
@@ -174,7 +188,7 @@ int32_t method_of(const gsofa_matrix* m);
 bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, void* ws,
               size_t* bytes, HubLaunch* L, HubCfg* c);
 // Consecutive sources per work item.
-long long chain_chunk(const gsofa_opts& o, long long total_sources, int grid, bool sym);
+long long chain_chunk(const gsofa_opts& o, long long total_sources, int32_t nmax, int grid, bool sym);
 // Result arrays of an n-row matrix, zero-initialised on `stream`.
 int result_alloc_on(gsofa_ctx* ctx, int32_t n, uint32_t flags, int32_t mss, cudaStream_t stream,
                     gsofa_result** out);

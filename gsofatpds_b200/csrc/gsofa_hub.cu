@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(kExtraThreads, 1024 / kExtraThreads) extra_ker
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) large_kernel(HubLaunch P) {
     extern __shared__ uint4 dyn_smem[];
-    __shared__ BfsSmem bfs;
+    __shared__ BfsSmem<BLOCK> bfs;
     __shared__ long long item;
     __shared__ unsigned long long red[BLOCK / 32][4];
     __shared__ int row[2];

@@ -75,6 +75,11 @@ struct MatDesc {
     // in the other direction reads it (see traverse_kernel: chained starts)
     uint8_t* link;
     long long item_base;        // first work item of this matrix
+    // gsofa_chain.cu: the chunks of the largest sources, taken by a launch of
+    // larger CTAs, and the first of them there
+    long long top_items;
+    long long top_base;
+    long long left_base;        // its first item in the launch of what gsofa_hub.cu leaves
     // gsofa_hub.cu: place of the matrix in its arrays (a multiple of 32), the
     // room there (n + 1 rounded up), first work item and items (a power of two)
     long long hub_off;
@@ -152,6 +157,11 @@ struct TraverseLaunch {
 // ints and gbm_count bitmaps of bitmap_words words in global memory (two that
 // are zero between uses; two more for the dense base when it does not fit in
 // shared memory).
+enum : int {
+    ITEMS_MAIN = 0,  // the matrices' chunks but the top_items
+    ITEMS_TOP = 1,   // those
+    ITEMS_LEFT = 2,  // the chunks of the matrices with a fallback flag
+};
 struct ChainLaunch {
     const MatDesc* mats;               // device array
     int32_t nmats;
@@ -163,12 +173,13 @@ struct ChainLaunch {
     int gbm_count;
     long long bitmap_words;            // covers the largest n + padding
     long long smem_words;              // bitmap words that fit in shared memory
+    int items;                         // ITEMS_*
     int sides;                         // directions with tables: 1 when every pattern is symmetric
     int chunk;                         // consecutive sources per work item
     int list_cap;                      // new ids of a search before the whole CTA takes it
     long long sample_stride;           // > 1: only every stride-th item (autotuner timing)
     int32_t* status;                   // device error word
-    const int32_t* fallback;           // or null: per matrix, gsofa_hub.cu left it to the chain
+    const int32_t* fallback;           // ITEMS_LEFT: per matrix, gsofa_hub.cu left it to the chain
     ServeLaunch serve;                 // serving kernel only
 };
 // sizes of a set relative to the current source: ids above it, ids below it,
