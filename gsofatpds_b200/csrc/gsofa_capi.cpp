@@ -496,7 +496,7 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
 // Smaller meshes lose more by the SMs those CTAs take (170 x 170: 0.82 -> 1.0 ms,
 // a batch of 64 matrices 5.9 -> 7.2).
 long long chain_top_items(const gsofa_opts& o, int32_t n, long long chunk, bool sym) {
-    if (!sym || o.threads_per_source > 0 || o.sources_in_flight > 0 || n < 131072) return 0;
+    if (!sym || o.sources_in_flight > 0 || n < 131072) return 0;
     const long long chunks = (n + chunk - 1) / chunk;
     return std::min(chunks - 1, (n / 50 + chunk - 1) / chunk);
 }
@@ -1216,9 +1216,6 @@ int gsofa_create(int device, size_t budget_bytes, gsofa_ctx** out) {
         if (ctx->side_stream) cudaStreamDestroy(ctx->side_stream);
         if (ctx->fork) cudaEventDestroy(ctx->fork);
         if (ctx->join) cudaEventDestroy(ctx->join);
-        if (ctx->hub_stream) cudaStreamDestroy(ctx->hub_stream);
-        if (ctx->hub_fork) cudaEventDestroy(ctx->hub_fork);
-        if (ctx->hub_join) cudaEventDestroy(ctx->hub_join);
         if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
         if (ctx->h_fallback) cudaFreeHost(ctx->h_fallback);
         if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
@@ -1243,10 +1240,7 @@ int gsofa_create(int device, size_t budget_bytes, gsofa_ctx** out) {
     if ((e = cudaEventCreate(&ctx->evt)) != cudaSuccess) return fail(e);
     if ((e = cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming)) != cudaSuccess ||
-        (e = cudaEventCreateWithFlags(&ctx->join, cudaEventDisableTiming)) != cudaSuccess ||
-        (e = cudaStreamCreateWithFlags(&ctx->hub_stream, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = cudaEventCreateWithFlags(&ctx->hub_fork, cudaEventDisableTiming)) != cudaSuccess ||
-        (e = cudaEventCreateWithFlags(&ctx->hub_join, cudaEventDisableTiming)) != cudaSuccess)
+        (e = cudaEventCreateWithFlags(&ctx->join, cudaEventDisableTiming)) != cudaSuccess)
         return fail(e);
     if (ensure_pinned(ctx, 1) != GSOFA_OK) return fail(cudaErrorMemoryAllocation);
     if ((e = cudaMallocHost((void**)&ctx->h_stage, kStageBytes)) != cudaSuccess) return fail(e);
@@ -1284,9 +1278,6 @@ int gsofa_destroy(gsofa_ctx* ctx) {
         cudaStreamDestroy(ctx->side_stream);
         cudaEventDestroy(ctx->fork);
         cudaEventDestroy(ctx->join);
-        cudaStreamDestroy(ctx->hub_stream);
-        cudaEventDestroy(ctx->hub_fork);
-        cudaEventDestroy(ctx->hub_join);
         cudaFreeHost(ctx->h_counters);
         cudaFreeHost(ctx->h_fallback);
         cudaFreeHost(ctx->h_stage);
@@ -1403,13 +1394,20 @@ int gsofa_factor_batch(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     return GSOFA_OK;
 }
 
+static gsofa_opts base_without_l_rows(gsofa_opts o) {
+    o.flags &= ~(uint32_t)GSOFA_L_ROW_STATS;
+    return o;
+}
+
 // Times candidate launch shapes on an evenly spread sample of the matrix's
 // work items (large matrices) or on the whole matrix (small ones) and keeps
 // the fastest.  The candidates differ only in speed: every setting gives the
 // same results.  Choices are cached per size class in the context.
-// Coordinate descent over the launch shape (CTA size, closure ring, chunk,
-// warp-walked row threshold), each candidate timed on the device as one
-// persistent launch over all `count` matrices.  Writes the best into *opts.
+// Coordinate descent over the launch shape, each candidate timed on the device
+// as one call over all `count` matrices: CTA size and chunk of the chain's
+// launch where it takes any of them, or CTA size, closure ring, chunk and
+// warp-walked row threshold of traverse_kernel's where that counts.  The hubs'
+// launches have no shape to choose.  Writes the best into *opts.
 static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
                          gsofa_opts* opts) {
     int rc = GSOFA_OK;
@@ -1421,7 +1419,10 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
         total_sources += chunk_weight(ctx, mats[i]);
     }
     gsofa_opts base = *opts;
-    base.flags &= ~(uint32_t)(GSOFA_SUPERNODES | GSOFA_PATTERN | GSOFA_L_ROW_STATS);
+    base.flags &= ~(uint32_t)(GSOFA_SUPERNODES | GSOFA_PATTERN);
+    if (chain_runs(*opts, mats, count) || !chain_runs(base_without_l_rows(*opts), mats, count))
+        base.flags &= ~(uint32_t)GSOFA_L_ROW_STATS;  // else they decide which kernel counts
+    const bool chain = chain_runs(base, mats, count);
     // reference timing with the defaults picks the sampling rate
     std::vector<gsofa_result*> rr((size_t)count, nullptr);
     auto free_all = [&]() {
@@ -1467,14 +1468,34 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
     double best_ms = 0;
     rc = time_opts(best, &best_ms);
     if (rc) { free_all(); return rc; }
+    long long auto_chunk = 64;
+    bool walks = !chain;  // some matrix's counting depends on the shape
     {
         LaunchCfg c0;
-        if (plan_launch(ctx, nmax, &base, &c0) == GSOFA_OK) best.threads_per_source = c0.block;
+        if (plan_launch(ctx, nmax, &base, &c0) == GSOFA_OK) {
+            best.threads_per_source = c0.block;
+            auto_chunk = default_chunk(total_sources, c0.grid);
+        }
+        long long chain_sources = 0;
+        bool chain_sym = true;
+        for (int32_t i = 0; i < count; i++) {
+            if (!chain || method_of(mats[i]) != METHOD_CHAIN) continue;
+            walks = true;
+            chain_sources += mats[i]->n;
+            chain_sym = chain_sym && mats[i]->host_sym > 0;
+        }
+        ChainCfg cc;
+        if (chain_sources > 0 &&
+            plan_chain(ctx, std::max(nmax, 1), chain_sources, chain_sym, &base, false, &cc) == GSOFA_OK) {
+            best.threads_per_source = cc.block;
+            auto_chunk = chain_chunk(base, chain_sources, nmax, cc.grid, chain_sym);
+            best.chunk_sources = (int32_t)auto_chunk;
+        }
         ctx->err.clear();
     }
     const int tps_c[] = {128, 256, 512, 1024};
     for (int tps : tps_c) {
-        if (tps == best.threads_per_source) continue;
+        if (tps == best.threads_per_source || !walks) continue;
         gsofa_opts p = best;
         p.threads_per_source = tps;
         double ms;
@@ -1485,7 +1506,7 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
     const int ring_now = best.cached_closures > 0 ? best.cached_closures : kDefaultRing;
     best.cached_closures = ring_now;
     for (int ring : ring_c) {
-        if (ring == ring_now) continue;
+        if (ring == ring_now || chain) continue;
         gsofa_opts p = best;
         p.cached_closures = ring;
         double ms;
@@ -1494,13 +1515,13 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
     }
     {
         LaunchCfg c;
-        long long auto_chunk = 64;
-        if (plan_launch(ctx, nmax, &best, &c) == GSOFA_OK) auto_chunk = default_chunk(total_sources, c.grid);
+        if (!chain && plan_launch(ctx, nmax, &best, &c) == GSOFA_OK)
+            auto_chunk = default_chunk(total_sources, c.grid);
         ctx->err.clear();
         if (best.chunk_sources <= 0) best.chunk_sources = (int32_t)auto_chunk;
         const long long cands[] = {auto_chunk / 8, auto_chunk / 4, auto_chunk / 2, auto_chunk * 2};
         for (long long ch : cands) {
-            if (ch < 16 || ch > 1024 || ch == best.chunk_sources) continue;
+            if (ch < 16 || ch > 1024 || ch == best.chunk_sources || !walks) continue;
             gsofa_opts p = best;
             p.chunk_sources = (int32_t)ch;
             double ms;
@@ -1512,7 +1533,7 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
     const int heavy_now = best.heavy_row > 0 ? best.heavy_row : kDefaultHeavyRow;
     best.heavy_row = heavy_now;
     for (int hr : {32, 64}) {
-        if (hr == heavy_now) continue;
+        if (hr == heavy_now || chain) continue;
         gsofa_opts p = best;
         p.heavy_row = hr;
         double ms;
@@ -1549,7 +1570,9 @@ int gsofa_autotune(gsofa_ctx* ctx, const gsofa_matrix* mat, gsofa_opts* opts) {
     if (ce != cudaSuccess) return cuda_fail(ctx, ce, "autotune locality");
     const double rel = mat->nnz > 0 ? (double)hsum / (double)mat->nnz / (double)mat->n : 0.0;
     const int loc = rel > 1e-9 ? std::max(-60, (int)std::floor(2.0 * std::log2(rel))) : -61;
-    const std::tuple<int, int, int> key(lg, deg, loc);
+    // and so do the kernels that may count them
+    const gsofa_matrix* const mats[1] = {mat};
+    const std::tuple<int, int, int, int> key(lg, deg, loc, chain_runs(*opts, mats, 1) ? method_of(mat) : -1);
     auto it = ctx->tuned.find(key);
     if (it != ctx->tuned.end()) {
         opts->threads_per_source = it->second.threads_per_source;
@@ -1558,7 +1581,6 @@ int gsofa_autotune(gsofa_ctx* ctx, const gsofa_matrix* mat, gsofa_opts* opts) {
         opts->heavy_row = it->second.heavy_row;
         return GSOFA_OK;
     }
-    const gsofa_matrix* const mats[1] = {mat};
     rc = autotune_impl(ctx, mats, 1, opts);
     if (rc == GSOFA_OK) ctx->tuned[key] = *opts;
     return rc;
@@ -1804,6 +1826,19 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     }
 
     // capture: reset -> traversal -> supernodes -> read-back
+    struct Fork {  // the hubs' branch: of use during the capture alone
+        cudaStream_t stream = nullptr;
+        cudaEvent_t fork = nullptr, join = nullptr;
+        ~Fork() {
+            if (stream) cudaStreamDestroy(stream);
+            if (fork) cudaEventDestroy(fork);
+            if (join) cudaEventDestroy(join);
+        }
+    } hf;
+    if (hub && ((e = cudaStreamCreateWithFlags(&hf.stream, cudaStreamNonBlocking)) != cudaSuccess ||
+                (e = cudaEventCreateWithFlags(&hf.fork, cudaEventDisableTiming)) != cudaSuccess ||
+                (e = cudaEventCreateWithFlags(&hf.join, cudaEventDisableTiming)) != cudaSuccess))
+        return fail(cuda_fail(ctx, e, "batch streams"));
     if ((e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed)) != cudaSuccess)
         return fail(cuda_fail(ctx, e, "cudaStreamBeginCapture"));
     e = cudaMemsetAsync(b->ws, 0, 128, ctx->stream);
@@ -1811,14 +1846,14 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     if (e == cudaSuccess && chain) {
         // the two traversals side by side, then what the first leaves to the chain
         if (hub) {
-            e = cudaEventRecord(ctx->hub_fork, ctx->stream);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->hub_stream, ctx->hub_fork, 0);
-            if (e == cudaSuccess) e = launch_hub(HL, hcfg, (o.flags & GSOFA_DIGESTS) != 0, ctx->hub_stream);
-            if (e == cudaSuccess) e = cudaEventRecord(ctx->hub_join, ctx->hub_stream);
+            e = cudaEventRecord(hf.fork, ctx->stream);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(hf.stream, hf.fork, 0);
+            if (e == cudaSuccess) e = launch_hub(HL, hcfg, (o.flags & GSOFA_DIGESTS) != 0, hf.stream);
+            if (e == cudaSuccess) e = cudaEventRecord(hf.join, hf.stream);
         }
         if (e == cudaSuccess) e = launch_chain_both(ctx, CL, ccfg, top_items);
         if (e == cudaSuccess && hub) {
-            e = cudaStreamWaitEvent(ctx->stream, ctx->hub_join, 0);
+            e = cudaStreamWaitEvent(ctx->stream, hf.join, 0);
             if (e == cudaSuccess) e = launch_chain(LL, lcfg.block, false, lcfg.grid, lcfg.smem, ctx->stream);
         }
     }

@@ -89,7 +89,7 @@ __device__ inline bool serve_claim(const ServeLaunch& V, int* slot_out, long lon
         int c0 = 0, c1 = 0, n = 0;
         unsigned r = 0;
         if (lane == 0) {
-            c1 = ld_vol_i32(V.ctrl + 1);
+            c1 = ld_vol_i32(V.ctrl + 1) | (V.launch_no < ld_vol_i32(V.ctrl + 3));
             c0 = ld_vol_i32(V.ctrl);
             n = min(ld_vol_i32(V.ctrl + 2), V.nslots);
             if (!c1 && n > 0) r = atomicAdd(V.rr, 1u);
@@ -157,8 +157,14 @@ __device__ inline bool serve_claim(const ServeLaunch& V, int* slot_out, long lon
     return false;
 }
 
-// Serving: takes a free per-CTA workspace slot, or returns -1.
+// Serving: takes a free per-CTA workspace slot, or returns -1.  None on the SMs
+// left to the uploads' and builds' kernels: four CTAs of 256 threads and 64
+// registers fill an SM's registers, and single holes spread over many SMs are
+// too small for a sort's CTA, which then waits for a serving CTA to leave.
 __device__ inline int take_cta_slot(const ServeLaunch& V) {
+    unsigned sm;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+    if (sm >= V.sm_limit) return -1;
     const int nw = (V.n_cta_slots + 31) >> 5;
     for (int w = 0; w < nw; w++) {
         unsigned v = ld_vol_i32(reinterpret_cast<const int32_t*>(V.cta_slots + w));

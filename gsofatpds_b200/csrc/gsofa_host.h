@@ -27,14 +27,11 @@ struct gsofa_ctx {
     // the chain's two launches run side by side
     cudaStream_t side_stream = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
-    // a captured batch runs the hubs' launches beside the chain's
-    cudaStream_t hub_stream = nullptr;
-    cudaEvent_t hub_fork = nullptr, hub_join = nullptr;
     std::recursive_mutex mu;
     std::string err;
     // autotuner choices per class (log2 n, mean row length, locality: half-
     // octaves of the mean |i - j| of the entries over n)
-    std::map<std::tuple<int, int, int>, gsofa_opts> tuned;
+    std::map<std::tuple<int, int, int, int>, gsofa_opts> tuned;
     // pinned staging: totals of h_counters_cap matrices, the status words and
     // h_fallback_cap flags, and results on their way to the caller's arrays
     unsigned long long* h_counters = nullptr;

@@ -109,7 +109,8 @@ struct MatDesc {
 struct ServeLaunch {
     unsigned long long* claim;            // per slot
     const unsigned long long* list;       // (slot << 32) | request number
-    const int32_t* ctrl;                  // [0] exit when idle, [1] take no more items, [2] list entries
+    const int32_t* ctrl;                  // [0] exit when idle, [1] take no more items, [2] list entries,
+                                          // [3] launches before this number take no more items
     unsigned int* rr;                     // rotating start of the list scan (tie order)
     const MatDesc* slots;                 // one descriptor per slot
     unsigned long long* items_done;       // per slot: finished items
@@ -126,6 +127,8 @@ struct ServeLaunch {
     unsigned int* cta_slots;
     int32_t n_cta_slots;
     int* alive;                           // CTAs holding a slot
+    int32_t launch_no;
+    unsigned sm_limit;                    // CTAs on SMs of this number or above leave at once
 };
 
 struct TraverseLaunch {
