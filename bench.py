@@ -9,8 +9,8 @@ stand-in), max supernode size 128.
   e2e     the same metric through the C-ABI with host buffers: H2D of the
           CSR, device ingest/transpose, factorization, D2H of the per-row
           counts, every step
-  roofline  traversal kernel: algorithmic bytes (8*E_alg + 16*V_alg +
-          4*W_out) per launch / its CUDA-event duration vs measured HBM peak
+  roofline  counting kernels: the DRAM bytes they move in one factorization
+          / their CUDA-event duration vs measured HBM peak
 
 Usage: python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 N > 1 runs under torchrun as independent replicas (one matrix per GPU, no
@@ -77,27 +77,27 @@ def read_peaks():
 
 
 def roofline_entry(edges, vertices_alg, edges_trav, n, kernel_ms, peak, peak_kind, traffic):
-    """The line's roofline object for the traversal kernel, whose bound is
+    """The line's roofline object for the counting kernels, whose bound is
     HBM (an irregular integer traversal; no tensor cores).  `achieved` is the
-    DRAM bytes one launch really moves (`traffic`: ncu dram__bytes_read.sum +
-    dram__bytes_write.sum of one full-size launch, from the committed
-    profile of this workload) per second of the kernel's CUDA-event time, and
+    DRAM bytes they really move (`traffic`: ncu dram__bytes_read.sum +
+    dram__bytes_write.sum over one full-size factorization, from the committed
+    profile of this workload) per second of their CUDA-event time, and
     frac = achieved / the measured HBM peak.  `work_equivalent` gives the
     algorithmic bytes 8 E_alg + 16 V_alg + 4 W_out of a search that expands
-    every reachable vertex of every source, per second: closure reuse and
-    chained starts do far less than that work, so that figure exceeds the
+    every reachable vertex of every source, per second: sets that are shared
+    between sources make it far less work, so that figure exceeds the
     peak and is not a bandwidth fraction."""
     w_out = 11 * n  # nnz_u, nz_row_u, nnz_lc, 2 digests (u64), 128-bit L-mask per row
     bytes_alg = 8 * edges + 16 * vertices_alg + 4 * w_out
     t = kernel_ms / 1e3
     roof = {"bound": "hbm", "achieved": None, "peak": peak, "unit": "GB/s", "frac": None,
             "traffic": traffic, "peak_kind": peak_kind + " (MEASURED_PEAKS hbm_gbs)",
-            "kernel": "traverse_kernel", "kernel_ms": kernel_ms,
-            "traffic_source": "ncu, one full-size launch (profiles/traverse_<workload>.md)",
+            "kernel": "counting kernels of gsofa_hub.cu / gsofa_chain.cu", "kernel_ms": kernel_ms,
+            "traffic_source": "ncu, one full-size factorization (profiles/traverse_<workload>.md)",
             "inspected_edges_per_s": edges_trav / t,
             "work_equivalent": {"bytes_alg": bytes_alg, "gbs": bytes_alg / t / 1e9,
                                 "note": "algorithmic bytes of an ideal label search per second; "
-                                        "the kernel reuses closures, so this exceeds the peak"}}
+                                        "sources share reach sets, so this exceeds the peak"}}
     if traffic:
         roof["achieved"] = traffic / t / 1e9
         roof["frac"] = roof["achieved"] / peak

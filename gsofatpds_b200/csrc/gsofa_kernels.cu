@@ -1,4 +1,9 @@
-// gsofa_kernels.cu -- sm_100a kernels of the fill-path symbolic factorization.
+// gsofa_kernels.cu -- sm_100a kernels of the fill-path symbolic factorization:
+// ingest, supernodes, and traverse_kernel, which walks every source's closure.
+// Plain counting is done by gsofa_hub.cu and gsofa_chain.cu; traverse_kernel has
+// the calls that need closures one by one: the pattern pass, per-row L
+// statistics of symmetric patterns, the no-allocation entry point, and the
+// switches that turn closure reuse or top-down search off.
 //
 // Fill-path rule (the reference's, SOA symbfact_warp_centric_new_scheduling.cuh
 // :842-1001): (s,m), s != m, is an entry of L+U iff A(s,m) != 0 or a path

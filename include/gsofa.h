@@ -65,8 +65,8 @@ typedef struct gsofa_opts {
     /* rows per supernode chunk; the reference's max_supernode_size, argv[5]
      * of the SOA command line (symbfact_warp_centric_new_scheduling.cuh:2540) */
     int32_t max_supernode_size;
-    /* threads cooperating on one source traversal (CTA size: 128..1024,
-     * multiple of 32); 0 = autotuned */
+    /* threads cooperating on one chunk of sources (CTA size: 128..1024,
+     * multiple of 32); 0 = by size */
     int32_t threads_per_source;
     /* concurrent source traversals (CTAs); 0 = as many as fit on the GPU.
      * The reference's N_src_group (Compute_Src_group, :1031-1048) */
@@ -83,16 +83,18 @@ typedef struct gsofa_opts {
     int32_t heavy_row;
     /* sources with a smaller id always stay top-down; 0 = default (2048) */
     int32_t bu_min_source;
-    /* consecutive sources one CTA takes as a work item (the previous source's
-     * closure is reused inside a chunk); 0 = default */
+    /* consecutive sources one CTA takes as a work item (the previous sources'
+     * sets are reused inside a chunk); 0 = default */
     int32_t chunk_sources;
     /* closures of recently finished sources each CTA keeps for reuse
-     * (rounded down to a power of 2, at most 64); 0 = default */
+     * (rounded down to a power of 2, at most 64); 0 = default.  Used where
+     * closures are kept: the pattern pass, per-row L statistics of symmetric
+     * patterns, the no-allocation entry point and the diagnostic switches */
     int32_t cached_closures;
     /* how long (microseconds) a source search may wait, when the search of
      * the same chunk in the other direction is one source behind, for the
      * result that lets it start from the previous source's closure; 0 =
-     * default, < 0 = never wait */
+     * default, < 0 = never wait.  Used where cached_closures is */
     int32_t chain_wait_us;
     int32_t reserved;
 } gsofa_opts;
@@ -246,7 +248,7 @@ typedef struct gsofa_counts {
     double ms_device;         /* device time of the factorization (CUDA events) */
     double ms_traverse;       /* device time of the traversal kernel alone      */
     uint64_t sources_chained; /* source searches (U rows and L columns) that
-                               * started from the previous source's closure    */
+                               * started from a set known before them         */
 } gsofa_counts;
 int gsofa_result_counts(const gsofa_result* res, gsofa_counts* out);
 
