@@ -44,6 +44,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include "gsofa_device.cuh"
+#include "gsofa_label.h"
 
 namespace gsofa {
 
@@ -54,7 +55,6 @@ constexpr int kHubs = 4;  // two for the first window, one for each other
 constexpr int kBases = 2;  // arrays of totals: a source has at most two hubs to choose from
 constexpr int kMaxRounds = 192;  // label rounds before a matrix is left to the chain
 constexpr int kLabelThreads = 1024;
-constexpr int kNoLabel = 0x7f7f7f7f;
 constexpr int kExtraThreads = 256;
 constexpr int kJudgeAfter = 512;  // searches before a matrix may be left to the chain
 
@@ -134,13 +134,10 @@ __device__ __forceinline__ int dsm_min(unsigned a, int v) {
     asm volatile("atom.relaxed.cluster.shared::cluster.min.s32 %0, [%1], %2;" : "=r"(x) : "r"(a), "r"(v) : "memory");
     return x;
 }
-__device__ __forceinline__ unsigned dsm_or(unsigned a, unsigned v) {
-    unsigned x;
+__device__ __forceinline__ int dsm_or(unsigned a, int v) {
+    int x;
     asm volatile("atom.relaxed.cluster.shared::cluster.or.b32 %0, [%1], %2;" : "=r"(x) : "r"(a), "r"(v) : "memory");
     return x;
-}
-__device__ __forceinline__ void dsm_and(unsigned a, unsigned v) {
-    asm volatile("red.relaxed.cluster.shared::cluster.and.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 __device__ __forceinline__ int dsm_add(unsigned a, int v) {
     int x;
@@ -149,10 +146,10 @@ __device__ __forceinline__ int dsm_add(unsigned a, int v) {
 }
 
 // Labels of one (matrix, hub, direction) by one thread block cluster, spread
-// over its CTAs' shared memory: the labels and one bit per id that is queued,
-// 32-id words dealt out in turn.  A round expands the ids queued in the one
-// before; an id's bit is cleared before its label is read, so an improvement
-// is either read there or queues the id again.  Queues are in global memory.
+// over its CTAs' shared memory: a word per id (gsofa_label.h), groups of 32 ids
+// dealt out in turn.  A round expands the ids queued in the one before; one
+// atomic operation marks an id idle and reads its label, so an improvement is
+// either read there or queues the id again.  Queues are in global memory.
 __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch P) {
     extern __shared__ uint4 dyn_smem[];
     __shared__ int cnt[3];  // of rank 0: queued ids per round, in turn
@@ -169,9 +166,7 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
     const long long at = lam_at(P, M, h, d);
     const int mine = (nw + (int)C - 1) >> shift;  // words of this CTA, at most
     int32_t* const lam = reinterpret_cast<int32_t*>(dyn_smem);
-    uint32_t* const inq = reinterpret_cast<uint32_t*>(lam + 32 * mine);
     const unsigned lam_a = (unsigned)__cvta_generic_to_shared(lam);
-    const unsigned inq_a = (unsigned)__cvta_generic_to_shared(inq);
     const unsigned cnt_a = at_rank((unsigned)__cvta_generic_to_shared(cnt), 0);
     auto group_sync = [&]() {
         if (C == 1) __syncthreads();
@@ -181,16 +176,11 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
         const unsigned w = (unsigned)v >> 5;
         return at_rank(lam_a + 4 * (32 * (w >> shift) + ((unsigned)v & 31)), w & (C - 1));
     };
-    auto inq_of = [&](int v) {
-        const unsigned w = (unsigned)v >> 5;
-        return at_rank(inq_a + 4 * (w >> shift), w & (C - 1));
-    };
     int32_t* const q[2] = {P.lq + 2 * at, P.lq + 2 * at + M.hub_len};
     const int lane = threadIdx.x & 31;
     const int gw = (int)(rank * kLabelThreads + threadIdx.x) >> 5;
     const int nwarps = (int)C * (kLabelThreads / 32);
-    for (int v = threadIdx.x; v < 32 * mine; v += kLabelThreads) lam[v] = kNoLabel;
-    for (int w = threadIdx.x; w < mine; w += kLabelThreads) inq[w] = 0u;
+    for (int v = threadIdx.x; v < 32 * mine; v += kLabelThreads) lam[v] = kNoLabelWord;
     if (threadIdx.x == 0) {
         cnt[0] = 1;
         cnt[1] = cnt[2] = 0;
@@ -198,7 +188,7 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
     group_sync();
     if (rank == 0 && threadIdx.x == 0) {
         const int hub = hub_of(P, mi, h);
-        dsm_min(lam_of(hub), hub);
+        dsm_min(lam_of(hub), label_queued(hub));
         __stcg(q[0], hub);
     }
     group_sync();
@@ -217,8 +207,7 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
             if (lane < per && base + lane < count) {
                 const int u = __ldcg(cur + base + lane);
                 const int a0 = __ldg(G.rp + u), a1 = __ldg(G.rp + u + 1);
-                dsm_and(inq_of(u), ~(1u << (u & 31)));
-                nl = max(dsm_ld(lam_of(u)), u);
+                nl = label_queued(max(label_of_word(dsm_or(lam_of(u), kLabelIdle)), u));
                 s0 = a0 & ~3;
                 its = ((a1 & ~3) - s0) >> 2;
             }
@@ -239,15 +228,13 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
 #pragma unroll
                 for (int c = 0; c < 4; c++) lw[c] = ws[c] >= 0 ? dsm_ld(lam_of(ws[c])) : -1;
 #pragma unroll
-                for (int c = 0; c < 4; c++) lw[c] = onl < lw[c] ? dsm_min(lam_of(ws[c]), onl) : -1;
-                unsigned was[4], bal[4];
-#pragma unroll
                 for (int c = 0; c < 4; c++)
-                    was[c] = lw[c] > onl && ws[c] < bound ? dsm_or(inq_of(ws[c]), 1u << (ws[c] & 31)) : ~0u;
+                    lw[c] = label_of_word(onl) < label_of_word(lw[c]) ? dsm_min(lam_of(ws[c]), onl) : -1;
+                unsigned bal[4];
                 int k = 0;
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                    bal[c] = __ballot_sync(FULL_MASK, !((was[c] >> (ws[c] & 31)) & 1u));
+                    bal[c] = __ballot_sync(FULL_MASK, label_queues(lw[c], onl) && ws[c] < bound);
                     k += __popc(bal[c]);
                 }
                 if (k) {
@@ -270,8 +257,8 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
     if (r == kMaxRounds && dsm_ld(cnt_a + 4 * (r % 3)) != 0 && rank == 0 && threadIdx.x == 0)
         atomicExch(P.fallback + mi, 1);  // unfinished labels are too large
     for (int w = (int)rank + (int)C * (threadIdx.x >> 5); w < nw; w += (int)C * (kLabelThreads / 32)) {
-        // whole words: the ids from n on keep kNoLabel
-        P.lam[at + 32ll * w + lane] = lam[32 * (w >> shift) + lane];
+        // whole groups: the ids from n on have no label
+        P.lam[at + 32ll * w + lane] = label_of_word(lam[32 * (w >> shift) + lane]);
     }
     group_sync();  // no CTA leaves while another may still read its counts
 }
@@ -904,7 +891,7 @@ int hub_bases() { return kBases; }
 // The largest cluster's shared memory per CTA for a matrix of order n.
 size_t label_smem_bytes(int32_t n, int cluster) {
     const size_t words = (((size_t)n + 31) / 32 + (size_t)cluster - 1) / (size_t)cluster;
-    return 33 * 4 * words + 16;
+    return 32 * 4 * words + 16;
 }
 
 size_t hub_scan_bytes(long long tots, long long uses) {
