@@ -1118,46 +1118,29 @@ int gsofa::host::matrix_build(gsofa_ctx* ctx, cudaStream_t stream, int32_t* dsta
 // four copying threads).
 int gsofa::host::fetch_all(gsofa_ctx* ctx, const Fetch* f, int count) {
     size_t total = 0;
-    for (int k = 0; k < count; k++) {
-        if (!f[k].dst) continue;
-        if (!f[k].src)
-            return set_err(ctx, GSOFA_ERR_ARG, "requested array was not computed (option off)");
-        total += f[k].bytes;
-    }
+    int missing = 0;  // the arrays before a missing one are still brought
+    for (; missing < count && (!f[missing].dst || f[missing].src); missing++)
+        if (f[missing].dst) total += f[missing].bytes;
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     cudaError_t e = cudaSuccess;
-    if (total + 256 * (size_t)count <= kStageBytes && count <= 8) {
-        // arrays that lie one after another (256-byte steps) share a copy too
-        size_t at[8] = {}, used = 0;
-        for (int k = 0; k < count && e == cudaSuccess;) {
-            if (!f[k].dst || !f[k].bytes) {
-                k++;
-                continue;
-            }
-            const char* first = static_cast<const char*>(f[k].src);
-            at[k] = used;
-            size_t span = f[k].bytes;
-            int next = k + 1;
-            for (; next < count && f[next].dst && f[next].bytes; next++) {
-                const char* s = static_cast<const char*>(f[next].src);
-                if (s < first + span || s - (first + span) >= 256) break;
-                at[next] = used + (size_t)(s - first);
-                span = (size_t)(s - first) + f[next].bytes;
-            }
-            e = cudaMemcpyAsync(ctx->h_stage + used, first, span, cudaMemcpyDeviceToHost, ctx->stream);
-            used += span;
-            k = next;
-        }
+    if (total + kFetchStep * (size_t)count <= kStageBytes) {
+        const FetchPlan p = plan_fetch(f, missing);
+        for (int c = 0; c < p.copies && e == cudaSuccess; c++)
+            e = cudaMemcpyAsync(ctx->h_stage + p.copy[c].at, p.copy[c].src, p.copy[c].bytes,
+                                cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess && p.copies) e = cudaStreamSynchronize(ctx->stream);
+        for (int k = 0; k < missing && e == cudaSuccess; k++)
+            if (f[k].dst && f[k].bytes) memcpy(f[k].dst, ctx->h_stage + p.at[k], f[k].bytes);
+    } else {
+        for (int k = 0; k < missing && e == cudaSuccess; k++)
+            if (f[k].dst && f[k].bytes)
+                e = cudaMemcpyAsync(f[k].dst, f[k].src, f[k].bytes, cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        for (int k = 0; k < count && e == cudaSuccess; k++)
-            if (f[k].dst && f[k].bytes) memcpy(f[k].dst, ctx->h_stage + at[k], f[k].bytes);
-        return e == cudaSuccess ? GSOFA_OK : cuda_fail(ctx, e, "result fetch");
     }
-    for (int k = 0; k < count && e == cudaSuccess; k++)
-        if (f[k].dst && f[k].bytes)
-            e = cudaMemcpyAsync(f[k].dst, f[k].src, f[k].bytes, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    return e == cudaSuccess ? GSOFA_OK : cuda_fail(ctx, e, "result fetch");
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "result fetch");
+    if (missing < count)
+        return set_err(ctx, GSOFA_ERR_ARG, "requested array was not computed (option off)");
+    return GSOFA_OK;
 }
 
 // ============================================================================
@@ -1935,7 +1918,7 @@ int gsofa_result_counts(const gsofa_result* r, gsofa_counts* out) {
 
 static int fetch(const gsofa_result* r, void* dst, const void* src, size_t bytes) {
     if (dst && !src) return set_err(r->ctx, GSOFA_ERR_ARG, "requested array was not computed (option off)");
-    const Fetch f{dst, src, bytes};
+    const Fetch f{dst, src, bytes, nullptr};
     return fetch_all(r->ctx, &f, 1);
 }
 
@@ -1943,15 +1926,19 @@ int gsofa_result_row_counts(const gsofa_result* r, int32_t* nnz_u_row, int32_t* 
                             int32_t* nnz_l_col, int32_t* nnz_l_row) {
     if (!r) return GSOFA_ERR_ARG;
     const size_t b = 4 * (size_t)r->n;
-    const Fetch f[4] = {{nnz_u_row, r->nnz_u, b}, {nz_row_u, r->nz_row_u, b},
-                        {nnz_l_col, r->nnz_lc, b}, {nnz_l_row, r->nnz_lr, b}};
+    const Fetch f[4] = {{nnz_u_row, r->nnz_u, b, r->arena},
+                        {nz_row_u, r->nz_row_u, b, r->arena},
+                        {nnz_l_col, r->nnz_lc, b, r->arena},
+                        {nnz_l_row, r->nnz_lr, b, r->arena}};
     return fetch_all(r->ctx, f, 4);
 }
 
 int gsofa_result_digests(const gsofa_result* r, uint64_t* du, uint64_t* dlc, uint64_t* dlr) {
     if (!r) return GSOFA_ERR_ARG;
     const size_t b = 8 * (size_t)r->n;
-    const Fetch f[3] = {{du, r->dig_u, b}, {dlc, r->dig_lc, b}, {dlr, r->dig_lr, b}};
+    const Fetch f[3] = {{du, r->dig_u, b, r->arena},
+                        {dlc, r->dig_lc, b, r->arena},
+                        {dlr, r->dig_lr, b, r->arena}};
     return fetch_all(r->ctx, f, 3);
 }
 

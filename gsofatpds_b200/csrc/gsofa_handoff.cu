@@ -300,10 +300,11 @@ extern "C" int gsofa_result_supernodal(const gsofa_result* res, int64_t* nblocks
     if (nl) *nl = r->sn_nl;
     if (nu) *nu = r->sn_nu;
     const size_t nb = (size_t)r->sn_nblocks + 1;
-    const Fetch f[5] = {{block_start, r->sn_start, 4 * nb},
-                        {lptr, r->sn_lptr, 8 * nb},
-                        {lrows, r->sn_lrows, 4 * (size_t)r->sn_nl},
-                        {uptr, r->sn_uptr, 8 * nb},
-                        {ucols, r->sn_ucols, 4 * (size_t)r->sn_nu}};
+    // five allocations: a copy each, one wait
+    const Fetch f[5] = {{block_start, r->sn_start, 4 * nb, nullptr},
+                        {lptr, r->sn_lptr, 8 * nb, nullptr},
+                        {lrows, r->sn_lrows, 4 * (size_t)r->sn_nl, nullptr},
+                        {uptr, r->sn_uptr, 8 * nb, nullptr},
+                        {ucols, r->sn_ucols, 4 * (size_t)r->sn_nu, nullptr}};
     return fetch_all(ctx, f, 5);
 }

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/gsofa.h"
+#include "gsofa_fetch.h"
 #include "gsofa_internal.h"
 
 struct gsofa_ctx {
@@ -252,12 +253,7 @@ struct DeviceScratch {
 };
 
 constexpr size_t kStageBytes = 2u << 20;  // ctx->h_stage
-// Device arrays to the caller's memory, complete on return.
-struct Fetch {
-    void* dst;
-    const void* src;
-    size_t bytes;
-};
+// Device arrays to the caller's memory, complete on return (at most kMaxFetch).
 int fetch_all(gsofa_ctx* ctx, const Fetch* f, int count);
 
 constexpr int kDefaultBuAlpha = 0;  // top-down only unless a caller asks
