@@ -150,7 +150,9 @@ __device__ inline bool serve_claim(const ServeLaunch& V, int* slot_out, long lon
             }
         }
         if (c0) return false;
-        if (global_ns() - t0 > (unsigned long long)V.idle_ns) return false;
+        // lane 0's clock decides for the warp
+        const int idle = global_ns() - t0 > (unsigned long long)V.idle_ns;
+        if (__shfl_sync(FULL_MASK, idle, 0)) return false;
         __nanosleep(ns);
         if (ns < 2048) ns <<= 1;
     }

@@ -533,7 +533,10 @@ __global__ void __launch_bounds__(kExtraThreads, 1024 / kExtraThreads) extra_ker
             mi = lo;
         }
         const MatDesc& M = P.mats[mi];
-        if (ld_vol_i32(P.fallback + mi)) continue;
+        // one lane looks: another warp may set the flag between two lanes' loads
+        int left = 0;
+        if (lane == 0) left = ld_vol_i32(P.fallback + mi);
+        if (__shfl_sync(FULL_MASK, left, 0)) continue;
         if (M.asym[1] != 0) {  // repeated entries: the chain counts a row's distinct ids
             if (lane == 0) atomicExch(P.fallback + mi, 1);
             continue;
