@@ -8,6 +8,7 @@
 #include <cmath>
 #include <map>
 #include <cerrno>
+#include <climits>
 #include <chrono>
 #include <cstdarg>
 #include <cstdio>
@@ -339,13 +340,17 @@ MatDesc make_desc(const gsofa_matrix* m, const gsofa_result* r, long long base) 
 // Whether the counting traversals (gsofa_chain.cu, gsofa_hub.cu) run these
 // options: they always reuse closures and search top-down, so the diagnostic
 // switches take traverse_kernel.  Per-row L statistics come from gsofa_hub.cu
-// alone: with them, only matrices that all go there.
+// alone: with them, only matrices that all go there.  The hubs' arrays of one
+// launch hold fewer than 2^31 entries, the count their scans take.
 bool chain_runs(const gsofa_opts& o, const gsofa_matrix* const* mats, int32_t count) {
     if ((o.flags & (GSOFA_NO_MERGE | GSOFA_NO_CHAIN)) || o.bu_alpha > 0) return false;
-    if (o.flags & GSOFA_L_ROW_STATS)
-        for (int32_t i = 0; i < count; i++)
-            if (method_of(mats[i]) == METHOD_CHAIN) return false;
-    return true;
+    long long hub_rows = 0;
+    for (int32_t i = 0; i < count; i++) {
+        const int32_t method = method_of(mats[i]);
+        if (method == METHOD_CHAIN && (o.flags & GSOFA_L_ROW_STATS)) return false;
+        if (method == METHOD_HUB) hub_rows += mats[i]->n + 32ll;
+    }
+    return hub_rows * std::max(hub_count(), 2 * hub_bases()) <= INT_MAX;
 }
 
 int plan_chain(gsofa_ctx* ctx, int32_t nmax, long long total_sources, bool all_sym, const gsofa_opts* o,
@@ -403,13 +408,15 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     *c = HubCfg{};
     long long sources = 0, off = 0, items = 0;
     int32_t n_max = 0;
-    int hubs = 0;
+    int hubs = 0, k = 0;
     for (MatDesc& d : *descs) {
+        k++;
         if (d.method == METHOD_CHAIN) continue;
         sources += 2ll * d.n;
         n_max = std::max(n_max, d.n);
         if (d.method != METHOD_HUB) continue;
         hubs++;
+        L->hub_mats = k;
         d.hub_off = off;
         d.hub_len = ((long long)d.n + 1 + 31) & ~31ll;
         off += d.hub_len;

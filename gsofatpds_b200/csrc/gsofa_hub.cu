@@ -264,8 +264,8 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
 }
 
 // The same by the whole GPU, one launch per round (labels, queues, counts in
-// global memory): blockIdx.y is the job, a launch that finds nothing queued
-// ends at once.  `last`: the matrix goes to the chain if this round leaves ids
+// global memory): `per` CTAs a job, a launch that finds nothing queued ends at
+// once.  `last`: the matrix goes to the chain if this round leaves ids
 // queued.
 __global__ void label_start_kernel(HubLaunch P) {
     const int job = blockIdx.x;
@@ -279,17 +279,17 @@ __global__ void label_start_kernel(HubLaunch P) {
     P.lcnt[4ll * job] = 1;
 }
 
-__global__ void __launch_bounds__(kLabelThreads) label_round_kernel(HubLaunch P, int r, int last) {
-    const int job = blockIdx.y;
+__global__ void __launch_bounds__(kLabelThreads) label_round_kernel(HubLaunch P, int per_job, int r, int last) {
+    const int job = blockIdx.x / per_job, part = blockIdx.x % per_job;
     int32_t* const cnt = P.lcnt + 4ll * job;
     const int count = cnt[r % 3];
-    if (blockIdx.x == 0 && threadIdx.x == 0) cnt[(r + 2) % 3] = 0;
+    if (part == 0 && threadIdx.x == 0) cnt[(r + 2) % 3] = 0;
     if (count == 0) return;
     const int mi = job / (2 * kHubs), h = (job >> 1) % kHubs, d = job & 1;
-    if (last && blockIdx.x == 0 && threadIdx.x == 0) atomicExch(P.fallback + mi, 1);
+    if (last && part == 0 && threadIdx.x == 0) atomicExch(P.fallback + mi, 1);
     const int lane = threadIdx.x & 31;
-    const int gw = (blockIdx.x * kLabelThreads + threadIdx.x) >> 5;
-    const int nwarps = (int)gridDim.x * (kLabelThreads / 32);
+    const int gw = (part * kLabelThreads + threadIdx.x) >> 5;
+    const int nwarps = per_job * (kLabelThreads / 32);
     // few ids queued: fewer per warp, so that more warps work
     const int per = count >= 32 * nwarps ? 32 : (count + nwarps - 1) / nwarps;
     if (gw * per >= count) return;
@@ -359,8 +359,9 @@ __global__ void __launch_bounds__(kLabelThreads) label_round_kernel(HubLaunch P,
 
 // The changes over s of the hub set's totals.  A warp per word: lane j is id
 // v = 32 w + j, in the set from s = label + 1 on, above s until s = v.
-__global__ void event_kernel(HubLaunch P, int digests) {
-    const int mi = blockIdx.y / (2 * kHubs), h = (blockIdx.y >> 1) % kHubs, d = blockIdx.y & 1;
+__global__ void event_kernel(HubLaunch P, int per_job, int digests) {
+    const int job = blockIdx.x / per_job, part = blockIdx.x % per_job;
+    const int mi = job / (2 * kHubs), h = (job >> 1) % kHubs, d = job & 1;
     const MatDesc& M = P.mats[mi];
     if (M.method != METHOD_HUB) return;
     const int n = M.n;
@@ -372,8 +373,7 @@ __global__ void event_kernel(HubLaunch P, int digests) {
     Tot* const D = P.base + (2ll * (h == 1) + d) * P.total + M.hub_off;
     const int lane = threadIdx.x & 31;
     const int nw = (n + 31) >> 5;
-    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nw;
-         w += (gridDim.x * blockDim.x) >> 5) {
+    for (int w = (part * blockDim.x + threadIdx.x) >> 5; w < nw; w += (per_job * blockDim.x) >> 5) {
         const int v = 32 * w + lane;
         const int lv = v < n ? __ldg(lam + v) : INT_MAX;
         int in = -1, out = -1, ve = -1, deg = 0;
@@ -856,12 +856,12 @@ struct UseSum {
 // Per-row L statistics from the hubs' sets: row v is in the set of column s
 // when label(v) < s < v, so it gains the columns that took hub h's set between
 // those two ids: a difference of prefix sums (l_use, scanned).
-__global__ void lrow_kernel(HubLaunch P) {
-    const int mi = blockIdx.y;
+__global__ void lrow_kernel(HubLaunch P, int per_mat) {
+    const int mi = blockIdx.x / per_mat, part = blockIdx.x % per_mat;
     const MatDesc& M = P.mats[mi];
     if (M.method != METHOD_HUB || P.fallback[mi]) return;
     const int d = M.asym[0] == 0 ? 0 : 1;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < M.n; v += gridDim.x * blockDim.x) {
+    for (int v = part * blockDim.x + threadIdx.x; v < M.n; v += per_mat * blockDim.x) {
         unsigned long long count = 0, dig = 0;
         for (int h = 0; h < kHubs; h++) {
             const int l = __ldg(P.lam + lam_at(P, M, h, d) + v);
@@ -919,12 +919,18 @@ int large_occupancy(int block, size_t smem) {
     return e == cudaSuccess ? occ : 0;
 }
 
+// CTAs for each of `jobs` jobs of at most `most` CTAs' work: together no more than
+// some tens of waves.
+static int parts(int most, int jobs) { return std::max(1, std::min({most, 1024, (1 << 17) / jobs})); }
+
 cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(L.zeroed, 0, c.zeroed_bytes, st);
     if (e != cudaSuccess) return e;
     if (c.any_hub) {
-        const int jobs = L.nmats * 2 * kHubs;
-        hub_kernel<<<dim3((unsigned)(L.nmats * kHubs), 16), 256, 0, st>>>(L);
+        // (grids are one-dimensional: a batch may have more jobs than the 65,535
+        // that a second dimension takes)
+        const int jobs = L.hub_mats * 2 * kHubs;
+        hub_kernel<<<dim3((unsigned)(L.hub_mats * kHubs), 16), 256, 0, st>>>(L);
         if (c.cluster > 0) {
             const size_t smem = label_smem_bytes(c.n_max, c.cluster);
             e = cudaFuncSetAttribute(label_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -947,12 +953,13 @@ cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStr
             e = cudaMemsetAsync(L.lam, 0x7f, 4ull * 2 * kHubs * (size_t)L.total, st);
             if (e != cudaSuccess) return e;
             label_start_kernel<<<jobs, 32, 0, st>>>(L);
-            const dim3 grid((unsigned)std::max(8, 2 * c.sm_count / std::min(L.nmats, 8)), (unsigned)jobs);
+            const int per = std::max(8, 2 * c.sm_count / std::min(L.hub_mats, 8));
             for (int r = 0; r < kMaxRounds; r++)
-                label_round_kernel<<<grid, kLabelThreads, 0, st>>>(L, r, r == kMaxRounds - 1);
+                label_round_kernel<<<per * jobs, kLabelThreads, 0, st>>>(L, per, r, r == kMaxRounds - 1);
         }
         const int words = (int)((c.n_max + 31) / 32);
-        event_kernel<<<dim3((unsigned)std::min((words + 7) / 8, 1024), (unsigned)jobs), 256, 0, st>>>(L, digests);
+        const int per = parts((words + 7) / 8, jobs);
+        event_kernel<<<per * jobs, 256, 0, st>>>(L, per, digests);
         size_t sb = c.scan_bytes;
         e = cub::DeviceScan::InclusiveScan(c.scan_tmp, sb, L.base, L.base, TotSum(), (int)(2 * kBases * L.total), st);
         if (e != cudaSuccess) return e;
@@ -968,7 +975,8 @@ cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStr
         size_t sb = c.scan_bytes;
         e = cub::DeviceScan::InclusiveScan(c.scan_tmp, sb, L.l_use, L.l_use, UseSum(), (int)(kHubs * L.total), st);
         if (e != cudaSuccess) return e;
-        lrow_kernel<<<dim3((unsigned)std::min((c.n_max + 255) / 256, 1024), (unsigned)L.nmats), 256, 0, st>>>(L);
+        const int per = parts((c.n_max + 255) / 256, L.hub_mats);
+        lrow_kernel<<<per * L.hub_mats, 256, 0, st>>>(L, per);
     }
     commit_kernel<<<L.nmats, 32, 0, st>>>(L);
     return cudaGetLastError();

@@ -211,6 +211,7 @@ constexpr int kDirectMax = 1024;
 struct HubLaunch {
     const MatDesc* mats;
     int32_t nmats;
+    int32_t hub_mats;                  // the matrices with a hub are among the first hub_mats
     int group;                         // consecutive sources per work item
     long long total;
     long long total_items;

@@ -1,7 +1,6 @@
 """Hub labels (csrc/gsofa_hub.cu) against the oracle, bit for bit: the label
 searches of one launch run in clusters of 1 to 16 CTAs, by how many matrices
 share it, and labels of a random pattern are lowered many times."""
-import numpy as np
 import pytest
 
 from gsofatpds_b200 import gen
