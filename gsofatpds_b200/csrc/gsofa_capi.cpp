@@ -51,10 +51,39 @@ int cuda_fail(gsofa_ctx* ctx, cudaError_t e, const char* where) {
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, #call); \
     } while (0)
 
+void dev_free_on(gsofa_ctx* ctx, void* p, size_t bytes, cudaStream_t stream) {
+    if (!p) return;
+    bytes = (bytes + 255) & ~(size_t)255;
+    cudaFreeAsync(p, stream);
+    ctx->used -= std::min(ctx->used, bytes);
+}
+
+size_t kept_workspace(const gsofa_ctx* ctx) {
+    return ctx->hub_ws_bytes + ctx->queue_bytes + ctx->gbitmap_bytes + ctx->gprev_bytes;
+}
+
+// Gives back the workspace that factorizations keep between calls.
+void drop_workspace(gsofa_ctx* ctx) {
+    struct {
+        void** p;
+        size_t* bytes;
+    } const kept[] = {{&ctx->hub_ws, &ctx->hub_ws_bytes},
+                      {&ctx->queue, &ctx->queue_bytes},
+                      {&ctx->gbitmap, &ctx->gbitmap_bytes},
+                      {&ctx->gprev, &ctx->gprev_bytes}};
+    for (const auto& k : kept) {
+        dev_free_on(ctx, *k.p, *k.bytes, ctx->stream);
+        *k.p = nullptr;
+        *k.bytes = 0;
+    }
+}
+
 int dev_alloc_on(gsofa_ctx* ctx, size_t bytes, void** p, cudaStream_t stream) {
     *p = nullptr;
     if (bytes == 0) return GSOFA_OK;
     bytes = (bytes + 255) & ~(size_t)255;
+    // a factorization's kept workspace gives way to what a caller asks for
+    if (ctx->used + bytes > ctx->budget && !ctx->factoring) drop_workspace(ctx);
     if (ctx->used + bytes > ctx->budget)
         return set_err(ctx, GSOFA_ERR_OOM_BUDGET,
                        "allocation of %zu bytes exceeds the budget (%zu of %zu bytes in use)",
@@ -66,13 +95,6 @@ int dev_alloc_on(gsofa_ctx* ctx, size_t bytes, void** p, cudaStream_t stream) {
     }
     ctx->used += bytes;
     return GSOFA_OK;
-}
-
-void dev_free_on(gsofa_ctx* ctx, void* p, size_t bytes, cudaStream_t stream) {
-    if (!p) return;
-    bytes = (bytes + 255) & ~(size_t)255;
-    cudaFreeAsync(p, stream);
-    ctx->used -= std::min(ctx->used, bytes);
 }
 
 int dev_alloc(gsofa_ctx* ctx, size_t bytes, void** p) {
@@ -403,7 +425,7 @@ int32_t method_of(const gsofa_matrix* m) {
 }
 
 bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, void* ws,
-              size_t* bytes, HubLaunch* L, HubCfg* c) {
+              size_t* bytes, size_t room, HubLaunch* L, HubCfg* c) {
     *L = HubLaunch{};
     *c = HubCfg{};
     long long sources = 0, off = 0, items = 0;
@@ -458,6 +480,11 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     int occ = large_occupancy(c->large_block, c->large_smem);
     if (occ <= 0) occ = 1;
     c->large_grid = occ * ctx->sm_count;
+    c->extra_grid = extra_ctas_per_sm() * ctx->sm_count;
+    if (o.sources_in_flight > 0) {
+        c->large_grid = std::min(c->large_grid, o.sources_in_flight);
+        c->extra_grid = std::min(c->extra_grid, o.sources_in_flight);
+    }
     L->queue_stride = n_max;
     if (o.flags & GSOFA_DEBUG_QUEUE_CAP) L->queue_stride = std::min<long long>(L->queue_stride, 64);
     c->l_rows = (o.flags & GSOFA_L_ROW_STATS) != 0;
@@ -488,6 +515,12 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     L->lq = static_cast<int32_t*>(place(8 * 2 * (size_t)W * T));
     L->large = static_cast<unsigned long long*>(place(8 * (size_t)sources));
     c->scan_tmp = place(c->scan_bytes);
+    // the large searches' CTAs, by far the most of it, take turns: as many as fit
+    auto large_bytes = [&]() {
+        return align256((size_t)c->large_grid * (size_t)L->queue_stride * 4) +
+               align256(L->large_smem ? 0 : (size_t)c->large_grid * (size_t)L->bitmap_words * 4);
+    };
+    while (c->large_grid > 1 && at + large_bytes() > room) c->large_grid = (c->large_grid + 1) / 2;
     L->queue = static_cast<int32_t*>(place((size_t)c->large_grid * (size_t)L->queue_stride * 4));
     L->gbm = static_cast<uint32_t*>(
         place(L->large_smem ? 0 : (size_t)c->large_grid * (size_t)L->bitmap_words * 4));
@@ -556,9 +589,10 @@ long long chain_chunk(const gsofa_opts& o, long long total_sources, int32_t nmax
 
 // Runs the traversal (and optionally supernodes / pattern) for `count`
 // matrices in one persistent launch.  results[i] must be freshly allocated.
-int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
-               const gsofa_opts* o, gsofa_result** res, long long sample_stride = 1,
-               bool counting = true) {
+// counting: by the counting traversals where chain_runs, else by traverse_kernel.
+int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
+                    const gsofa_opts* o, gsofa_result** res, long long sample_stride,
+                    bool counting) {
     int32_t nmax = 0;
     long long total_sources = 0, weight = 0;
     bool all_sym = true;
@@ -623,14 +657,20 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
             top_items += d.top_items;
             items += (m->n + CL.chunk - 1) / CL.chunk - d.top_items;
         }
+        ccfg.grid = (int)std::max(1ll, std::min<long long>(ccfg.grid, items));
         size_t hub_bytes = 0;
-        if (plan_hub(ctx, &descs, *o, nullptr, &hub_bytes, &HL, &hcfg)) {
+        // the hubs' workspace may take what the budget leaves beside the chain's
+        const size_t chain_bytes = align256(chain_queue_bytes(ctx, ccfg, nmax, top_items > 0)) +
+                                   align256(chain_gbm_bytes(ctx, ccfg, top_items > 0)) +
+                                   align256(sizeof(MatDesc) * (size_t)count);
+        const size_t others = ctx->used - std::min(ctx->used, ctx->hub_ws_bytes + ctx->queue_bytes + ctx->gbitmap_bytes);
+        const size_t room = ctx->budget > others + chain_bytes ? ctx->budget - others - chain_bytes : 0;
+        if (plan_hub(ctx, &descs, *o, nullptr, &hub_bytes, room, &HL, &hcfg)) {
             rc = ensure(ctx, &ctx->hub_ws, &ctx->hub_ws_bytes, hub_bytes);
             if (rc) return rc;
-            hub = plan_hub(ctx, &descs, *o, ctx->hub_ws, &hub_bytes, &HL, &hcfg);
+            hub = plan_hub(ctx, &descs, *o, ctx->hub_ws, &hub_bytes, room, &HL, &hcfg);
             HL.status = dstatus;
         }
-        ccfg.grid = (int)std::max(1ll, std::min<long long>(ccfg.grid, items));
         rc = ensure(ctx, &ctx->queue, &ctx->queue_bytes, chain_queue_bytes(ctx, ccfg, nmax, top_items > 0));
         if (!rc)
             rc = ensure(ctx, &ctx->gbitmap, &ctx->gbitmap_bytes, chain_gbm_bytes(ctx, ccfg, top_items > 0));
@@ -740,7 +780,7 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
     if (any && (o->flags & GSOFA_L_ROW_STATS)) {
         // the chain does not make them: all of it again
         for (int32_t i = 0; i < count; i++) CK(result_clear(res[i], ctx->stream));
-        return run_factor(ctx, mats, count, o, res, sample_stride, false);
+        return run_factor_with(ctx, mats, count, o, res, sample_stride, false);
     }
     if (any) {
         long long items = 0, sources = 0;
@@ -841,6 +881,32 @@ int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
         k.ms_traverse = (double)ms_trav;
     }
     return GSOFA_OK;
+}
+
+// The same, within the budget: when the counting traversals' workspace does not
+// fit, nothing of earlier calls is kept and traverse_kernel, whose workspace is
+// smaller, counts.
+int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count, const gsofa_opts* o,
+               gsofa_result** res, long long sample_stride = 1) {
+    ctx->factoring = true;
+    int rc = run_factor_with(ctx, mats, count, o, res, sample_stride, true);
+    if (rc == GSOFA_ERR_OOM_BUDGET) {
+        drop_workspace(ctx);
+        rc = GSOFA_OK;
+        for (int32_t i = 0; i < count && rc == GSOFA_OK; i++) {
+            gsofa_result* r = res[i];
+            dev_free(ctx, r->parena, r->pbytes);
+            r->parena = nullptr;
+            r->pbytes = 0;
+            r->uptr = r->lptr = nullptr;
+            r->ucols = r->lrows = nullptr;
+            const cudaError_t e = result_clear(r, ctx->stream);
+            if (e != cudaSuccess) rc = cuda_fail(ctx, e, "result arrays");
+        }
+        if (rc == GSOFA_OK) rc = run_factor_with(ctx, mats, count, o, res, sample_stride, false);
+    }
+    ctx->factoring = false;
+    return rc;
 }
 
 int validate_opts(gsofa_ctx* ctx, const gsofa_opts* o) {
@@ -1620,26 +1686,16 @@ static void batch_free(gsofa_batch* b) {
     delete b;
 }
 
-int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
-                       const gsofa_opts* opts, gsofa_batch** out) {
-    if (!ctx || !out || count <= 0 || !mats) return GSOFA_ERR_ARG;
-    *out = nullptr;
-    std::lock_guard<std::recursive_mutex> g(ctx->mu);
-    gsofa_opts o;
-    if (opts) o = *opts; else gsofa_opts_default(&o);
-    int rc = validate_opts(ctx, &o);
-    if (rc) return rc;
-    if (o.flags & GSOFA_PATTERN)
-        return set_err(ctx, GSOFA_ERR_UNSUPPORTED, "a captured batch cannot materialise patterns");
+// counting: by the counting traversals where chain_runs, else by traverse_kernel.
+static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
+                             const gsofa_opts& o, bool counting, gsofa_batch** out) {
+    int rc = GSOFA_OK;
     int32_t nmax = 1;
-    for (int32_t i = 0; i < count; i++) {
-        if (!mats[i] || mats[i]->ctx != ctx)
-            return set_err(ctx, GSOFA_ERR_ARG, "matrix %d is null or from another context", i);
-        nmax = std::max(nmax, mats[i]->n);
-    }
-    if (cudaSetDevice(ctx->device) != cudaSuccess) return set_err(ctx, GSOFA_ERR_CUDA, "cudaSetDevice");
     long long weight = 0;
-    for (int32_t i = 0; i < count; i++) weight += chunk_weight(ctx, mats[i]);
+    for (int32_t i = 0; i < count; i++) {
+        nmax = std::max(nmax, mats[i]->n);
+        weight += chunk_weight(ctx, mats[i]);
+    }
     gsofa_batch* b = new (std::nothrow) gsofa_batch();
     if (!b) return set_err(ctx, GSOFA_ERR_OOM_BUDGET, "host allocation failed");
     b->ctx = ctx;
@@ -1656,7 +1712,7 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
         b->res[(size_t)i]->batch_owned = true;
     }
     // (per-row L statistics could not be made again inside the captured launch)
-    const bool chain = !(o.flags & GSOFA_L_ROW_STATS) && chain_runs(o, mats, count);
+    const bool chain = counting && !(o.flags & GSOFA_L_ROW_STATS) && chain_runs(o, mats, count);
     ChainCfg ccfg;
     LaunchCfg cfg;
     // the chain's shape for the symmetric matrices it takes, and for those that
@@ -1721,7 +1777,6 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
         }
         b->items = items;
     }
-    if (chain) hub = plan_hub(ctx, &descs, o, nullptr, &sz_hub, &HL, &hcfg);
     const size_t sz_small = 256;
     const size_t sz_desc = align256(sizeof(MatDesc) * (size_t)count);
     const size_t sz_seg = align256(sizeof(long long) * ((size_t)count + 1));
@@ -1734,7 +1789,11 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     const size_t sz_gbm =
         chain ? align256(std::max(chain_gbm_bytes(ctx, ccfg, top_items > 0), chain_gbm_bytes(ctx, lcfg, false)))
         : cfg.smem_bitmap ? 0 : align256((size_t)cfg.grid * (size_t)cfg.words * 4);
-    b->ws_bytes = sz_small + sz_desc + sz_seg + sz_cnt + sz_q + sz_ring + sz_gbm + sz_hub;
+    b->ws_bytes = sz_small + sz_desc + sz_seg + sz_cnt + sz_q + sz_ring + sz_gbm;
+    const size_t taken = ctx->used - std::min(ctx->used, kept_workspace(ctx)) + b->ws_bytes;
+    const size_t room = ctx->budget > taken ? ctx->budget - taken : 0;
+    if (chain) hub = plan_hub(ctx, &descs, o, nullptr, &sz_hub, room, &HL, &hcfg);
+    b->ws_bytes += sz_hub;
     rc = dev_alloc(ctx, b->ws_bytes, &b->ws);
     if (rc) return fail(rc);
     char* p = reinterpret_cast<char*>(b->ws);
@@ -1754,7 +1813,7 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
     uint32_t* dgbm = sz_gbm ? reinterpret_cast<uint32_t*>(p) : nullptr;
     p += sz_gbm;
     if (hub) {
-        plan_hub(ctx, &descs, o, p, &sz_hub, &HL, &hcfg);
+        plan_hub(ctx, &descs, o, p, &sz_hub, room, &HL, &hcfg);
         HL.mats = ddesc;
         HL.status = dstatus;
     }
@@ -1868,6 +1927,27 @@ int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t 
         return fail(cuda_fail(ctx, e, "cudaGraphInstantiate"));
     *out = b;
     return GSOFA_OK;
+}
+
+int gsofa_batch_create(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
+                       const gsofa_opts* opts, gsofa_batch** out) {
+    if (!ctx || !out || count <= 0 || !mats) return GSOFA_ERR_ARG;
+    *out = nullptr;
+    std::lock_guard<std::recursive_mutex> g(ctx->mu);
+    gsofa_opts o;
+    if (opts) o = *opts; else gsofa_opts_default(&o);
+    int rc = validate_opts(ctx, &o);
+    if (rc) return rc;
+    if (o.flags & GSOFA_PATTERN)
+        return set_err(ctx, GSOFA_ERR_UNSUPPORTED, "a captured batch cannot materialise patterns");
+    for (int32_t i = 0; i < count; i++)
+        if (!mats[i] || mats[i]->ctx != ctx)
+            return set_err(ctx, GSOFA_ERR_ARG, "matrix %d is null or from another context", i);
+    if (cudaSetDevice(ctx->device) != cudaSuccess) return set_err(ctx, GSOFA_ERR_CUDA, "cudaSetDevice");
+    rc = batch_create_with(ctx, mats, count, o, true, out);
+    // the counting traversals' workspace does not fit: traverse_kernel's is smaller
+    if (rc == GSOFA_ERR_OOM_BUDGET) rc = batch_create_with(ctx, mats, count, o, false, out);
+    return rc;
 }
 
 int gsofa_batch_run(gsofa_batch* b) {

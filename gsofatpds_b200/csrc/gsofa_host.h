@@ -55,6 +55,7 @@ struct gsofa_ctx {
     size_t scan_tmp_bytes = 0;
     void* hub_ws = nullptr;
     size_t hub_ws_bytes = 0;
+    bool factoring = false;  // the workspace above is in use
 };
 
 struct gsofa_matrix {
@@ -181,10 +182,10 @@ void fill_chain_launch(ChainLaunch* L, const ChainCfg& c, const gsofa_opts& o, i
 // Which counting traversal a matrix takes (its host_sym must be known).
 int32_t method_of(const gsofa_matrix* m);
 // A launch of gsofa_hub.cu over descriptors whose methods are set: fills their
-// hub_* fields, `L` and `c`, and places the workspace of *bytes in `ws` (null:
-// sizes only).  False: no matrix takes it.
+// hub_* fields, `L` and `c`, and places the workspace of *bytes, at most `room`
+// if fewer CTAs for large searches can bring it there, in `ws` (null: sizes only).  False: no matrix takes it.
 bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, void* ws,
-              size_t* bytes, HubLaunch* L, HubCfg* c);
+              size_t* bytes, size_t room, HubLaunch* L, HubCfg* c);
 // Consecutive sources per work item.
 long long chain_chunk(const gsofa_opts& o, long long total_sources, int32_t nmax, int grid, bool sym);
 // Result arrays of an n-row matrix, zero-initialised on `stream`.

@@ -890,6 +890,7 @@ __global__ void commit_kernel(HubLaunch P) {
 
 int hub_count() { return kHubs; }
 int hub_bases() { return kBases; }
+int extra_ctas_per_sm() { return 1024 / kExtraThreads; }
 
 // The largest cluster's shared memory per CTA for a matrix of order n.
 size_t label_smem_bytes(int32_t n, int cluster) {
@@ -968,7 +969,7 @@ cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStr
     if ((e = cudaFuncSetAttribute(extra_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
         return e;
     const long long want = (L.total_items + kExtraThreads / 32 - 1) / (kExtraThreads / 32);
-    extra_kernel<<<(int)std::min<long long>(want, (long long)c.sm_count * (1024 / kExtraThreads)), kExtraThreads, smem, st>>>(L);
+    extra_kernel<<<(int)std::min<long long>(want, c.extra_grid), kExtraThreads, smem, st>>>(L);
     if (c.large_block == 256) large_kernel<256><<<c.large_grid, 256, c.large_smem, st>>>(L);
     else large_kernel<1024><<<c.large_grid, 1024, c.large_smem, st>>>(L);
     if (c.any_hub && c.l_rows) {
