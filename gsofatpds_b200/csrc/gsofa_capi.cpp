@@ -535,8 +535,8 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
 // at most one per SM, beside the rest (3.55 ms; the 64^3 mesh 3.3 either way).
 // Smaller meshes lose more by the SMs those CTAs take (170 x 170: 0.82 -> 1.0 ms,
 // a batch of 64 matrices 5.9 -> 7.2).
-long long chain_top_items(const gsofa_opts& o, int32_t n, long long chunk, bool sym) {
-    if (!sym || o.sources_in_flight > 0 || n < 131072) return 0;
+long long chain_top_items(const gsofa_opts& o, int32_t n, long long chunk) {
+    if (o.sources_in_flight > 0 || n < 131072) return 0;
     const long long chunks = (n + chunk - 1) / chunk;
     return std::min(chunks - 1, (n / 50 + chunk - 1) / chunk);
 }
@@ -573,17 +573,13 @@ cudaError_t launch_chain_both(gsofa_ctx* ctx, const ChainLaunch& L, const ChainC
     return e;
 }
 
-long long chain_chunk(const gsofa_opts& o, long long total_sources, int32_t nmax, int grid, bool sym) {
+long long chain_chunk(const gsofa_opts& o, long long total_sources, int32_t nmax, int grid) {
     if (o.chunk_sources > 0) return o.chunk_sources;
-    // A chunk's first source is searched from nothing.  Symmetric patterns:
-    // about two items per CTA, at most 128 sources each, since their items
-    // differ in cost (64^3 mesh: 3.3 ms with 128 sources, 4.0 with 443; 40^3:
-    // 0.92 with 54, 1.09 with 108).  The others come here without a core that a
-    // hub lies in, and such first searches may read most of the matrix: one
-    // item per CTA.
-    if (!sym) return std::max(1ll, (total_sources + grid - 1) / grid);
-    // (64 where no matrix has the 1,024-thread launch: a batch's meshes of up to
-    // 30,000 rows 5.9 -> 5.3 ms)
+    // A chunk's first source is searched from nothing: about two items per CTA,
+    // at most 128 sources each, since items differ in cost (64^3 mesh: 3.3 ms with
+    // 128 sources, 4.0 with 443; 40^3: 0.92 with 54, 1.09 with 108).  At most 64
+    // where no matrix has the 1,024-thread launch (a batch's meshes of up to
+    // 30,000 rows 5.9 -> 5.3 ms).
     return std::max(1ll, std::min(nmax < 131072 ? 64ll : 128ll, (total_sources + 2ll * grid - 1) / (2ll * grid)));
 }
 
@@ -595,12 +591,10 @@ int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t cou
                     bool counting) {
     int32_t nmax = 0;
     long long total_sources = 0, weight = 0;
-    bool all_sym = true;
     for (int32_t i = 0; i < count; i++) {
         nmax = std::max(nmax, mats[i]->n);
         weight += chunk_weight(ctx, mats[i]);
         total_sources += mats[i]->n;
-        all_sym = all_sym && mats[i]->host_sym > 0;
     }
     const bool chain = counting && chain_runs(*o, mats, count);
     const bool pattern = (o->flags & GSOFA_PATTERN) != 0;
@@ -630,20 +624,11 @@ int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t cou
     long long top_items = 0;
     if (chain) {
         long long chain_sources = 0;
-        bool chain_sym = true;
-        for (int32_t i = 0; i < count; i++) {
-            if (method_of(mats[i]) != METHOD_CHAIN) continue;
-            chain_sources += mats[i]->n;
-            chain_sym = chain_sym && mats[i]->host_sym > 0;
-        }
-        // with none of its own, the chain's shape is that of what it may be left
-        if (chain_sources == 0) {
-            chain_sources = total_sources;
-            chain_sym = all_sym;
-        }
-        rc = plan_chain(ctx, std::max(nmax, 1), chain_sources, chain_sym, o, false, &ccfg);
+        for (int32_t i = 0; i < count; i++)
+            if (method_of(mats[i]) == METHOD_CHAIN) chain_sources += mats[i]->n;
+        rc = plan_chain(ctx, std::max(nmax, 1), chain_sources, true, o, false, &ccfg);
         if (rc) return rc;
-        CL.chunk = (int)chain_chunk(*o, chain_sources, nmax, ccfg.grid, chain_sym);
+        CL.chunk = (int)chain_chunk(*o, chain_sources, nmax, ccfg.grid);
         long long items = 0;
         place(CL.chunk, 1);
         for (int32_t k = 0; k < count; k++) {
@@ -653,7 +638,7 @@ int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t cou
             d.item_base = items;
             d.top_base = top_items;
             if (d.method != METHOD_CHAIN) continue;
-            d.top_items = stride > 1 ? 0 : chain_top_items(*o, m->n, CL.chunk, m->host_sym > 0);
+            d.top_items = stride > 1 ? 0 : chain_top_items(*o, m->n, CL.chunk);
             top_items += d.top_items;
             items += (m->n + CL.chunk - 1) / CL.chunk - d.top_items;
         }
@@ -741,26 +726,6 @@ int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t cou
     CK(cudaMemsetAsync(ctx->small, 0, 128, ctx->stream));
     L.mats = CL.mats = HL.mats = reinterpret_cast<const MatDesc*>(ddesc);
 
-    // the supernodes and the read-back of the matrices of `mine` (all: null)
-    auto finish = [&](const std::vector<char>* mine) -> int {
-        for (int32_t k = 0; k < count; k++) {
-            const int32_t i = order[(size_t)k];
-            if (mine && !(*mine)[(size_t)k]) continue;
-            if ((o->flags & GSOFA_SUPERNODES) && mats[i]->n > 0)
-                CK(launch_supernodes(mats[i]->n, o->max_supernode_size, res[i]->nz_row_u, res[i]->lmask,
-                                     res[i]->sflags, res[i]->counters, ctx->stream));
-        }
-        CK(cudaEventRecord(ctx->ev1, ctx->stream));
-        for (int32_t k = 0; k < count; k++) {
-            const int32_t i = order[(size_t)k];
-            if (mine && !(*mine)[(size_t)k]) continue;
-            CK(cudaMemcpyAsync(ctx->h_counters + (size_t)i * CNT_SLOTS, res[i]->counters, 8 * CNT_SLOTS,
-                               cudaMemcpyDeviceToHost, ctx->stream));
-        }
-        CK(cudaMemcpyAsync(ctx->h_status, dstatus, 4, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        return check_status(ctx);
-    };
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     if (hub) {
         CK(launch_hub(HL, hcfg, (o->flags & GSOFA_DIGESTS) != 0, ctx->stream));
@@ -771,66 +736,59 @@ int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t cou
     if (!chain && L.total_items > 0)
         CK(launch_traverse(L, cfg.block, cfg.grid, cfg.smem_bitmap, cfg.smem, ctx->stream));
     CK(cudaEventRecord(ctx->evt, ctx->stream));
-    rc = finish(nullptr);
+    for (int32_t k = 0; k < count; k++) {
+        const int32_t i = order[(size_t)k];
+        if ((o->flags & GSOFA_SUPERNODES) && mats[i]->n > 0)
+            CK(launch_supernodes(mats[i]->n, o->max_supernode_size, res[i]->nz_row_u, res[i]->lmask,
+                                 res[i]->sflags, res[i]->counters, ctx->stream));
+    }
+    CK(cudaEventRecord(ctx->ev1, ctx->stream));
+    for (int32_t i = 0; i < count; i++)
+        CK(cudaMemcpyAsync(ctx->h_counters + (size_t)i * CNT_SLOTS, res[i]->counters, 8 * CNT_SLOTS,
+                           cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->h_status, dstatus, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    rc = check_status(ctx);
     if (rc) return rc;
-    // matrices the hubs' launch left to the chain (few: no core, repeated entries)
-    std::vector<char> left((size_t)count, 0);
-    bool any = false;
-    for (int32_t k = 0; k < count && hub; k++) any |= (left[(size_t)k] = ctx->h_fallback[k] != 0);
-    if (any && (o->flags & GSOFA_L_ROW_STATS)) {
-        // the chain does not make them: all of it again
-        for (int32_t i = 0; i < count; i++) CK(result_clear(res[i], ctx->stream));
-        return run_factor_with(ctx, mats, count, o, res, sample_stride, false);
-    }
-    if (any) {
-        long long items = 0, sources = 0;
-        bool sym = true;
-        for (int32_t k = 0; k < count; k++) {
-            if (!left[(size_t)k]) continue;
-            sources += descs[(size_t)k].n;
-            sym = sym && mats[order[(size_t)k]]->host_sym > 0;
+    float ms_f = 0.f, ms_trav_f = 0.f;
+    CK(cudaEventElapsedTime(&ms_f, ctx->ev0, ctx->ev1));
+    CK(cudaEventElapsedTime(&ms_trav_f, ctx->ev0, ctx->evt));
+    double ms = ms_f, ms_trav = ms_trav_f;
+    std::vector<unsigned long long> totals(ctx->h_counters, ctx->h_counters + (size_t)count * CNT_SLOTS);
+
+    // matrices that the hubs' launch left: traverse_kernel counts them
+    std::vector<int32_t> left;
+    for (int32_t k = 0; k < count && hub; k++)
+        if (ctx->h_fallback[k]) left.push_back(order[(size_t)k]);
+    if (!left.empty()) {
+        std::vector<const gsofa_matrix*> lm;
+        std::vector<gsofa_result*> lr;
+        for (const int32_t i : left) {
+            lm.push_back(mats[i]);
+            lr.push_back(res[i]);
+            CK(result_clear(res[i], ctx->stream));
         }
-        rc = plan_chain(ctx, std::max(nmax, 1), sources, sym, o, false, &ccfg);
+        gsofa_opts lo = *o;
+        lo.flags &= ~(uint32_t)GSOFA_PATTERN;  // made below, with the others'
+        rc = run_factor_with(ctx, lm.data(), (int32_t)lm.size(), &lo, lr.data(), sample_stride, false);
         if (rc) return rc;
-        CL.chunk = (int)chain_chunk(*o, sources, nmax, ccfg.grid, sym);
-        for (int32_t k = 0; k < count; k++) {
-            MatDesc& d = descs[(size_t)k];
-            // the others have no items now
-            d.method = left[(size_t)k] ? METHOD_CHAIN : d.method;
-            d.item_base = items;
-            d.top_items = 0;
-            if (!left[(size_t)k]) continue;
-            items += (d.n + CL.chunk - 1) / CL.chunk;
-            CK(cudaMemsetAsync(res[order[(size_t)k]]->counters, 0, 8 * CNT_SLOTS, ctx->stream));
-        }
-        ccfg.grid = (int)std::max(1ll, std::min<long long>(ccfg.grid, items));
-        rc = ensure(ctx, &ctx->queue, &ctx->queue_bytes, (size_t)ccfg.grid * (size_t)std::max(nmax, 1) * 4);
-        if (!rc)
-            rc = ensure(ctx, &ctx->gbitmap, &ctx->gbitmap_bytes,
-                        (size_t)ccfg.grid * (size_t)ccfg.gbm_count * (size_t)ccfg.words * 4);
-        if (rc) return rc;
-        fill_chain_launch(&CL, ccfg, *o, nmax);
-        CL.queue = L.queue = reinterpret_cast<int32_t*>(ctx->queue);
-        CL.gbm = L.gbitmap = reinterpret_cast<uint32_t*>(ctx->gbitmap);
-        CL.total_items = (items + stride - 1) / stride;
-        CK(cudaMemsetAsync(ctx->small, 0, 128, ctx->stream));
-        CK(cudaMemcpyAsync(ddesc, descs.data(), sizeof(MatDesc) * (size_t)count, cudaMemcpyHostToDevice,
-                           ctx->stream));
-        CK(launch_chain(CL, ccfg.block, false, ccfg.grid, ccfg.smem, ctx->stream));
-        CK(cudaEventRecord(ctx->evt, ctx->stream));
-        rc = finish(&left);
-        if (rc) return rc;
+        for (size_t j = 0; j < left.size(); j++)
+            std::copy_n(ctx->h_counters + j * CNT_SLOTS, (size_t)CNT_SLOTS,
+                        totals.data() + (size_t)left[j] * CNT_SLOTS);
+        ms += lr[0]->counts.ms_device;
+        ms_trav += lr[0]->counts.ms_traverse;
+        // the buffers may have grown
+        L.queue = reinterpret_cast<int32_t*>(ctx->queue);
+        L.gbitmap = reinterpret_cast<uint32_t*>(ctx->gbitmap);
+        L.gprev = reinterpret_cast<uint32_t*>(ctx->gprev);
     }
-    float ms = 0.f, ms_trav = 0.f;
-    CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
-    CK(cudaEventElapsedTime(&ms_trav, ctx->ev0, ctx->evt));
 
     // pattern pass (second traversal writing sorted ids)
     if (pattern) {
         for (int32_t k = 0; k < count; k++) {
             const int32_t i = order[(size_t)k];
             gsofa_result* r = res[i];
-            const unsigned long long* c = ctx->h_counters + (size_t)i * CNT_SLOTS;
+            const unsigned long long* c = totals.data() + (size_t)i * CNT_SLOTS;
             const size_t N = (size_t)r->n + 1;
             const size_t nu = c[CNT_NNZ_U], nl = c[CNT_NNZ_L];
             size_t total = align256(8 * N) * 2 + align256(4 * std::max<size_t>(nu, 1)) +
@@ -865,7 +823,7 @@ int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t cou
 
     for (int32_t i = 0; i < count; i++) {
         gsofa_result* r = res[i];
-        const unsigned long long* c = ctx->h_counters + (size_t)i * CNT_SLOTS;
+        const unsigned long long* c = totals.data() + (size_t)i * CNT_SLOTS;
         gsofa_counts& k = r->counts;
         k.n = r->n;
         k.fill_count = c[CNT_FILLS];
@@ -1533,18 +1491,16 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
             auto_chunk = default_chunk(total_sources, c0.grid);
         }
         long long chain_sources = 0;
-        bool chain_sym = true;
         for (int32_t i = 0; i < count; i++) {
             if (!chain || method_of(mats[i]) != METHOD_CHAIN) continue;
             walks = true;
             chain_sources += mats[i]->n;
-            chain_sym = chain_sym && mats[i]->host_sym > 0;
         }
         ChainCfg cc;
         if (chain_sources > 0 &&
-            plan_chain(ctx, std::max(nmax, 1), chain_sources, chain_sym, &base, false, &cc) == GSOFA_OK) {
+            plan_chain(ctx, std::max(nmax, 1), chain_sources, true, &base, false, &cc) == GSOFA_OK) {
             best.threads_per_source = cc.block;
-            auto_chunk = chain_chunk(base, chain_sources, nmax, cc.grid, chain_sym);
+            auto_chunk = chain_chunk(base, chain_sources, nmax, cc.grid);
             best.chunk_sources = (int32_t)auto_chunk;
         }
         ctx->err.clear();
@@ -1715,27 +1671,22 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
     const bool chain = counting && !(o.flags & GSOFA_L_ROW_STATS) && chain_runs(o, mats, count);
     ChainCfg ccfg;
     LaunchCfg cfg;
-    // the chain's shape for the symmetric matrices it takes, and for those that
-    // the hubs' launch may leave it
-    long long chain_sources = 0, left_sources = 0;
+    // the chain's shape for the symmetric matrices, and traverse_kernel's for
+    // those that the hubs' launch may leave it
+    long long chain_sources = 0, left_weight = 0;
     int32_t chain_nmax = 1, left_nmax = 1;
     for (int32_t i = 0; i < count; i++) {
         const bool mine = method_of(mats[i]) == METHOD_CHAIN;
-        (mine ? chain_sources : left_sources) += mats[i]->n;
+        if (mine) chain_sources += mats[i]->n;
+        else left_weight += chunk_weight(ctx, mats[i]);
         (mine ? chain_nmax : left_nmax) = std::max(mine ? chain_nmax : left_nmax, mats[i]->n);
     }
-    ChainCfg lcfg;
-    if (chain) {
-        rc = plan_chain(ctx, chain_nmax, chain_sources, true, &o, false, &ccfg);
-        if (!rc) rc = plan_chain(ctx, left_nmax, left_sources, false, &o, false, &lcfg);
-    } else {
-        rc = plan_launch(ctx, nmax, &o, &cfg);
-    }
+    if (chain) rc = plan_chain(ctx, chain_nmax, chain_sources, true, &o, false, &ccfg);
+    if (!rc) rc = plan_launch(ctx, chain ? left_nmax : nmax, &o, &cfg);
     if (rc) return fail(rc);
-    const long long chunk = chain ? chain_chunk(o, chain_sources, chain_nmax, ccfg.grid, true)
-                            : o.chunk_sources > 0 ? o.chunk_sources
-                                                  : default_chunk(weight, cfg.grid);
-    const long long left_chunk = chain_chunk(o, left_sources, left_nmax, lcfg.grid > 0 ? lcfg.grid : 1, false);
+    const long long walk_chunk =
+        o.chunk_sources > 0 ? o.chunk_sources : default_chunk(chain ? left_weight : weight, cfg.grid);
+    const long long chunk = chain ? chain_chunk(o, chain_sources, chain_nmax, ccfg.grid) : walk_chunk;
     const long long per_chunk = chain ? 1 : 2;  // work items
     const bool merge = !(o.flags & GSOFA_NO_MERGE);
     int ring = o.cached_closures > 0 ? o.cached_closures : kDefaultRing;
@@ -1758,6 +1709,7 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
     size_t sz_hub = 0;
     bool hub = false;
     long long top_items = 0, left_items = 0;
+    std::vector<MatDesc> left;  // of traverse_kernel's launch beside the chain
     if (chain) {
         long long items = 0;
         for (int32_t k = 0; k < count; k++) {
@@ -1766,29 +1718,28 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
             d.method = method_of(m);
             d.item_base = items;
             d.top_base = top_items;
-            d.left_base = left_items;
             if (d.method == METHOD_CHAIN) {
-                d.top_items = chain_top_items(o, m->n, chunk, true);
+                d.top_items = chain_top_items(o, m->n, chunk);
                 top_items += d.top_items;
                 items += (m->n + chunk - 1) / chunk - d.top_items;
-            } else {
-                left_items += (m->n + left_chunk - 1) / left_chunk;
+            } else if (m->n > 0) {
+                left_items += 2 * ((m->n + walk_chunk - 1) / walk_chunk);
             }
         }
         b->items = items;
+        cfg.grid = (int)std::min<long long>(cfg.grid, left_items);
     }
     const size_t sz_small = 256;
-    const size_t sz_desc = align256(sizeof(MatDesc) * (size_t)count);
+    const size_t sz_desc = align256(sizeof(MatDesc) * (size_t)count) * (left_items ? 2 : 1);
     const size_t sz_seg = align256(sizeof(long long) * ((size_t)count + 1));
     const size_t sz_cnt = align256(8ull * CNT_SLOTS * (size_t)count);
-    const size_t sz_q = align256(chain ? std::max(chain_queue_bytes(ctx, ccfg, chain_nmax, top_items > 0),
-                                                  chain_queue_bytes(ctx, lcfg, left_nmax, false))
-                                       : (size_t)cfg.grid * (size_t)nmax * 4);
-    const size_t sz_ring =
-        merge && !chain ? align256((size_t)cfg.grid * (size_t)ring * (size_t)cfg.words * 4) : 0;
+    const size_t walk_q = (size_t)cfg.grid * (size_t)(chain ? left_nmax : nmax) * 4;
+    const size_t walk_gbm = cfg.smem_bitmap ? 0 : (size_t)cfg.grid * (size_t)cfg.words * 4;
+    const size_t sz_q =
+        align256(chain ? std::max(chain_queue_bytes(ctx, ccfg, chain_nmax, top_items > 0), walk_q) : walk_q);
+    const size_t sz_ring = merge ? align256((size_t)cfg.grid * (size_t)ring * (size_t)cfg.words * 4) : 0;
     const size_t sz_gbm =
-        chain ? align256(std::max(chain_gbm_bytes(ctx, ccfg, top_items > 0), chain_gbm_bytes(ctx, lcfg, false)))
-        : cfg.smem_bitmap ? 0 : align256((size_t)cfg.grid * (size_t)cfg.words * 4);
+        align256(chain ? std::max(chain_gbm_bytes(ctx, ccfg, top_items > 0), walk_gbm) : walk_gbm);
     b->ws_bytes = sz_small + sz_desc + sz_seg + sz_cnt + sz_q + sz_ring + sz_gbm;
     const size_t taken = ctx->used - std::min(ctx->used, kept_workspace(ctx)) + b->ws_bytes;
     const size_t room = ctx->budget > taken ? ctx->budget - taken : 0;
@@ -1801,6 +1752,7 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
     int32_t* dstatus = reinterpret_cast<int32_t*>(p + 64);
     p += sz_small;
     MatDesc* ddesc = reinterpret_cast<MatDesc*>(p);
+    MatDesc* dleft = reinterpret_cast<MatDesc*>(p + align256(sizeof(MatDesc) * (size_t)count));
     p += sz_desc;
     long long* dseg = reinterpret_cast<long long*>(p);
     p += sz_seg;
@@ -1819,9 +1771,20 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
     }
     for (int32_t k = 0; k < count; k++)  // matrix i's counters at slot i, whatever its launch order
         descs[(size_t)k].counters = dcnt + (size_t)order[(size_t)k] * CNT_SLOTS;
+    long long left_base = 0;
+    for (int32_t k = 0; k < count && left_items; k++) {
+        MatDesc d = descs[(size_t)k];
+        if (d.method == METHOD_CHAIN || d.n <= 0) continue;
+        d.item_base = left_base;
+        left_base += 2 * ((d.n + walk_chunk - 1) / walk_chunk);
+        d.only_if = HL.fallback + k;
+        left.push_back(d);
+    }
     cudaError_t e;
     if ((e = cudaMemcpyAsync(ddesc, descs.data(), sizeof(MatDesc) * (size_t)count,
                              cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess ||
+        (!left.empty() && (e = cudaMemcpyAsync(dleft, left.data(), sizeof(MatDesc) * left.size(),
+                                               cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess) ||
         (e = cudaMemcpyAsync(dseg, seg.data(), sizeof(long long) * ((size_t)count + 1),
                              cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess ||
@@ -1832,12 +1795,12 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
         return fail(cuda_fail(ctx, e, "batch set-up"));
 
     TraverseLaunch L{};
-    L.mats = ddesc;
-    L.nmats = count;
-    L.total_items = b->items;
-    L.work_counter = wc;
+    L.mats = chain ? dleft : ddesc;
+    L.nmats = chain ? (int32_t)left.size() : count;
+    L.total_items = chain ? left_items : b->items;
+    L.work_counter = chain ? wc + 2 : wc;
     L.queue = dq;
-    L.queue_stride = nmax;
+    L.queue_stride = chain ? left_nmax : nmax;
     L.gbitmap = dgbm;
     L.bitmap_words = cfg.words;
     L.status = dstatus;
@@ -1847,7 +1810,7 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
     L.bu_min_src = o.bu_min_source > 0 ? o.bu_min_source : kBuMinSource;
     L.heavy_len = o.heavy_row > 0 ? ((o.heavy_row + 3) & ~3) : kDefaultHeavyRow;
     L.gprev = dring;
-    L.chunk = (int)chunk;
+    L.chunk = (int)walk_chunk;
     L.merge = merge ? 1 : 0;
     L.chain = merge && !(o.flags & GSOFA_NO_CHAIN) ? 1 : 0;
     L.chain_wait_ns = chain_wait_ns(o);
@@ -1863,16 +1826,7 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
     CL.chunk = (int)chunk;
     CL.sample_stride = 1;
     CL.status = dstatus;
-    ChainLaunch LL = CL;  // what the hubs' launch leaves
-    if (chain) {
-        fill_chain_launch(&CL, ccfg, o, chain_nmax);
-        fill_chain_launch(&LL, lcfg, o, left_nmax);
-        LL.chunk = (int)left_chunk;
-        LL.items = ITEMS_LEFT;
-        LL.total_items = left_items;
-        LL.work_counter = wc + 2;
-        LL.fallback = HL.fallback;
-    }
+    if (chain) fill_chain_launch(&CL, ccfg, o, chain_nmax);
 
     // capture: reset -> traversal -> supernodes -> read-back
     struct Fork {  // the hubs' branch: of use during the capture alone
@@ -1893,7 +1847,7 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
     e = cudaMemsetAsync(b->ws, 0, 128, ctx->stream);
     if (e == cudaSuccess) e = launch_batch_reset(ddesc, count, ctx->stream);
     if (e == cudaSuccess && chain) {
-        // the two traversals side by side, then what the first leaves to the chain
+        // the two traversals side by side, then what the hubs' launch leaves
         if (hub) {
             e = cudaEventRecord(hf.fork, ctx->stream);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(hf.stream, hf.fork, 0);
@@ -1903,10 +1857,9 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
         if (e == cudaSuccess) e = launch_chain_both(ctx, CL, ccfg, top_items);
         if (e == cudaSuccess && hub) {
             e = cudaStreamWaitEvent(ctx->stream, hf.join, 0);
-            if (e == cudaSuccess) e = launch_chain(LL, lcfg.block, false, lcfg.grid, lcfg.smem, ctx->stream);
         }
     }
-    if (e == cudaSuccess && b->items > 0 && !chain)
+    if (e == cudaSuccess && L.total_items > 0)
         e = launch_traverse(L, cfg.block, cfg.grid, cfg.smem_bitmap, cfg.smem, ctx->stream);
     if (e == cudaSuccess && (o.flags & GSOFA_SUPERNODES))
         e = launch_supernodes_batch(ddesc, count, o.max_supernode_size, dseg, seg[(size_t)count],

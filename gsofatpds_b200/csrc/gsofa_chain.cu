@@ -879,11 +879,10 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) chain_kernel(ChainLaunch 
             const unsigned long long c = atomicAdd(P.work_counter, 1ull);
             const long long it = (long long)c < P.total_items ? (long long)c * stride : -1;
             if (it >= 0) {
-                SM.mi = P.items == ITEMS_TOP    ? find_matrix<&MatDesc::top_base>(P.mats, P.nmats, it)
-                        : P.items == ITEMS_LEFT ? find_matrix<&MatDesc::left_base>(P.mats, P.nmats, it)
-                                                : find_matrix(P.mats, P.nmats, it);
+                SM.mi = P.items == ITEMS_TOP ? find_matrix<&MatDesc::top_base>(P.mats, P.nmats, it)
+                                             : find_matrix(P.mats, P.nmats, it);
                 copy_desc<false>(&SD, P.mats + SM.mi);
-                SM.skip = P.items == ITEMS_LEFT && !P.fallback[SM.mi];
+                SM.skip = 0;
                 SM.sym = SD.asym[0] == 0;
                 SM.dup = SD.asym[1] != 0;
             }
@@ -897,10 +896,9 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) chain_kernel(ChainLaunch 
         const long long clen = SERVE ? (long long)M.chunk : (long long)P.chunk;
         const long long nchunks = ((long long)n + clen - 1) / clen;
         // largest sources first; M.top_items of them are the other launch's
-        const long long local = SERVE                   ? SM.item
-                                : P.items == ITEMS_TOP  ? SM.item - M.top_base
-                                : P.items == ITEMS_LEFT ? SM.item - M.left_base
-                                                        : SM.item - M.item_base + M.top_items;
+        const long long local = SERVE                  ? SM.item
+                                : P.items == ITEMS_TOP ? SM.item - M.top_base
+                                                       : SM.item - M.item_base + M.top_items;
         const long long chunk = nchunks - 1 - local;
         const int s_first = (int)(chunk * clen);
         const int s_end = SM.skip ? s_first : (int)min((long long)n, (chunk + 1) * clen);

@@ -170,7 +170,7 @@ bool chain_runs(const gsofa_opts& o, const gsofa_matrix* const* mats, int32_t co
 int plan_chain(gsofa_ctx* ctx, int32_t nmax, long long total_sources, bool all_sym, const gsofa_opts* o,
                bool serve, ChainCfg* c);
 // The chunks of a matrix of n rows that the launch of larger CTAs takes.
-long long chain_top_items(const gsofa_opts& o, int32_t n, long long chunk, bool sym);
+long long chain_top_items(const gsofa_opts& o, int32_t n, long long chunk);
 // Both launches of the chain on ctx->stream and beside it: `top` (`top_items`
 // items, workspace after the first launch's) and the rest.
 cudaError_t launch_chain_both(gsofa_ctx* ctx, const ChainLaunch& L, const ChainCfg& c, long long top_items);
@@ -187,7 +187,7 @@ int32_t method_of(const gsofa_matrix* m);
 bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, void* ws,
               size_t* bytes, size_t room, HubLaunch* L, HubCfg* c);
 // Consecutive sources per work item.
-long long chain_chunk(const gsofa_opts& o, long long total_sources, int32_t nmax, int grid, bool sym);
+long long chain_chunk(const gsofa_opts& o, long long total_sources, int32_t nmax, int grid);
 // Result arrays of an n-row matrix, zero-initialised on `stream`.
 int result_alloc_on(gsofa_ctx* ctx, int32_t n, uint32_t flags, int32_t mss, cudaStream_t stream,
                     gsofa_result** out);

@@ -36,8 +36,11 @@
 //
 // A matrix of at most kDirectMax rows has every source searched alone, without
 // a hub.  A matrix in which more than a quarter of the searches outgrow the
-// table (no core that the hub lies in: meshes) is left to gsofa_chain.cu, and
-// so are matrices with repeated entries in a row.
+// table (no core that the hub lies in: meshes) is left, and so are matrices with
+// repeated entries in a row: traverse_kernel counts them, whose reuse of closures
+// does not need a core (200,000-row band of 4 without one: 13 ms, 248 by
+// gsofa_chain.cu; 90,000-row mesh with a third of its couplings one-sided: 16 ms,
+// 26 by it).
 #include <algorithm>
 #include <climits>
 
@@ -53,10 +56,10 @@ namespace {
 constexpr int kWindows = 3;
 constexpr int kHubs = 4;  // two for the first window, one for each other
 constexpr int kBases = 2;  // arrays of totals: a source has at most two hubs to choose from
-constexpr int kMaxRounds = 192;  // label rounds before a matrix is left to the chain
+constexpr int kMaxRounds = 192;  // label rounds before a matrix is left to traverse_kernel
 constexpr int kLabelThreads = 1024;
 constexpr int kExtraThreads = 256;
-constexpr int kJudgeAfter = 512;  // searches before a matrix may be left to the chain
+constexpr int kJudgeAfter = 512;  // searches before a matrix may be left
 
 struct WarpTable {
     uint32_t key[kSlots];
@@ -265,8 +268,7 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
 
 // The same by the whole GPU, one launch per round (labels, queues, counts in
 // global memory): `per` CTAs a job, a launch that finds nothing queued ends at
-// once.  `last`: the matrix goes to the chain if this round leaves ids
-// queued.
+// once.  `last`: the matrix is left if this round leaves ids queued.
 __global__ void label_start_kernel(HubLaunch P) {
     const int job = blockIdx.x;
     const int mi = job / (2 * kHubs), h = (job >> 1) % kHubs, d = job & 1;
@@ -537,7 +539,7 @@ __global__ void __launch_bounds__(kExtraThreads, 1024 / kExtraThreads) extra_ker
         int left = 0;
         if (lane == 0) left = ld_vol_i32(P.fallback + mi);
         if (__shfl_sync(FULL_MASK, left, 0)) continue;
-        if (M.asym[1] != 0) {  // repeated entries: the chain counts a row's distinct ids
+        if (M.asym[1] != 0) {  // repeated entries: traverse_kernel counts a row's distinct ids
             if (lane == 0) atomicExch(P.fallback + mi, 1);
             continue;
         }
@@ -877,7 +879,7 @@ __global__ void lrow_kernel(HubLaunch P, int per_mat) {
     }
 }
 
-// The counters of every matrix that was not left to the chain.
+// The counters of every matrix that was not left.
 __global__ void commit_kernel(HubLaunch P) {
     const int mi = blockIdx.x;
     const MatDesc& M = P.mats[mi];

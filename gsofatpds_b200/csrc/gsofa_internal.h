@@ -79,7 +79,9 @@ struct MatDesc {
     // larger CTAs, and the first of them there
     long long top_items;
     long long top_base;
-    long long left_base;        // its first item in the launch of what gsofa_hub.cu leaves
+    // traverse_kernel: only when this device word is not 0 (null: always).  Set
+    // in a batch's launch of what gsofa_hub.cu may leave
+    const int32_t* only_if;
     // gsofa_hub.cu: place of the matrix in its arrays (a multiple of 32), the
     // room there (n + 1 rounded up), first work item and items (a power of two)
     long long hub_off;
@@ -163,7 +165,6 @@ struct TraverseLaunch {
 enum : int {
     ITEMS_MAIN = 0,  // the matrices' chunks but the top_items
     ITEMS_TOP = 1,   // those
-    ITEMS_LEFT = 2,  // the chunks of the matrices with a fallback flag
 };
 struct ChainLaunch {
     const MatDesc* mats;               // device array
@@ -182,7 +183,6 @@ struct ChainLaunch {
     int list_cap;                      // new ids of a search before the whole CTA takes it
     long long sample_stride;           // > 1: only every stride-th item (autotuner timing)
     int32_t* status;                   // device error word
-    const int32_t* fallback;           // ITEMS_LEFT: per matrix, gsofa_hub.cu left it to the chain
     ServeLaunch serve;                 // serving kernel only
 };
 // sizes of a set relative to the current source: ids above it, ids below it,
@@ -223,7 +223,7 @@ struct HubLaunch {
     Tot* base;                         // per base, direction and source: the hub set's totals
     int32_t* stamp;                    // as lam
     int32_t* lcnt;                     // 4 per label job
-    int32_t* fallback;                 // per matrix: left to the chain
+    int32_t* fallback;                 // per matrix: left to traverse_kernel
     int32_t* judged;                   // per matrix: searches done, searches too large
     unsigned long long* counters;      // per matrix, CNT_SLOTS
     int* large_count;

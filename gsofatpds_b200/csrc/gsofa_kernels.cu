@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) traverse_kernel(TraverseL
             if (it >= 0) {
                 SM.mi = find_matrix(P.mats, P.nmats, it * stride);
                 copy_desc<false>(&SD, P.mats + SM.mi);
-                SM.skip = 0;
+                SM.skip = SD.only_if != nullptr && *SD.only_if == 0;
                 SM.sym = SD.asym != nullptr && *SD.asym == 0;
             }
             SM.item = it;

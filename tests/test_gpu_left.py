@@ -1,0 +1,98 @@
+"""What the hubs' launch leaves (matrices without a core, repeated entries) is
+counted by traverse_kernel: the same results as the oracle, beside matrices that
+it does not leave; no slower than that kernel alone by more than the attempt;
+and its device time holds both."""
+import time
+
+import numpy as np
+import pytest
+
+from gsofatpds_b200 import gen
+from tests.helpers import scrambled_csr
+from tests.test_gpu_parity import check_full, ctx, oracle_full  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def oriented(t):
+    """A mesh with a third of its couplings from lower to higher ids only."""
+    n, rp, col = t
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    keep = (rows == col) | ((rows + col) % 3 == 0) | (rows > col)
+    return gen.from_coo(n, rows[keep], col[keep])
+
+
+def doubled(t, seed):
+    n, rp, col = t
+    return scrambled_csr(np.random.default_rng(seed), [set(col[rp[v]:rp[v + 1]]) for v in range(n)],
+                         shuffle_rows=False, dup_prob=0.2)
+
+
+def plain(t):
+    beg, end = gen.csr_to_beg_end(t[1])
+    return beg, end, t[2]
+
+
+MIX = [
+    lambda: plain(gen.circuit_like(3000, target_nnz=27000, seed=31)),
+    lambda: plain(gen.random_banded(5000, bw=2, extra=0, seed=9)),
+    lambda: plain(gen.grid_nd((40, 40), "5")),
+    lambda: doubled(gen.random_extra(2500, 3, seed=32), 1),
+    lambda: plain(oriented(gen.grid_nd((60, 60), "5"))),
+    lambda: doubled(gen.random_extra(600, 2, seed=33), 2),
+    lambda: doubled(gen.grid_nd((35, 33), "5"), 3),
+    lambda: plain(gen.random_extra(900, 2, seed=34)),
+]
+
+
+def test_left_beside_the_others(ctx):  # noqa: F811
+    ts = [f() for f in MIX]
+    refs = [oracle_full(*t, pattern=True) for t in ts]
+    mats = [ctx.load_csr(*t) for t in ts]
+    for kw in (dict(), dict(l_row_stats=True), dict(pattern=True)):
+        for group in ([0, 1, 2, 3, 4, 5, 6, 7], [0, 1, 3, 4, 5, 7], [1], [3], [5]):
+            results = ctx.factor_batch([mats[i] for i in group], **kw)
+            for i, res in zip(group, results):
+                check_full(res, *refs[i], l_rows="l_row_stats" in kw)
+                if "pattern" in kw:
+                    np.testing.assert_array_equal(res.pattern_u()[1], refs[i][0]["Ucols"])
+                    np.testing.assert_array_equal(res.pattern_l()[1], refs[i][1]["Ucols"])
+                res.close()
+    for kw in (dict(), dict(l_row_stats=True)):
+        b = ctx.batch(mats, **kw)
+        for _ in range(3):
+            b.run()
+            for i, ref in enumerate(refs):
+                check_full(b.result(i), *ref, l_rows="l_row_stats" in kw)
+        b.close()
+    for m in mats:
+        m.close()
+
+
+def best(ctx, m, **kw):  # noqa: F811
+    wall, dev = [], []
+    for _ in range(5):
+        t = time.perf_counter()
+        res = ctx.factor(m, **kw)
+        wall.append((time.perf_counter() - t) * 1e3)
+        dev.append(res.counts["ms_device"])
+        res.close()
+    return min(wall), min(dev)
+
+
+@pytest.mark.parametrize("name", ["band", "mesh"])
+def test_no_core_costs_little_more_than_traverse_kernel(ctx, name):  # noqa: F811
+    t = gen.random_banded(80000, bw=4, extra=0, seed=6) if name == "band" else oriented(
+        gen.grid_nd((170, 170), "5"))
+    m = ctx.load_rowptr(*t[1:])
+    _, default = best(ctx, m)
+    _, alone = best(ctx, m, bu_alpha=1, bu_min_source=1 << 30)  # a diagnostic option: traverse_kernel
+    m.close()
+    assert default < 2 * alone + 3
+
+
+def test_device_time_holds_the_attempt(ctx):  # noqa: F811
+    m = ctx.load_rowptr(*oriented(gen.grid_nd((43, 43, 43), "7"))[1:])
+    wall, dev = best(ctx, m, l_row_stats=True)
+    m.close()
+    assert dev > 0.85 * wall
