@@ -503,7 +503,7 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     L->base = static_cast<Tot*>(place(sizeof(Tot) * 2 * (size_t)hub_bases() * T));
     L->l_use = static_cast<LRowUse*>(place(sizeof(LRowUse) * (size_t)uses));
     L->stamp = static_cast<int32_t*>(place(4 * 2 * (size_t)W * T));
-    L->lcnt = static_cast<int32_t*>(place(16 * 2 * (size_t)W * (size_t)nm));
+    L->lcnt = static_cast<int32_t*>(place(32 * 2 * (size_t)W * (size_t)nm));
     L->fallback = static_cast<int32_t*>(place(4 * (size_t)nm));
     L->judged = static_cast<int32_t*>(place(8 * (size_t)nm));
     L->counters = static_cast<unsigned long long*>(place(8 * CNT_SLOTS * (size_t)nm));

@@ -56,8 +56,23 @@ namespace {
 constexpr int kWindows = 3;
 constexpr int kHubs = 4;  // two for the first window, one for each other
 constexpr int kBases = 2;  // arrays of totals: a source has at most two hubs to choose from
-constexpr int kMaxRounds = 192;  // label rounds before a matrix is left to traverse_kernel
+// Label rounds before a matrix is left: 24 at n = 5,000, 103 to 192 at 20,000 and
+// 96 at 40,000 were enough for matrices with a core (random and banded with
+// uniform entries, circuit-like); a band without one uses up all of them, which
+// at 192 was 0.6 of 2.6 ms at n = 5,000.
+constexpr int kMaxRounds = 192;
+__host__ __device__ __forceinline__ int label_rounds(int n) { return n / 64 < kMaxRounds - 64 ? 64 + n / 64 : kMaxRounds; }
+// A core is reached within a few tens of rounds, the rest only lower labels; in
+// a mesh the hub's set still grows then.  The ids first reached in the rounds up
+// to kSpread, in the next 16 and in the 16 after that are counted; a matrix is
+// left when the last are more than half of those before them and more than n/64
+// (see spreads): a 40^3 mesh with a third of its couplings one-sided 8.2 -> 6.5 ms,
+// 6.1 by traverse_kernel alone.
+constexpr int kSpread = 32, kSpreadStep = 16;
+constexpr int kSpreadEnd = kSpread + 2 * kSpreadStep;
+constexpr int kLook = 16;  // rounds between looks whether another search has left the matrix
 constexpr int kLabelThreads = 1024;
+constexpr int kNoLabel = 0x7f7f7f7f;  // label_round_kernel's arrays are set bytewise
 constexpr int kExtraThreads = 256;
 constexpr int kJudgeAfter = 512;  // searches before a matrix may be left
 
@@ -81,6 +96,11 @@ __host__ __device__ __forceinline__ int window_of_hub(int h) { return h < 2 ? 0 
 __device__ __forceinline__ long long lam_at(const HubLaunch& P, const MatDesc& M, int h, int d) {
     return (2ll * h + d) * P.total + M.hub_off;
 }
+
+// The count that round r adds to: 0 up to kSpread, 1 and 2 for the steps after it.
+__device__ __forceinline__ int spread_part(int r) { return r < kSpread ? 0 : r < kSpread + kSpreadStep ? 1 : 2; }
+
+__device__ __forceinline__ bool spreads(int n, int before, int last) { return 2 * last > before && 64 * (long long)last > n; }
 
 // Per matrix and hub, several CTAs: the largest key (degree product, then
 // smallest id).  The first window's two hubs are the best of the even and of
@@ -155,7 +175,9 @@ __device__ __forceinline__ int dsm_add(unsigned a, int v) {
 // either read there or queues the id again.  Queues are in global memory.
 __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch P) {
     extern __shared__ uint4 dyn_smem[];
-    __shared__ int cnt[3];  // of rank 0: queued ids per round, in turn
+    // of rank 0: queued ids per round, in turn; whether the matrix is left, every
+    // kLook rounds in turn; ids first reached
+    __shared__ int cnt[3], quit[2], reached[3];
     const unsigned C = cluster_size(), rank = cluster_rank();
     const unsigned shift = 31 - __clz(C);
     const int job = blockIdx.x / C;
@@ -171,6 +193,8 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
     int32_t* const lam = reinterpret_cast<int32_t*>(dyn_smem);
     const unsigned lam_a = (unsigned)__cvta_generic_to_shared(lam);
     const unsigned cnt_a = at_rank((unsigned)__cvta_generic_to_shared(cnt), 0);
+    const unsigned quit_a = at_rank((unsigned)__cvta_generic_to_shared(quit), 0);
+    const unsigned reached_a = at_rank((unsigned)__cvta_generic_to_shared(reached), 0);
     auto group_sync = [&]() {
         if (C == 1) __syncthreads();
         else cluster_sync();
@@ -187,6 +211,8 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
     if (threadIdx.x == 0) {
         cnt[0] = 1;
         cnt[1] = cnt[2] = 0;
+        quit[0] = quit[1] = 0;
+        reached[0] = reached[1] = reached[2] = 0;
     }
     group_sync();
     if (rank == 0 && threadIdx.x == 0) {
@@ -195,10 +221,12 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
         __stcg(q[0], hub);
     }
     group_sync();
-    int r = 0, count = 0;
-    for (; r < kMaxRounds; r++) {
+    const int rounds = label_rounds(n);
+    int r = 0, count = 0, got = 0;
+    for (; r < rounds; r++) {
         count = dsm_ld(cnt_a + 4 * (r % 3));
         if (count == 0) break;
+        if (r && r % kLook == 0 && dsm_ld(quit_a + 4 * (r / kLook % 2))) break;
         const int32_t* cur = q[r & 1];
         int32_t* const next = q[(r + 1) & 1];
         const unsigned nc = cnt_a + 4 * ((r + 1) % 3);
@@ -233,6 +261,8 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
 #pragma unroll
                 for (int c = 0; c < 4; c++)
                     lw[c] = label_of_word(onl) < label_of_word(lw[c]) ? dsm_min(lam_of(ws[c]), onl) : -1;
+#pragma unroll
+                for (int c = 0; c < 4; c++) got += lw[c] == kNoLabelWord;
                 unsigned bal[4];
                 int k = 0;
 #pragma unroll
@@ -255,9 +285,21 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
                 e = en;
             }
         }
+        if (l == 0 && r < kSpreadEnd && spread_part(r) != spread_part(r + 1 < kSpreadEnd ? r + 1 : 0)) {
+            got = __reduce_add_sync(FULL_MASK, got);
+            if (lane == 0 && got) dsm_add(reached_a + 4 * spread_part(r), got);
+            got = 0;
+        }
+        // another search of the matrix may have found it to be left
+        if (r % kLook == kLook - 1 && rank == 0 && threadIdx.x == 0)
+            quit[(r + 1) / kLook % 2] = ld_vol_i32(P.fallback + mi);
         group_sync();
+        if (l == 0 && r == kSpreadEnd - 1 && spreads(n, dsm_ld(reached_a + 4), dsm_ld(reached_a + 8))) {
+            if (rank == 0 && threadIdx.x == 0) atomicExch(P.fallback + mi, 1);
+            break;
+        }
     }
-    if (r == kMaxRounds && dsm_ld(cnt_a + 4 * (r % 3)) != 0 && rank == 0 && threadIdx.x == 0)
+    if (r == rounds && dsm_ld(cnt_a + 4 * (r % 3)) != 0 && rank == 0 && threadIdx.x == 0)
         atomicExch(P.fallback + mi, 1);  // unfinished labels are too large
     for (int w = (int)rank + (int)C * (threadIdx.x >> 5); w < nw; w += (int)C * (kLabelThreads / 32)) {
         // whole groups: the ids from n on have no label
@@ -268,7 +310,7 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
 
 // The same by the whole GPU, one launch per round (labels, queues, counts in
 // global memory): `per` CTAs a job, a launch that finds nothing queued ends at
-// once.  `last`: the matrix is left if this round leaves ids queued.
+// once.  The matrix is left if its last round finds ids queued.
 __global__ void label_start_kernel(HubLaunch P) {
     const int job = blockIdx.x;
     const int mi = job / (2 * kHubs), h = (job >> 1) % kHubs, d = job & 1;
@@ -278,18 +320,26 @@ __global__ void label_start_kernel(HubLaunch P) {
     const int hub = hub_of(P, mi, h);
     P.lam[at + hub] = hub;
     P.lq[2 * at] = hub;
-    P.lcnt[4ll * job] = 1;
+    P.lcnt[8ll * job] = 1;
 }
 
-__global__ void __launch_bounds__(kLabelThreads) label_round_kernel(HubLaunch P, int per_job, int r, int last) {
+__global__ void __launch_bounds__(kLabelThreads) label_round_kernel(HubLaunch P, int per_job, int r) {
     const int job = blockIdx.x / per_job, part = blockIdx.x % per_job;
-    int32_t* const cnt = P.lcnt + 4ll * job;
+    int32_t* const cnt = P.lcnt + 8ll * job;
+    int32_t* const reached = cnt + 4;  // ids first reached (see spreads)
     const int count = cnt[r % 3];
     if (part == 0 && threadIdx.x == 0) cnt[(r + 2) % 3] = 0;
     if (count == 0) return;
     const int mi = job / (2 * kHubs), h = (job >> 1) % kHubs, d = job & 1;
-    if (last && part == 0 && threadIdx.x == 0) atomicExch(P.fallback + mi, 1);
     const int lane = threadIdx.x & 31;
+    int left = 0;
+    if (lane == 0) left = ld_vol_i32(P.fallback + mi);
+    if (__shfl_sync(FULL_MASK, left, 0)) return;
+    const int l = window_of_hub(h);
+    if (part == 0 && threadIdx.x == 0 &&
+        (r >= label_rounds(P.mats[mi].n) - 1 ||
+         (l == 0 && r == kSpreadEnd && spreads(P.mats[mi].n, reached[1], reached[2]))))
+        atomicExch(P.fallback + mi, 1);
     const int gw = (part * kLabelThreads + threadIdx.x) >> 5;
     const int nwarps = per_job * (kLabelThreads / 32);
     // few ids queued: fewer per warp, so that more warps work
@@ -297,10 +347,10 @@ __global__ void __launch_bounds__(kLabelThreads) label_round_kernel(HubLaunch P,
     if (gw * per >= count) return;
     const MatDesc& M = P.mats[mi];
     const int n = M.n;
-    const int l = window_of_hub(h);
     const int bound = l == 0 ? n : window_end(n, l) + 1;
     const Graph G = d ? Graph{M.trowptr, M.tcol} : Graph{M.rowptr, M.col};
     const long long at = lam_at(P, M, h, d);
+    int got = 0;
     int32_t* const lam = P.lam + at;
     int32_t* const stamp = P.stamp + at;
     const int32_t* cur = P.lq + 2 * at + (r & 1) * M.hub_len;
@@ -333,6 +383,8 @@ __global__ void __launch_bounds__(kLabelThreads) label_round_kernel(HubLaunch P,
 #pragma unroll
             for (int c = 0; c < 4; c++) old[c] = onl < lw[c] ? atomicMin(lam + ws[c], onl) : -1;
 #pragma unroll
+            for (int c = 0; c < 4; c++) got += old[c] == kNoLabel;
+#pragma unroll
             for (int c = 0; c < 4; c++)
                 old[c] = old[c] > onl && ws[c] < bound ? atomicExch(stamp + ws[c], r + 1) : r + 1;
             unsigned bal[4];
@@ -357,6 +409,10 @@ __global__ void __launch_bounds__(kLabelThreads) label_round_kernel(HubLaunch P,
             e = en;
         }
     }
+    if (l == 0 && r < kSpreadEnd) {
+        got = __reduce_add_sync(FULL_MASK, got);
+        if (lane == 0 && got) atomicAdd(reached + spread_part(r), got);
+    }
 }
 
 // The changes over s of the hub set's totals.  A warp per word: lane j is id
@@ -365,7 +421,7 @@ __global__ void event_kernel(HubLaunch P, int per_job, int digests) {
     const int job = blockIdx.x / per_job, part = blockIdx.x % per_job;
     const int mi = job / (2 * kHubs), h = (job >> 1) % kHubs, d = job & 1;
     const MatDesc& M = P.mats[mi];
-    if (M.method != METHOD_HUB) return;
+    if (M.method != METHOD_HUB || P.fallback[mi]) return;
     const int n = M.n;
     const int l = window_of_hub(h);
     const int lo = l == kWindows - 1 ? 0 : window_end(n, l + 1) + 1;  // the window's sources
@@ -957,8 +1013,8 @@ cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStr
             if (e != cudaSuccess) return e;
             label_start_kernel<<<jobs, 32, 0, st>>>(L);
             const int per = std::max(8, 2 * c.sm_count / std::min(L.hub_mats, 8));
-            for (int r = 0; r < kMaxRounds; r++)
-                label_round_kernel<<<per * jobs, kLabelThreads, 0, st>>>(L, per, r, r == kMaxRounds - 1);
+            for (int r = 0; r < label_rounds(c.n_max); r++)
+                label_round_kernel<<<per * jobs, kLabelThreads, 0, st>>>(L, per, r);
         }
         const int words = (int)((c.n_max + 31) / 32);
         const int per = parts((words + 7) / 8, jobs);

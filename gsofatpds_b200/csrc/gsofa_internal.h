@@ -222,7 +222,7 @@ struct HubLaunch {
     LRowUse* l_use;                    // per hub and source (with per-row L statistics): see lrow_kernel
     Tot* base;                         // per base, direction and source: the hub set's totals
     int32_t* stamp;                    // as lam
-    int32_t* lcnt;                     // 4 per label job
+    int32_t* lcnt;                     // 8 per label job
     int32_t* fallback;                 // per matrix: left to traverse_kernel
     int32_t* judged;                   // per matrix: searches done, searches too large
     unsigned long long* counters;      // per matrix, CNT_SLOTS
