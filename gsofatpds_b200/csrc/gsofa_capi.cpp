@@ -160,15 +160,18 @@ std::vector<int32_t> batch_order(const gsofa_matrix* const* mats, int32_t count)
 
 long long chunk_weight(gsofa_ctx* ctx, const gsofa_matrix* m) {
     if (m->host_sym < 0) {
-        int sym = 0;
+        int sym = 0, dup = 1;
         if (m->n > 0 &&
-            cudaMemcpyAsync(ctx->h_status + 1, m->asym, 4, cudaMemcpyDeviceToHost, ctx->stream) ==
+            cudaMemcpyAsync(ctx->h_status + 1, m->asym, 8, cudaMemcpyDeviceToHost, ctx->stream) ==
                 cudaSuccess &&
-            cudaStreamSynchronize(ctx->stream) == cudaSuccess)
+            cudaStreamSynchronize(ctx->stream) == cudaSuccess) {
             sym = ctx->h_status[1] == 0;
-        else
+            dup = ctx->h_status[2] != 0;
+        } else {
             cudaGetLastError();
+        }
         m->host_sym = sym;
+        m->host_dup = dup;
     }
     return m->host_sym ? m->n / 4 : 2ll * m->n;
 }
@@ -367,12 +370,14 @@ MatDesc make_desc(const gsofa_matrix* m, const gsofa_result* r, long long base) 
 bool chain_runs(const gsofa_opts& o, const gsofa_matrix* const* mats, int32_t count) {
     if ((o.flags & (GSOFA_NO_MERGE | GSOFA_NO_CHAIN)) || o.bu_alpha > 0) return false;
     long long hub_rows = 0;
+    bool any = count == 0;
     for (int32_t i = 0; i < count; i++) {
         const int32_t method = method_of(mats[i]);
+        any |= method != METHOD_WALK;
         if (method == METHOD_CHAIN && (o.flags & GSOFA_L_ROW_STATS)) return false;
         if (method == METHOD_HUB) hub_rows += mats[i]->n + 32ll;
     }
-    return hub_rows * std::max(hub_count(), 2 * hub_bases()) <= INT_MAX;
+    return any && hub_rows * std::max(hub_count(), 2 * hub_bases()) <= INT_MAX;
 }
 
 int plan_chain(gsofa_ctx* ctx, int32_t nmax, long long total_sources, bool all_sym, const gsofa_opts* o,
@@ -420,6 +425,8 @@ void fill_chain_launch(ChainLaunch* L, const ChainCfg& c, const gsofa_opts& o, i
 }
 
 int32_t method_of(const gsofa_matrix* m) {
+    // the hubs' launch does not count a row's distinct ids, the chain does
+    if (m->host_dup != 0 && (m->n <= kDirectMax || m->host_sym <= 0)) return METHOD_WALK;
     if (m->n <= kDirectMax) return METHOD_DIRECT;
     return m->host_sym > 0 ? METHOD_CHAIN : METHOD_HUB;
 }
@@ -433,7 +440,7 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     int hubs = 0, k = 0;
     for (MatDesc& d : *descs) {
         k++;
-        if (d.method == METHOD_CHAIN) continue;
+        if (d.method != METHOD_HUB && d.method != METHOD_DIRECT) continue;
         sources += 2ll * d.n;
         n_max = std::max(n_max, d.n);
         if (d.method != METHOD_HUB) continue;
@@ -465,7 +472,7 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     for (MatDesc& d : *descs) {
         d.hub_item = items;
         d.hub_slots = 0;
-        if (d.method == METHOD_CHAIN || d.n == 0) continue;
+        if ((d.method != METHOD_HUB && d.method != METHOD_DIRECT) || d.n == 0) continue;
         d.hub_slots = 1;
         while (d.hub_slots < 2 * ((d.n + g - 1) / g)) d.hub_slots *= 2;
         items += d.hub_slots;
@@ -756,10 +763,11 @@ int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t cou
     double ms = ms_f, ms_trav = ms_trav_f;
     std::vector<unsigned long long> totals(ctx->h_counters, ctx->h_counters + (size_t)count * CNT_SLOTS);
 
-    // matrices that the hubs' launch left: traverse_kernel counts them
+    // those that neither traversal takes and those that the hubs' launch left
     std::vector<int32_t> left;
-    for (int32_t k = 0; k < count && hub; k++)
-        if (ctx->h_fallback[k]) left.push_back(order[(size_t)k]);
+    for (int32_t k = 0; k < count && chain; k++)
+        if (descs[(size_t)k].method == METHOD_WALK || (hub && ctx->h_fallback[k]))
+            left.push_back(order[(size_t)k]);
     if (!left.empty()) {
         std::vector<const gsofa_matrix*> lm;
         std::vector<gsofa_result*> lr;
@@ -1336,9 +1344,12 @@ int gsofa_load_csr(gsofa_ctx* ctx, int32_t n, int64_t nnz, const int32_t* row_be
     if (rc) return rc;
     cudaError_t e = cudaMemcpyAsync(ctx->h_status, dstatus, 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(ctx->h_status + 1, m->asym, 4, cudaMemcpyDeviceToHost, ctx->stream);
+        e = cudaMemcpyAsync(ctx->h_status + 1, m->asym, 8, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e == cudaSuccess) m->host_sym = n > 0 && ctx->h_status[1] == 0;
+    if (e == cudaSuccess) {
+        m->host_sym = n > 0 && ctx->h_status[1] == 0;
+        m->host_dup = n > 0 && ctx->h_status[2] != 0;
+    }
     rc = e != cudaSuccess ? cuda_fail(ctx, e, "load") : check_status(ctx);
     if (rc) {
         dev_free(ctx, m->rowptr, m->bytes);
@@ -1583,6 +1594,7 @@ int gsofa_autotune(gsofa_ctx* ctx, const gsofa_matrix* mat, gsofa_opts* opts) {
     const double rel = mat->nnz > 0 ? (double)hsum / (double)mat->nnz / (double)mat->n : 0.0;
     const int loc = rel > 1e-9 ? std::max(-60, (int)std::floor(2.0 * std::log2(rel))) : -61;
     // and so do the kernels that may count them
+    chunk_weight(ctx, mat);
     const gsofa_matrix* const mats[1] = {mat};
     const std::tuple<int, int, int, int> key(lg, deg, loc, chain_runs(*opts, mats, 1) ? method_of(mat) : -1);
     auto it = ctx->tuned.find(key);
@@ -1777,7 +1789,7 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
         if (d.method == METHOD_CHAIN || d.n <= 0) continue;
         d.item_base = left_base;
         left_base += 2 * ((d.n + walk_chunk - 1) / walk_chunk);
-        d.only_if = HL.fallback + k;
+        d.only_if = d.method == METHOD_WALK ? nullptr : HL.fallback + k;
         left.push_back(d);
     }
     cudaError_t e;

@@ -72,7 +72,8 @@ struct gsofa_matrix {
     // device words: [0] 0 iff the pattern is symmetric, [1] non-zero when a row may hold an id twice
     int32_t* asym = nullptr;
     size_t bytes = 0;
-    mutable int host_sym = -1;  // the device word read back once (-1: not yet)
+    mutable int host_sym = -1;  // the device words read back once (-1: not yet)
+    mutable int host_dup = -1;
 };
 
 struct gsofa_result {
@@ -179,7 +180,7 @@ size_t chain_queue_bytes(const gsofa_ctx* ctx, const ChainCfg& c, int32_t nmax, 
 size_t chain_gbm_bytes(const gsofa_ctx* ctx, const ChainCfg& c, bool top);
 // The launch's fields that follow from the shape, the options and the largest order.
 void fill_chain_launch(ChainLaunch* L, const ChainCfg& c, const gsofa_opts& o, int32_t nmax);
-// Which counting traversal a matrix takes (its host_sym must be known).
+// Which counting traversal a matrix takes (its host_sym and host_dup must be known).
 int32_t method_of(const gsofa_matrix* m);
 // A launch of gsofa_hub.cu over descriptors whose methods are set: fills their
 // hub_* fields, `L` and `c`, and places the workspace of *bytes, at most `room`

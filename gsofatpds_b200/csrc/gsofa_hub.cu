@@ -36,9 +36,8 @@
 //
 // A matrix of at most kDirectMax rows has every source searched alone, without
 // a hub.  A matrix in which more than a quarter of the searches outgrow the
-// table (no core that the hub lies in: meshes) is left, and so are matrices with
-// repeated entries in a row: traverse_kernel counts them, whose reuse of closures
-// does not need a core (200,000-row band of 4 without one: 13 ms, 248 by
+// table (no core that the hub lies in: meshes) is left: traverse_kernel counts
+// it, whose reuse of closures does not need a core (200,000-row band of 4 without one: 13 ms, 248 by
 // gsofa_chain.cu; 90,000-row mesh with a third of its couplings one-sided: 16 ms,
 // 26 by it).
 #include <algorithm>
@@ -595,10 +594,6 @@ __global__ void __launch_bounds__(kExtraThreads, 1024 / kExtraThreads) extra_ker
         int left = 0;
         if (lane == 0) left = ld_vol_i32(P.fallback + mi);
         if (__shfl_sync(FULL_MASK, left, 0)) continue;
-        if (M.asym[1] != 0) {  // repeated entries: traverse_kernel counts a row's distinct ids
-            if (lane == 0) atomicExch(P.fallback + mi, 1);
-            continue;
-        }
         const int n = M.n;
         const bool sym = M.asym[0] == 0;
         const bool digests = M.dig_u != nullptr;
@@ -939,7 +934,7 @@ __global__ void lrow_kernel(HubLaunch P, int per_mat) {
 __global__ void commit_kernel(HubLaunch P) {
     const int mi = blockIdx.x;
     const MatDesc& M = P.mats[mi];
-    if (M.method != METHOD_CHAIN && !P.fallback[mi] && threadIdx.x < CNT_SLOTS)
+    if ((M.method == METHOD_HUB || M.method == METHOD_DIRECT) && !P.fallback[mi] && threadIdx.x < CNT_SLOTS)
         M.counters[threadIdx.x] += P.counters[(long long)mi * CNT_SLOTS + threadIdx.x];
 }
 

@@ -202,6 +202,7 @@ enum : int32_t {
     METHOD_CHAIN = 0,   // gsofa_chain.cu
     METHOD_HUB = 1,     // gsofa_hub.cu
     METHOD_DIRECT = 2,  // gsofa_hub.cu without a hub: every source searched alone
+    METHOD_WALK = 3,    // traverse_kernel: repeated entries, whose rows those two do not count
 };
 // A matrix of at most this many rows is METHOD_DIRECT.
 constexpr int kDirectMax = 1024;

@@ -954,6 +954,7 @@ extern "C" int gsofa_matrix_permute(gsofa_ctx* ctx, const gsofa_matrix* mat, con
         return rc;
     }
     m->host_sym = mat->host_sym;
+    m->host_dup = mat->host_dup;
     *out = m;
     return GSOFA_OK;
 }
