@@ -1197,17 +1197,16 @@ cudaError_t launch_serve(const TraverseLaunch& L, int block, int grid, size_t sm
 //
 // The host computes A's padded row pointers (pad counts in the low 2 bits).
 // One warp per row copies the row into its padded slot, writes the padding
-// (the row's own id) and counts the entries per column for A^T.  *dup becomes
-// non-zero when a row holds an id twice: a strictly increasing row cannot;
-// the others are compared pairwise up to kDupCheckMaxRow entries, and longer
-// unsorted rows count as holding one (a matrix so marked has its rows'
-// distinct ids counted in every search: slower, the same results).
-constexpr int kDupCheckMaxRow = 1024;
+// (the row's own id) and counts the entries per column for A^T.  dup[0] becomes
+// non-zero when a row holds an id twice: a strictly increasing row cannot, the
+// others are matched within the warp up to 32 entries, and longer ones are
+// listed (dup[1] of them in `list`) for repeated_kernel.
 
 __global__ void gather_rows_kernel(int32_t n, long long nnz_in, const int32_t* __restrict__ beg,
                                    const int32_t* __restrict__ rp,
                                    const int32_t* __restrict__ col_in, int32_t* __restrict__ col_out,
-                                   int32_t* __restrict__ tcount, int32_t* dup, int32_t* status) {
+                                   int32_t* __restrict__ tcount, int32_t* dup,
+                                   int32_t* __restrict__ list, int32_t* status) {
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -1218,6 +1217,7 @@ __global__ void gather_rows_kernel(int32_t n, long long nnz_in, const int32_t* _
         const long long plen = (long long)(r1 & ~3) - o;
         const long long d = plen - (r1 & 3);
         bool unsorted = false;
+        int mine = -1 - lane;  // the lane's last valid entry, or a value of its own
         for (long long j = lane; j < plen; j += 32) {
             if (j >= d) {
                 col_out[o + j] = (int32_t)v;
@@ -1241,16 +1241,67 @@ __global__ void gather_rows_kernel(int32_t n, long long nnz_in, const int32_t* _
             }
             col_out[o + j] = c;
             atomicAdd(&tcount[c], 1);
+            mine = c;
             unsorted |= j > 0 && src > 0 && col_in[src - 1] >= c;
         }
         if (!dup || !__any_sync(FULL_MASK, unsorted)) continue;
-        bool twice = d > kDupCheckMaxRow;
-        for (long long j = lane; j < d && !twice; j += 32) {
-            if (b + j < 0 || b + j >= nnz_in) break;  // reported above
-            const int32_t c = col_in[b + j];
-            for (long long i = 0; i < j && !twice; i++) twice = b + i >= 0 && col_in[b + i] == c;
+        if (d > 32) {
+            if (lane == 0) list[atomicAdd(dup + 1, 1)] = (int32_t)v;  // at most once a row
+        } else if (__any_sync(FULL_MASK, __popc(__match_any_sync(FULL_MASK, mine)) > 1)) {
+            if (lane == 0) atomicOr(dup, 1);
         }
-        if (twice) atomicOr(dup, 1);
+    }
+}
+
+// The listed rows, a CTA each: entries into a hash table in shared memory; an id
+// met again is one held twice.  Rows above half the table go in passes over
+// classes of ids.  A table that fills up all the same counts as an id held twice:
+// slower searches, the same results.  (Every pair of entries compared by the
+// gather's warp: loads of 100,000 circuit-like rows with entries twice took 2.0
+// instead of 1.1 ms; rows above 1,024 entries were not compared at all.)
+constexpr int kHashSlots = 8192;
+constexpr int kHashThreads = 256;
+
+__global__ void __launch_bounds__(kHashThreads) repeated_kernel(int32_t n, long long nnz_in,
+                                                                const int32_t* __restrict__ beg,
+                                                                const int32_t* __restrict__ rp,
+                                                                const int32_t* __restrict__ col_in,
+                                                                const int32_t* __restrict__ list, int32_t* dup) {
+    __shared__ int key[kHashSlots];
+    __shared__ int stop;
+    const int count = min(dup[1], n);
+    for (int i = blockIdx.x; i < count; i += gridDim.x) {
+        __syncthreads();
+        if (threadIdx.x == 0) stop = ld_vol_i32(dup);
+        __syncthreads();
+        if (stop) return;
+        const int v = list[i];
+        const long long b = beg[v];
+        const int r0 = rp[v], r1 = rp[v + 1];
+        const int d = (r1 & ~3) - (r0 & ~3) - (r1 & 3);
+        const unsigned passes = ((unsigned)d + kHashSlots / 2 - 1) / (kHashSlots / 2);
+        int size = 64;  // a power of two, twice the row's entries or all of the table
+        while (size < kHashSlots && size < 2 * d) size *= 2;
+        for (unsigned p = 0; p < passes; p++) {
+            for (int k = threadIdx.x; k < size; k += kHashThreads) key[k] = -1;
+            __syncthreads();
+            for (int j = threadIdx.x; j < d; j += kHashThreads) {
+                const long long src = b + j;
+                if (src < 0 || src >= nnz_in) continue;  // reported by the gather
+                const int c = col_in[src];
+                if (c < 0 || c >= n) continue;
+                if (passes > 1 && ((unsigned)c * 0x85EBCA6Bu >> 8) % passes != p) continue;
+                int s = (int)((unsigned)c * 0x9E3779B1u >> 8) & (size - 1), tries = 0;
+                for (; tries < size; tries++) {
+                    const int was = atomicCAS(key + s, -1, c);
+                    if (was == -1) break;
+                    if (was == c) tries = size;
+                    s = (s + 1) & (size - 1);
+                }
+                if (tries >= size) atomicOr(dup, 1);
+            }
+            __syncthreads();
+        }
     }
 }
 
@@ -1393,7 +1444,7 @@ cudaError_t launch_canonicalize(int32_t n, long long nnz_in, const int32_t* beg,
                                 int32_t* asym, int check_symmetry, int check_dup, void* scan_tmp,
                                 size_t scan_tmp_bytes, int32_t* status, cudaStream_t st) {
     cudaError_t e0 = cudaMemsetAsync(asym, check_symmetry ? 0 : 1, 4, st);
-    if (e0 == cudaSuccess) e0 = cudaMemsetAsync(asym + 1, check_dup ? 0 : 1, 4, st);
+    if (e0 == cudaSuccess) e0 = cudaMemsetAsync(asym + 1, check_dup ? 0 : 1, 8, st);
     if (e0 != cudaSuccess) return e0;
     if (n <= 0) return cudaSuccess;
     const int threads = 256;
@@ -1402,9 +1453,13 @@ cudaError_t launch_canonicalize(int32_t n, long long nnz_in, const int32_t* beg,
     long long grid_t = ((long long)n + threads) / threads;
     int gridt = (int)(grid_t > 148 * 16 ? 148 * 16 : grid_t);
     gather_rows_kernel<<<grid, threads, 0, st>>>(n, nnz_in, beg, rp, col_in, col_out, tcount,
-                                                 check_dup ? asym + 1 : nullptr, status);
+                                                 check_dup ? asym + 1 : nullptr, tpad, status);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
+    if (check_dup) {  // (the list lies in tpad, which is not made yet)
+        repeated_kernel<<<n < 148 * 4 ? n : 148 * 4, kHashThreads, 0, st>>>(n, nnz_in, beg, rp, col_in, tpad, asym + 1);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     pad_counts_kernel<<<gridt, threads, 0, st>>>(n, tcount, tpad);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     size_t bytes = scan_tmp_bytes;
