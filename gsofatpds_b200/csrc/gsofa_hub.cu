@@ -58,9 +58,12 @@ constexpr int kBases = 2;  // arrays of totals: a source has at most two hubs to
 // Label rounds before a matrix is left: 24 at n = 5,000, 103 to 192 at 20,000 and
 // 96 at 40,000 were enough for matrices with a core (random and banded with
 // uniform entries, circuit-like); a band without one uses up all of them, which
-// at 192 was 0.6 of 2.6 ms at n = 5,000.
-constexpr int kMaxRounds = 192;
-__host__ __device__ __forceinline__ int label_rounds(int n) { return n / 64 < kMaxRounds - 64 ? 64 + n / 64 : kMaxRounds; }
+// at 192 was 0.6 of 2.6 ms at n = 5,000.  Far larger ones need more: a band with
+// one uniform entry per row at n = 1,200,000 more than 192 (left: 582 ms).
+__host__ __device__ __forceinline__ int label_rounds(int n) {
+    const int a = 64 + n / 64, b = n / 2048 < 192 ? 192 : n / 2048;
+    return a < b ? a : b;
+}
 // A core is reached within a few tens of rounds, the rest only lower labels; in
 // a mesh the hub's set still grows then.  The ids first reached in the rounds up
 // to kSpread, in the next 16 and in the 16 after that are counted; a matrix is
@@ -1007,7 +1010,9 @@ cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStr
             e = cudaMemsetAsync(L.lam, 0x7f, 4ull * 2 * kHubs * (size_t)L.total, st);
             if (e != cudaSuccess) return e;
             label_start_kernel<<<jobs, 32, 0, st>>>(L);
-            const int per = std::max(8, 2 * c.sm_count / std::min(L.hub_mats, 8));
+            // two CTAs per SM over a matrix's eight jobs: a round without work costs
+            // its CTAs' launch (n = 1,200,000: 16 CTAs per SM 38 ms, two 33)
+            const int per = std::max(8, c.sm_count / (4 * std::min(L.hub_mats, 8)));
             for (int r = 0; r < label_rounds(c.n_max); r++)
                 label_round_kernel<<<per * jobs, kLabelThreads, 0, st>>>(L, per, r);
         }
