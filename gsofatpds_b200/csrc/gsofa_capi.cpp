@@ -458,11 +458,16 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     c->sm_count = ctx->sm_count;
     // labels in the shared memory of a cluster: of as many CTAs as leave every
     // job's cluster room on the GPU at once, and hold the largest matrix's labels
+    const int widest = ctx->label_cluster;
     c->cluster = 1;
-    while (c->cluster < 16 && 2 * W * hubs * 2 * c->cluster <= ctx->sm_count) c->cluster *= 2;
-    while (c->cluster < 16 && label_smem_bytes(n_max, c->cluster) + 2048 > (size_t)ctx->smem_optin)
+    while (c->cluster < widest && 2 * W * hubs * 2 * c->cluster <= ctx->sm_count) c->cluster *= 2;
+    while (c->cluster < widest && label_smem_bytes(n_max, c->cluster) + 2048 > (size_t)ctx->smem_optin)
         c->cluster *= 2;
-    if (label_smem_bytes(n_max, c->cluster) + 2048 > (size_t)ctx->smem_optin) c->cluster = 0;
+    // by the whole GPU in global memory: matrices too large for that, GPUs that
+    // place no cluster, and with the diagnostic GSOFA_FORCE_GLOBAL_BITMAP
+    if (widest == 0 || label_smem_bytes(n_max, c->cluster) + 2048 > (size_t)ctx->smem_optin ||
+        (o.flags & GSOFA_FORCE_GLOBAL_BITMAP))
+        c->cluster = 0;
     L->nmats = nm;
     L->total = off;
     // sources per warp and turn: few enough that the GPU's warps all have some
@@ -478,13 +483,12 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
         items += d.hub_slots;
     }
     L->total_items = items;
-    // large_kernel: small CTAs for small matrices, whole SMs for large ones
+    // large_kernel: its bitmap in shared memory where four CTAs' fit an SM
     L->bitmap_words = bitmap_words(n_max);
     const size_t bm = ((size_t)L->bitmap_words * 4 + 15) & ~(size_t)15;
-    c->large_block = 256;
     L->large_smem = 4 * (bm + 2048) <= (size_t)ctx->smem_per_sm && !(o.flags & GSOFA_FORCE_GLOBAL_BITMAP);
     c->large_smem = L->large_smem ? bm : 0;
-    int occ = large_occupancy(c->large_block, c->large_smem);
+    int occ = large_occupancy(c->large_smem);
     if (occ <= 0) occ = 1;
     c->large_grid = occ * ctx->sm_count;
     c->extra_grid = extra_ctas_per_sm() * ctx->sm_count;
@@ -1260,6 +1264,7 @@ int gsofa_create(int device, size_t budget_bytes, gsofa_ctx** out) {
     if ((e = cudaEventCreate(&ctx->ev0)) != cudaSuccess) return fail(e);
     if ((e = cudaEventCreate(&ctx->ev1)) != cudaSuccess) return fail(e);
     if ((e = cudaEventCreate(&ctx->evt)) != cudaSuccess) return fail(e);
+    ctx->label_cluster = label_max_cluster(((size_t)ctx->smem_optin - 2048) & ~(size_t)127);
     if ((e = cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&ctx->join, cudaEventDisableTiming)) != cudaSuccess)

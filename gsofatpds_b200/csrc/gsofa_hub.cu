@@ -76,6 +76,7 @@ constexpr int kLook = 16;  // rounds between looks whether another search has le
 constexpr int kLabelThreads = 1024;
 constexpr int kNoLabel = 0x7f7f7f7f;  // label_round_kernel's arrays are set bytewise
 constexpr int kExtraThreads = 256;
+constexpr int kLargeThreads = 256;
 constexpr int kJudgeAfter = 512;  // searches before a matrix may be left
 
 struct WarpTable {
@@ -962,18 +963,45 @@ size_t hub_scan_bytes(long long tots, long long uses) {
     return std::max(b, c);
 }
 
-int large_occupancy(int block, size_t smem) {
+int large_occupancy(size_t smem) {
     int occ = 0;
-    cudaError_t e;
-    if (block == 256) {
-        e = cudaFuncSetAttribute(large_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, large_kernel<256>, 256, smem);
-    } else {
-        e = cudaFuncSetAttribute(large_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, large_kernel<1024>, 1024, smem);
-    }
+    cudaError_t e = cudaFuncSetAttribute(large_kernel<kLargeThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, large_kernel<kLargeThreads>, kLargeThreads, smem);
     if (e != cudaSuccess) cudaGetLastError();
     return e == cudaSuccess ? occ : 0;
+}
+
+static cudaError_t label_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int jobs, int cluster,
+                                size_t smem, cudaStream_t st) {
+    cudaError_t e = cudaFuncSetAttribute(label_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && cluster > 8)
+        e = cudaFuncSetAttribute(label_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    *cfg = cudaLaunchConfig_t{};
+    cfg->gridDim = dim3((unsigned)(jobs * cluster));
+    cfg->blockDim = dim3(kLabelThreads);
+    cfg->dynamicSmemBytes = smem;
+    cfg->stream = st;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)cluster;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg->attrs = attr;
+    cfg->numAttrs = 1;
+    return e;
+}
+
+// The widest cluster that this GPU can place with `smem` bytes per CTA; 0: none.
+int label_max_cluster(size_t smem) {
+    for (int c = 16; c > 0; c /= 2) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr;
+        int n = 0;
+        cudaError_t e = label_config(&cfg, &attr, 1, c, smem, nullptr);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, label_cluster_kernel, &cfg);
+        if (e == cudaSuccess && n > 0) return c;
+        cudaGetLastError();
+    }
+    return 0;
 }
 
 // CTAs for each of `jobs` jobs of at most `most` CTAs' work: together no more than
@@ -989,23 +1017,11 @@ cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStr
         const int jobs = L.hub_mats * 2 * kHubs;
         hub_kernel<<<dim3((unsigned)(L.hub_mats * kHubs), 16), 256, 0, st>>>(L);
         if (c.cluster > 0) {
-            const size_t smem = label_smem_bytes(c.n_max, c.cluster);
-            e = cudaFuncSetAttribute(label_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e == cudaSuccess && c.cluster > 8)
-                e = cudaFuncSetAttribute(label_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            cudaLaunchConfig_t cfg;
+            cudaLaunchAttribute attr;
+            e = label_config(&cfg, &attr, jobs, c.cluster, label_smem_bytes(c.n_max, c.cluster), st);
+            if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, label_cluster_kernel, L);
             if (e != cudaSuccess) return e;
-            cudaLaunchConfig_t cfg{};
-            cudaLaunchAttribute attr{};
-            cfg.gridDim = dim3((unsigned)(jobs * c.cluster));
-            cfg.blockDim = dim3(kLabelThreads);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = st;
-            attr.id = cudaLaunchAttributeClusterDimension;
-            attr.val.clusterDim.x = (unsigned)c.cluster;
-            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-            cfg.attrs = &attr;
-            cfg.numAttrs = 1;
-            if ((e = cudaLaunchKernelEx(&cfg, label_cluster_kernel, L)) != cudaSuccess) return e;
         } else {
             e = cudaMemsetAsync(L.lam, 0x7f, 4ull * 2 * kHubs * (size_t)L.total, st);
             if (e != cudaSuccess) return e;
@@ -1028,8 +1044,7 @@ cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStr
         return e;
     const long long want = (L.total_items + kExtraThreads / 32 - 1) / (kExtraThreads / 32);
     extra_kernel<<<(int)std::min<long long>(want, c.extra_grid), kExtraThreads, smem, st>>>(L);
-    if (c.large_block == 256) large_kernel<256><<<c.large_grid, 256, c.large_smem, st>>>(L);
-    else large_kernel<1024><<<c.large_grid, 1024, c.large_smem, st>>>(L);
+    large_kernel<kLargeThreads><<<c.large_grid, kLargeThreads, c.large_smem, st>>>(L);
     if (c.any_hub && c.l_rows) {
         size_t sb = c.scan_bytes;
         e = cub::DeviceScan::InclusiveScan(c.scan_tmp, sb, L.l_use, L.l_use, UseSum(), (int)(kHubs * L.total), st);

@@ -247,7 +247,7 @@ struct HubCfg {
     size_t zeroed_bytes = 0;
     void* scan_tmp = nullptr;
     size_t scan_bytes = 0;
-    int large_block = 256, large_grid = 0;
+    int large_grid = 0;
     int extra_grid = 0;       // CTAs of the warps' searches at most
     size_t large_smem = 0;
     bool l_rows = false;      // per-row L statistics are wanted
@@ -256,7 +256,8 @@ int hub_count();  // hubs per matrix
 int hub_bases();  // arrays of totals per direction
 size_t label_smem_bytes(int32_t n, int cluster);
 size_t hub_scan_bytes(long long tots, long long uses);
-int large_occupancy(int block, size_t smem);
+int large_occupancy(size_t smem);
+int label_max_cluster(size_t smem);
 int extra_ctas_per_sm();
 cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStream_t stream);
 

@@ -46,7 +46,8 @@ typedef struct gsofa_batch gsofa_batch;
 #define GSOFA_PATTERN (1u << 2)     /* materialise L (by columns) and U (by rows)    */
 #define GSOFA_DIGESTS (1u << 3)     /* per-row/column 64-bit column-set digests      */
 /* Diagnostic: keep the traversal's seen-bitmap in global memory even when
- * it fits in shared memory (the variant used for orders above ~1.8M). */
+ * it fits in shared memory (the variant used for orders above ~1.8M), and
+ * the hubs' labels too (used above ~900,000 rows). */
 #define GSOFA_FORCE_GLOBAL_BITMAP (1u << 30)
 /* Diagnostic: never reuse the previous source's closure (every source is
  * searched from scratch). */
