@@ -74,13 +74,21 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
+// Whether this CTA's SM belongs to the other serving kernel now.
+__device__ __forceinline__ bool serve_elsewhere(const ServeLaunch& V) {
+    unsigned sm;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+    return V.kind == SERVE_CHAIN ? (int)sm >= ld_vol_i32(V.ctrl + 5) : (int)sm < ld_vol_i32(V.ctrl + 6);
+}
+
 // Serving, called by all 32 lanes of warp 0: claims a work item of any
-// published request.  Each lane checks one list entry (rotating start); the
-// claimable entry with the fewest unclaimed items is taken with
-// compare-and-swap on its claim word.  Returns false (in every
-// lane) when the host says to take no more items (ctrl[1]), when nothing is
-// claimable and the host asks idle CTAs to exit (ctrl[0]), after idle_ns of
-// finding nothing, or after max_idle_polls polls.
+// published request of the launch's kind.  Each lane checks one list entry
+// (rotating start); the claimable entry with the fewest unclaimed items is taken
+// with compare-and-swap on its claim word.  Returns false (in every lane) when
+// the host says to take no more items (ctrl[1], or by launch: ctrl[3], ctrl[4]),
+// when the SM is the other kernel's now, when nothing is claimable and the host
+// asks idle CTAs to exit (ctrl[0]), after idle_ns of finding nothing, or after
+// max_idle_polls polls.
 __device__ inline bool serve_claim(const ServeLaunch& V, int* slot_out, long long* item_out) {
     const int lane = threadIdx.x & 31;
     unsigned ns = 32;
@@ -89,7 +97,8 @@ __device__ inline bool serve_claim(const ServeLaunch& V, int* slot_out, long lon
         int c0 = 0, c1 = 0, n = 0;
         unsigned r = 0;
         if (lane == 0) {
-            c1 = ld_vol_i32(V.ctrl + 1) | (V.launch_no < ld_vol_i32(V.ctrl + 3));
+            c1 = ld_vol_i32(V.ctrl + 1) | (V.launch_no < ld_vol_i32(V.ctrl + (V.kind == SERVE_CHAIN ? 3 : 4))) |
+                 serve_elsewhere(V);
             c0 = ld_vol_i32(V.ctrl);
             n = min(ld_vol_i32(V.ctrl + 2), V.nslots);
             if (!c1 && n > 0) r = atomicAdd(V.rr, 1u);
@@ -114,8 +123,9 @@ __device__ inline bool serve_claim(const ServeLaunch& V, int* slot_out, long lon
                     v = ld_vol64(V.claim + slot);
                     if ((unsigned)(v >> 32) == seq) {
                         __threadfence();  // the descriptor was written before the claim word
-                        nit = __ldcg(&V.slots[slot].n_items);
-                        ok = (long long)(v & 0xffffffffull) < nit;
+                        nit = __ldcg(V.kind == SERVE_CHAIN ? &V.slots[slot].n_items : &V.slots[slot].walk_items);
+                        ok = (long long)(v & 0xffffffffull) < nit &&
+                             (V.kind == SERVE_ALL || (__ldcg(V.asym + slot) == 0) == (V.kind == SERVE_CHAIN));
                     }
                 }
             }
@@ -166,7 +176,7 @@ __device__ inline bool serve_claim(const ServeLaunch& V, int* slot_out, long lon
 __device__ inline int take_cta_slot(const ServeLaunch& V) {
     unsigned sm;
     asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
-    if (sm >= V.sm_limit) return -1;
+    if (sm >= V.sm_limit || serve_elsewhere(V)) return -1;
     const int nw = (V.n_cta_slots + 31) >> 5;
     for (int w = 0; w < nw; w++) {
         unsigned v = ld_vol_i32(reinterpret_cast<const int32_t*>(V.cta_slots + w));

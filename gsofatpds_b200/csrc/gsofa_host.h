@@ -146,6 +146,9 @@ int32_t* work_counter_status(gsofa_ctx* ctx, unsigned long long** wc);
 int check_status(gsofa_ctx* ctx);
 // Pool allocation with budget accounting, ordered on `stream`; the caller
 // holds ctx->mu.
+// Bytes of the workspace that factorizations keep between calls; an allocation
+// that the budget has no other room for takes their place.
+size_t kept_workspace(const gsofa_ctx* ctx);
 int dev_alloc_on(gsofa_ctx* ctx, size_t bytes, void** p, cudaStream_t stream);
 void dev_free_on(gsofa_ctx* ctx, void* p, size_t bytes, cudaStream_t stream);
 size_t align256(size_t x);

@@ -89,10 +89,13 @@ struct MatDesc {
     long long hub_item;
     long long hub_slots;
     // serving only (zero elsewhere)
-    long long n_items;          // work items of this request
+    long long n_items;          // work items of this request, for either kernel
+    long long walk_items;
     unsigned long long seq;     // request number (claim word tag, done flag value)
-    int32_t chunk;              // consecutive sources per work item
+    int32_t chunk;              // consecutive sources per work item, for either kernel
+    int32_t walk_chunk;
     int32_t slot;               // slot of the serving tables
+    int32_t pad1;
 };
 
 // The serving kernel's view of the request loop.  Each admitted request
@@ -108,11 +111,20 @@ struct MatDesc {
 // (mapped host memory, the one place the kernel touches host memory).
 // Every wait is bounded: a CTA that finds nothing to claim for idle_ns (or
 // max_idle_polls polls) exits, which also returns its SM to other work.
+enum : int32_t {
+    SERVE_CHAIN = 0,  // chain_kernel: requests with a symmetric pattern
+    SERVE_WALK = 1,   // traverse_kernel: the others
+    SERVE_ALL = 2,    // traverse_kernel, where it serves alone
+};
 struct ServeLaunch {
     unsigned long long* claim;            // per slot
     const unsigned long long* list;       // (slot << 32) | request number
     const int32_t* ctrl;                  // [0] exit when idle, [1] take no more items, [2] list entries,
-                                          // [3] launches before this number take no more items
+                                          // [3], [4] chain_kernel's, traverse_kernel's launches before this
+                                          // number take no more items; [5] chain_kernel's SMs end and [6]
+                                          // traverse_kernel's begin here
+    int32_t kind;                         // SERVE_*: the requests it takes
+    const int32_t* asym;                  // per slot: not 0 when the request's pattern is unsymmetric
     unsigned int* rr;                     // rotating start of the list scan (tie order)
     const MatDesc* slots;                 // one descriptor per slot
     unsigned long long* items_done;       // per slot: finished items

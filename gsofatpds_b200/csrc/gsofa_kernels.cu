@@ -695,7 +695,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) traverse_kernel(TraverseL
         const int mi = MODE == 2 ? 0 : SM.mi;
         const long long item = MODE == 2 ? SM.item : SM.item * stride;
         const int32_t n = M.n;
-        const long long clen = MODE == 2 ? (long long)M.chunk : (long long)P.chunk;
+        const long long clen = MODE == 2 ? (long long)M.walk_chunk : (long long)P.chunk;
         const long long local = item - M.item_base;
         const int dir = (int)(local & 1);
         const long long nchunks = ((long long)n + clen - 1) / clen;
@@ -1093,7 +1093,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) traverse_kernel(TraverseL
                 flush_counters(M.counters, acc);
                 __threadfence();
                 const unsigned long long d = atomicAdd(P.serve.items_done + M.slot, 1ull) + 1ull;
-                if (d == (unsigned long long)M.n_items) {
+                if (d == (unsigned long long)M.walk_items) {
                     __threadfence_system();
                     *reinterpret_cast<volatile unsigned long long*>(P.serve.done_flags + M.slot) =
                         M.seq;

@@ -1,8 +1,11 @@
 // gsofa_server.cpp -- the serving request loop (continuous batching).
 //
 // One host thread per server drives:
-//   * a persistent traversal kernel (chain_kernel; traverse_kernel for the
-//     diagnostic options and per-row L statistics) on the kernel stream.  Its CTAs claim work items of every published request;
+//   * two persistent traversal kernels, chain_kernel for requests with a
+//     symmetric pattern and traverse_kernel for the others (for all of them with
+//     the diagnostic options, per-row L statistics, or a budget without room for
+//     both workspaces).  Their CTAs claim work items of every published request;
+//     while both have work each uses half of the SMs;
 //     it stays on the device while published work is waiting and ends by
 //     itself when its CTAs have found nothing to claim for a short while;
 //   * a side stream for everything else: the upload and padded-CSR build of
@@ -68,7 +71,6 @@ struct Request {
     int state = R_QUEUED;
     int status = GSOFA_ERR_BUSY;
     int slot = -1;
-    long long item_base = 0;
     long long n_items = 0;
     unsigned long long seq = 0;
     size_t footprint = 0;
@@ -77,10 +79,11 @@ struct Request {
     bool handed_out = false;
     double t_submit = 0, t_admit = 0, t_publish = 0, t_done = 0;
     bool published = false;  // the claim word copy has executed
+    int engine = 0;          // then: the kernel that takes its items
 };
 
 constexpr int kSlots = 256;
-constexpr int kKernelStreams = 8;  // serving launches that may run at once
+constexpr int kKernelStreams = 4;  // serving launches of a kernel that may run at once
 constexpr int kReserveSms = 4;
 constexpr long long kMaxIdlePolls = 1000000;  // a cap far above idle_ns worth of polls
 constexpr long long kIdleNs = 300000;         // a CTA with nothing to claim for 0.3 ms exits
@@ -89,6 +92,52 @@ constexpr double kAdmitSliceMs = 1.0;         // admissions per loop pass stop a
 constexpr size_t kDefaultBudget = 40ull << 30;
 constexpr double kShutdownGraceMs = 120000.0;  // destroy waits this long for queued work
 
+// SMs that serving CTAs use; the rest are the uploads' and builds'.
+unsigned serve_sms(const gsofa_ctx* ctx) {
+    return ctx->sm_count > kReserveSms ? (unsigned)(ctx->sm_count - kReserveSms) : (unsigned)ctx->sm_count;
+}
+
+// A serving kernel's launch shape for requests of up to max_n rows and the
+// workspace its CTAs need.
+struct ServeShape {
+    bool chain = false;
+    int block = 0, occ = 0, grid = 0;
+    size_t smem = 0;  // dynamic, in all
+    long long smem_words = 0;
+    int32_t max_n = 0;
+    int ring = 0;
+
+    size_t queues() const { return align256((size_t)grid * (size_t)max_n * 4); }
+    size_t rings(long long words) const {
+        return chain ? 0 : align256((size_t)grid * (size_t)ring * (size_t)words * 4);
+    }
+    // the chain's four, or one for traverse_kernel where shared memory has no room for it
+    size_t bitmaps(long long words) const {
+        return chain || words > smem_words ? align256((size_t)grid * (chain ? 4 : 1) * (size_t)words * 4) : 0;
+    }
+    size_t bytes(long long words) const { return queues() + rings(words) + bitmaps(words); }
+};
+
+// One of the two serving kernels: its shape, launches and workspace.
+enum : int { E_CHAIN = 0, E_WALK = 1, kEngines = 2 };
+struct Engine {
+    bool on = false;
+    ServeShape shape;
+    cudaStream_t ks[kKernelStreams] = {};  // launches (low priority)
+    cudaEvent_t kdone[kKernelStreams] = {};
+    bool krun[kKernelStreams] = {};
+    int32_t kno[kKernelStreams] = {};  // the launch's number
+    int32_t launches = 0;
+    void* ws = nullptr;
+    size_t ws_bytes = 0;
+    int32_t* queue = nullptr;
+    uint32_t* rings = nullptr;
+    uint32_t* gbm = nullptr;
+    unsigned int* d_cta_slots = nullptr;
+    int* d_alive = nullptr;
+    double alive_checked = -1.0;
+};
+
 }  // namespace
 
 struct gsofa_server {
@@ -96,41 +145,29 @@ struct gsofa_server {
     gsofa_opts opts{};
     int32_t max_n = 0;
     size_t budget = 0;
-    int block = 256, grid = 0, occ = 0;
-    size_t smem = 0;
-    long long smem_words = 0, words = 0;
+    long long words = 0;
     int ring = 32;
     bool merge = true;
-    bool chain = true;  // gsofa_chain.cu serves; else traverse_kernel (diagnostics, per-row L statistics)
-    cudaStream_t ks[kKernelStreams] = {};  // serving launches (low priority)
-    cudaEvent_t kdone[kKernelStreams] = {};
-    bool krun[kKernelStreams] = {};
-    int32_t kno[kKernelStreams] = {};  // the launch's number
-    int32_t launches = 0;
+    Engine eng[kEngines];
     cudaStream_t as = nullptr, cs = nullptr, fs = nullptr;
     std::vector<cudaEvent_t> slot_ev;  // per slot: read-back done
     std::vector<cudaEvent_t> pub_ev;   // per slot: claim word written
-    // device workspace (one block)
-    void* ws = nullptr;
-    size_t ws_bytes = 0;
-    int32_t* queue = nullptr;
-    uint32_t* rings = nullptr;
-    uint32_t* gbm = nullptr;
+    // device tables (one block; each kernel has a workspace of its own)
+    void* tab = nullptr;
+    size_t tab_bytes = 0;
     MatDesc* d_slots = nullptr;
     unsigned long long* d_claim = nullptr;
     unsigned long long* d_items_done = nullptr;
     int32_t* d_slot_status = nullptr;
     unsigned int* d_rr = nullptr;
-    unsigned int* d_cta_slots = nullptr;
-    int* d_alive = nullptr;
-    int* h_alive = nullptr;  // pinned read-back of *d_alive
-    double alive_checked = -1.0;
+    int* h_alive = nullptr;  // pinned read-back of an engine's *d_alive
+    int32_t* d_asym = nullptr;  // per slot: the request's symmetry word
+    int32_t* h_asym = nullptr;
     unsigned long long* d_work = nullptr;
     int32_t* d_status = nullptr;
-    // control table: int32 ctrl[4] ([0] exit when idle, [1] take no more
-    // items, [2] list entries, [3] launches before this number take no more
-    // items), then u64 list[kSlots] = (slot << 32) | request
-    // number.  Master copy in pinned host memory, pushed whole.
+    // control table: int32 ctrl[8] (ServeLaunch says what they hold), then u64
+    // list[kSlots] = (slot << 32) | request number.  Master copy in pinned host
+    // memory, pushed whole.
     void* d_ctl = nullptr;
     void* h_ctl = nullptr;
     // mapped host memory
@@ -158,9 +195,10 @@ struct gsofa_server {
     int nlist = 0;
     bool kernel_running = false;
     bool launch_failed = false;
+    bool shed = false;  // the chain's workspace has to make room
     int live = 0;
     // accounting
-    size_t fixed = 0, in_use = 0, peak = 0;
+    size_t fixed = 0, least = 0, in_use = 0, peak = 0;  // least: fixed without the chain's workspace
     gsofa_server_stats st{};
     std::string err;
     std::chrono::steady_clock::time_point t0;
@@ -189,40 +227,86 @@ size_t request_footprint(const gsofa_server* s, int32_t n, int64_t nnz) {
     return kept + staging + result_bytes(n, s->opts.flags);
 }
 
-// Consecutive sources per work item: about four items per CTA for this
+// Consecutive sources per work item of traverse_kernel: about four items per CTA for this
 // order and grid (requests share the CTAs, so items stay shorter than the
 // plain path's), capped so that chunk * n stays near 2^28 -- one item of a
 // large request then holds its CTA for a bounded time, not for a large part
 // of the request, and a request that arrives meanwhile finds CTAs soon.  The
 // cap is no tighter because every item's first source starts cold.
-int request_chunk(const gsofa_server* s, int32_t n) {
+int walk_chunk(const gsofa_server* s, int32_t n) {
     if (s->opts.chunk_sources > 0) return s->opts.chunk_sources;
-    if (s->chain) {
-        // about one item per CTA; an item's first source is searched from nothing
-        return (int)std::max(8ll, std::min(128ll, ((long long)n + s->grid - 1) / s->grid));
-    }
     long long cap = 512;
     while (cap > 16 && cap * (long long)std::max(n, 1) > (1ll << 28)) cap >>= 1;
-    return (int)std::min<long long>(default_chunk(2ll * n, 4 * s->grid), cap);
+    return (int)std::min<long long>(default_chunk(2ll * n, 4 * s->eng[E_WALK].shape.grid), cap);
 }
 
-// Marks a request finished (done or failed) and releases its slot and memory.
-void finish(gsofa_server* s, const std::shared_ptr<Request>& r, int status) {
-    gsofa_ctx* ctx = s->ctx;
-    {
-        std::lock_guard<std::recursive_mutex> g(ctx->mu);
-        if (r->mat) {
-            dev_free_on(ctx, r->mat->rowptr, r->mat->bytes, s->as);
-            delete r->mat;
-            r->mat = nullptr;
-        }
-        if (status != GSOFA_OK && r->res) {
-            dev_free_on(ctx, r->res->arena, r->res->bytes, s->as);
-            delete r->res;
-            r->res = nullptr;
-        }
+// The chain's: about one item per CTA; an item's first source is searched from
+// nothing.
+int chain_item(const gsofa_server* s, int32_t n) {
+    if (s->opts.chunk_sources > 0) return s->opts.chunk_sources;
+    const long long grid = std::max(1, s->eng[E_CHAIN].shape.grid);
+    return (int)std::max(8ll, std::min(128ll, ((long long)n + grid - 1) / grid));
+}
+
+// Default CTA size of traverse_kernel: the plain path's for the largest order
+// served (the widest bitmap then fits in shared memory up to n of about 1.8M).
+// The chain's throughput is its CTAs' number, whatever max_n: four of 256 threads
+// per SM, or as many as keep one bitmap of max_n in shared memory while that
+// takes at most 64 KB (a symmetric pattern's only one: the 64^3 mesh at
+// max_n = 300,000 took 11.8 ms with it in global memory); wider ones are in
+// global memory.
+ServeShape serve_shape(const gsofa_ctx* ctx, const gsofa_server& s, bool chain) {
+    const gsofa_opts& o = s.opts;
+    ServeShape r;
+    r.chain = chain;
+    r.max_n = s.max_n;
+    r.ring = s.merge ? s.ring : 0;
+    r.block = o.threads_per_source > 0 ? o.threads_per_source
+              : chain                  ? 256
+                                       : std::max(256, default_block(s.max_n, ctx->smem_per_sm));
+    // shared-memory bitmap: the widest that keeps the block's full residency
+    // (none with the diagnostic GSOFA_FORCE_GLOBAL_BITMAP)
+    const int occ_target = 1024 / r.block;
+    const size_t fixed = chain ? (chain_sparse_bytes(2) + 15) & ~(size_t)15 : 0;
+    auto occupancy = [&](size_t bytes) {
+        return chain ? chain_occupancy(r.block, true, fixed + bytes) : serve_occupancy(r.block, bytes);
+    };
+    size_t smem = 0;
+    if (!(o.flags & GSOFA_FORCE_GLOBAL_BITMAP)) {
+        smem = (size_t)std::min(ctx->smem_optin, ctx->smem_per_sm / occ_target - 8 * 1024);
+        smem &= ~(size_t)1023;
+        while (smem >= 4096 && occupancy(smem) < occ_target) smem -= 1024;
+        if (smem < 4096) smem = 0;
+        const size_t one = ((size_t)s.words * 4 + 1023) & ~(size_t)1023;
+        if (chain && one <= 64 * 1024 && smem < one && occupancy(one) > 0) smem = one;
     }
-    std::lock_guard<std::mutex> g(s->mu);
+    if (chain) smem = std::min(smem, ((size_t)s.words * 8 + 1023) & ~(size_t)1023);  // both directions
+    r.occ = occupancy(smem);
+    r.smem = fixed + smem;
+    r.smem_words = (long long)(smem / 4);
+    r.grid = r.occ * std::max(1, ctx->sm_count - kReserveSms);
+    if (o.sources_in_flight > 0) r.grid = std::min(r.grid, o.sources_in_flight);
+    return r;
+}
+
+// Gives a request's device memory back, but for a result that is kept.
+void drop_buffers(gsofa_server* s, const std::shared_ptr<Request>& r, bool keep_result = false) {
+    gsofa_ctx* ctx = s->ctx;
+    std::lock_guard<std::recursive_mutex> g(ctx->mu);
+    if (r->mat) {
+        dev_free_on(ctx, r->mat->rowptr, r->mat->bytes, s->as);
+        delete r->mat;
+        r->mat = nullptr;
+    }
+    if (!keep_result && r->res) {
+        dev_free_on(ctx, r->res->arena, r->res->bytes, s->as);
+        delete r->res;
+        r->res = nullptr;
+    }
+}
+
+// (with s->mu held)
+void release_slot(gsofa_server* s, const std::shared_ptr<Request>& r) {
     if (r->slot >= 0) {
         s->slot_req[(size_t)r->slot].reset();
         s->free_slots.push_back(r->slot);
@@ -230,6 +314,13 @@ void finish(gsofa_server* s, const std::shared_ptr<Request>& r, int status) {
         s->live--;
     }
     s->in_use -= std::min(s->in_use, r->footprint);
+}
+
+// Marks a request finished (done or failed) and releases its slot and memory.
+void finish(gsofa_server* s, const std::shared_ptr<Request>& r, int status) {
+    drop_buffers(s, r, status == GSOFA_OK);
+    std::lock_guard<std::mutex> g(s->mu);
+    release_slot(s, r);
     r->t_done = now_ms(s);
     r->status = status;
     r->state = status == GSOFA_OK ? R_DONE : R_FAILED;
@@ -238,11 +329,12 @@ void finish(gsofa_server* s, const std::shared_ptr<Request>& r, int status) {
     s->cv_done.notify_all();
 }
 
-constexpr size_t kCtlBytes = 16 + 8 * (size_t)kSlots;
+constexpr size_t kCtlFlags = 32;
+constexpr size_t kCtlBytes = kCtlFlags + 8 * (size_t)kSlots;
 
 int32_t* ctl_flags(gsofa_server* s) { return static_cast<int32_t*>(s->h_ctl); }
 unsigned long long* ctl_list(gsofa_server* s) {
-    return reinterpret_cast<unsigned long long*>(static_cast<char*>(s->h_ctl) + 16);
+    return reinterpret_cast<unsigned long long*>(static_cast<char*>(s->h_ctl) + kCtlFlags);
 }
 
 // Copies the control table to the device and waits for the copy (tens of
@@ -278,20 +370,58 @@ void set_control(gsofa_server* s, int which, int32_t value) {
     push_control(s);
 }
 
+// With nothing in flight and a request waiting for room: the chain's workspace
+// goes, and traverse_kernel serves alone from here on.
+void shed_chain(gsofa_server* s) {
+    Engine& C = s->eng[E_CHAIN];
+    set_control(s, 3, C.launches);  // its CTAs find nothing to claim: they leave at once
+    set_control(s, 4, s->eng[E_WALK].launches);
+    for (Engine& E : s->eng)
+        for (int k = 0; k < kKernelStreams; k++) {
+            if (E.krun[k]) cudaEventSynchronize(E.kdone[k]);
+            E.krun[k] = false;
+        }
+    {
+        std::lock_guard<std::recursive_mutex> g(s->ctx->mu);
+        dev_free_on(s->ctx, C.ws, C.ws_bytes, s->as);
+    }
+    std::lock_guard<std::mutex> g(s->mu);
+    s->fixed -= C.ws_bytes;
+    s->in_use -= C.ws_bytes;
+    C.ws = nullptr;
+    C.on = false;
+    s->shed = false;
+    s->st.grid = s->eng[E_WALK].shape.grid;
+    s->st.block = s->eng[E_WALK].shape.block;
+}
+
 // Admits the request at the head of the queue if it fits; queues its upload,
 // build, table writes and publication on the side stream.
 bool admit_one(gsofa_server* s) {
     std::shared_ptr<Request> r;
     int slot = -1;
-    long long items = 0;
-    int chunk = 0;
+    bool clear = false;
     {
         std::lock_guard<std::mutex> g(s->mu);
         if (s->queued.empty() || s->free_slots.empty()) return false;
+        const bool fits = s->in_use + s->queued.front()->footprint <= s->budget;
+        if (!fits || s->shed) {
+            if (!s->eng[E_CHAIN].on || s->live > 0) return false;
+            clear = true;
+        }
+    }
+    if (clear) shed_chain(s);
+    const bool both = s->eng[E_CHAIN].on;
+    long long items = 0, walk_items = 0;
+    int chunk = 0, walk = 0;
+    {
+        std::lock_guard<std::mutex> g(s->mu);
+        if (s->queued.empty()) return false;
         r = s->queued.front();
-        if (s->in_use + r->footprint > s->budget) return false;
-        chunk = request_chunk(s, r->n);
-        items = (s->chain ? 1ll : 2ll) * (((long long)r->n + chunk - 1) / chunk);
+        walk = walk_chunk(s, r->n);
+        walk_items = 2 * (((long long)r->n + walk - 1) / walk);
+        chunk = both ? chain_item(s, r->n) : 1;
+        items = both ? ((long long)r->n + chunk - 1) / chunk : walk_items;
         s->queued.pop_front();
         slot = s->free_slots.back();
         s->free_slots.pop_back();
@@ -320,24 +450,45 @@ bool admit_one(gsofa_server* s) {
             rc = result_alloc_on(ctx, r->n, flags, s->opts.max_supernode_size, s->as, &r->res);
         if (rc != GSOFA_OK) why = ctx->err;
     }
+    if (rc == GSOFA_ERR_OOM_BUDGET && both) {
+        // the context has no room: again without the chain's workspace, once the
+        // requests in flight are done
+        drop_buffers(s, r);
+        std::lock_guard<std::mutex> g(s->mu);
+        release_slot(s, r);
+        r->state = R_QUEUED;
+        s->queued.push_front(r);
+        s->shed = true;
+        return true;
+    }
     if (rc != GSOFA_OK) {
         server_err(s, "ticket %llu: %s", (unsigned long long)r->ticket, why.c_str());
         finish(s, r, rc);
         return true;
     }
-    r->item_base = 0;
     r->n_items = items;
     r->seq = ++s->seq;
+    r->engine = E_WALK;
     MatDesc d = make_desc(r->mat, r->res, 0);
     d.n_items = items;
+    d.walk_items = walk_items;
     d.seq = r->seq;
     d.chunk = chunk;
+    d.walk_chunk = walk;
     d.slot = slot;
     s->h_desc[slot] = d;
     s->h_done[slot] = 0ull;
     s->h_claim[slot] = (r->seq & 0xffffffffull) << 32;
     e = cudaMemcpyAsync(s->d_slots + slot, s->h_desc + slot, sizeof(MatDesc),
                         cudaMemcpyHostToDevice, s->as);
+    if (both) {
+        // which of the two takes the request: read there by a CTA before it
+        // claims, here to keep that kernel running
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(s->d_asym + slot, r->mat->asym, 4, cudaMemcpyDeviceToDevice, s->as);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(s->h_asym + slot, r->mat->asym, 4, cudaMemcpyDeviceToHost, s->as);
+    }
     // the publication: the claim word (request number, 0 claimed), ordered
     // after the build and the descriptor
     if (e == cudaSuccess)
@@ -365,73 +516,76 @@ bool admit_one(gsofa_server* s) {
     return true;
 }
 
-bool launch_kernel(gsofa_server* s, int k, int grid) {
-    TraverseLaunch L{};
-    L.work_counter = s->d_work;
-    L.queue = s->queue;
-    L.queue_stride = std::max(s->max_n, 1);
-    L.gbitmap = s->gbm;
-    L.gprev = s->rings;
-    L.chunk = 1;
-    L.merge = s->merge ? 1 : 0;
-    L.chain = s->merge && !(s->opts.flags & GSOFA_NO_CHAIN) ? 1 : 0;
-    L.chain_wait_ns = chain_wait_ns(s->opts);
-    L.ring = s->ring;
-    L.sample_stride = 1;
-    L.bitmap_words = s->words;
-    L.status = s->d_status;
-    L.pattern_pass = 0;
+bool launch_kernel(gsofa_server* s, Engine& E, int k, int grid) {
     const gsofa_opts& o = s->opts;
-    L.bu_alpha = o.bu_alpha > 0 ? o.bu_alpha : 0;
-    L.bu_beta = o.bu_beta > 0 ? o.bu_beta : kDefaultBuBeta;
-    L.bu_min_src = o.bu_min_source > 0 ? o.bu_min_source : kBuMinSource;
-    L.heavy_len = o.heavy_row > 0 ? ((o.heavy_row + 3) & ~3) : kDefaultHeavyRow;
-    ServeLaunch& V = L.serve;
+    ServeLaunch V{};
     V.claim = s->d_claim;
-    V.list = reinterpret_cast<const unsigned long long*>(static_cast<char*>(s->d_ctl) + 16);
+    V.list = reinterpret_cast<const unsigned long long*>(static_cast<char*>(s->d_ctl) + kCtlFlags);
     V.ctrl = static_cast<const int32_t*>(s->d_ctl);
+    V.kind = E.shape.chain ? SERVE_CHAIN : s->eng[E_CHAIN].on ? SERVE_WALK : SERVE_ALL;
+    V.asym = s->d_asym;
     V.rr = s->d_rr;
     V.nslots = kSlots;
     V.slots = s->d_slots;
     V.items_done = s->d_items_done;
     V.slot_status = s->d_slot_status;
     V.done_flags = s->d_done;
-    V.smem_words = s->smem_words;
+    V.smem_words = E.shape.smem_words;
     V.max_idle_polls = kMaxIdlePolls;
     V.idle_ns = kIdleNs;
-    V.cta_slots = s->d_cta_slots;
-    V.n_cta_slots = s->grid;
-    V.alive = s->d_alive;
-    V.launch_no = s->launches;
-    V.sm_limit = s->ctx->sm_count > kReserveSms ? (unsigned)(s->ctx->sm_count - kReserveSms) : ~0u;
+    V.cta_slots = E.d_cta_slots;
+    V.n_cta_slots = E.shape.grid;
+    V.alive = E.d_alive;
+    V.launch_no = E.launches;
+    V.sm_limit = serve_sms(s->ctx);
     cudaError_t e;
-    if (s->chain) {
+    if (E.shape.chain) {
         ChainLaunch C{};
         C.work_counter = s->d_work;
-        C.queue = s->queue;
+        C.queue = E.queue;
         C.queue_stride = std::max(s->max_n, 1);
-        C.gbm = s->gbm;
+        C.gbm = E.gbm;
         C.gbm_count = 4;
         C.bitmap_words = s->words;
-        C.smem_words = s->smem_words;
+        C.smem_words = E.shape.smem_words;
         C.sides = 2;
         C.chunk = 1;
         C.list_cap = (int)std::min<long long>(chain_list_cap(), C.queue_stride);
         C.sample_stride = 1;
         C.status = s->d_status;
         C.serve = V;
-        e = launch_chain(C, s->block, true, grid, s->smem, s->ks[k]);
+        e = launch_chain(C, E.shape.block, true, grid, E.shape.smem, E.ks[k]);
     } else {
-        e = launch_serve(L, s->block, grid, s->smem, s->ks[k]);
+        TraverseLaunch L{};
+        L.work_counter = s->d_work;
+        L.queue = E.queue;
+        L.queue_stride = std::max(s->max_n, 1);
+        L.gbitmap = E.gbm;
+        L.gprev = E.rings;
+        L.chunk = 1;
+        L.merge = s->merge ? 1 : 0;
+        L.chain = s->merge && !(o.flags & GSOFA_NO_CHAIN) ? 1 : 0;
+        L.chain_wait_ns = chain_wait_ns(o);
+        L.ring = s->ring;
+        L.sample_stride = 1;
+        L.bitmap_words = s->words;
+        L.status = s->d_status;
+        L.pattern_pass = 0;
+        L.bu_alpha = o.bu_alpha > 0 ? o.bu_alpha : 0;
+        L.bu_beta = o.bu_beta > 0 ? o.bu_beta : kDefaultBuBeta;
+        L.bu_min_src = o.bu_min_source > 0 ? o.bu_min_source : kBuMinSource;
+        L.heavy_len = o.heavy_row > 0 ? ((o.heavy_row + 3) & ~3) : kDefaultHeavyRow;
+        L.serve = V;
+        e = launch_serve(L, E.shape.block, grid, E.shape.smem, E.ks[k]);
     }
-    if (e == cudaSuccess) e = cudaEventRecord(s->kdone[k], s->ks[k]);
+    if (e == cudaSuccess) e = cudaEventRecord(E.kdone[k], E.ks[k]);
     if (e != cudaSuccess) {
         server_err(s, "serving kernel launch: %s", cudaGetErrorString(e));
         s->launch_failed = true;
         return false;
     }
-    s->krun[k] = true;
-    s->kno[k] = s->launches++;
+    E.krun[k] = true;
+    E.kno[k] = E.launches++;
     s->kernel_running = true;
     std::lock_guard<std::mutex> g(s->mu);
     s->st.kernel_launches++;
@@ -439,47 +593,74 @@ bool launch_kernel(gsofa_server* s, int k, int grid) {
 }
 
 // CTAs currently holding a workspace slot (a short synchronous read).
-int alive_ctas(gsofa_server* s) {
-    cudaError_t e = cudaMemcpyAsync(s->h_alive, s->d_alive, 4, cudaMemcpyDeviceToHost, s->cs);
+int alive_ctas(gsofa_server* s, const Engine& E) {
+    cudaError_t e = cudaMemcpyAsync(s->h_alive, E.d_alive, 4, cudaMemcpyDeviceToHost, s->cs);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->cs);
-    return e == cudaSuccess ? *s->h_alive : s->grid;
+    return e == cudaSuccess ? *s->h_alive : E.shape.grid;
 }
 
-// Keeps CTAs on the device while published work is waiting.  A CTA leaves
-// once it has found nothing to claim for kIdleNs, which hands its SM back to
-// the side stream (uploads and builds of later requests).  When work is
-// waiting and fewer CTAs than workspace slots are alive -- none at all, or
-// the rest left during a large request's last items -- another launch of
-// the missing CTAs goes out on a free kernel stream (CTAs that find no free
-// slot exit at once, so a stale count costs nothing).  With every stream
-// taken, the oldest launch is told to take no more items: a few CTAs of each
-// launch would otherwise keep all streams for as long as there is work, and
-// nothing could replace those that left (48 requests at once, largest n = 10^6:
-// 0.42, 1.2 and 3.2 s in three runs of 22, 0.13-0.18 s in the others).
-bool manage_kernel(gsofa_server* s, bool claimable) {
+// Which SMs each kernel may use: all of them, or half each while there is work
+// for both.  (Halves of every SM's room would never hold a 1,024-thread CTA.)  A
+// CTA on the wrong side leaves after its item.
+void share_sms(gsofa_server* s, const bool* claimable) {
+    const int sms = (int)serve_sms(s->ctx), half = sms / 2;
+    int end = sms, begin = 0;
+    if (claimable[E_CHAIN] && claimable[E_WALK]) end = begin = half;
+    else if (claimable[E_CHAIN]) begin = sms;
+    else if (claimable[E_WALK]) end = 0;
+    else return;
+    if (!s->eng[E_CHAIN].on) begin = 0;
+    int32_t* f = ctl_flags(s);
+    if (f[5] == end && f[6] == begin) return;
+    f[5] = end;
+    f[6] = begin;
+    push_control(s);
+    for (Engine& E : s->eng) E.alive_checked = -1.0;
+}
+
+// Keeps a kernel's CTAs on the device while published work is waiting for it.
+// A CTA leaves once it has found nothing to claim for kIdleNs, which hands its
+// SM back to the side stream (uploads and builds of later requests) and to the
+// other kernel.  When work is waiting and fewer CTAs than its SMs hold are
+// alive -- none at all, or the rest left during a large request's last items --
+// another launch goes out on a free kernel stream (CTAs that find no free slot,
+// or are on the other kernel's SMs, exit at once, so a stale count costs
+// nothing; with half of the SMs a launch has twice the CTAs that are missing).
+// With every stream taken, the oldest launch is told to take no more items: a few
+// CTAs of each launch would otherwise keep all streams for as long as there is
+// work, and nothing could replace those that left (48 requests at once, largest
+// n = 10^6: 0.42, 1.2 and 3.2 s in three runs of 22, 0.13-0.18 s in the others).
+bool manage_kernel(gsofa_server* s, int e, bool claimable) {
+    Engine& E = s->eng[e];
+    if (!E.on) return false;
     bool progress = false;
     bool any = false;
     int free_k = -1;
     for (int k = 0; k < kKernelStreams; k++) {
-        if (s->krun[k] && cudaEventQuery(s->kdone[k]) == cudaSuccess) {
-            s->krun[k] = false;
+        if (E.krun[k] && cudaEventQuery(E.kdone[k]) == cudaSuccess) {
+            E.krun[k] = false;
             progress = true;
         }
-        if (s->krun[k]) any = true;
+        if (E.krun[k]) any = true;
         else if (free_k < 0) free_k = k;
     }
-    s->kernel_running = any;
+    s->kernel_running |= any;
     if (!claimable) return progress;
-    if (!any) return launch_kernel(s, free_k, s->grid) || progress;
+    if (!any) return launch_kernel(s, E, free_k, E.shape.grid) || progress;
     const double t = now_ms(s);
-    if (t - s->alive_checked < kTopUpCheckMs) return progress;
-    s->alive_checked = t;
-    const int missing = s->grid - alive_ctas(s);
-    if (missing < std::max(8, s->grid / 16)) return progress;
-    if (free_k >= 0) return launch_kernel(s, free_k, missing) || progress;
-    int32_t oldest = s->kno[0];
-    for (int k = 1; k < kKernelStreams; k++) oldest = std::min(oldest, s->kno[k]);
-    if (ctl_flags(s)[3] <= oldest) set_control(s, 3, oldest + 1);
+    if (t - E.alive_checked < kTopUpCheckMs) return progress;
+    E.alive_checked = t;
+    const int sms = (int)serve_sms(s->ctx);
+    const int mine = e == E_CHAIN ? ctl_flags(s)[5] : sms - ctl_flags(s)[6];
+    const bool part = mine < sms;
+    const int full = part ? std::min(E.shape.grid, E.shape.occ * std::max(mine, 1)) : E.shape.grid;
+    const int missing = full - alive_ctas(s, E);
+    if (missing < std::max(full < 8 ? 1 : 8, full / 16)) return progress;
+    if (free_k >= 0)
+        return launch_kernel(s, E, free_k, part ? std::min(E.shape.grid, 2 * missing) : missing) || progress;
+    int32_t oldest = E.kno[0];
+    for (int k = 1; k < kKernelStreams; k++) oldest = std::min(oldest, E.kno[k]);
+    if (ctl_flags(s)[3 + e] <= oldest) set_control(s, 3 + e, oldest + 1);
     return progress;
 }
 
@@ -589,7 +770,7 @@ void loop(gsofa_server* s) {
         }
         // requests whose claim word is on the device and whose items are not
         // all finished
-        bool claimable = false;
+        bool claimable[kEngines] = {};
         {
             std::lock_guard<std::mutex> g(s->mu);
             for (auto& r : s->slot_req) {
@@ -598,11 +779,14 @@ void loop(gsofa_server* s) {
                     cudaEventQuery(s->pub_ev[(size_t)r->slot]) == cudaSuccess) {
                     r->published = true;
                     r->t_publish = now_ms(s);
+                    if (s->eng[E_CHAIN].on && s->h_asym[r->slot] == 0) r->engine = E_CHAIN;
                 }
-                if (r->published) claimable = true;
+                if (r->published) claimable[r->engine] = true;
             }
         }
-        progress |= manage_kernel(s, claimable);
+        share_sms(s, claimable);
+        s->kernel_running = false;
+        for (int e = 0; e < kEngines; e++) progress |= manage_kernel(s, e, claimable[e]);
         if (s->launch_failed) {
             // no kernel can run: nothing admitted can finish
             fail_live(s, GSOFA_ERR_CUDA);
@@ -623,8 +807,9 @@ void loop(gsofa_server* s) {
             // CTAs finish the ones they hold, and fail whatever is left
             lk.unlock();
             set_control(s, 1, 1);
-            for (int k = 0; k < kKernelStreams; k++)
-                if (s->krun[k]) cudaEventSynchronize(s->kdone[k]);
+            for (Engine& E : s->eng)
+                for (int k = 0; k < kKernelStreams; k++)
+                    if (E.krun[k]) cudaEventSynchronize(E.kdone[k]);
             s->kernel_running = false;
             reap(s);
             fail_live(s, GSOFA_ERR_TIMEOUT);
@@ -655,24 +840,29 @@ void loop(gsofa_server* s) {
 void release(gsofa_server* s) {
     gsofa_ctx* ctx = s->ctx;
     cudaSetDevice(ctx->device);
-    if (s->ws) {
+    for (Engine& E : s->eng)
+        for (int k = 0; k < kKernelStreams; k++)
+            if (E.ks[k]) cudaStreamSynchronize(E.ks[k]);
+    {
         std::lock_guard<std::recursive_mutex> g(ctx->mu);
-        dev_free_on(ctx, s->ws, s->ws_bytes, s->as ? s->as : ctx->stream);
+        cudaStream_t st = s->as ? s->as : ctx->stream;
+        dev_free_on(ctx, s->tab, s->tab_bytes, st);
+        for (Engine& E : s->eng) dev_free_on(ctx, E.ws, E.ws_bytes, st);
     }
     if (s->as) cudaStreamSynchronize(s->as);
-    for (int k = 0; k < kKernelStreams; k++)
-        if (s->ks[k]) cudaStreamSynchronize(s->ks[k]);
     if (s->cs) cudaStreamSynchronize(s->cs);
     if (s->fs) cudaStreamSynchronize(s->fs);
     for (cudaEvent_t e : s->slot_ev)
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : s->pub_ev)
         if (e) cudaEventDestroy(e);
-    for (int k = 0; k < kKernelStreams; k++)
-        if (s->kdone[k]) cudaEventDestroy(s->kdone[k]);
+    for (Engine& E : s->eng)
+        for (int k = 0; k < kKernelStreams; k++) {
+            if (E.kdone[k]) cudaEventDestroy(E.kdone[k]);
+            if (E.ks[k]) cudaStreamDestroy(E.ks[k]);
+        }
     if (s->as) cudaStreamDestroy(s->as);
-    for (int k = 0; k < kKernelStreams; k++)
-        if (s->ks[k]) cudaStreamDestroy(s->ks[k]);
+    if (s->h_asym) cudaFreeHost(s->h_asym);
     if (s->h_alive) cudaFreeHost(s->h_alive);
     if (s->cs) cudaStreamDestroy(s->cs);
     if (s->fs) cudaStreamDestroy(s->fs);
@@ -701,18 +891,8 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
         return set_err(ctx, GSOFA_ERR_ARG, "invalid serving options");
     if (o.flags & GSOFA_PATTERN)
         return set_err(ctx, GSOFA_ERR_UNSUPPORTED, "GSOFA_PATTERN is not served");
-    const bool chain = chain_runs(o, nullptr, 0) && !(o.flags & GSOFA_L_ROW_STATS);
-    // default CTA size of traverse_kernel: the plain path's for the largest
-    // order served (the widest bitmap then fits in shared memory up to n of
-    // about 1.8M).  The chain's throughput is its CTAs' number, whatever max_n:
-    // four of 256 threads per SM, or as many as keep one bitmap of max_n in shared
-    // memory while that takes at most 64 KB (a symmetric pattern's only one: the
-    // 64^3 mesh at max_n = 300,000 took 11.8 ms with it in global memory); wider
-    // ones are in global memory.
-    const int block = o.threads_per_source > 0 ? o.threads_per_source
-                      : chain ? 256
-                              : std::max(256, default_block(max_n, ctx->smem_per_sm));
-    if (block != 256 && block != 512 && block != 1024)
+    if (o.threads_per_source > 0 && o.threads_per_source != 256 && o.threads_per_source != 512 &&
+        o.threads_per_source != 1024)
         return set_err(ctx, GSOFA_ERR_ARG, "serving threads_per_source must be 256, 512 or 1024");
     if (cudaSetDevice(ctx->device) != cudaSuccess) return set_err(ctx, GSOFA_ERR_CUDA, "cudaSetDevice");
 
@@ -722,8 +902,6 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
     s->opts = o;
     s->max_n = max_n;
     s->budget = budget_bytes ? budget_bytes : kDefaultBudget;
-    s->block = block;
-    s->chain = chain;
     s->merge = !(o.flags & GSOFA_NO_MERGE);
     s->ring = o.cached_closures > 0 ? std::min(o.cached_closures, kMaxRing) : kDefaultRing;
     while (s->ring & (s->ring - 1)) s->ring &= s->ring - 1;
@@ -736,50 +914,34 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
         return rc;
     };
 
-    // shared-memory bitmap: the widest that keeps the block's full residency
-    // (none with the diagnostic GSOFA_FORCE_GLOBAL_BITMAP)
     s->words = (((long long)max_n + 31) >> 5) + 6;
-    const int occ_target = 1024 / block;
-    const size_t fixed = chain ? (chain_sparse_bytes(2) + 15) & ~(size_t)15 : 0;
-    auto occupancy = [&](size_t bytes) {
-        return chain ? chain_occupancy(block, true, fixed + bytes) : serve_occupancy(block, bytes);
-    };
-    size_t smem = 0;
-    if (!(o.flags & GSOFA_FORCE_GLOBAL_BITMAP)) {
-        smem = (size_t)std::min(ctx->smem_optin, ctx->smem_per_sm / occ_target - 8 * 1024);
-        smem &= ~(size_t)1023;
-        while (smem >= 4096 && occupancy(smem) < occ_target) smem -= 1024;
-        if (smem < 4096) smem = 0;
-        const size_t one = ((size_t)s->words * 4 + 1023) & ~(size_t)1023;
-        if (chain && one <= 64 * 1024 && smem < one && occupancy(one) > 0) smem = one;
-    }
-    if (chain) smem = std::min(smem, ((size_t)s->words * 8 + 1023) & ~(size_t)1023);  // both directions
-    s->occ = occupancy(smem);
-    if (s->occ <= 0)
+    const bool counting = chain_runs(o, nullptr, 0) && !(o.flags & GSOFA_L_ROW_STATS);
+    // traverse_kernel always, and the chain for symmetric patterns where it can
+    // be resident and the budgets have room for its workspace too; that goes
+    // again when a request needs its room (shed_chain)
+    s->eng[E_WALK].shape = serve_shape(ctx, *s, false);
+    s->eng[E_WALK].on = true;
+    if (s->eng[E_WALK].shape.occ <= 0)
         return fail(GSOFA_ERR_UNSUPPORTED, "serving kernel cannot be resident", cudaSuccess);
-    s->smem = fixed + smem;
-    s->smem_words = (long long)(smem / 4);
-    s->grid = s->occ * std::max(1, ctx->sm_count - kReserveSms);
-    if (o.sources_in_flight > 0) s->grid = std::min(s->grid, o.sources_in_flight);
+    if (counting) s->eng[E_CHAIN].shape = serve_shape(ctx, *s, true);
+    s->eng[E_CHAIN].on = counting && s->eng[E_CHAIN].shape.occ > 0;
 
     // the side and control streams outrank the kernel stream: when an SM
     // frees up, their pending blocks are placed first
     cudaError_t e;
     int prio_low = 0, prio_high = 0;
     cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
-    for (int k = 0; k < kKernelStreams; k++)
-        if ((e = cudaStreamCreateWithPriority(&s->ks[k], cudaStreamNonBlocking, prio_low)) !=
-            cudaSuccess)
-            return fail(GSOFA_ERR_CUDA, "stream", e);
+    for (Engine& E : s->eng)
+        for (int k = 0; k < kKernelStreams && E.on; k++)
+            if ((e = cudaStreamCreateWithPriority(&E.ks[k], cudaStreamNonBlocking, prio_low)) != cudaSuccess ||
+                (e = cudaEventCreateWithFlags(&E.kdone[k], cudaEventDisableTiming)) != cudaSuccess)
+                return fail(GSOFA_ERR_CUDA, "stream", e);
     if ((e = cudaStreamCreateWithPriority(&s->as, cudaStreamNonBlocking, prio_high)) != cudaSuccess)
         return fail(GSOFA_ERR_CUDA, "stream", e);
     if ((e = cudaStreamCreateWithPriority(&s->cs, cudaStreamNonBlocking, prio_high)) != cudaSuccess)
         return fail(GSOFA_ERR_CUDA, "stream", e);
     if ((e = cudaStreamCreateWithPriority(&s->fs, cudaStreamNonBlocking, prio_high)) != cudaSuccess)
         return fail(GSOFA_ERR_CUDA, "stream", e);
-    for (int k = 0; k < kKernelStreams; k++)
-        if ((e = cudaEventCreateWithFlags(&s->kdone[k], cudaEventDisableTiming)) != cudaSuccess)
-            return fail(GSOFA_ERR_CUDA, "event", e);
     s->slot_ev.assign(kSlots, nullptr);
     s->pub_ev.assign(kSlots, nullptr);
     for (auto& ev : s->slot_ev)
@@ -794,10 +956,11 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
     if ((e = cudaHostGetDevicePointer((void**)&s->d_done, s->h_done, 0)) != cudaSuccess)
         return fail(GSOFA_ERR_CUDA, "mapped host memory", e);
     if ((e = cudaMallocHost(&s->h_ctl, kCtlBytes)) != cudaSuccess ||
+        (e = cudaMallocHost((void**)&s->h_asym, 4 * kSlots)) != cudaSuccess ||
         (e = cudaMallocHost((void**)&s->h_alive, 64)) != cudaSuccess)
         return fail(GSOFA_ERR_CUDA, "pinned host memory", e);
-    memset(s->h_ctl, 0, 16);
-    memset(static_cast<char*>(s->h_ctl) + 16, 0xff, kCtlBytes - 16);
+    memset(s->h_ctl, 0, kCtlFlags);
+    memset(static_cast<char*>(s->h_ctl) + kCtlFlags, 0xff, kCtlBytes - kCtlFlags);
     if ((e = cudaMallocHost((void**)&s->h_desc, sizeof(MatDesc) * kSlots)) != cudaSuccess ||
         (e = cudaMallocHost((void**)&s->h_claim, 8 * kSlots)) != cudaSuccess ||
         (e = cudaMallocHost((void**)&s->h_cnt, 8 * CNT_SLOTS * kSlots)) != cudaSuccess ||
@@ -805,36 +968,30 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
         (e = s->stager.init()) != cudaSuccess)
         return fail(GSOFA_ERR_CUDA, "pinned host memory", e);
 
-    // device workspace: per-CTA queues, closure rings and global bitmaps
-    // (only when max_n's bitmap exceeds shared memory), then the tables
-    const bool need_gbm = chain || s->words > s->smem_words;
-    const size_t G = (size_t)s->grid;
-    const size_t qb = align256(G * (size_t)max_n * 4);
-    const size_t rb = s->merge && !chain ? align256(G * (size_t)s->ring * (size_t)s->words * 4) : 0;
-    const size_t gb = need_gbm ? align256(G * (chain ? 4 : 1) * (size_t)s->words * 4) : 0;
-    const size_t tb = align256(sizeof(MatDesc) * kSlots) + align256(8 * kSlots) * 2 +
-                      align256(4 * kSlots) + 256 + align256(4 * (size_t)((s->grid + 31) / 32)) +
-                      align256(kCtlBytes);
-    s->ws_bytes = qb + rb + gb + tb;
-    if (s->ws_bytes > s->budget)
+    // the device tables, then per kernel: per-CTA queues, closure rings and
+    // global bitmaps, the CTA slots' bits and the count of those taken
+    s->tab_bytes = align256(sizeof(MatDesc) * kSlots) + align256(8 * kSlots) * 2 +
+                   align256(4 * kSlots) * 2 + 256 + align256(kCtlBytes);
+    auto slot_bytes = [](const Engine& E) { return align256(4 * (size_t)((E.shape.grid + 31) / 32)); };
+    for (Engine& E : s->eng)
+        if (E.on) E.ws_bytes = E.shape.bytes(s->words) + slot_bytes(E) + 256;
+    s->least = s->tab_bytes + s->eng[E_WALK].ws_bytes;
+    if (s->least > s->budget)
         return fail(GSOFA_ERR_OOM_BUDGET, "serving workspace exceeds the budget", cudaSuccess);
+    if (s->least + s->eng[E_CHAIN].ws_bytes > s->budget) s->eng[E_CHAIN].on = false;
     {
         std::lock_guard<std::recursive_mutex> g(ctx->mu);
-        int rc = dev_alloc_on(ctx, s->ws_bytes, &s->ws, s->as);
+        int rc = dev_alloc_on(ctx, s->tab_bytes, &s->tab, s->as);
+        if (rc == GSOFA_OK) rc = dev_alloc_on(ctx, s->eng[E_WALK].ws_bytes, &s->eng[E_WALK].ws, s->as);
         if (rc) {
-            s->ws = nullptr;
             release(s);
             delete s;
             return rc;
         }
+        Engine& C = s->eng[E_CHAIN];
+        if (C.on && dev_alloc_on(ctx, C.ws_bytes, &C.ws, s->as) != GSOFA_OK) C.on = false;
     }
-    char* b = static_cast<char*>(s->ws);
-    s->queue = reinterpret_cast<int32_t*>(b);
-    b += qb;
-    s->rings = rb ? reinterpret_cast<uint32_t*>(b) : nullptr;
-    b += rb;
-    s->gbm = need_gbm ? reinterpret_cast<uint32_t*>(b) : nullptr;
-    b += gb;
+    char* b = static_cast<char*>(s->tab);
     s->d_slots = reinterpret_cast<MatDesc*>(b);
     b += align256(sizeof(MatDesc) * kSlots);
     s->d_claim = reinterpret_cast<unsigned long long*>(b);
@@ -843,32 +1000,48 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
     b += align256(8 * kSlots);
     s->d_slot_status = reinterpret_cast<int32_t*>(b);
     b += align256(4 * kSlots);
+    s->d_asym = reinterpret_cast<int32_t*>(b);
+    b += align256(4 * kSlots);
     s->d_work = reinterpret_cast<unsigned long long*>(b);
     s->d_rr = reinterpret_cast<unsigned int*>(s->d_work + 1);
     s->d_status = reinterpret_cast<int32_t*>(s->d_work + 2);
-    s->d_alive = reinterpret_cast<int*>(s->d_work + 3);
     b += 256;
-    s->d_cta_slots = reinterpret_cast<unsigned int*>(b);
-    b += align256(4 * (size_t)((s->grid + 31) / 32));
     s->d_ctl = b;
-    if (need_gbm && (e = cudaMemsetAsync(s->gbm, 0, gb, s->as)) != cudaSuccess)
-        return fail(GSOFA_ERR_CUDA, "workspace init", e);
+    int32_t* const flags = ctl_flags(s);
+    flags[5] = (int32_t)serve_sms(ctx);
+    for (Engine& E : s->eng) {
+        if (!E.on) continue;
+        char* w = static_cast<char*>(E.ws);
+        E.queue = reinterpret_cast<int32_t*>(w);
+        w += E.shape.queues();
+        E.rings = E.shape.rings(s->words) ? reinterpret_cast<uint32_t*>(w) : nullptr;
+        w += E.shape.rings(s->words);
+        const size_t gb = E.shape.bitmaps(s->words);
+        E.gbm = gb ? reinterpret_cast<uint32_t*>(w) : nullptr;
+        w += gb;
+        E.d_cta_slots = reinterpret_cast<unsigned int*>(w);
+        w += slot_bytes(E);
+        E.d_alive = reinterpret_cast<int*>(w);
+        if ((gb && (e = cudaMemsetAsync(E.gbm, 0, gb, s->as)) != cudaSuccess) ||
+            (e = cudaMemsetAsync(E.d_cta_slots, 0, slot_bytes(E) + 256, s->as)) != cudaSuccess)
+            return fail(GSOFA_ERR_CUDA, "workspace init", e);
+    }
     // claim words start at request number 0 (never used): nothing claimable
     if ((e = cudaMemsetAsync(s->d_claim, 0, 8 * kSlots, s->as)) != cudaSuccess ||
+        (e = cudaMemsetAsync(s->d_asym, 0, 4 * kSlots, s->as)) != cudaSuccess ||
         (e = cudaMemsetAsync(s->d_work, 0, 256, s->as)) != cudaSuccess ||
-        (e = cudaMemsetAsync(s->d_cta_slots, 0, 4 * (size_t)((s->grid + 31) / 32), s->as)) !=
-            cudaSuccess ||
         (e = cudaMemcpyAsync(s->d_ctl, s->h_ctl, kCtlBytes, cudaMemcpyHostToDevice, s->as)) !=
             cudaSuccess)
         return fail(GSOFA_ERR_CUDA, "workspace init", e);
     if ((e = cudaStreamSynchronize(s->as)) != cudaSuccess)
         return fail(GSOFA_ERR_CUDA, "workspace init", e);
-    s->fixed = s->ws_bytes;
+    s->fixed = s->least + (s->eng[E_CHAIN].on ? s->eng[E_CHAIN].ws_bytes : 0);
     s->in_use = s->peak = s->fixed;
     s->slot_req.assign(kSlots, nullptr);
     for (int i = kSlots - 1; i >= 0; i--) s->free_slots.push_back(i);
-    s->st.grid = s->grid;
-    s->st.block = s->block;
+    const ServeShape& lead = s->eng[s->eng[E_CHAIN].on ? E_CHAIN : E_WALK].shape;
+    s->st.grid = lead.grid;
+    s->st.block = lead.block;
     try {
         s->th = std::thread(loop, s);
     } catch (...) {
@@ -892,7 +1065,7 @@ int gsofa_server_submit(gsofa_server* s, int32_t n, int64_t nnz, const int32_t* 
     r->end = row_end;
     r->col = col;
     r->footprint = request_footprint(s, n, nnz);
-    if (r->footprint + s->fixed > s->budget) return GSOFA_ERR_OOM_BUDGET;
+    if (r->footprint + s->least > s->budget) return GSOFA_ERR_OOM_BUDGET;
     std::lock_guard<std::mutex> g(s->mu);
     if (s->shutdown) return GSOFA_ERR_ARG;
     r->ticket = s->next_ticket++;
