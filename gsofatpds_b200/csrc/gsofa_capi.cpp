@@ -432,7 +432,7 @@ int32_t method_of(const gsofa_matrix* m) {
 }
 
 bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, void* ws,
-              size_t* bytes, size_t room, HubLaunch* L, HubCfg* c) {
+              size_t* bytes, size_t room, HubLaunch* L, HubCfg* c, int most) {
     *L = HubLaunch{};
     *c = HubCfg{};
     long long sources = 0, off = 0, items = 0;
@@ -458,7 +458,7 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     c->sm_count = ctx->sm_count;
     // labels in the shared memory of a cluster: of as many CTAs as leave every
     // job's cluster room on the GPU at once, and hold the largest matrix's labels
-    const int widest = ctx->label_cluster;
+    const int widest = std::min(ctx->label_cluster, most);
     c->cluster = 1;
     while (c->cluster < widest && 2 * W * hubs * 2 * c->cluster <= ctx->sm_count) c->cluster *= 2;
     while (c->cluster < widest && label_smem_bytes(n_max, c->cluster) + 2048 > (size_t)ctx->smem_optin)

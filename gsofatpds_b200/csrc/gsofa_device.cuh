@@ -78,7 +78,9 @@ __device__ __forceinline__ unsigned long long global_ns() {
 __device__ __forceinline__ bool serve_elsewhere(const ServeLaunch& V) {
     unsigned sm;
     asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
-    return V.kind == SERVE_CHAIN ? (int)sm >= ld_vol_i32(V.ctrl + 5) : (int)sm < ld_vol_i32(V.ctrl + 6);
+    return V.kind == SERVE_CHAIN
+               ? (int)sm >= ld_vol_i32(V.ctrl + 5)
+               : (int)sm < ld_vol_i32(V.ctrl + 6) || (int)sm >= ld_vol_i32(V.ctrl + 7);
 }
 
 // Serving, called by all 32 lanes of warp 0: claims a work item of any
@@ -125,7 +127,8 @@ __device__ inline bool serve_claim(const ServeLaunch& V, int* slot_out, long lon
                         __threadfence();  // the descriptor was written before the claim word
                         nit = __ldcg(V.kind == SERVE_CHAIN ? &V.slots[slot].n_items : &V.slots[slot].walk_items);
                         ok = (long long)(v & 0xffffffffull) < nit &&
-                             (V.kind == SERVE_ALL || (__ldcg(V.asym + slot) == 0) == (V.kind == SERVE_CHAIN));
+                             (V.kind == SERVE_ALL ||
+                              __ldcg(V.route + slot) == (V.kind == SERVE_CHAIN ? ROUTE_CHAIN : ROUTE_WALK));
                     }
                 }
             }

@@ -188,9 +188,10 @@ void fill_chain_launch(ChainLaunch* L, const ChainCfg& c, const gsofa_opts& o, i
 int32_t method_of(const gsofa_matrix* m);
 // A launch of gsofa_hub.cu over descriptors whose methods are set: fills their
 // hub_* fields, `L` and `c`, and places the workspace of *bytes, at most `room`
-// if fewer CTAs for large searches can bring it there, in `ws` (null: sizes only).  False: no matrix takes it.
+// if fewer CTAs for large searches can bring it there, in `ws` (null: sizes only).
+// Label searches get clusters of at most `widest` CTAs.  False: no matrix takes it.
 bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, void* ws,
-              size_t* bytes, size_t room, HubLaunch* L, HubCfg* c);
+              size_t* bytes, size_t room, HubLaunch* L, HubCfg* c, int widest = 16);
 // Consecutive sources per work item.
 long long chain_chunk(const gsofa_opts& o, long long total_sources, int32_t nmax, int grid);
 // Result arrays of an n-row matrix, zero-initialised on `stream`.

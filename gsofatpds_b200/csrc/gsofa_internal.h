@@ -112,19 +112,23 @@ struct MatDesc {
 // Every wait is bounded: a CTA that finds nothing to claim for idle_ns (or
 // max_idle_polls polls) exits, which also returns its SM to other work.
 enum : int32_t {
-    SERVE_CHAIN = 0,  // chain_kernel: requests with a symmetric pattern
-    SERVE_WALK = 1,   // traverse_kernel: the others
-    SERVE_ALL = 2,    // traverse_kernel, where it serves alone
+    SERVE_CHAIN = 0,  // chain_kernel: requests routed to it
+    SERVE_WALK = 1,   // traverse_kernel: the same
+    SERVE_ALL = 2,    // traverse_kernel, where it serves alone: any request
 };
+// A slot's route.  The symmetry word of the request's matrix is copied there
+// with its build, so that a symmetric request is the chain's at once; the host
+// sends others to traverse_kernel.
+enum : int32_t { ROUTE_CHAIN = 0, ROUTE_WALK = -2 };
 struct ServeLaunch {
     unsigned long long* claim;            // per slot
     const unsigned long long* list;       // (slot << 32) | request number
     const int32_t* ctrl;                  // [0] exit when idle, [1] take no more items, [2] list entries,
                                           // [3], [4] chain_kernel's, traverse_kernel's launches before this
-                                          // number take no more items; [5] chain_kernel's SMs end and [6]
-                                          // traverse_kernel's begin here
+                                          // number take no more items; [5] chain_kernel's SMs end, [6]
+                                          // traverse_kernel's begin and [7] end here
     int32_t kind;                         // SERVE_*: the requests it takes
-    const int32_t* asym;                  // per slot: not 0 when the request's pattern is unsymmetric
+    const int32_t* route;                 // per slot: ROUTE_*, else nobody claims the request's items
     unsigned int* rr;                     // rotating start of the list scan (tie order)
     const MatDesc* slots;                 // one descriptor per slot
     unsigned long long* items_done;       // per slot: finished items

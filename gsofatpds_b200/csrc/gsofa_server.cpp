@@ -2,12 +2,15 @@
 //
 // One host thread per server drives:
 //   * two persistent traversal kernels, chain_kernel for requests with a
-//     symmetric pattern and traverse_kernel for the others (for all of them with
-//     the diagnostic options, per-row L statistics, or a budget without room for
-//     both workspaces).  Their CTAs claim work items of every published request;
-//     while both have work each uses half of the SMs;
+//     symmetric pattern and traverse_kernel for those without one that the hubs'
+//     launch leaves (for all of them with the diagnostic options, per-row L
+//     statistics, or a budget without room for both workspaces).  Their CTAs claim
+//     work items of every published request;
 //     it stays on the device while published work is waiting and ends by
 //     itself when its CTAs have found nothing to claim for a short while;
+//   * a few lanes for the other requests: each the hubs' launch of a plain call
+//     (gsofa_hub.cu) on a stream and in a workspace of its own.  The SMs are
+//     shared out among the two kernels and the lanes while they have work;
 //   * a side stream for everything else: the upload and padded-CSR build of
 //     each admitted request, its descriptor, the copy that publishes it (its
 //     claim word), and, once the kernel reports the request finished, its
@@ -59,6 +62,7 @@ using namespace gsofa::host;
 
 namespace {
 
+enum ReqRoute { TO_NONE, TO_CHAIN, TO_LANE, TO_WALK };
 enum ReqState { R_QUEUED, R_RUNNING, R_FINISHING, R_DONE, R_FAILED };
 
 struct Request {
@@ -79,12 +83,16 @@ struct Request {
     bool handed_out = false;
     double t_submit = 0, t_admit = 0, t_publish = 0, t_done = 0;
     bool published = false;  // the claim word copy has executed
-    int engine = 0;          // then: the kernel that takes its items
+    int route = 0;           // TO_*: then, who counts it
 };
 
 constexpr int kSlots = 256;
-constexpr int kKernelStreams = 4;  // serving launches of a kernel that may run at once
+constexpr int kKernelStreams = 8;  // launches of a kernel that may run at once (4: 48 requests 126-182 ms, 8: 114-154)
 constexpr int kReserveSms = 4;
+constexpr int kLanes = 3;                      // hubs' launches that may run at once
+constexpr int kLaneCluster = 4;                // CTAs of a lane's label search at most: its SMs are shared
+constexpr size_t kLaneBytes = 16u << 20;       // a lane's workspace for large searches, or that of 64 CTAs
+constexpr double kLaneHoldMs = 1.0;            // the lanes' SMs stay free this long after their last work
 constexpr long long kMaxIdlePolls = 1000000;  // a cap far above idle_ns worth of polls
 constexpr long long kIdleNs = 300000;         // a CTA with nothing to claim for 0.3 ms exits
 constexpr double kTopUpCheckMs = 0.5;         // how often a partial launch is topped up
@@ -138,6 +146,17 @@ struct Engine {
     double alive_checked = -1.0;
 };
 
+// A hubs' launch for one request, and what it needs.
+struct Lane {
+    cudaStream_t st = nullptr;
+    cudaEvent_t done = nullptr;
+    std::shared_ptr<Request> r;  // null: free
+    void* ws = nullptr;
+    size_t bytes = 0;
+    MatDesc* h_desc = nullptr;  // pinned
+    int32_t* h_left = nullptr;  // pinned: the launch left the request
+};
+
 }  // namespace
 
 struct gsofa_server {
@@ -149,6 +168,9 @@ struct gsofa_server {
     int ring = 32;
     bool merge = true;
     Engine eng[kEngines];
+    Lane lanes[kLanes];
+    std::deque<std::shared_ptr<Request>> lane_queue;
+    double lanes_until = -1.0;
     cudaStream_t as = nullptr, cs = nullptr, fs = nullptr;
     std::vector<cudaEvent_t> slot_ev;  // per slot: read-back done
     std::vector<cudaEvent_t> pub_ev;   // per slot: claim word written
@@ -161,8 +183,10 @@ struct gsofa_server {
     int32_t* d_slot_status = nullptr;
     unsigned int* d_rr = nullptr;
     int* h_alive = nullptr;  // pinned read-back of an engine's *d_alive
-    int32_t* d_asym = nullptr;  // per slot: the request's symmetry word
-    int32_t* h_asym = nullptr;
+    int32_t* d_route = nullptr;  // per slot
+    // pinned, 4 words a slot: the matrix's symmetry and repeated-entry words, the
+    // build's status, and ROUTE_WALK to be copied from
+    int32_t* h_words = nullptr;
     unsigned long long* d_work = nullptr;
     int32_t* d_status = nullptr;
     // control table: int32 ctrl[8] (ServeLaunch says what they hold), then u64
@@ -468,7 +492,7 @@ bool admit_one(gsofa_server* s) {
     }
     r->n_items = items;
     r->seq = ++s->seq;
-    r->engine = E_WALK;
+    r->route = TO_NONE;
     MatDesc d = make_desc(r->mat, r->res, 0);
     d.n_items = items;
     d.walk_items = walk_items;
@@ -482,12 +506,15 @@ bool admit_one(gsofa_server* s) {
     e = cudaMemcpyAsync(s->d_slots + slot, s->h_desc + slot, sizeof(MatDesc),
                         cudaMemcpyHostToDevice, s->as);
     if (both) {
-        // which of the two takes the request: read there by a CTA before it
-        // claims, here to keep that kernel running
+        // who counts the request: read there by a CTA before it claims, here to
+        // send it on
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(s->d_asym + slot, r->mat->asym, 4, cudaMemcpyDeviceToDevice, s->as);
+            e = cudaMemcpyAsync(s->d_route + slot, r->mat->asym, 4, cudaMemcpyDeviceToDevice, s->as);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(s->h_asym + slot, r->mat->asym, 4, cudaMemcpyDeviceToHost, s->as);
+            e = cudaMemcpyAsync(s->h_words + 4 * slot, r->mat->asym, 8, cudaMemcpyDeviceToHost, s->as);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(s->h_words + 4 * slot + 2, s->d_slot_status + slot, 4, cudaMemcpyDeviceToHost,
+                                s->as);
     }
     // the publication: the claim word (request number, 0 claimed), ordered
     // after the build and the descriptor
@@ -523,7 +550,7 @@ bool launch_kernel(gsofa_server* s, Engine& E, int k, int grid) {
     V.list = reinterpret_cast<const unsigned long long*>(static_cast<char*>(s->d_ctl) + kCtlFlags);
     V.ctrl = static_cast<const int32_t*>(s->d_ctl);
     V.kind = E.shape.chain ? SERVE_CHAIN : s->eng[E_CHAIN].on ? SERVE_WALK : SERVE_ALL;
-    V.asym = s->d_asym;
+    V.route = s->d_route;
     V.rr = s->d_rr;
     V.nslots = kSlots;
     V.slots = s->d_slots;
@@ -599,23 +626,112 @@ int alive_ctas(gsofa_server* s, const Engine& E) {
     return e == cudaSuccess ? *s->h_alive : E.shape.grid;
 }
 
-// Which SMs each kernel may use: all of them, or half each while there is work
-// for both.  (Halves of every SM's room would never hold a 1,024-thread CTA.)  A
-// CTA on the wrong side leaves after its item.
-void share_sms(gsofa_server* s, const bool* claimable) {
-    const int sms = (int)serve_sms(s->ctx), half = sms / 2;
-    int end = sms, begin = 0;
-    if (claimable[E_CHAIN] && claimable[E_WALK]) end = begin = half;
-    else if (claimable[E_CHAIN]) begin = sms;
-    else if (claimable[E_WALK]) end = 0;
-    else return;
-    if (!s->eng[E_CHAIN].on) begin = 0;
+// Shares the SMs out among the chain, traverse_kernel and the lanes: equal parts
+// for those that have work.  (Parts of every SM's room would never hold a
+// 1,024-thread CTA or a cluster.)  A CTA on another's SM leaves after its item.
+void share_sms(gsofa_server* s, bool chain, bool walk, bool lanes) {
+    const int parts = (chain ? 1 : 0) + (walk ? 1 : 0) + (lanes ? 1 : 0);
+    if (!parts) return;
+    const int each = (int)serve_sms(s->ctx) / parts;
+    const int end = chain ? each : 0, begin = end;
+    const int walk_end = walk ? (lanes ? begin + each : (int)serve_sms(s->ctx)) : begin;
     int32_t* f = ctl_flags(s);
-    if (f[5] == end && f[6] == begin) return;
-    f[5] = end;
+    const int chain_end = chain && parts == 1 ? (int)serve_sms(s->ctx) : end;
+    if (f[5] == chain_end && f[6] == begin && f[7] == walk_end) return;
+    f[5] = chain_end;
     f[6] = begin;
+    f[7] = walk_end;
     push_control(s);
     for (Engine& E : s->eng) E.alive_checked = -1.0;
+}
+
+// traverse_kernel takes the request.
+void to_walk(gsofa_server* s, const std::shared_ptr<Request>& r) {
+    r->route = TO_WALK;
+    if (!s->eng[E_CHAIN].on) return;  // it takes any
+    s->h_words[4 * r->slot + 3] = ROUTE_WALK;
+    const cudaError_t e = cudaMemcpyAsync(s->d_route + r->slot, s->h_words + 4 * r->slot + 3, 4,
+                                          cudaMemcpyHostToDevice, s->cs);
+    if (e != cudaSuccess) server_err(s, "ticket %llu: %s", (unsigned long long)r->ticket, cudaGetErrorString(e));
+}
+
+// Starts the hubs' launch of a request; false: no room for its workspace.
+bool lane_start(gsofa_server* s, Lane& l, const std::shared_ptr<Request>& r) {
+    gsofa_ctx* ctx = s->ctx;
+    size_t room;
+    {
+        std::lock_guard<std::mutex> g(s->mu);
+        room = s->budget - std::min(s->budget, s->in_use);
+    }
+    std::vector<MatDesc> d(1, make_desc(r->mat, r->res, 0));
+    d[0].method = r->n <= kDirectMax ? METHOD_DIRECT : METHOD_HUB;
+    const size_t head = align256(sizeof(MatDesc));
+    HubLaunch L;
+    HubCfg c;
+    size_t bytes = 0;
+    std::lock_guard<std::recursive_mutex> g(ctx->mu);
+    // the labels, totals and queues take less than 256 bytes a row
+    const size_t want = 256 * (size_t)r->n + std::max(kLaneBytes, 64 * 5 * (size_t)r->n);
+    const size_t fit = std::min(room - std::min(room, head), want);
+    plan_hub(ctx, &d, s->opts, nullptr, &bytes, fit, &L, &c, kLaneCluster);
+    if (head + bytes > room || dev_alloc_on(ctx, head + bytes, &l.ws, l.st) != GSOFA_OK) {
+        l.ws = nullptr;
+        return false;
+    }
+    l.bytes = head + bytes;
+    plan_hub(ctx, &d, s->opts, static_cast<char*>(l.ws) + head, &bytes, fit, &L, &c, kLaneCluster);
+    *l.h_desc = d[0];
+    L.mats = static_cast<const MatDesc*>(l.ws);
+    L.status = s->d_status;
+    cudaError_t e = cudaMemcpyAsync(l.ws, l.h_desc, sizeof(MatDesc), cudaMemcpyHostToDevice, l.st);
+    if (e == cudaSuccess) e = launch_hub(L, c, (s->opts.flags & GSOFA_DIGESTS) != 0, l.st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(l.h_left, L.fallback, 4, cudaMemcpyDeviceToHost, l.st);
+    if (e == cudaSuccess) e = cudaEventRecord(l.done, l.st);
+    if (e != cudaSuccess) {
+        cudaStreamSynchronize(l.st);
+        server_err(s, "ticket %llu: %s", (unsigned long long)r->ticket, cudaGetErrorString(e));
+        dev_free_on(ctx, l.ws, l.bytes, l.st);
+        l.ws = nullptr;
+        return false;
+    }
+    l.r = r;
+    std::lock_guard<std::mutex> gs(s->mu);
+    s->in_use += l.bytes;
+    s->peak = std::max(s->peak, s->in_use);
+    s->st.kernel_launches++;
+    return true;
+}
+
+// Lanes whose launch is over; then the next requests for those that are free.
+bool manage_lanes(gsofa_server* s) {
+    bool progress = false;
+    for (Lane& l : s->lanes) {
+        if (l.r) {
+            const cudaError_t q = cudaEventQuery(l.done);
+            if (q == cudaErrorNotReady) continue;
+            progress = true;
+            const std::shared_ptr<Request> r = l.r;
+            l.r.reset();
+            {
+                std::lock_guard<std::recursive_mutex> g(s->ctx->mu);
+                dev_free_on(s->ctx, l.ws, l.bytes, l.st);
+                l.ws = nullptr;
+            }
+            {
+                std::lock_guard<std::mutex> g(s->mu);
+                s->in_use -= std::min(s->in_use, l.bytes);
+            }
+            if (q == cudaSuccess && *l.h_left == 0) s->h_done[r->slot] = r->seq;
+            else to_walk(s, r);
+        }
+        if (!s->lane_queue.empty()) {
+            const std::shared_ptr<Request> r = s->lane_queue.front();
+            s->lane_queue.pop_front();
+            if (!lane_start(s, l, r)) to_walk(s, r);
+            progress = true;
+        }
+    }
+    return progress;
 }
 
 // Keeps a kernel's CTAs on the device while published work is waiting for it.
@@ -651,7 +767,7 @@ bool manage_kernel(gsofa_server* s, int e, bool claimable) {
     if (t - E.alive_checked < kTopUpCheckMs) return progress;
     E.alive_checked = t;
     const int sms = (int)serve_sms(s->ctx);
-    const int mine = e == E_CHAIN ? ctl_flags(s)[5] : sms - ctl_flags(s)[6];
+    const int mine = e == E_CHAIN ? ctl_flags(s)[5] : ctl_flags(s)[7] - ctl_flags(s)[6];
     const bool part = mine < sms;
     const int full = part ? std::min(E.shape.grid, E.shape.occ * std::max(mine, 1)) : E.shape.grid;
     const int missing = full - alive_ctas(s, E);
@@ -740,8 +856,26 @@ bool reap(gsofa_server* s) {
     return progress;
 }
 
+// Waits for the lanes' launches and drops their requests.
+void lanes_stop(gsofa_server* s) {
+    s->lane_queue.clear();
+    for (Lane& l : s->lanes) {
+        if (!l.r) continue;
+        cudaStreamSynchronize(l.st);
+        l.r.reset();
+        {
+            std::lock_guard<std::recursive_mutex> g(s->ctx->mu);
+            dev_free_on(s->ctx, l.ws, l.bytes, l.st);
+            l.ws = nullptr;
+        }
+        std::lock_guard<std::mutex> g(s->mu);
+        s->in_use -= std::min(s->in_use, l.bytes);
+    }
+}
+
 // Fails every admitted request (the kernel is not running).
 void fail_live(gsofa_server* s, int status) {
+    lanes_stop(s);
     std::vector<std::shared_ptr<Request>> act;
     {
         std::lock_guard<std::mutex> g(s->mu);
@@ -771,6 +905,7 @@ void loop(gsofa_server* s) {
         // requests whose claim word is on the device and whose items are not
         // all finished
         bool claimable[kEngines] = {};
+        std::vector<std::shared_ptr<Request>> walk;  // repeated entries, or a build that failed
         {
             std::lock_guard<std::mutex> g(s->mu);
             for (auto& r : s->slot_req) {
@@ -779,12 +914,24 @@ void loop(gsofa_server* s) {
                     cudaEventQuery(s->pub_ev[(size_t)r->slot]) == cudaSuccess) {
                     r->published = true;
                     r->t_publish = now_ms(s);
-                    if (s->eng[E_CHAIN].on && s->h_asym[r->slot] == 0) r->engine = E_CHAIN;
+                    const int32_t* w = s->h_words + 4 * r->slot;
+                    if (!s->eng[E_CHAIN].on) r->route = TO_WALK;
+                    else if (w[0] == 0) r->route = TO_CHAIN;
+                    else if (w[1] == 0 && w[2] == 0) r->route = TO_LANE;
+                    if (r->route == TO_LANE) s->lane_queue.push_back(r);
+                    else if (r->route == TO_NONE) walk.push_back(r);
                 }
-                if (r->published) claimable[r->engine] = true;
+                if (r->route == TO_CHAIN) claimable[E_CHAIN] = true;
+                if (r->route == TO_WALK) claimable[E_WALK] = true;
             }
         }
-        share_sms(s, claimable);
+        for (auto& r : walk) to_walk(s, r);
+        progress |= manage_lanes(s);
+        bool lanes = !s->lane_queue.empty();
+        for (const Lane& l : s->lanes) lanes |= l.r != nullptr;
+        if (lanes) s->lanes_until = now_ms(s) + kLaneHoldMs;
+        const bool held = (claimable[E_CHAIN] || claimable[E_WALK]) && now_ms(s) < s->lanes_until;
+        share_sms(s, claimable[E_CHAIN], claimable[E_WALK], lanes || held);
         s->kernel_running = false;
         for (int e = 0; e < kEngines; e++) progress |= manage_kernel(s, e, claimable[e]);
         if (s->launch_failed) {
@@ -843,6 +990,12 @@ void release(gsofa_server* s) {
     for (Engine& E : s->eng)
         for (int k = 0; k < kKernelStreams; k++)
             if (E.ks[k]) cudaStreamSynchronize(E.ks[k]);
+    for (Lane& l : s->lanes) {
+        if (l.st) cudaStreamSynchronize(l.st);
+        if (l.done) cudaEventDestroy(l.done);
+        if (l.st) cudaStreamDestroy(l.st);
+        if (l.h_desc) cudaFreeHost(l.h_desc);
+    }
     {
         std::lock_guard<std::recursive_mutex> g(ctx->mu);
         cudaStream_t st = s->as ? s->as : ctx->stream;
@@ -862,7 +1015,7 @@ void release(gsofa_server* s) {
             if (E.ks[k]) cudaStreamDestroy(E.ks[k]);
         }
     if (s->as) cudaStreamDestroy(s->as);
-    if (s->h_asym) cudaFreeHost(s->h_asym);
+    if (s->h_words) cudaFreeHost(s->h_words);
     if (s->h_alive) cudaFreeHost(s->h_alive);
     if (s->cs) cudaStreamDestroy(s->cs);
     if (s->fs) cudaStreamDestroy(s->fs);
@@ -936,6 +1089,16 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
             if ((e = cudaStreamCreateWithPriority(&E.ks[k], cudaStreamNonBlocking, prio_low)) != cudaSuccess ||
                 (e = cudaEventCreateWithFlags(&E.kdone[k], cudaEventDisableTiming)) != cudaSuccess)
                 return fail(GSOFA_ERR_CUDA, "stream", e);
+    // (the lanes' kernels end by themselves: they go before CTAs of the two that stay)
+    for (Lane& l : s->lanes) {
+        if (!s->eng[E_CHAIN].on) break;
+        if ((e = cudaStreamCreateWithPriority(&l.st, cudaStreamNonBlocking, (prio_low + prio_high) / 2)) !=
+                cudaSuccess ||
+            (e = cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming)) != cudaSuccess ||
+            (e = cudaMallocHost((void**)&l.h_desc, align256(sizeof(MatDesc)) + 64)) != cudaSuccess)
+            return fail(GSOFA_ERR_CUDA, "lane", e);
+        l.h_left = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(l.h_desc) + align256(sizeof(MatDesc)));
+    }
     if ((e = cudaStreamCreateWithPriority(&s->as, cudaStreamNonBlocking, prio_high)) != cudaSuccess)
         return fail(GSOFA_ERR_CUDA, "stream", e);
     if ((e = cudaStreamCreateWithPriority(&s->cs, cudaStreamNonBlocking, prio_high)) != cudaSuccess)
@@ -956,7 +1119,7 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
     if ((e = cudaHostGetDevicePointer((void**)&s->d_done, s->h_done, 0)) != cudaSuccess)
         return fail(GSOFA_ERR_CUDA, "mapped host memory", e);
     if ((e = cudaMallocHost(&s->h_ctl, kCtlBytes)) != cudaSuccess ||
-        (e = cudaMallocHost((void**)&s->h_asym, 4 * kSlots)) != cudaSuccess ||
+        (e = cudaMallocHost((void**)&s->h_words, 16 * kSlots)) != cudaSuccess ||
         (e = cudaMallocHost((void**)&s->h_alive, 64)) != cudaSuccess)
         return fail(GSOFA_ERR_CUDA, "pinned host memory", e);
     memset(s->h_ctl, 0, kCtlFlags);
@@ -1000,7 +1163,7 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
     b += align256(8 * kSlots);
     s->d_slot_status = reinterpret_cast<int32_t*>(b);
     b += align256(4 * kSlots);
-    s->d_asym = reinterpret_cast<int32_t*>(b);
+    s->d_route = reinterpret_cast<int32_t*>(b);
     b += align256(4 * kSlots);
     s->d_work = reinterpret_cast<unsigned long long*>(b);
     s->d_rr = reinterpret_cast<unsigned int*>(s->d_work + 1);
@@ -1008,7 +1171,7 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
     b += 256;
     s->d_ctl = b;
     int32_t* const flags = ctl_flags(s);
-    flags[5] = (int32_t)serve_sms(ctx);
+    flags[5] = flags[7] = (int32_t)serve_sms(ctx);
     for (Engine& E : s->eng) {
         if (!E.on) continue;
         char* w = static_cast<char*>(E.ws);
@@ -1028,7 +1191,7 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
     }
     // claim words start at request number 0 (never used): nothing claimable
     if ((e = cudaMemsetAsync(s->d_claim, 0, 8 * kSlots, s->as)) != cudaSuccess ||
-        (e = cudaMemsetAsync(s->d_asym, 0, 4 * kSlots, s->as)) != cudaSuccess ||
+        (e = cudaMemsetAsync(s->d_route, 0, 4 * kSlots, s->as)) != cudaSuccess ||
         (e = cudaMemsetAsync(s->d_work, 0, 256, s->as)) != cudaSuccess ||
         (e = cudaMemcpyAsync(s->d_ctl, s->h_ctl, kCtlBytes, cudaMemcpyHostToDevice, s->as)) !=
             cudaSuccess)

@@ -349,7 +349,7 @@ typedef struct gsofa_ticket_info {
 int gsofa_server_ticket_info(gsofa_server* srv, uint64_t ticket, gsofa_ticket_info* info);
 typedef struct gsofa_server_stats {
     uint64_t submitted, completed, failed;
-    uint64_t kernel_launches;   /* persistent kernel (re)launches          */
+    uint64_t kernel_launches;   /* of the persistent kernels and the hubs   */
     uint64_t items_published;
     uint64_t bytes_in_use;      /* workspace + admitted requests            */
     uint64_t peak_bytes;

@@ -1,12 +1,16 @@
-"""The request loop's two kernels: symmetric requests by the chain, the others
-by traverse_kernel, side by side; few CTAs; budgets that were enough for
-traverse_kernel's workspace alone, where the chain's makes room."""
+"""The request loop's routes: symmetric requests by the chain, the others by the
+hubs' launch in a lane, what that leaves by traverse_kernel, side by side; few
+CTAs; budgets that were enough for traverse_kernel's workspace alone, where the
+chain's makes room."""
 import threading
 import time
 
+import numpy as np
 import pytest
 
-from gsofatpds_b200 import Context, gen
+from gsofatpds_b200 import _lib as C
+from gsofatpds_b200 import Context, GsofaError, gen
+from tests.helpers import scrambled_csr
 from tests.test_gpu_serving import _alone, _cuda, _same, _submit
 
 pytestmark = pytest.mark.gpu
@@ -75,6 +79,36 @@ def test_neither_kind_waits_for_the_other(ctx, refs):
             stop.set()
             th.join()
         assert done[0] > 0
+
+
+def test_every_route(ctx):
+    """Unsymmetric requests of a lane's own making: few rows, entries twice, a
+    malformed one, none at all; beside symmetric ones."""
+    rng = np.random.default_rng(84)
+    few = gen.random_extra(700, 2, seed=85)[1:]
+    _, rp, col = gen.random_extra(2000, 3, seed=86)
+    twice = scrambled_csr(rng, [set(col[rp[v]:rp[v + 1]]) for v in range(2000)], dup_prob=0.3)
+    one = gen.from_coo(1, [0], [0])[1:]
+    large = gen.random_banded(90000, bw=6, extra=2, seed=87)[1:]
+    specs = [few, twice, one, MESH, BAND, large]
+    want = [_alone(ctx, x) for x in specs]
+    bad = col.copy()
+    bad[11] = 1 << 30
+    with ctx.server(max_n=100000) as srv:
+        for _ in range(2):
+            tickets = [_submit(srv, x) for x in specs]
+            t_bad = srv.submit_rowptr(rp, bad)
+            t_none = srv.submit_rowptr(np.zeros(1, np.int64), np.zeros(0, np.int32))
+            for t, w in zip(tickets, want):
+                got = srv.wait(t, 60000)
+                _same("route", got, w)
+                got.close()
+            with pytest.raises(GsofaError) as e:
+                srv.wait(t_bad, 60000)
+            assert e.value.status == C.ERR_ARG
+            got = srv.wait(t_none, 60000)
+            assert got.counts["nnz_u"] == 0
+            got.close()
 
 
 def workspaces(ctx, max_n, spec):
