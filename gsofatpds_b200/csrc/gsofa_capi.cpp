@@ -772,6 +772,7 @@ int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t cou
     for (int32_t k = 0; k < count && chain; k++)
         if (descs[(size_t)k].method == METHOD_WALK || (hub && ctx->h_fallback[k]))
             left.push_back(order[(size_t)k]);
+    const int walked = chain ? (int)left.size() : count;
     if (!left.empty()) {
         std::vector<const gsofa_matrix*> lm;
         std::vector<gsofa_result*> lr;
@@ -833,6 +834,7 @@ int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t cou
         if (rc) return rc;
     }
 
+    ctx->walked = walked;
     for (int32_t i = 0; i < count; i++) {
         gsofa_result* r = res[i];
         const unsigned long long* c = totals.data() + (size_t)i * CNT_SLOTS;
@@ -859,6 +861,7 @@ int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t cou
 int run_factor(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count, const gsofa_opts* o,
                gsofa_result** res, long long sample_stride = 1) {
     ctx->factoring = true;
+    ctx->walked = 0;
     int rc = run_factor_with(ctx, mats, count, o, res, sample_stride, true);
     if (rc == GSOFA_ERR_OOM_BUDGET) {
         drop_workspace(ctx);
@@ -1434,10 +1437,10 @@ static gsofa_opts base_without_l_rows(gsofa_opts o) {
 // the fastest.  The candidates differ only in speed: every setting gives the
 // same results.  Choices are cached per size class in the context.
 // Coordinate descent over the launch shape, each candidate timed on the device
-// as one call over all `count` matrices: CTA size and chunk of the chain's
-// launch where it takes any of them, or CTA size, closure ring, chunk and
-// warp-walked row threshold of traverse_kernel's where that counts.  The hubs'
-// launches have no shape to choose.  Writes the best into *opts.
+// as one call over all `count` matrices: CTA size and chunk where the chain or
+// traverse_kernel counts any of them (in a list with both, one choice for both),
+// and closure ring and warp-walked row threshold where traverse_kernel does.  The
+// hubs' launches have no shape to choose.  Writes the best into *opts.
 static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t count,
                          gsofa_opts* opts) {
     int rc = GSOFA_OK;
@@ -1464,6 +1467,7 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
     }
     rc = run_factor(ctx, mats, count, &base, rr.data());
     if (rc) { free_all(); return rc; }
+    const bool walked = ctx->walked > 0;
     const double full_ms = rr[0]->counts.ms_traverse;  // the launch's time
     // Full runs while they are short; above 2 s time every stride-th work
     // item, keeping at least 16 items per CTA so the tail does not dominate.
@@ -1499,14 +1503,14 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
     rc = time_opts(best, &best_ms);
     if (rc) { free_all(); return rc; }
     long long auto_chunk = 64;
-    bool walks = !chain;  // some matrix's counting depends on the shape
+    long long chain_sources = 0;
+    bool walks = walked;  // some matrix's counting depends on the shape
     {
         LaunchCfg c0;
         if (plan_launch(ctx, nmax, &base, &c0) == GSOFA_OK) {
             best.threads_per_source = c0.block;
             auto_chunk = default_chunk(total_sources, c0.grid);
         }
-        long long chain_sources = 0;
         for (int32_t i = 0; i < count; i++) {
             if (!chain || method_of(mats[i]) != METHOD_CHAIN) continue;
             walks = true;
@@ -1534,7 +1538,7 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
     const int ring_now = best.cached_closures > 0 ? best.cached_closures : kDefaultRing;
     best.cached_closures = ring_now;
     for (int ring : ring_c) {
-        if (ring == ring_now || chain) continue;
+        if (ring == ring_now || !walked) continue;
         gsofa_opts p = best;
         p.cached_closures = ring;
         double ms;
@@ -1543,7 +1547,7 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
     }
     {
         LaunchCfg c;
-        if (!chain && plan_launch(ctx, nmax, &best, &c) == GSOFA_OK)
+        if (chain_sources == 0 && plan_launch(ctx, nmax, &best, &c) == GSOFA_OK)
             auto_chunk = default_chunk(total_sources, c.grid);
         ctx->err.clear();
         if (best.chunk_sources <= 0) best.chunk_sources = (int32_t)auto_chunk;
@@ -1561,7 +1565,7 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
     const int heavy_now = best.heavy_row > 0 ? best.heavy_row : kDefaultHeavyRow;
     best.heavy_row = heavy_now;
     for (int hr : {32, 64}) {
-        if (hr == heavy_now || chain) continue;
+        if (hr == heavy_now || !walked) continue;
         gsofa_opts p = best;
         p.heavy_row = hr;
         double ms;

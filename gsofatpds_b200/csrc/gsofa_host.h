@@ -56,6 +56,7 @@ struct gsofa_ctx {
     void* hub_ws = nullptr;
     size_t hub_ws_bytes = 0;
     bool factoring = false;  // the workspace above is in use
+    int walked = 0;          // matrices of the last counting call that traverse_kernel counted
     int label_cluster = 0;   // CTAs of the widest cluster a label search may have
 };
 

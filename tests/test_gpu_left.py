@@ -112,3 +112,26 @@ def test_a_mesh_is_left_early(ctx):  # noqa: F811
         b.close()
     m.close()
     assert default < 1.2 * min(alone) + 0.2
+
+
+@pytest.mark.parametrize("name", ["mesh", "band", "twice"])
+def test_autotuned_shapes_for_what_is_left(ctx, name):  # noqa: F811
+    """The autotuner times traverse_kernel's shapes where that counts: the
+    tuned call is no slower than the default one, and as exact."""
+    t = {"mesh": lambda: plain(oriented(gen.grid_nd((170, 170), "5"))),
+         "band": lambda: plain(gen.random_banded(30000, bw=4, extra=0, seed=6)),
+         "twice": lambda: doubled(gen.random_extra(2500, 3, seed=32), 1)}[name]()
+    m = ctx.load_csr(*t)
+    tuned = ctx.autotune(m)
+    _, default = best(ctx, m)
+    _, fast = best(ctx, m, **tuned)
+    a, b = ctx.factor(m), ctx.factor(m, **tuned)
+    for x, y in zip(list(a.row_counts().values()) + list(a.digests().values()),
+                    list(b.row_counts().values()) + list(b.digests().values())):
+        np.testing.assert_array_equal(x, y)
+    a.close()
+    b.close()
+    m.close()
+    assert fast < 1.1 * default + 0.1
+    if name == "mesh":
+        assert fast < 0.9 * default  # 16-source chunks by 128 threads
