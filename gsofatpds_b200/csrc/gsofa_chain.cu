@@ -972,7 +972,7 @@ template <int BLOCK, bool SERVE>
 int occupancy_one(size_t smem) {
     auto k = chain_kernel<BLOCK, SERVE>;
     int blocks = 0;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if (allow_shared_memory<chain_kernel<BLOCK, SERVE>>() != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, BLOCK, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -983,7 +983,7 @@ int occupancy_one(size_t smem) {
 template <int BLOCK, bool SERVE>
 cudaError_t launch_one(const ChainLaunch& L, int grid, size_t smem, cudaStream_t st) {
     auto k = chain_kernel<BLOCK, SERVE>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory<chain_kernel<BLOCK, SERVE>>();
     if (e != cudaSuccess) return e;
     k<<<grid, BLOCK, smem, st>>>(L);
     return cudaGetLastError();

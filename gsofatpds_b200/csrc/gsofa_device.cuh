@@ -1,11 +1,35 @@
 // Device helpers shared by the traversal kernels (gsofa_kernels.cu,
 // gsofa_chain.cu): loads, digests, work-item lookup and serving claims.
 #pragma once
+#include <atomic>
+
 #include "gsofa_internal.h"
 
 namespace gsofa {
 
 #define FULL_MASK 0xffffffffu
+
+// Lets a kernel's launches ask for all the dynamic shared memory a CTA may
+// have.  The limit belongs to the function, for every thread of the process: one
+// set to a launch's own need could be lowered by another thread before that
+// launch.
+template <auto KERNEL>
+cudaError_t allow_shared_memory() {
+    static std::atomic<int> limits[64];  // per device, once known
+    int dev = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    int limit = dev < 64 ? limits[dev].load(std::memory_order_relaxed) : 0;
+    if (limit == 0) {
+        cudaFuncAttributes fa;
+        e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, KERNEL);
+        if (e != cudaSuccess) return e;
+        limit = most - (int)fa.sharedSizeBytes;
+        if (dev < 64) limits[dev].store(limit, std::memory_order_relaxed);
+    }
+    return cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+}
 
 // Digest mixing: splitmix64 finaliser (Steele, Lea, Flood 2014).  A U-row
 // or L-column digest sums mix64((w << 32) | mask) over the set's non-zero

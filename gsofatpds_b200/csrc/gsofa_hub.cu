@@ -965,7 +965,7 @@ size_t hub_scan_bytes(long long tots, long long uses) {
 
 int large_occupancy(size_t smem) {
     int occ = 0;
-    cudaError_t e = cudaFuncSetAttribute(large_kernel<kLargeThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory<large_kernel<kLargeThreads>>();
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, large_kernel<kLargeThreads>, kLargeThreads, smem);
     if (e != cudaSuccess) cudaGetLastError();
@@ -974,7 +974,7 @@ int large_occupancy(size_t smem) {
 
 static cudaError_t label_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int jobs, int cluster,
                                 size_t smem, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(label_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared_memory<label_cluster_kernel>();
     if (e == cudaSuccess && cluster > 8)
         e = cudaFuncSetAttribute(label_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     *cfg = cudaLaunchConfig_t{};
@@ -1040,8 +1040,7 @@ cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStr
         if (e != cudaSuccess) return e;
     }
     const size_t smem = sizeof(WarpTable) * (kExtraThreads / 32);
-    if ((e = cudaFuncSetAttribute(extra_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
-        return e;
+    if ((e = allow_shared_memory<extra_kernel>()) != cudaSuccess) return e;
     const long long want = (L.total_items + kExtraThreads / 32 - 1) / (kExtraThreads / 32);
     extra_kernel<<<(int)std::min<long long>(want, c.extra_grid), kExtraThreads, smem, st>>>(L);
     large_kernel<kLargeThreads><<<c.large_grid, kLargeThreads, c.large_smem, st>>>(L);

@@ -1115,8 +1115,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) traverse_kernel(TraverseL
 template <int BLOCK, int MODE>
 static cudaError_t launch_one(const TraverseLaunch& L, int grid, size_t smem, cudaStream_t st) {
     auto k = traverse_kernel<BLOCK, MODE>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(MODE == 0 ? 0 : smem));
+    cudaError_t e = allow_shared_memory<traverse_kernel<BLOCK, MODE>>();
     if (e != cudaSuccess) return e;
     k<<<grid, BLOCK, MODE == 0 ? 0 : smem, st>>>(L);
     return cudaGetLastError();
@@ -1125,8 +1124,7 @@ static cudaError_t launch_one(const TraverseLaunch& L, int grid, size_t smem, cu
 template <int BLOCK, int MODE>
 static int occ_one(size_t smem) {
     auto k = traverse_kernel<BLOCK, MODE>;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(MODE == 0 ? 0 : smem)) != cudaSuccess) {
+    if (allow_shared_memory<traverse_kernel<BLOCK, MODE>>() != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
