@@ -91,7 +91,7 @@ constexpr int kKernelStreams = 8;  // launches of a kernel that may run at once 
 constexpr int kReserveSms = 4;
 constexpr int kLanes = 3;                      // hubs' launches that may run at once
 constexpr int kLaneCluster = 4;                // CTAs of a lane's label search at most: its SMs are shared
-constexpr size_t kLaneBytes = 16u << 20;       // a lane's workspace for large searches, or that of 64 CTAs
+constexpr size_t kLaneBytes = 64u << 20;       // a lane's workspace for large searches, or that of 296 CTAs
 constexpr double kLaneHoldMs = 1.0;            // the lanes' SMs stay free this long after their last work
 constexpr long long kMaxIdlePolls = 1000000;  // a cap far above idle_ns worth of polls
 constexpr long long kIdleNs = 300000;         // a CTA with nothing to claim for 0.3 ms exits
@@ -671,7 +671,7 @@ bool lane_start(gsofa_server* s, Lane& l, const std::shared_ptr<Request>& r) {
     size_t bytes = 0;
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     // the labels, totals and queues take less than 256 bytes a row
-    const size_t want = 256 * (size_t)r->n + std::max(kLaneBytes, 64 * 5 * (size_t)r->n);
+    const size_t want = 256 * (size_t)r->n + std::max(kLaneBytes, 296 * 5 * (size_t)r->n);
     const size_t fit = std::min(room - std::min(room, head), want);
     plan_hub(ctx, &d, s->opts, nullptr, &bytes, fit, &L, &c, kLaneCluster);
     if (head + bytes > room || dev_alloc_on(ctx, head + bytes, &l.ws, l.st) != GSOFA_OK) {
