@@ -77,7 +77,11 @@ constexpr int kLabelThreads = 1024;
 constexpr int kNoLabel = 0x7f7f7f7f;  // label_round_kernel's arrays are set bytewise
 constexpr int kExtraThreads = 256;
 constexpr int kLargeThreads = 256;
-constexpr int kJudgeAfter = 512;  // searches before a matrix may be left
+// A matrix is left when more than half of at least kJudgeEarly searches, or more
+// than a quarter of kJudgeAfter, have outgrown the table: looked at with every
+// such search, and what is under way then ends with it (at the end of every
+// item instead, a batch of 48 bands without a core spent 10 of 28 ms there).
+constexpr int kJudgeEarly = 64, kJudgeAfter = 512;
 
 struct WarpTable {
     uint32_t key[kSlots];
@@ -613,7 +617,8 @@ __global__ void __launch_bounds__(kExtraThreads, 1024 / kExtraThreads) extra_ker
         const Graph G = d ? Graph{M.trowptr, M.tcol} : Graph{M.rowptr, M.col};
         const int s_first = g * P.group, s_end = min(n, s_first + P.group);
         unsigned long long a_fill = 0, a_e = 0, a_v = 0, a_nnz = 0, a_trav = 0;
-        int a_hub = 0, a_large = 0;
+        int a_hub = 0, judged = s_first;  // the item's sources below `judged` have been counted
+        bool abandoned = false;
         int r0 = __ldg(G.rp + s_first), r1 = __ldg(G.rp + s_first + 1);
         int4 pre = make_int4(-1, -1, -1, -1);
         if (4 * lane < (r1 & ~3) - (r0 & ~3)) pre = ld_row4<false>(G.cl + (r0 & ~3) + 4 * lane);
@@ -716,12 +721,21 @@ __global__ void __launch_bounds__(kExtraThreads, 1024 / kExtraThreads) extra_ker
                 h = min(h + 32, end);
             }
             if (large) {
-                a_large++;
+                int left = 0;
                 if (lane == 0) {
                     // room for every (source, direction) of the launch
                     const int p = atomicAdd(P.large_count, 1);
                     P.large[p] = (unsigned long long)mi << 33 | (unsigned long long)d << 32 | (unsigned)s;
+                    const int done = atomicAdd(P.judged + 2 * mi, s + 1 - judged) + s + 1 - judged;
+                    const int big = atomicAdd(P.judged + 2 * mi + 1, 1) + 1;
+                    if (n > kDirectMax && ((done >= kJudgeEarly && 2ll * big > done) ||
+                                           (done >= kJudgeAfter && 4ll * big > done)))
+                        atomicExch(P.fallback + mi, 1);
+                    left = ld_vol_i32(P.fallback + mi);
                 }
+                judged = s + 1;
+                abandoned = __shfl_sync(FULL_MASK, left, 0) != 0;
+                if (abandoned) break;
             } else {
                 Tot t = B.t;
                 raw = __reduce_add_sync(FULL_MASK, raw);
@@ -778,7 +792,7 @@ __global__ void __launch_bounds__(kExtraThreads, 1024 / kExtraThreads) extra_ker
             r0 = r1;
             r1 = r2;
         }
-        if (lane == 0) {
+        if (lane == 0 && !abandoned) {
             unsigned long long* c = P.counters + (long long)mi * CNT_SLOTS;
             atomicAdd(c + CNT_FILLS, a_fill);
             atomicAdd(c + CNT_EDGES_TRAV, a_trav);
@@ -789,11 +803,7 @@ __global__ void __launch_bounds__(kExtraThreads, 1024 / kExtraThreads) extra_ker
             }
             if (d == 1 || sym) atomicAdd(c + CNT_NNZ_L, a_nnz);
             if (a_hub) atomicAdd(c + CNT_CHAINED, (unsigned long long)a_hub);
-            const int done = atomicAdd(P.judged + 2 * mi, s_end - s_first) + s_end - s_first;
-            if (a_large) {
-                const int big = atomicAdd(P.judged + 2 * mi + 1, a_large) + a_large;
-                if (M.n > kDirectMax && done >= kJudgeAfter && 4ll * big > done) atomicExch(P.fallback + mi, 1);
-            }
+            atomicAdd(P.judged + 2 * mi, s_end - judged);
         }
     }
 }
