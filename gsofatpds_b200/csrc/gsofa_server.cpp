@@ -533,13 +533,6 @@ bool admit_one(gsofa_server* s) {
         std::lock_guard<std::mutex> g(s->mu);
         s->st.items_published += (uint64_t)items;
     }
-    if (items == 0) {
-        // nothing for the kernel: read back at once
-        std::lock_guard<std::mutex> g(s->mu);
-        r->published = true;
-        r->t_publish = now_ms(s);
-        s->h_done[slot] = r->seq;
-    }
     return true;
 }
 
@@ -909,11 +902,15 @@ void loop(gsofa_server* s) {
         {
             std::lock_guard<std::mutex> g(s->mu);
             for (auto& r : s->slot_req) {
-                if (!r || r->state != R_RUNNING || r->n_items == 0) continue;
+                if (!r || r->state != R_RUNNING) continue;
                 if (!r->published &&
                     cudaEventQuery(s->pub_ev[(size_t)r->slot]) == cudaSuccess) {
                     r->published = true;
                     r->t_publish = now_ms(s);
+                    if (r->n_items == 0) {  // no rows: to be read back, now that its totals are zeroed
+                        s->h_done[r->slot] = r->seq;
+                        continue;
+                    }
                     const int32_t* w = s->h_words + 4 * r->slot;
                     if (!s->eng[E_CHAIN].on) r->route = TO_WALK;
                     else if (w[0] == 0) r->route = TO_CHAIN;
