@@ -516,6 +516,7 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     L->stamp = static_cast<int32_t*>(place(4 * 2 * (size_t)W * T));
     L->lcnt = static_cast<int32_t*>(place(32 * 2 * (size_t)W * (size_t)nm));
     L->fallback = static_cast<int32_t*>(place(4 * (size_t)nm));
+    L->given_up = static_cast<int32_t*>(place(4 * (size_t)nm));
     L->judged = static_cast<int32_t*>(place(8 * (size_t)nm));
     L->counters = static_cast<unsigned long long*>(place(8 * CNT_SLOTS * (size_t)nm));
     L->hubs = static_cast<unsigned long long*>(place(8 * (size_t)W * (size_t)nm));

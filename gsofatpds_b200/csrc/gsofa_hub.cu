@@ -55,15 +55,22 @@ namespace {
 constexpr int kWindows = 3;
 constexpr int kHubs = 4;  // two for the first window, one for each other
 constexpr int kBases = 2;  // arrays of totals: a source has at most two hubs to choose from
-// Label rounds before a matrix is left: 24 at n = 5,000, 103 to 192 at 20,000 and
-// 96 at 40,000 were enough for matrices with a core (random and banded with
-// uniform entries, circuit-like); a band without one uses up all of them, which
-// at 192 was 0.6 of 2.6 ms at n = 5,000.  Far larger ones need more: a band with
-// one uniform entry per row at n = 1,200,000 more than 192 (left: 582 ms).
-__host__ __device__ __forceinline__ int label_rounds(int n) {
+// Label rounds after which a hub is given up.  First window: 24 at n = 5,000, 39
+// to 284 at 20,000 and 96 at 40,000 for matrices with a core (random and banded
+// with uniform entries, circuit-like), and seldom both of its hubs above 192; a
+// band without a core uses up all of them, which at 192 was 0.6 of 2.6 ms at
+// n = 5,000.  Far larger ones need more: a band with one uniform entry per row at
+// n = 1,200,000 more than 192 (left: 582 ms).  The other windows' few ids are a
+// band with hardly an entry besides, where labels travel along: up to 278 at
+// 20,000.  (With 192 for all, and a matrix left with its first such hub, 9 of 40
+// random n = 20,000 matrices were left, at 2.2 ms; now none, 0.5 to 0.9.)
+__host__ __device__ __forceinline__ int label_rounds(int n, int window) {
+    if (window) return 64 + n / 32;
     const int a = 64 + n / 64, b = n / 2048 < 192 ? 192 : n / 2048;
     return a < b ? a : b;
 }
+// The first window's limit once its set has stopped growing (see settled).
+__host__ __device__ __forceinline__ int label_rounds_settled(int n) { return 128 + n / 64; }
 // A core is reached within a few tens of rounds, the rest only lower labels; in
 // a mesh the hub's set still grows then.  The ids first reached in the rounds up
 // to kSpread, in the next 16 and in the 16 after that are counted; a matrix is
@@ -107,7 +114,20 @@ __device__ __forceinline__ long long lam_at(const HubLaunch& P, const MatDesc& M
 // The count that round r adds to: 0 up to kSpread, 1 and 2 for the steps after it.
 __device__ __forceinline__ int spread_part(int r) { return r < kSpread ? 0 : r < kSpread + kSpreadStep ? 1 : 2; }
 
+// Less than an eighth of the set came in the last step: a core has been reached,
+// and the rounds that are left lower labels.
+__device__ __forceinline__ bool settled(int all, int last) { return 8ll * last <= all; }
+
 __device__ __forceinline__ bool spreads(int n, int before, int last) { return 2 * last > before && 64 * (long long)last > n; }
+
+// A label search of hub h did not finish.  The hub's labels in that direction
+// become none, so that no search starts from it or finds anything in its set; the
+// first window has another hub.  Without that one, or another window's only
+// hub, the matrix is left.
+__device__ __forceinline__ void give_up(const HubLaunch& P, int mi, int h) {
+    const int before = atomicOr(P.given_up + mi, 1 << h);
+    if (h > 1 || ((before | 1 << h) & 3) == 3) atomicExch(P.fallback + mi, 1);
+}
 
 // Per matrix and hub, several CTAs: the largest key (degree product, then
 // smallest id).  The first window's two hubs are the best of the even and of
@@ -228,8 +248,7 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
         __stcg(q[0], hub);
     }
     group_sync();
-    const int rounds = label_rounds(n);
-    int r = 0, count = 0, got = 0;
+    int rounds = label_rounds(n, l), r = 0, count = 0, got = 0;
     for (; r < rounds; r++) {
         count = dsm_ld(cnt_a + 4 * (r % 3));
         if (count == 0) break;
@@ -301,23 +320,28 @@ __global__ void __launch_bounds__(kLabelThreads) label_cluster_kernel(HubLaunch 
         if (r % kLook == kLook - 1 && rank == 0 && threadIdx.x == 0)
             quit[(r + 1) / kLook % 2] = ld_vol_i32(P.fallback + mi);
         group_sync();
-        if (l == 0 && r == kSpreadEnd - 1 && spreads(n, dsm_ld(reached_a + 4), dsm_ld(reached_a + 8))) {
-            if (rank == 0 && threadIdx.x == 0) atomicExch(P.fallback + mi, 1);
-            break;
+        if (l == 0 && r == kSpreadEnd - 1) {
+            const int first = dsm_ld(reached_a), before = dsm_ld(reached_a + 4), last = dsm_ld(reached_a + 8);
+            if (spreads(n, before, last)) {
+                if (rank == 0 && threadIdx.x == 0) atomicExch(P.fallback + mi, 1);
+                break;
+            }
+            if (settled(first + before + last, last)) rounds = max(rounds, label_rounds_settled(n));
         }
     }
-    if (r == rounds && dsm_ld(cnt_a + 4 * (r % 3)) != 0 && rank == 0 && threadIdx.x == 0)
-        atomicExch(P.fallback + mi, 1);  // unfinished labels are too large
+    // unfinished labels are too large: the hub reaches nothing
+    const bool none = r == rounds && dsm_ld(cnt_a + 4 * (r % 3)) != 0;
+    if (none && rank == 0 && threadIdx.x == 0) give_up(P, mi, h);
     for (int w = (int)rank + (int)C * (threadIdx.x >> 5); w < nw; w += (int)C * (kLabelThreads / 32)) {
         // whole groups: the ids from n on have no label
-        P.lam[at + 32ll * w + lane] = label_of_word(lam[32 * (w >> shift) + lane]);
+        P.lam[at + 32ll * w + lane] = label_of_word(none ? kNoLabelWord : lam[32 * (w >> shift) + lane]);
     }
     group_sync();  // no CTA leaves while another may still read its counts
 }
 
 // The same by the whole GPU, one launch per round (labels, queues, counts in
 // global memory): `per` CTAs a job, a launch that finds nothing queued ends at
-// once.  The matrix is left if its last round finds ids queued.
+// once; after the last, label_drop_kernel looks for unfinished searches.
 __global__ void label_start_kernel(HubLaunch P) {
     const int job = blockIdx.x;
     const int mi = job / (2 * kHubs), h = (job >> 1) % kHubs, d = job & 1;
@@ -343,9 +367,8 @@ __global__ void __launch_bounds__(kLabelThreads) label_round_kernel(HubLaunch P,
     if (lane == 0) left = ld_vol_i32(P.fallback + mi);
     if (__shfl_sync(FULL_MASK, left, 0)) return;
     const int l = window_of_hub(h);
-    if (part == 0 && threadIdx.x == 0 &&
-        (r >= label_rounds(P.mats[mi].n) - 1 ||
-         (l == 0 && r == kSpreadEnd && spreads(P.mats[mi].n, reached[1], reached[2]))))
+    if (part == 0 && threadIdx.x == 0 && l == 0 && r == kSpreadEnd &&
+        spreads(P.mats[mi].n, reached[1], reached[2]))
         atomicExch(P.fallback + mi, 1);
     const int gw = (part * kLabelThreads + threadIdx.x) >> 5;
     const int nwarps = per_job * (kLabelThreads / 32);
@@ -420,6 +443,17 @@ __global__ void __launch_bounds__(kLabelThreads) label_round_kernel(HubLaunch P,
         got = __reduce_add_sync(FULL_MASK, got);
         if (lane == 0 && got) atomicAdd(reached + spread_part(r), got);
     }
+}
+
+// Searches with ids still queued after the last round.
+__global__ void label_drop_kernel(HubLaunch P, int per_job, int rounds) {
+    const int job = blockIdx.x / per_job, part = blockIdx.x % per_job;
+    if (P.lcnt[8ll * job + rounds % 3] == 0) return;
+    const int mi = job / (2 * kHubs), h = (job >> 1) % kHubs, d = job & 1;
+    const MatDesc& M = P.mats[mi];
+    if (part == 0 && threadIdx.x == 0) give_up(P, mi, h);
+    int32_t* const lam = P.lam + lam_at(P, M, h, d);
+    for (long long v = part * blockDim.x + threadIdx.x; v < M.hub_len; v += per_job * blockDim.x) lam[v] = kNoLabel;
 }
 
 // The changes over s of the hub set's totals.  A warp per word: lane j is id
@@ -1039,8 +1073,9 @@ cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStr
             // two CTAs per SM over a matrix's eight jobs: a round without work costs
             // its CTAs' launch (n = 1,200,000: 16 CTAs per SM 38 ms, two 33)
             const int per = std::max(8, c.sm_count / (4 * std::min(L.hub_mats, 8)));
-            for (int r = 0; r < label_rounds(c.n_max); r++)
-                label_round_kernel<<<per * jobs, kLabelThreads, 0, st>>>(L, per, r);
+            const int rounds = label_rounds(c.n_max, 0);
+            for (int r = 0; r < rounds; r++) label_round_kernel<<<per * jobs, kLabelThreads, 0, st>>>(L, per, r);
+            label_drop_kernel<<<per * jobs, kLabelThreads, 0, st>>>(L, per, rounds);
         }
         const int words = (int)((c.n_max + 31) / 32);
         const int per = parts((words + 7) / 8, jobs);

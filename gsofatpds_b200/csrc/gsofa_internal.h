@@ -241,6 +241,7 @@ struct HubLaunch {
     int32_t* stamp;                    // as lam
     int32_t* lcnt;                     // 8 per label job
     int32_t* fallback;                 // per matrix: left to traverse_kernel
+    int32_t* given_up;                 // per matrix: bit h when hub h has been given up
     int32_t* judged;                   // per matrix: searches done, searches too large
     unsigned long long* counters;      // per matrix, CNT_SLOTS
     int* large_count;

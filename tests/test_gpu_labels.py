@@ -56,3 +56,19 @@ def test_labels_by_the_whole_gpu(ctx, name):  # noqa: F811
         res.close()
     for x in mats[:2]:
         x.close()
+
+
+@pytest.mark.parametrize("seed", [8, 32])
+def test_a_hub_that_is_given_up(ctx, seed):  # noqa: F811
+    """Random patterns whose labels take more than 192 rounds for one of the
+    first window's hubs: given up in the whole GPU's rounds (which end there),
+    finished by the clusters (whose limit is higher once the set has settled)."""
+    n, rp, col = gen.random_extra(20000, 3, seed=seed)
+    beg, end = gen.csr_to_beg_end(rp)
+    r, rt = oracle_full(beg, end, col)
+    m = ctx.load_rowptr(rp, col)
+    for kw in (dict(), dict(global_bitmap=True), dict(l_row_stats=True), dict(global_bitmap=True, l_row_stats=True)):
+        res = ctx.factor(m, **kw)
+        check_full(res, r, rt, l_rows="l_row_stats" in kw)
+        res.close()
+    m.close()
