@@ -380,17 +380,14 @@ bool chain_runs(const gsofa_opts& o, const gsofa_matrix* const* mats, int32_t co
     return any && hub_rows * std::max(hub_count(), 2 * hub_bases()) <= INT_MAX;
 }
 
-int plan_chain(gsofa_ctx* ctx, int32_t nmax, long long total_sources, bool all_sym, const gsofa_opts* o,
-               bool serve, ChainCfg* c) {
+int plan_chain(gsofa_ctx* ctx, int32_t nmax, long long total_sources, const gsofa_opts* o, ChainCfg* c) {
     c->words = bitmap_words(nmax);
-    const long long need = (all_sym ? 1 : 2) * c->words;  // X of each direction
-    c->sides = all_sym ? 1 : 2;
-    const size_t fixed = (chain_sparse_bytes(c->sides) + 15) & ~(size_t)15;
-    size_t bytes = ((size_t)need * 4 + 15) & ~(size_t)15;
+    const size_t fixed = (chain_sparse_bytes() + 15) & ~(size_t)15;
+    size_t bytes = ((size_t)c->words * 4 + 15) & ~(size_t)15;
     if (fixed + bytes + 20 * 1024 > (size_t)ctx->smem_optin || (o->flags & GSOFA_FORCE_GLOBAL_BITMAP))
         bytes = 0;
-    c->smem_words = bytes ? need : 0;
-    c->gbm_count = bytes ? 2 : 4;
+    c->smem_words = bytes ? c->words : 0;
+    c->gbm_count = bytes ? 1 : 2;
     c->smem = fixed + bytes;
     c->block = o->threads_per_source;
     if (c->block <= 0) {
@@ -400,11 +397,10 @@ int plan_chain(gsofa_ctx* ctx, int32_t nmax, long long total_sources, bool all_s
         // are the longest chain, shorter with more threads (170 x 170 mesh:
         // 0.97 against 0.82 ms).
         c->block = fit >= 8 && total_sources >= 8ll * nmax ? 128 : fit >= 4 ? 256 : fit >= 2 ? 512 : 1024;
-
     }
     if (c->block != 128 && c->block != 256 && c->block != 512 && c->block != 1024)
         return set_err(ctx, GSOFA_ERR_ARG, "threads_per_source must be 128, 256, 512 or 1024");
-    const int occ = chain_occupancy(c->block, serve, c->smem);
+    const int occ = chain_occupancy(c->block, false, c->smem);
     if (occ <= 0)
         return set_err(ctx, GSOFA_ERR_UNSUPPORTED,
                        "traversal kernel cannot be resident (block %d, %zu B shared)", c->block,
@@ -421,7 +417,6 @@ void fill_chain_launch(ChainLaunch* L, const ChainCfg& c, const gsofa_opts& o, i
     L->gbm_count = c.gbm_count;
     L->bitmap_words = c.words;
     L->smem_words = c.smem_words;
-    L->sides = c.sides;
 }
 
 int32_t method_of(const gsofa_matrix* m) {
@@ -638,7 +633,7 @@ int run_factor_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_t cou
         long long chain_sources = 0;
         for (int32_t i = 0; i < count; i++)
             if (method_of(mats[i]) == METHOD_CHAIN) chain_sources += mats[i]->n;
-        rc = plan_chain(ctx, std::max(nmax, 1), chain_sources, true, o, false, &ccfg);
+        rc = plan_chain(ctx, std::max(nmax, 1), chain_sources, o, &ccfg);
         if (rc) return rc;
         CL.chunk = (int)chain_chunk(*o, chain_sources, nmax, ccfg.grid);
         long long items = 0;
@@ -1519,7 +1514,7 @@ static int autotune_impl(gsofa_ctx* ctx, const gsofa_matrix* const* mats, int32_
         }
         ChainCfg cc;
         if (chain_sources > 0 &&
-            plan_chain(ctx, std::max(nmax, 1), chain_sources, true, &base, false, &cc) == GSOFA_OK) {
+            plan_chain(ctx, std::max(nmax, 1), chain_sources, &base, &cc) == GSOFA_OK) {
             best.threads_per_source = cc.block;
             auto_chunk = chain_chunk(base, chain_sources, nmax, cc.grid);
             best.chunk_sources = (int32_t)auto_chunk;
@@ -1703,7 +1698,7 @@ static int batch_create_with(gsofa_ctx* ctx, const gsofa_matrix* const* mats, in
         else left_weight += chunk_weight(ctx, mats[i]);
         (mine ? chain_nmax : left_nmax) = std::max(mine ? chain_nmax : left_nmax, mats[i]->n);
     }
-    if (chain) rc = plan_chain(ctx, chain_nmax, chain_sources, true, &o, false, &ccfg);
+    if (chain) rc = plan_chain(ctx, chain_nmax, chain_sources, &o, &ccfg);
     if (!rc) rc = plan_launch(ctx, chain ? left_nmax : nmax, &o, &cfg);
     if (rc) return fail(rc);
     const long long walk_chunk =

@@ -169,12 +169,10 @@ struct ChainCfg {
     size_t smem = 0;
     long long words = 0;       // of the largest matrix's bitmap
     long long smem_words = 0;  // bitmap words in shared memory (0: bitmaps in global memory)
-    int gbm_count = 2;         // global bitmaps per CTA
-    int sides = 2;
+    int gbm_count = 1;         // global bitmaps per CTA
 };
 bool chain_runs(const gsofa_opts& o, const gsofa_matrix* const* mats, int32_t count);
-int plan_chain(gsofa_ctx* ctx, int32_t nmax, long long total_sources, bool all_sym, const gsofa_opts* o,
-               bool serve, ChainCfg* c);
+int plan_chain(gsofa_ctx* ctx, int32_t nmax, long long total_sources, const gsofa_opts* o, ChainCfg* c);
 // The chunks of a matrix of n rows that the launch of larger CTAs takes.
 long long chain_top_items(const gsofa_opts& o, int32_t n, long long chunk);
 // Both launches of the chain on ctx->stream and beside it: `top` (`top_items`

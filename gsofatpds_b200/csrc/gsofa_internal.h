@@ -175,9 +175,9 @@ struct TraverseLaunch {
 };
 
 // The counting traversal (gsofa_chain.cu).  Per CTA: a queue of queue_stride
-// ints and gbm_count bitmaps of bitmap_words words in global memory (two that
-// are zero between uses; two more for the dense base when it does not fit in
-// shared memory).
+// ints and gbm_count bitmaps of bitmap_words words in global memory (one that is
+// zero between uses; another for the dense base when it does not fit in shared
+// memory).
 enum : int {
     ITEMS_MAIN = 0,  // the matrices' chunks but the top_items
     ITEMS_TOP = 1,   // those
@@ -194,7 +194,6 @@ struct ChainLaunch {
     long long bitmap_words;            // covers the largest n + padding
     long long smem_words;              // bitmap words that fit in shared memory
     int items;                         // ITEMS_*
-    int sides;                         // directions with tables: 1 when every pattern is symmetric
     int chunk;                         // consecutive sources per work item
     int list_cap;                      // new ids of a search before the whole CTA takes it
     long long sample_stride;           // > 1: only every stride-th item (autotuner timing)
@@ -279,7 +278,7 @@ int extra_ctas_per_sm();
 cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStream_t stream);
 
 // Shared memory of a CTA besides its bitmaps; the largest list_cap.
-size_t chain_sparse_bytes(int sides);
+size_t chain_sparse_bytes();
 int chain_list_cap();
 // Resident CTAs per SM with `smem` dynamic bytes (0 = cannot run).
 int chain_occupancy(int block, bool serve, size_t smem);

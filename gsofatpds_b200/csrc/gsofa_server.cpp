@@ -119,9 +119,9 @@ struct ServeShape {
     size_t rings(long long words) const {
         return chain ? 0 : align256((size_t)grid * (size_t)ring * (size_t)words * 4);
     }
-    // the chain's four, or one for traverse_kernel where shared memory has no room for it
+    // the chain's two, or one for traverse_kernel where shared memory has no room for it
     size_t bitmaps(long long words) const {
-        return chain || words > smem_words ? align256((size_t)grid * (chain ? 4 : 1) * (size_t)words * 4) : 0;
+        return chain || words > smem_words ? align256((size_t)grid * (chain ? 2 : 1) * (size_t)words * 4) : 0;
     }
     size_t bytes(long long words) const { return queues() + rings(words) + bitmaps(words); }
 };
@@ -291,7 +291,7 @@ ServeShape serve_shape(const gsofa_ctx* ctx, const gsofa_server& s, bool chain) 
     // shared-memory bitmap: the widest that keeps the block's full residency
     // (none with the diagnostic GSOFA_FORCE_GLOBAL_BITMAP)
     const int occ_target = 1024 / r.block;
-    const size_t fixed = chain ? (chain_sparse_bytes(2) + 15) & ~(size_t)15 : 0;
+    const size_t fixed = chain ? (chain_sparse_bytes() + 15) & ~(size_t)15 : 0;
     auto occupancy = [&](size_t bytes) {
         return chain ? chain_occupancy(r.block, true, fixed + bytes) : serve_occupancy(r.block, bytes);
     };
@@ -304,7 +304,7 @@ ServeShape serve_shape(const gsofa_ctx* ctx, const gsofa_server& s, bool chain) 
         const size_t one = ((size_t)s.words * 4 + 1023) & ~(size_t)1023;
         if (chain && one <= 64 * 1024 && smem < one && occupancy(one) > 0) smem = one;
     }
-    if (chain) smem = std::min(smem, ((size_t)s.words * 8 + 1023) & ~(size_t)1023);  // both directions
+    if (chain) smem = std::min(smem, ((size_t)s.words * 4 + 1023) & ~(size_t)1023);
     r.occ = occupancy(smem);
     r.smem = fixed + smem;
     r.smem_words = (long long)(smem / 4);
@@ -565,10 +565,9 @@ bool launch_kernel(gsofa_server* s, Engine& E, int k, int grid) {
         C.queue = E.queue;
         C.queue_stride = std::max(s->max_n, 1);
         C.gbm = E.gbm;
-        C.gbm_count = 4;
+        C.gbm_count = 2;
         C.bitmap_words = s->words;
         C.smem_words = E.shape.smem_words;
-        C.sides = 2;
         C.chunk = 1;
         C.list_cap = (int)std::min<long long>(chain_list_cap(), C.queue_stride);
         C.sample_stride = 1;
