@@ -1048,6 +1048,26 @@ int label_max_cluster(size_t smem) {
     return 0;
 }
 
+size_t hub_load_bytes() { return hub_scan_bytes(2, 2) + 256 + 2 * sizeof(Tot); }
+
+cudaError_t hub_load(void* scratch, cudaStream_t st) {
+    cudaFuncAttributes fa;
+    const void* const kernels[] = {(const void*)hub_kernel,        (const void*)label_cluster_kernel,
+                                   (const void*)label_start_kernel, (const void*)label_round_kernel,
+                                   (const void*)label_drop_kernel,  (const void*)event_kernel,
+                                   (const void*)extra_kernel,       (const void*)large_kernel<kLargeThreads>,
+                                   (const void*)commit_kernel};
+    cudaError_t e = cudaSuccess;
+    for (const void* k : kernels)
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k);
+    Tot* const two = static_cast<Tot*>(scratch);
+    size_t sb = hub_scan_bytes(2, 2);
+    if (e == cudaSuccess) e = cudaMemsetAsync(two, 0, 2 * sizeof(Tot), st);
+    if (e == cudaSuccess)
+        e = cub::DeviceScan::InclusiveScan(static_cast<char*>(scratch) + 256, sb, two, two, TotSum(), 2, st);
+    return e;
+}
+
 // CTAs for each of `jobs` jobs of at most `most` CTAs' work: together no more than
 // some tens of waves.
 static int parts(int most, int jobs) { return std::max(1, std::min({most, 1024, (1 << 17) / jobs})); }

@@ -274,6 +274,10 @@ size_t label_smem_bytes(int32_t n, int cluster);
 size_t hub_scan_bytes(long long tots, long long uses);
 int large_occupancy(size_t smem);
 int label_max_cluster(size_t smem);
+// Loads every kernel of launch_hub, with hub_load_bytes() of device memory for a
+// scan of nothing.
+size_t hub_load_bytes();
+cudaError_t hub_load(void* scratch, cudaStream_t stream);
 int extra_ctas_per_sm();
 cudaError_t launch_hub(const HubLaunch& L, const HubCfg& c, int digests, cudaStream_t stream);
 
@@ -309,6 +313,7 @@ size_t canonicalize_scan_bytes(int32_t n);
 // *sum (zeroed by the caller) += sum over A's entries (v, c) of |v - c|.
 cudaError_t launch_index_distance(int32_t n, const int32_t* rp, const int32_t* col,
                                   unsigned long long* sum, cudaStream_t stream);
+cudaError_t load_supernodes();
 cudaError_t launch_supernodes(int32_t n, int32_t mss, const int32_t* nz_row_u,
                               const uint32_t* lmask, int8_t* flags,
                               unsigned long long* counters, cudaStream_t stream);

@@ -1621,6 +1621,11 @@ long long supernode_segment_count(int32_t n, int32_t mss) {
     return n <= 0 ? 0 : (((long long)n + mss - 1) / mss) * (((long long)mss + 127) / 128);
 }
 
+cudaError_t load_supernodes() {
+    cudaFuncAttributes fa;
+    return cudaFuncGetAttributes(&fa, supernode_kernel);
+}
+
 cudaError_t launch_supernodes(int32_t n, int32_t mss, const int32_t* nzu, const uint32_t* lmask,
                               int8_t* flags, unsigned long long* counters, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;

@@ -92,6 +92,7 @@ constexpr int kReserveSms = 4;
 constexpr int kLanes = 3;                      // hubs' launches that may run at once
 constexpr int kLaneCluster = 4;                // CTAs of a lane's label search at most: its SMs are shared
 constexpr size_t kLaneBytes = 64u << 20;       // a lane's workspace for large searches, or that of 296 CTAs
+constexpr size_t kAhead = 2ull << 30;          // memory the pool gets before the first request, at most
 constexpr double kLaneHoldMs = 1.0;            // the lanes' SMs stay free this long after their last work
 constexpr long long kMaxIdlePolls = 1000000;  // a cap far above idle_ns worth of polls
 constexpr long long kIdleNs = 300000;         // a CTA with nothing to claim for 0.3 ms exits
@@ -144,6 +145,8 @@ struct Engine {
     unsigned int* d_cta_slots = nullptr;
     int* d_alive = nullptr;
     double alive_checked = -1.0;
+
+    int streams() const { return shape.chain ? kKernelStreams : kKernelStreams / 2; }
 };
 
 // A hubs' launch for one request, and what it needs.
@@ -647,6 +650,9 @@ void to_walk(gsofa_server* s, const std::shared_ptr<Request>& r) {
     if (e != cudaSuccess) server_err(s, "ticket %llu: %s", (unsigned long long)r->ticket, cudaGetErrorString(e));
 }
 
+// A lane's workspace: labels, totals and queues take less than 256 bytes a row.
+size_t lane_bytes(int32_t n) { return 256 * (size_t)n + std::max(kLaneBytes, 296 * 5 * (size_t)n); }
+
 // Starts the hubs' launch of a request; false: no room for its workspace.
 bool lane_start(gsofa_server* s, Lane& l, const std::shared_ptr<Request>& r) {
     gsofa_ctx* ctx = s->ctx;
@@ -662,9 +668,7 @@ bool lane_start(gsofa_server* s, Lane& l, const std::shared_ptr<Request>& r) {
     HubCfg c;
     size_t bytes = 0;
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
-    // the labels, totals and queues take less than 256 bytes a row
-    const size_t want = 256 * (size_t)r->n + std::max(kLaneBytes, 296 * 5 * (size_t)r->n);
-    const size_t fit = std::min(room - std::min(room, head), want);
+    const size_t fit = std::min(room - std::min(room, head), lane_bytes(r->n));
     plan_hub(ctx, &d, s->opts, nullptr, &bytes, fit, &L, &c, kLaneCluster);
     if (head + bytes > room || dev_alloc_on(ctx, head + bytes, &l.ws, l.st) != GSOFA_OK) {
         l.ws = nullptr;
@@ -744,7 +748,7 @@ bool manage_kernel(gsofa_server* s, int e, bool claimable) {
     bool progress = false;
     bool any = false;
     int free_k = -1;
-    for (int k = 0; k < kKernelStreams; k++) {
+    for (int k = 0; k < E.streams(); k++) {
         if (E.krun[k] && cudaEventQuery(E.kdone[k]) == cudaSuccess) {
             E.krun[k] = false;
             progress = true;
@@ -767,7 +771,7 @@ bool manage_kernel(gsofa_server* s, int e, bool claimable) {
     if (free_k >= 0)
         return launch_kernel(s, E, free_k, part ? std::min(E.shape.grid, 2 * missing) : missing) || progress;
     int32_t oldest = E.kno[0];
-    for (int k = 1; k < kKernelStreams; k++) oldest = std::min(oldest, E.kno[k]);
+    for (int k = 1; k < E.streams(); k++) oldest = std::min(oldest, E.kno[k]);
     if (ctl_flags(s)[3 + e] <= oldest) set_control(s, 3 + e, oldest + 1);
     return progress;
 }
@@ -1081,7 +1085,7 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
     int prio_low = 0, prio_high = 0;
     cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
     for (Engine& E : s->eng)
-        for (int k = 0; k < kKernelStreams && E.on; k++)
+        for (int k = 0; k < E.streams() && E.on; k++)
             if ((e = cudaStreamCreateWithPriority(&E.ks[k], cudaStreamNonBlocking, prio_low)) != cudaSuccess ||
                 (e = cudaEventCreateWithFlags(&E.kdone[k], cudaEventDisableTiming)) != cudaSuccess)
                 return fail(GSOFA_ERR_CUDA, "stream", e);
@@ -1149,7 +1153,30 @@ int gsofa_server_create(gsofa_ctx* ctx, const gsofa_opts* opts, int32_t max_n,
         }
         Engine& C = s->eng[E_CHAIN];
         if (C.on && dev_alloc_on(ctx, C.ws_bytes, &C.ws, s->as) != GSOFA_OK) C.on = false;
+        // The pool grows now, for the lanes' workspaces and a few requests of max_n
+        // rows: while serving kernels run, its growth waits until they have no work
+        // (a request behind a large one's last item; of 56 bursts of 48 requests 3 took
+        // about 1 s, of 60 now none took more than 0.15 s).
+        size_t ahead[kLanes + 1];
+        std::fill_n(ahead, kLanes, C.on ? std::min(lane_bytes(max_n), kAhead / 8) : 0);
+        ahead[kLanes] = std::min(4 * request_footprint(s, max_n, 16ll * max_n), kAhead);
+        void* warm[kLanes + 1] = {};
+        for (int k = 0; k <= kLanes; k++)
+            if (s->least + C.ws_bytes + ahead[k] > s->budget ||
+                dev_alloc_on(ctx, ahead[k], &warm[k], s->as) != GSOFA_OK)
+                warm[k] = nullptr;
+        for (int k = 0; k <= kLanes; k++) dev_free_on(ctx, warm[k], ahead[k], s->as);
+        // kernels that a request would load while serving kernels run, which its
+        // launch then waits for (the first burst of 48 requests of up to 10^6 rows
+        // took 0.33-0.75 s, now 0.13)
+        void* few = nullptr;
+        if (C.on && dev_alloc_on(ctx, hub_load_bytes(), &few, s->as) == GSOFA_OK) {
+            e = hub_load(few, s->as);
+            dev_free_on(ctx, few, hub_load_bytes(), s->as);
+        }
+        if (e == cudaSuccess) e = load_supernodes();
     }
+    if (e != cudaSuccess) return fail(GSOFA_ERR_CUDA, "serving kernels", e);
     char* b = static_cast<char*>(s->tab);
     s->d_slots = reinterpret_cast<MatDesc*>(b);
     b += align256(sizeof(MatDesc) * kSlots);
