@@ -537,13 +537,17 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
 
 // The last separators of a mesh in nested-dissection order reach almost
 // everything: their chunks' first searches, from nothing, take as long as all
-// the rest of the launch (500 x 500 mesh: 4.0 of 4.6 ms by 256 threads).  From
-// 131,072 rows on, the chunks of the last 2 % of them go to CTAs of 1,024 threads,
-// at most one per SM, beside the rest (3.55 ms; the 64^3 mesh 3.3 either way).
-// Smaller meshes lose more by the SMs those CTAs take (170 x 170: 0.82 -> 1.0 ms,
-// a batch of 64 matrices 5.9 -> 7.2).
+// the rest of the launch.  From 65,536 rows on, the chunks of the last 2 % of them
+// go to CTAs of 1,024 threads, at most one per SM, beside the rest.  Times of a
+// call without and with them: 9-point meshes of 260 x 260 1.43 and 1.15 ms, 300 x
+// 300 1.83 and 1.36, 362 x 362 2.50 and 1.88, 500 x 500 4.25 and 3.03; 7-point of
+// 46^3 1.32 and 1.34, 50^3 1.63 and 1.57, 64^3 2.97 and 2.80; 16 meshes of 300 x 300
+// 10.6 and 10.1.  Below, there is little to gain (170 x 170: 0.78 and 0.74) and a
+// batch of 64 matrices of up to 30,000 rows loses more by the SMs those CTAs take
+// (5.9 and 7.2).
+constexpr int32_t kTopRows = 65536;
 long long chain_top_items(const gsofa_opts& o, int32_t n, long long chunk) {
-    if (o.sources_in_flight > 0 || n < 131072) return 0;
+    if (o.sources_in_flight > 0 || n < kTopRows) return 0;
     const long long chunks = (n + chunk - 1) / chunk;
     return std::min(chunks - 1, (n / 50 + chunk - 1) / chunk);
 }
@@ -585,8 +589,7 @@ long long chain_chunk(const gsofa_opts& o, long long total_sources, int32_t nmax
     // A chunk's first source is searched from nothing: about two items per CTA,
     // at most 128 sources each, since items differ in cost (64^3 mesh: 3.3 ms with
     // 128 sources, 4.0 with 443; 40^3: 0.92 with 54, 1.09 with 108).  At most 64
-    // where no matrix has the 1,024-thread launch (a batch's meshes of up to
-    // 30,000 rows 5.9 -> 5.3 ms).
+    // below 131,072 rows (a batch's meshes of up to 30,000 rows 5.9 -> 5.3 ms).
     return std::max(1ll, std::min(nmax < 131072 ? 64ll : 128ll, (total_sources + 2ll * grid - 1) / (2ll * grid)));
 }
 
