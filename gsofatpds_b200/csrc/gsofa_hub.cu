@@ -17,16 +17,17 @@
 // average, and no source waits for another.  gsofa_chain.cu, where a chunk's
 // sources are a chain, took 450 ms on that matrix.
 //
-// Three hubs serve three windows of s (above n/16, n/16 down to n/256, below),
-// each among the ids below its window's, so that early sources have one too;
-// the smaller windows' labels expand only ids below their end.
+// Four hubs serve three windows of s (above n/16, n/16 down to n/256, below), two
+// of them the first, each among the ids below its window's, so that early sources
+// have one too; the smaller windows' labels expand only ids below their end.
 //
 //   hub_kernel     per matrix and window: the vertex of largest in-degree times
 //                  out-degree below the window's start
-//   label_*_kernel label-correcting rounds, by one CTA per (matrix, window,
-//                  direction) in shared memory up to 50,000 rows, else one launch
-//                  of the whole GPU per round (46 and 93 rounds on the
-//                  circuit-like matrix, 3.5 to 5.2 reads per entry)
+//   label_*_kernel label-correcting rounds: by a cluster of up to 16 CTAs per
+//                  (matrix, hub, direction) in shared memory, which takes n up to
+//                  893,000, else one launch of the whole GPU per round (46 and 93
+//                  rounds for the first window of the circuit-like matrix, 3.5 to
+//                  5.2 reads per entry)
 //   event_kernel   a warp per word of 32 ids: the changes of the totals
 //   (a scan)       the totals of the hub's set for every s
 //   extra_kernel   a warp per (source, direction): the search beyond, in a
@@ -37,9 +38,9 @@
 // A matrix of at most kDirectMax rows has every source searched alone, without
 // a hub.  A matrix in which more than a quarter of the searches outgrow the
 // table (no core that the hub lies in: meshes) is left: traverse_kernel counts
-// it, whose reuse of closures does not need a core (200,000-row band of 4 without one: 13 ms, 248 by
-// gsofa_chain.cu; 90,000-row mesh with a third of its couplings one-sided: 16 ms,
-// 26 by it).
+// it, whose reuse of closures does not need a core (200,000-row band of 4 without
+// one: 13 ms, 248 searched source by source along a chain; 90,000-row mesh with a
+// third of its couplings one-sided: 16 ms and 26).
 #include <algorithm>
 #include <climits>
 
@@ -87,7 +88,10 @@ constexpr int kLargeThreads = 256;
 // A matrix is left when more than half of at least kJudgeEarly searches, or more
 // than a quarter of kJudgeAfter, have outgrown the table: looked at with every
 // such search, and what is under way then ends with it (at the end of every
-// item instead, a batch of 48 bands without a core spent 10 of 28 ms there).
+// item instead, a batch of 48 bands without a core spent 10 of 28 ms there).  An
+// eighth or a half instead of the quarter changes no time by more than 1 %: one-sided
+// meshes of 4,900 to 90,000 rows, a 200,000-row band, random n = 80,000 with 0.9 to
+// 2.5 entries a row.
 constexpr int kJudgeEarly = 64, kJudgeAfter = 512;
 
 struct WarpTable {

@@ -4,18 +4,18 @@
 //   * two persistent traversal kernels, chain_kernel for requests with a
 //     symmetric pattern and traverse_kernel for those without one that the hubs'
 //     launch leaves (for all of them with the diagnostic options, per-row L
-//     statistics, or a budget without room for both workspaces).  Their CTAs claim
-//     work items of every published request;
-//     it stays on the device while published work is waiting and ends by
-//     itself when its CTAs have found nothing to claim for a short while;
+//     statistics, or a budget without room for both workspaces).  Their CTAs
+//     claim work items of every published request; a kernel stays on the device
+//     while published work is waiting and ends by itself when its CTAs have
+//     found nothing to claim for a short while;
 //   * a few lanes for the other requests: each the hubs' launch of a plain call
 //     (gsofa_hub.cu) on a stream and in a workspace of its own.  The SMs are
 //     shared out among the two kernels and the lanes while they have work;
 //   * a side stream for everything else: the upload and padded-CSR build of
 //     each admitted request, its descriptor, the copy that publishes it (its
-//     claim word), and, once the kernel reports the request finished, its
+//     claim word), and, once the request is reported finished, its
 //     supernode detection and the read-back of its totals;
-//   * a control stream for the small table the kernel polls (the list of live
+//   * a control stream for the small table the kernels poll (the list of live
 //     requests the CTAs pick from, the "exit when idle" and "take no more
 //     items" controls): the host keeps the master copy in pinned memory and
 //     pushes it whole, synchronously, after each change;

@@ -89,8 +89,10 @@ typedef struct gsofa_opts {
     int32_t chunk_sources;
     /* closures of recently finished sources each CTA keeps for reuse
      * (rounded down to a power of 2, at most 64); 0 = default.  Used where
-     * closures are kept: the pattern pass, per-row L statistics of symmetric
-     * patterns, the no-allocation entry point and the diagnostic switches */
+     * closures are kept: unsymmetric matrices without a large strongly
+     * connected core or with rows that hold an id twice, the pattern pass,
+     * per-row L statistics of symmetric patterns, the no-allocation entry
+     * point and the diagnostic switches */
     int32_t cached_closures;
     /* how long (microseconds) a source search may wait, when the search of
      * the same chunk in the other direction is one source behind, for the
@@ -302,15 +304,17 @@ int gsofa_result_destroy(gsofa_result* res);
 
 /* ---- serving: a request loop with continuous batching ------------------------ */
 /* No counterpart in the reference, which factors one matrix per run.  A server
- * owns a host thread, three streams and a persistent traversal kernel that
- * stays on the device while published work is waiting.  Each submitted matrix is a
+ * owns a host thread, its streams and two persistent traversal kernels (for
+ * symmetric patterns and for others) that stay on the device while published
+ * work is waiting.  Each submitted matrix is a
  * request; the loop admits requests in arrival order as slots and memory free
  * up (its workspace footprint -- the padded CSR of A and A^T and its result
  * arrays -- must fit the budget next to the requests already admitted),
  * uploads and builds the matrix on a side stream, then publishes its work
- * items to the running kernel.  The kernel's CTAs take items of every admitted
- * request as they free up, so requests that arrive while others run share the
- * device.  When a request's last item is done the loop runs its supernode
+ * items to the running kernels, or launches the hubs' kernels for it where its
+ * pattern is unsymmetric.  A kernel's CTAs take items of every admitted request
+ * as they free up, so requests that arrive while others run share the device.
+ * When a request's last item is done the loop runs its supernode
  * detection and hands out a result identical to gsofa_factor_symbolic's
  * (gsofa_result_* getters; the caller destroys it).
  *
