@@ -519,6 +519,7 @@ bool plan_hub(gsofa_ctx* ctx, std::vector<MatDesc>* descs, const gsofa_opts& o, 
     L->fallback = static_cast<int32_t*>(place(4 * (size_t)nm));
     L->given_up = static_cast<int32_t*>(place(4 * (size_t)nm));
     L->judged = static_cast<int32_t*>(place(8 * (size_t)nm));
+    L->large_work = static_cast<unsigned long long*>(place(16 * (size_t)nm));
     L->counters = static_cast<unsigned long long*>(place(8 * CNT_SLOTS * (size_t)nm));
     L->hubs = static_cast<unsigned long long*>(place(8 * (size_t)W * (size_t)nm));
     L->large_count = static_cast<int*>(place(4));

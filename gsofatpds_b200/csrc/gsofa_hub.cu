@@ -93,6 +93,15 @@ constexpr int kLargeThreads = 256;
 // meshes of 4,900 to 90,000 rows, a 200,000-row band, random n = 80,000 with 0.9 to
 // 2.5 entries a row.
 constexpr int kJudgeEarly = 64, kJudgeAfter = 512;
+// A matrix is also left when its large searches, by the mean of those done so
+// far, will read more than kLargePerRow entries for each of its rows: large_kernel
+// reads 220 G entries/s, traverse_kernel takes 0.3 to 0.5 us a row.  The circuit-like
+// n = 659,033 after the hybrid ordering, whose sources below the top separators
+// reach no hub, would read 115,000 a row: 355 ms, 210 by traverse_kernel alone.
+// After the level-set ordering it reads 4,200 (44 ms against 326), ordered random
+// and banded matrices of 20,000 rows 10,000 to 15,000 (1.7-2.0 ms against 2.7-3.9).
+constexpr unsigned long long kLargeSample = 1024;
+constexpr double kLargePerRow = 65536.0;
 
 struct WarpTable {
     uint32_t key[kSlots];
@@ -865,12 +874,14 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) large_kernel(HubLaunch P)
         if (threadIdx.x == 0) {
             const unsigned long long k = atomicAdd(P.work_counter + 1, 1ull);
             item = k < (unsigned long long)count ? (long long)P.large[k] : -1;
+            // (one thread looks: another CTA may set the flag)
+            if (item >= 0 && ld_vol_i32(P.fallback + (int)(item >> 33))) item = -2;
         }
         __syncthreads();
-        if (item < 0) return;
+        if (item == -1) return;
+        if (item < 0) continue;
         const int mi = (int)(item >> 33), d = (int)(item >> 32) & 1, s = (int)(item & 0xffffffff);
         const MatDesc& M = P.mats[mi];
-        if (P.fallback[mi]) continue;
         const int n = M.n, nw = (n + 31) >> 5;
         const bool sym = M.asym[0] == 0;
         const bool digests = M.dig_u != nullptr;
@@ -945,6 +956,12 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) large_kernel(HubLaunch P)
                 }
                 if (d == 1 || sym) atomicAdd(c + CNT_NNZ_L, (unsigned long long)(unsigned)t.gt);
                 if (B.lam) atomicAdd(c + CNT_CHAINED, 1ull);
+                // how many of the matrix's large searches are done, and the entries they read
+                const unsigned long long done = atomicAdd(P.large_work + 2 * mi, 1ull) + 1;
+                const unsigned long long read = atomicAdd(P.large_work + 2 * mi + 1, bfs.rtrav) + bfs.rtrav;
+                if (n > kDirectMax && done >= kLargeSample &&
+                    (double)read / (double)done * P.judged[2 * mi + 1] > kLargePerRow * n)
+                    atomicExch(P.fallback + mi, 1);
             }
         }
         __syncthreads();

@@ -233,7 +233,7 @@ struct HubLaunch {
     long long total_items;
     unsigned long long* work_counter;  // [0] extra_kernel, [1] large_kernel
     // zeroed before every launch, in one block: Tot base[2 * hub_bases() * total], stamp,
-    // label counts, fallback, judged, counters, large_count
+    // label counts, fallback, judged, large_work, counters, large_count
     void* zeroed;
     LRowUse* l_use;                    // per hub and source (with per-row L statistics): see lrow_kernel
     Tot* base;                         // per base, direction and source: the hub set's totals
@@ -242,6 +242,7 @@ struct HubLaunch {
     int32_t* fallback;                 // per matrix: left to traverse_kernel
     int32_t* given_up;                 // per matrix: bit h when hub h has been given up
     int32_t* judged;                   // per matrix: searches done, searches too large
+    unsigned long long* large_work;    // per matrix: large searches done, entries they read
     unsigned long long* counters;      // per matrix, CNT_SLOTS
     int* large_count;
     int32_t* lam;                      // labels: hubs x 2 directions x total
